@@ -39,7 +39,7 @@ FLAG_D_PRECOMPUTED = 1 << 4
 FLAG_REUSE_FWD_ROUNDED = 1 << 5
 FLAG_DROPOUT_SCALED = 1 << 6  # inverted dropout (kept terms / (1 - p), normaliser over all keys)
 FLAG_CONTINUE_SOFTMAX_STATE = 1 << 7  # forward: O, LSE hold the result over earlier keys; fold this call's keys in
-FLAG_ROUND_IN_HBM = 1 << 8  # always round operands with the HBM pre-pass (default: in shared memory for short sequences)
+FLAG_ROUND_IN_HBM = 1 << 8  # asks for the forward's workspace at every size; the operands are rounded by the copies that load them
 FLAG_DETERMINISTIC_DQ = 1 << 9  # backward: dQ through per-KV-tile slabs added in a fixed order (same bits on every run)
 
 _f32p = C.POINTER(C.c_float)
@@ -120,6 +120,7 @@ def lib() -> C.CDLL:
         L.hk_status_string.argtypes = [C.c_int]
         L.hk_attn_forward.argtypes = [C.POINTER(MemEfficientFwdParams), C.c_void_p]
         L.hk_attn_backward.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
+        L.hk_attn_zero_dq.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
         L.hk_attn_bwd_precompute_D.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
         L.hk_attn_bwd_precompute_D_hd.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_int, C.c_void_p]
         L.hk_attn_fwd_workspace_bytes.restype = C.c_size_t
@@ -266,16 +267,9 @@ def attention_forward(Q, K, V, scale: float, causal: bool, *, dropout_p: float =
         flags |= FLAG_ROUND_IN_HBM
     p.flags = flags
     need = fwd_workspace_bytes(p)
-    if need == 0 and workspace is not None and not prerounded:
-        # nothing is required (operands rounded in shared memory), but a workspace that is given receives the rounded
-        # Q for a backward call with reuse_fwd_rounded
-        base = workspace.data_ptr()
-        off = (-base) % 256
-        p.workspace, p.workspace_bytes = base + off, workspace.numel() - off
-    else:
-        ws = _workspace(need, Q, workspace)
-        if ws is not None:
-            p.workspace, p.workspace_bytes = ws[1], need
+    ws = _workspace(need, Q, workspace)
+    if ws is not None:
+        p.workspace, p.workspace_bytes = ws[1], need
     fused_attn_forward(p, stream)
     return O, LSE
 
@@ -339,6 +333,14 @@ def attention_backward(Q, K, V, O, dO, LSE, scale: float, causal: bool, *, dropo
         p.workspace, p.workspace_bytes = ws[1], bwd_workspace_bytes(p)
     mem_efficient_bwd_unified(p, stream)
     return dQ, dK, dV, D
+
+
+def zero_dq(dQ, stream=None) -> None:
+    """Zeroes a [B, H, T, 64] dQ on a stream of the caller's choice, for a backward with accum_dq."""
+    p = MemEfficientBwdParams()
+    p.dQ, (p.B, p.nh, p.T) = dQ.data_ptr(), dQ.shape[:3]
+    _set3(p, "dq", dQ)
+    _check(lib().hk_attn_zero_dq(C.byref(p), _stream_handle(stream)), "hk_attn_zero_dq")
 
 
 def round_tf32(x, out=None, stream=None):

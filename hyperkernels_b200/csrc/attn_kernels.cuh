@@ -18,9 +18,6 @@ struct FwdArgs {
     int dropout_mode;  // 0 none, 1 dense mask, 2 Philox
     int drop_scaled;   // 1: inverted dropout (normaliser over all visible keys, kept terms times keep_scale)
     int continue_state;  // 1: O, LSE hold the result over earlier keys and are the starting state
-    int round_in_smem;   // 1: Q, K, V arrive unrounded and are rounded to TF32 in shared memory after the TMA landing
-    int store_q;         // with round_in_smem: the rounded Q, K and V tiles are also written out (maps mqw, mkw, mvw), where
-                         // the HBM pre-pass would have put them, for a backward call that reuses them
     float keep_scale;  // 1/(1-p) when drop_scaled, else 1
     uint32_t drop_thr;
     uint32_t bh_pos0;  // added to the local (batch, head) index in the Philox counter
@@ -30,9 +27,8 @@ struct FwdArgs {
     int timeline_block;
 };
 
-// mq, mk, mv: TMA maps of the (rounded) operands; mo: map of O, the destination of the kernel's bulk stores.
+// mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                    const CUtensorMap& mqw, const CUtensorMap& mkw, const CUtensorMap& mvw,
                     const FwdArgs& a, cudaStream_t stream);
 
 struct BwdArgs {
@@ -51,7 +47,6 @@ struct BwdArgs {
     float scale, scale_log2e;
     int causal;
     int accum_dkdv;
-    int round_kv;      // 1: K and V arrive unrounded; the compute warps round them to TF32 once they have landed
     int det_dq;        // 1: dQ tiles are stored (map dQ = the slabs [n_kvtiles * B, H, Tq, 64]) instead of added; B below
     int B;
     int dropout_mode;
@@ -75,6 +70,16 @@ struct BwdMaps {
 };
 
 int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream);
+
+// What hk_attn_forward / hk_attn_backward run.  check_scratch: ask for the workspace the C ABI documents; without it the
+// forward takes none and `workspace` of a deterministic backward holds the slabs of partial dQ alone.
+int attn_forward(const hk_attn_fwd_params& p, cudaStream_t stream, bool check_scratch);
+int attn_backward(const hk_attn_bwd_params& p, cudaStream_t stream, bool check_scratch);
+// the same for callers in this package, by name (dlsym)
+extern "C" int hk_attn_forward_noscratch(const hk_attn_fwd_params* p, void* stream);
+extern "C" int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* stream);
+// zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ
+extern "C" int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream);
 
 int run_umma_selftest(int which, const float* A, const float* B, float* out, cudaStream_t stream);
 

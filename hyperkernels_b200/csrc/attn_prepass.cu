@@ -8,46 +8,25 @@
 namespace hk {
 
 // ---------------------------------------------------------------------------
-// TF32 operand rounding.  The reference adds 0x1000 to the bit pattern of every
-// MMA operand as it loads it from shared memory
-// (fused_attn_forward_kernel_tc_sm89.cu:197,209-210,219;
-//  mem_efficient_bwd_unified_kernel_exp12.cu:118,127,136), i.e. round to
-// nearest, ties away.  tcgen05.mma reads its operands straight from the bytes
-// TMA wrote, so the rounding is applied once here, into contiguous
-// [BH, T, 64] copies in the caller's workspace.
+// TF32 rounding of contiguous rows (hk_attn_round_tf32).  The reference adds 0x1000 to the bit pattern of every MMA
+// operand as it loads it from shared memory (fused_attn_forward_kernel_tc_sm89.cu:197,209-210,219;
+// mem_efficient_bwd_unified_kernel_exp12.cu:118,127,136), i.e. round to nearest, ties away.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) round_tf32_kernel(const RoundJob job) {
-    const int t = blockIdx.y;
-    const int T = job.T[t];
-    const int H = job.H;
-    const View4 v = job.src[t];
-    uint4* dst = reinterpret_cast<uint4*>(job.dst[t]);
-    const long long nvec = (long long)job.BH * T * 16;  // 16 float4 per 64-float row
+__global__ void __launch_bounds__(256) round_tf32_kernel(const float* src, float* dst_, long long nvec) {
+    uint4* dst = reinterpret_cast<uint4*>(dst_);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
          i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i >> 4;
-        const int c4 = (int)(i & 15);
-        const int bh = (int)(row / T);
-        const int r = (int)(row - (long long)bh * T);
-        const int b = bh / H, h = bh - b * H;
-        // plain load: dst may be src (hk_attn_round_tf32 in place), which rules the read-only path out
-        const float4 x =
-            *(reinterpret_cast<const float4*>(v.ptr + (int64_t)b * v.sB + (int64_t)h * v.sH + (int64_t)r * v.sM) + c4);
-        uint4 y;
-        y.x = tf32_round_bits(__float_as_uint(x.x));
-        y.y = tf32_round_bits(__float_as_uint(x.y));
-        y.z = tf32_round_bits(__float_as_uint(x.z));
-        y.w = tf32_round_bits(__float_as_uint(x.w));
-        dst[i] = y;
+        // plain load: dst may be src, which rules the read-only path out
+        const uint4 x = reinterpret_cast<const uint4*>(src)[i];
+        dst[i] = make_uint4(tf32_round_bits(x.x), tf32_round_bits(x.y), tf32_round_bits(x.z), tf32_round_bits(x.w));
     }
 }
 
-int launch_round_tf32(const RoundJob& job, cudaStream_t stream) {
-    long long max_vec = 0;
-    for (int t = 0; t < job.n; ++t) max_vec = std::max(max_vec, (long long)job.BH * job.T[t] * 16);
-    if (max_vec == 0 || job.n == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((max_vec + 255) / 256, 148 * 8);
-    round_tf32_kernel<<<dim3(blocks, job.n), 256, 0, stream>>>(job);
+int launch_round_tf32(const float* src, float* dst, int64_t rows, cudaStream_t stream) {
+    const long long nvec = (long long)rows * 16;  // 16 float4 per 64-float row
+    if (nvec == 0) return HK_OK;
+    const int blocks = (int)std::min<long long>((nvec + 255) / 256, 148 * 8);
+    round_tf32_kernel<<<blocks, 256, 0, stream>>>(src, dst, nvec);
     count_launch();
     return check_launch();
 }
@@ -55,9 +34,8 @@ int launch_round_tf32(const RoundJob& job, cudaStream_t stream) {
 // ---------------------------------------------------------------------------
 // D[b,h,i] = sum_k dO[i,k] * O[i,k]  (mem_efficient_bwd_precompute_D_sm89.cu:45-91),
 // 16 lanes per row, one float4 of each operand per lane.  Optionally also
-// writes the TF32-rounded copy of dO the backward MMAs consume, so dO is read
-// from HBM once, and zeroes the matching rows of dQ (the reference leaves that
-// to its caller, kernels_test.cu:562).
+// zeroes the matching rows of dQ (the reference leaves that to its caller,
+// kernels_test.cu:562).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) precompute_D_kernel(const DJob j) {
     const long long nrows = (long long)j.BH * j.T;
@@ -75,14 +53,6 @@ __global__ void __launch_bounds__(256) precompute_D_kernel(const DJob j) {
             const float4 o = __ldg(
                 reinterpret_cast<const float4*>(j.O.ptr + (int64_t)b * j.O.sB + (int64_t)h * j.O.sH + (int64_t)r * j.O.sM) + sub);
             s = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
-            if (j.dO_rounded) {
-                uint4 y;
-                y.x = tf32_round_bits(__float_as_uint(g.x));
-                y.y = tf32_round_bits(__float_as_uint(g.y));
-                y.z = tf32_round_bits(__float_as_uint(g.z));
-                y.w = tf32_round_bits(__float_as_uint(g.w));
-                reinterpret_cast<uint4*>(j.dO_rounded)[row * 16 + sub] = y;
-            }
             if (j.dQ_zero)
                 reinterpret_cast<float4*>(j.dQ_zero + (int64_t)b * j.dq_sB + (int64_t)h * j.dq_sH + (int64_t)r * j.dq_sM)[sub] =
                     make_float4(0.f, 0.f, 0.f, 0.f);

@@ -4,26 +4,18 @@
 
 namespace hk {
 
-struct RoundJob {
-    View4 src[4];
-    float* dst[4];  // contiguous [BH, T[t], 64]
-    int T[4];
-    int H, BH;
-    int n;
-};
-int launch_round_tf32(const RoundJob& job, cudaStream_t stream);
+int launch_round_tf32(const float* src, float* dst, int64_t rows, cudaStream_t stream);
 
 struct DJob {
     View4 dO, O;
     float* D;
     int64_t d_sB, d_sH;
-    float* dO_rounded;  // contiguous [BH, T, 64] or nullptr
     float* dQ_zero;     // if set: the same rows of dQ are zeroed on the way (dQ is accumulated with atomics)
     int64_t dq_sB, dq_sM, dq_sH;
     int H, BH, T;
 };
 int launch_precompute_D(const DJob& j, cudaStream_t stream);
-// D only, head dimension 16, 32, 48, 64, 80, 96, 128, 160, 192 or 256 (dO_rounded and dQ_zero are ignored)
+// D only, head dimension 16, 32, 48, 64, 80, 96, 128, 160, 192 or 256 (dQ_zero is ignored)
 int launch_precompute_D_hd(const DJob& j, int head_dim, cudaStream_t stream);
 
 int launch_zero_rows(float* ptr, int64_t sB, int64_t sM, int64_t sH, int B, int H, int T, cudaStream_t stream);

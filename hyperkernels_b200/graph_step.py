@@ -1,12 +1,13 @@
 """Forward + backward captured once in a CUDA graph and replayed.
 
-A training step of the attention path is four launches (TF32 rounding pre-pass,
-forward, D pre-pass with dO rounding and dQ zeroing, backward).  At small sizes
+A training step of the attention path is four launches (dQ zeroing, forward, D
+pre-pass, backward).  At small sizes
 the gaps between dependent launches are a large part of the step (B=2, H=4,
 T=256: 0.064 ms issued launch by launch, 0.033 ms replayed from a graph); at
-B=8, H=12, T=1024 the graph saves about 2 %.  The graph holds exactly the
-launches the two C-ABI calls make: capture goes through ``hk_attn_forward`` and
-``hk_attn_backward`` on a side stream after one eager warm-up step (which sets
+B=8, H=12, T=1024 the graph saves about 2 %.  Zeroing dQ depends on nothing, so it is a
+branch of its own beside the forward: its stores (25 MB at B=8, H=12, T=1024) leave the
+D pre-pass and fill SMs the forward's last wave leaves idle.  Capture goes through
+``hk_attn_forward`` and ``hk_attn_backward`` on a side stream after one eager warm-up step (which sets
 the kernels' attributes and resolves the library's device symbols -- neither is
 allowed during capture).
 """
@@ -48,10 +49,16 @@ class GraphedAttentionStep:
             drop = dict(dropout_p=dropout_p, philox_seed=philox_seed, philox_offset=philox_offset,
                         dropout_scaled=dropout_scaled, bh_pos0=bh_pos0)
 
+        zero_stream = torch.cuda.Stream(device=dev)
+
         def step():
+            main = torch.cuda.current_stream(dev)
+            zero_stream.wait_stream(main)
             att.attention_forward(Q, K, V, scale, causal, workspace=self._ws, out=self.O, lse=self.LSE, **drop)
+            att.zero_dq(self.dQ, zero_stream)
+            main.wait_stream(zero_stream)
             att.attention_backward(Q, K, V, self.O, dO, self.LSE, scale, causal, workspace=self._ws, D=self.D,
-                                   dQ=self.dQ, dK=self.dK, dV=self.dV, reuse_fwd_rounded=True, **drop)
+                                   dQ=self.dQ, dK=self.dK, dV=self.dV, reuse_fwd_rounded=True, accum_dq=True, **drop)
 
         n0 = att.launch_count()
         side = torch.cuda.Stream(device=dev)

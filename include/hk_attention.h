@@ -12,8 +12,9 @@
  *
  * Conventions
  *   - head_dim is 64, I/O is fp32, MMA operands are TF32 rounded to nearest
- *     exactly as the reference rounds them (bit pattern + 0x1000, low 13 bits
- *     dropped), accumulation is fp32.
+ *     (Q, K, V, dO by the TMA copies that load them, ties to even; P and dS in
+ *     registers by bit pattern + 0x1000, as the reference rounds everything),
+ *     accumulation is fp32.
  *   - All pointers are device pointers owned by the caller; the library never
  *     allocates device memory.  Scratch comes from `workspace`.
  *   - Strides are in elements; the last-dimension stride is 1.  Every pointer
@@ -56,7 +57,7 @@ typedef enum hk_status {
     HK_ERR_STATIC_SCRATCH = -9  /* problem too large for the built-in scratch of hk_attn_forward_static_scratch */
 } hk_status;
 
-/* Size of the scratch array built into the library for hk_attn_forward_static_scratch. */
+/* Size limit of hk_attn_forward_static_scratch. */
 #define HK_STATIC_SCRATCH_BYTES ((size_t)24 << 20)
 
 enum {
@@ -64,7 +65,7 @@ enum {
      * with Philox4x32-10; see hk_attn_dropout_mask for the host twin. */
     HK_FLAG_PHILOX_DROPOUT = 1u << 0,
     /* Q, K, V (and dO) already hold TF32-representable values (low 13 mantissa
-     * bits zero): skip the operand rounding and its workspace. */
+     * bits zero): no workspace is asked for. */
     HK_FLAG_OPERANDS_PREROUNDED = 1u << 1,
     /* backward: add into dK/dV instead of overwriting them (a K/V block that
      * travels round a sequence-sharded ring carries its gradients with it). */
@@ -74,9 +75,8 @@ enum {
     /* backward: D is supplied by the caller (reference behaviour of the unified
      * kernel taken alone); otherwise hk_attn_backward computes it from dO and O. */
     HK_FLAG_D_PRECOMPUTED = 1u << 4,
-    /* backward: `workspace` is the one hk_attn_forward was given for these same Q, K, V
-     * (same shapes, same is_causal, same rounding flags) and still holds what that call left
-     * there: do not round again what it holds. */
+    /* backward: `workspace` is the one hk_attn_forward was given for these same Q, K, V.  Accepted and without
+     * effect: the operands are rounded as they are loaded, there is nothing to reuse. */
     HK_FLAG_REUSE_FWD_ROUNDED = 1u << 5,
     /* forward and backward: inverted dropout instead of the reference's drop-then-renormalise
      * (no reference counterpart).  The softmax is normalised over ALL visible keys, the kept
@@ -90,12 +90,9 @@ enum {
      * key sequence (a KV ring) chains its calls this way instead of merging partial results afterwards.  Not
      * available together with HK_FLAG_DROPOUT_SCALED.  No counterpart in the reference. */
     HK_FLAG_CONTINUE_SOFTMAX_STATE = 1u << 7,
-    /* forward and backward: always round the operands with the HBM pre-pass into the workspace.  By default
-     * problems of 512 <= T <= 2048 (causal) or <= 1024 (otherwise) are rounded in shared memory after the TMA has
-     * landed a tile -- forward: Q, K, V, and no workspace is needed (one that is given and large enough receives
-     * the rounded tensors for a backward with HK_FLAG_REUSE_FWD_ROUNDED); stand-alone backward: K and V (Q and dO
-     * are still rounded into the workspace) -- because there the pre-pass costs more than the extra
-     * shared-memory traffic; both ways give the same bits. */
+    /* forward: ask for the workspace at every size.  The operands are rounded to TF32 by the TMA copies that load
+     * them and the workspace is not touched; by default it is required except for 512 <= T <= 2048 (causal) or
+     * <= 1024 (otherwise). */
     HK_FLAG_ROUND_IN_HBM = 1u << 8,
     /* backward: deterministic dQ.  By default the KV-tile CTAs add their dQ tiles into dQ with bulk reductions whose
      * order is not fixed (run-to-run differences of the order of 1e-5); with this flag every CTA stores its tiles
@@ -196,16 +193,12 @@ int hk_attn_forward(const hk_attn_fwd_params* p, void* stream);
 
 /* hk_attn_forward for callers that cannot allocate device memory (it has no
  * counterpart in the reference, whose kernels need no scratch).  Same arguments
- * and results as hk_attn_forward, but `workspace`/`workspace_bytes` are ignored:
- * the TF32-rounded operand copies go into a 24 MiB array that is part of the
- * library's device image, so the call itself allocates nothing (no cudaMalloc,
- * no cudaFree).  Meant for plug-ins living inside a framework that owns all
- * device memory, and for serving loops where an allocation would stall the GPU.
+ * and results as hk_attn_forward, but `workspace`/`workspace_bytes` are ignored and
+ * the call allocates nothing (no cudaMalloc, no cudaFree).  Meant for plug-ins
+ * living inside a framework that owns all device memory, and for serving loops
+ * where an allocation would stall the GPU.
  * Limits: B*nh*(T + 2*kv_len)*256 bytes must fit in HK_STATIC_SCRATCH_BYTES,
- * otherwise HK_ERR_STATIC_SCRATCH; every GPU that loads the library carries the
- * array until exit; all calls on a GPU share it, so calls that overlap in time
- * on one GPU race (serialise them); the first call on each device resolves the
- * array's address and should be made before any stream capture begins. */
+ * otherwise HK_ERR_STATIC_SCRATCH. */
 int hk_attn_forward_static_scratch(const hk_attn_fwd_params* p, void* stream);
 
 /* Replaces the launch of mem_efficient_bwd_precompute_D_sm89<64>
@@ -228,11 +221,9 @@ int hk_attn_bwd_precompute_D_hd(const hk_attn_bwd_params* p, int head_dim, void*
  * Writes dQ, dK, dV (and D). */
 int hk_attn_backward(const hk_attn_bwd_params* p, void* stream);
 
-/* Scratch the two calls need for the given block, flags included (0 when none).  Forward: the rounded Q, K, V
- * (3 tensors) when the HBM pre-pass rounds them, nothing when the kernel rounds in shared memory -- though a workspace
- * of hk_attn_bwd_workspace_bytes given to it then receives the rounded tensors for HK_FLAG_REUSE_FWD_ROUNDED.
- * Backward: the rounded Q, K, V, dO (4 tensors, in the forward's order followed by dO), then, with
- * HK_FLAG_DETERMINISTIC_DQ, one slab of partial dQ per 128-key tile. */
+/* Scratch the two calls ask for with the given block, flags included (0 when none).  Forward: room for Q, K, V, by size
+ * (HK_FLAG_ROUND_IN_HBM).  Backward: room for Q, K, V, dO, then, with HK_FLAG_DETERMINISTIC_DQ, one slab of partial dQ
+ * per 128-key tile.  The slabs are the only part that is written. */
 size_t hk_attn_fwd_workspace_bytes(const hk_attn_fwd_params* p);
 size_t hk_attn_bwd_workspace_bytes(const hk_attn_bwd_params* p);
 
