@@ -32,48 +32,69 @@ int launch_round_tf32(const float* src, float* dst, int64_t rows, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------
+// Row bookkeeping of the kernels below: row -> (b, h, r) with 32-bit divisions (a 64-bit one costs more instructions than
+// the rest of a row's work).  The launchers cut anything of 2^31 rows or more into runs of batches.
+// ---------------------------------------------------------------------------
+struct RowPos {
+    int b, h, r;
+};
+__device__ __forceinline__ RowPos row_pos(uint32_t row, uint32_t T, uint32_t H) {
+    const uint32_t bh = row / T, b = bh / H;
+    return {(int)b, (int)(bh - b * H), (int)(row - bh * T)};
+}
+__device__ __forceinline__ int64_t row_off(const RowPos& p, int64_t sB, int64_t sM, int64_t sH) {
+    return (int64_t)p.b * sB + (int64_t)p.h * sH + (int64_t)p.r * sM;
+}
+// batches that fit one launch
+static int batches_per_launch(int B, int H, int T) {
+    const long long per = (long long)H * T;
+    return (int)std::max<long long>(1, std::min<long long>(B, ((1LL << 31) - 1) / per));
+}
+
+constexpr int ROWS_PER_BLOCK = 64;  // 256 threads: 16 lanes per row, four rows per lane
+
+// ---------------------------------------------------------------------------
 // D[b,h,i] = sum_k dO[i,k] * O[i,k]  (mem_efficient_bwd_precompute_D_sm89.cu:45-91),
 // 16 lanes per row, one float4 of each operand per lane.  Optionally also
 // zeroes the matching rows of dQ (the reference leaves that to its caller,
-// kernels_test.cu:562).
+// kernels_test.cu:562).  HBM-bound: a lane issues the eight loads of its four rows before it uses the first.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) precompute_D_kernel(const DJob j) {
-    const long long nrows = (long long)j.BH * j.T;
+__global__ void __launch_bounds__(256) precompute_D_kernel(const DJob j, uint32_t nrows) {
     const int sub = threadIdx.x & 15;
-    for (long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4; row < ((nrows + 15) & ~15ll);
-         row += ((long long)gridDim.x * blockDim.x) >> 4) {
-        float s = 0.f;
-        if (row < nrows) {
-            const int bh = (int)(row / j.T);
-            const int r = (int)(row - (long long)bh * j.T);
-            const int b = bh / j.H, h = bh - b * j.H;
-            const float4 g = __ldg(
-                reinterpret_cast<const float4*>(j.dO.ptr + (int64_t)b * j.dO.sB + (int64_t)h * j.dO.sH + (int64_t)r * j.dO.sM) +
-                sub);
-            const float4 o = __ldg(
-                reinterpret_cast<const float4*>(j.O.ptr + (int64_t)b * j.O.sB + (int64_t)h * j.O.sH + (int64_t)r * j.O.sM) + sub);
-            s = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
-            if (j.dQ_zero)
-                reinterpret_cast<float4*>(j.dQ_zero + (int64_t)b * j.dq_sB + (int64_t)h * j.dq_sH + (int64_t)r * j.dq_sM)[sub] =
-                    make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    const uint32_t row0 = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 4);
+    float4 g[4], o[4];
+    RowPos p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint32_t row = min(row0 + 16 * u, nrows - 1);  // rows past the end are computed and not stored
+        p[u] = row_pos(row, j.T, j.H);
+        g[u] = __ldg(reinterpret_cast<const float4*>(j.dO.ptr + row_off(p[u], j.dO.sB, j.dO.sM, j.dO.sH)) + sub);
+        o[u] = __ldg(reinterpret_cast<const float4*>(j.O.ptr + row_off(p[u], j.O.sB, j.O.sM, j.O.sH)) + sub);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const bool valid = row0 + 16 * u < nrows;
+        if (j.dQ_zero && valid)
+            reinterpret_cast<float4*>(j.dQ_zero + row_off(p[u], j.dq_sB, j.dq_sM, j.dq_sH))[sub] = make_float4(0.f, 0.f, 0.f, 0.f);
+        float s = g[u].x * o[u].x + g[u].y * o[u].y + g[u].z * o[u].z + g[u].w * o[u].w;
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (row < nrows && sub == 0) {
-            const int bh = (int)(row / j.T);
-            const int r = (int)(row - (long long)bh * j.T);
-            const int b = bh / j.H, h = bh - b * j.H;
-            j.D[(int64_t)b * j.d_sB + (int64_t)h * j.d_sH + r] = s;
-        }
+        if (sub == 0 && valid) j.D[(int64_t)p[u].b * j.d_sB + (int64_t)p[u].h * j.d_sH + p[u].r] = s;
     }
 }
 
-int launch_precompute_D(const DJob& j, cudaStream_t stream) {
-    const long long nrows = (long long)j.BH * j.T;
-    if (nrows == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((nrows * 16 + 255) / 256, 148 * 8);
-    precompute_D_kernel<<<blocks, 256, 0, stream>>>(j);
-    count_launch();
+int launch_precompute_D(const DJob& job, cudaStream_t stream) {
+    const int B = job.BH / job.H, step = batches_per_launch(B, job.H, job.T);
+    for (int b = 0; b < B; b += step) {
+        DJob j = job;
+        j.dO.ptr += b * j.dO.sB;
+        j.O.ptr += b * j.O.sB;
+        j.D += b * j.d_sB;
+        if (j.dQ_zero) j.dQ_zero += b * j.dq_sB;
+        const uint32_t nrows = (uint32_t)std::min(step, B - b) * j.H * j.T;
+        precompute_D_kernel<<<(nrows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 256, 0, stream>>>(j, nrows);
+        count_launch();
+    }
     return check_launch();
 }
 
@@ -155,69 +176,70 @@ int launch_precompute_D_hd(const DJob& j, int head_dim, cudaStream_t stream) {
 // reference leaves this to its caller, kernels_test.cu:562)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) zero_rows_kernel(float* ptr, int64_t sB, int64_t sM, int64_t sH, int H, int T,
-                                                        long long nvec) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i >> 4;
-        const int c4 = (int)(i & 15);
-        const int bh = (int)(row / T);
-        const int r = (int)(row - (long long)bh * T);
-        const int b = bh / H, h = bh - b * H;
-        reinterpret_cast<float4*>(ptr + (int64_t)b * sB + (int64_t)h * sH + (int64_t)r * sM)[c4] =
-            make_float4(0.f, 0.f, 0.f, 0.f);
+                                                        uint32_t nrows) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint32_t row = blockIdx.x * ROWS_PER_BLOCK + 16 * u + (threadIdx.x >> 4);
+        if (row < nrows)
+            reinterpret_cast<float4*>(ptr + row_off(row_pos(row, T, H), sB, sM, sH))[threadIdx.x & 15] =
+                make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
 int launch_zero_rows(float* ptr, int64_t sB, int64_t sM, int64_t sH, int B, int H, int T, cudaStream_t stream) {
-    const long long nvec = (long long)B * H * T * 16;
-    if (nvec == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((nvec + 255) / 256, 148 * 8);
-    zero_rows_kernel<<<blocks, 256, 0, stream>>>(ptr, sB, sM, sH, H, T, nvec);
-    count_launch();
+    const int step = batches_per_launch(B, H, T);
+    for (int b = 0; b < B; b += step) {
+        const uint32_t nrows = (uint32_t)std::min(step, B - b) * H * T;
+        zero_rows_kernel<<<(nrows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 256, 0, stream>>>(ptr + b * sB, sB, sM, sH, H, T, nrows);
+        count_launch();
+    }
     return check_launch();
 }
 
 // ---------------------------------------------------------------------------
 // Deterministic dQ: add the per-KV-tile slabs in KV-tile order.  A query tile is in the slab of KV tile kt only if
-// the backward CTA of kt visited it: under the causal mask that is every query tile from
-// it0(kt) = clamp((kt*128 + k_pos0 - q_pos0) / 128) on (attn_bwd_sm100.cu computes the same bound).
+// the backward CTA of kt visited it (attn_bwd_sm100.cu computes the same bound).  HBM-bound: the slabs are read four at
+// a time, all loads before the first addition.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) reduce_dq_slabs_kernel(DqReduceJob j, long long nvec) {
-    const long long slab = (long long)j.B * j.H * j.T * 16;  // float4 per slab
-    const int n_qtiles = (j.T + TILE - 1) / TILE;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i >> 4;
-        const int c4 = (int)(i & 15);
-        const int bh = (int)(row / j.T);
-        const int r = (int)(row - (long long)bh * j.T);
-        const int b = bh / j.H, h = bh - b * j.H;
-        const int qt = r / TILE;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4* out = reinterpret_cast<float4*>(j.dQ + (int64_t)b * j.dq_sB + (int64_t)h * j.dq_sH + (int64_t)r * j.dq_sM) + c4;
-        if (j.accumulate) acc = *out;
-        const float4* src = reinterpret_cast<const float4*>(j.slabs) + i;
-        for (int kt = 0; kt < j.n_kvtiles; ++kt) {
-            int it0 = 0;
-            if (j.causal) {
-                const long long first_q = (long long)kt * TILE + j.k_pos0 - j.q_pos0;
-                if (first_q > 0) it0 = (int)min((long long)n_qtiles, first_q / TILE);
-            }
-            if (qt >= it0) {
-                const float4 v = __ldg(src + (long long)kt * slab);
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-            }
-        }
-        *out = acc;
+__global__ void __launch_bounds__(256) reduce_dq_slabs_kernel(DqReduceJob j, uint32_t nrows) {
+    const uint32_t row = blockIdx.x * 16u + (threadIdx.x >> 4);
+    if (row >= nrows) return;
+    const int sub = threadIdx.x & 15;
+    const RowPos p = row_pos(row, j.T, j.H);
+    // KV tiles 0 .. n-1 visited this row's query tile: under the causal mask those whose first key is not past its end
+    int n = j.n_kvtiles;
+    if (j.causal) {
+        const long long end = (long long)(p.r / TILE + 1) * TILE + j.q_pos0 - j.k_pos0;
+        n = (int)max(0ll, min((long long)n, (end + TILE - 1) / TILE));
     }
+    float4* out = reinterpret_cast<float4*>(j.dQ + row_off(p, j.dq_sB, j.dq_sM, j.dq_sH)) + sub;
+    float4 acc = j.accumulate ? *out : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t slab = (int64_t)j.slab_rows * 16;  // float4 per slab
+    const float4* src = reinterpret_cast<const float4*>(j.slabs) + (int64_t)row * 16 + sub;
+    for (int kt = 0; kt < n; kt += 4) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            v[u] = kt + u < n ? __ldcs(src + (kt + u) * slab) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
+        }
+    }
+    *out = acc;
 }
 
-int launch_reduce_dq_slabs(const DqReduceJob& j, cudaStream_t stream) {
-    const long long nvec = (long long)j.B * j.H * j.T * 16;
-    if (nvec == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((nvec + 255) / 256, 148 * 8);
-    reduce_dq_slabs_kernel<<<blocks, 256, 0, stream>>>(j, nvec);
-    count_launch();
+int launch_reduce_dq_slabs(const DqReduceJob& job, cudaStream_t stream) {
+    const int step = batches_per_launch(job.B, job.H, job.T);
+    for (int b = 0; b < job.B; b += step) {
+        DqReduceJob j = job;
+        j.slab_rows = (int64_t)job.B * j.H * j.T;
+        j.slabs += (int64_t)b * j.H * j.T * 64;
+        j.dQ += b * j.dq_sB;
+        const uint32_t nrows = (uint32_t)std::min(step, job.B - b) * j.H * j.T;
+        reduce_dq_slabs_kernel<<<(nrows + 15) / 16, 256, 0, stream>>>(j, nrows);
+        count_launch();
+    }
     return check_launch();
 }
 

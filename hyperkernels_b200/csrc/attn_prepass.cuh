@@ -29,6 +29,7 @@ struct DqReduceJob {
     int B, H, T, n_kvtiles;
     int causal, q_pos0, k_pos0;
     int accumulate;  // 1: add to what dQ holds (HK_FLAG_ACCUM_DQ)
+    int64_t slab_rows;  // rows of one slab; set by the launcher
 };
 int launch_reduce_dq_slabs(const DqReduceJob& j, cudaStream_t stream);
 
