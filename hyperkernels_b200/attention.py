@@ -18,8 +18,8 @@ Here the same blocks are ``ctypes.Structure`` classes with the same field names
 functions ``fused_attn_forward``, ``mem_efficient_bwd_precompute_D`` and
 ``mem_efficient_bwd_unified``, which call the C ABI of ``libhk_attention.so``.
 ``attention_forward`` / ``attention_backward`` are conveniences that fill the
-blocks from torch CUDA tensors; torch is used only to own device memory and
-streams.
+blocks from torch CUDA tensors in native code (``csrc/hk_torch.cpp``); torch is
+used only to own device memory and streams.
 """
 from __future__ import annotations
 
@@ -120,7 +120,6 @@ def lib() -> C.CDLL:
         L.hk_status_string.argtypes = [C.c_int]
         L.hk_attn_forward.argtypes = [C.POINTER(MemEfficientFwdParams), C.c_void_p]
         L.hk_attn_backward.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
-        L.hk_attn_zero_dq.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
         L.hk_attn_bwd_precompute_D.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_void_p]
         L.hk_attn_bwd_precompute_D_hd.argtypes = [C.POINTER(MemEfficientBwdParams), C.c_int, C.c_void_p]
         L.hk_attn_fwd_workspace_bytes.restype = C.c_size_t
@@ -205,30 +204,26 @@ def dropout_keep_mask(BH: int, Tq: int, Tk: int, p: float, seed: int, offset: in
 
 
 # ---- conveniences over torch tensors -----------------------------------------
-def _strides_bmh(t):
-    """(strideB, strideM, strideH) in elements of a [B, H, T, 64] tensor view."""
-    assert t.dim() == 4 and t.shape[-1] == 64 and t.stride(-1) == 1, "expected [B,H,T,64] with unit last stride"
-    return t.stride(0), t.stride(2), t.stride(1)
+_native = None
 
 
-def _set3(p, name, t):
-    sB, sM, sH = _strides_bmh(t)
-    setattr(p, f"{name}_strideB", sB)
-    setattr(p, f"{name}_strideM", sM)
-    setattr(p, f"{name}_strideH", sH)
+def _torch_calls():
+    """The native call path over torch tensors (csrc/hk_torch.cpp), bound to the library lib() loads."""
+    global _native
+    if _native is None:
+        import importlib.util
 
+        import torch  # noqa: F401  (the module links against its libraries)
 
-def _workspace(nbytes: int, like, workspace):
-    import torch
-
-    if nbytes == 0:
-        return None
-    if workspace is None:
-        workspace = torch.empty(nbytes + 256, dtype=torch.uint8, device=like.device)
-    base = workspace.data_ptr()
-    off = (-base) % 256
-    assert workspace.numel() - off >= nbytes, "workspace too small"
-    return workspace, base + off
+        path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "_hk_torch.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `make -C hyperkernels_b200/csrc`. There is no fallback.")
+        spec = importlib.util.spec_from_file_location("_hk_torch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind(lib()._handle)
+        _native = mod
+    return _native
 
 
 def attention_forward(Q, K, V, scale: float, causal: bool, *, dropout_p: float = 0.0, dropout_mask=None,
@@ -236,26 +231,9 @@ def attention_forward(Q, K, V, scale: float, causal: bool, *, dropout_p: float =
                       bh_pos0: int = 0, prerounded: bool = False, dropout_scaled: bool = False, continue_state: bool = False,
                       round_in_hbm: bool = False, workspace=None, out=None, lse=None, stream=None):
     """O, LSE = fused attention forward of [B,H,Tq,64] Q against [B,H,Tk,64] K, V (fp32 CUDA tensors)."""
-    import torch
-
-    B, H, Tq, _ = Q.shape
-    Tk = K.shape[2]
-    O = out if out is not None else torch.empty((B, H, Tq, 64), dtype=torch.float32, device=Q.device)
-    LSE = lse if lse is not None else torch.empty((B, H, Tq), dtype=torch.float32, device=Q.device)
-    p = MemEfficientFwdParams()
-    p.Q, p.K, p.V, p.O, p.LSE = Q.data_ptr(), K.data_ptr(), V.data_ptr(), O.data_ptr(), LSE.data_ptr()
-    p.B, p.nh, p.T = B, H, Tq
-    p.scale, p.is_causal, p.dropout_p = scale, bool(causal), dropout_p
-    p.dropout_mask = dropout_mask.data_ptr() if dropout_mask is not None else None
-    for name, t in (("q", Q), ("k", K), ("v", V), ("o", O)):
-        _set3(p, name, t)
-    p.lse_strideB, p.lse_strideH = LSE.stride(0), LSE.stride(1)
-    p.kv_len = Tk if Tk != Tq else 0
-    p.q_pos0, p.k_pos0, p.bh_pos0 = q_pos0, k_pos0, bh_pos0
     flags = 0
     if philox_seed is not None:
         flags |= FLAG_PHILOX_DROPOUT
-        p.dropout_seed, p.dropout_offset = philox_seed, philox_offset
     if prerounded:
         flags |= FLAG_OPERANDS_PREROUNDED
     if dropout_scaled:
@@ -265,13 +243,12 @@ def attention_forward(Q, K, V, scale: float, causal: bool, *, dropout_p: float =
         flags |= FLAG_CONTINUE_SOFTMAX_STATE
     if round_in_hbm:
         flags |= FLAG_ROUND_IN_HBM
-    p.flags = flags
-    need = fwd_workspace_bytes(p)
-    ws = _workspace(need, Q, workspace)
-    if ws is not None:
-        p.workspace, p.workspace_bytes = ws[1], need
-    fused_attn_forward(p, stream)
-    return O, LSE
+    r = (_native or _torch_calls()).forward(
+        Q, K, V, scale, causal, dropout_p, dropout_mask, philox_seed, philox_offset, q_pos0, k_pos0, bh_pos0, flags,
+        workspace, out, lse, stream if stream is None else _stream_handle(stream))
+    if type(r) is int:
+        raise HKError(r, "hk_attn_forward")
+    return r
 
 
 def attention_backward(Q, K, V, O, dO, LSE, scale: float, causal: bool, *, dropout_p: float = 0.0, dropout_mask=None,
@@ -281,35 +258,9 @@ def attention_backward(Q, K, V, O, dO, LSE, scale: float, causal: bool, *, dropo
                        round_in_hbm: bool = False, deterministic_dq: bool = False, workspace=None, dQ=None, dK=None, dV=None,
                        stream=None):
     """dQ, dK, dV, D = fused attention backward (fp32 CUDA tensors, [B,H,T,64])."""
-    import torch
-
-    B, H, Tq, _ = Q.shape
-    Tk = K.shape[2]
-    dev = Q.device
-    dQ = dQ if dQ is not None else torch.empty((B, H, Tq, 64), dtype=torch.float32, device=dev)
-    dK = dK if dK is not None else torch.empty((B, H, Tk, 64), dtype=torch.float32, device=dev)
-    dV = dV if dV is not None else torch.empty((B, H, Tk, 64), dtype=torch.float32, device=dev)
-    D = D if D is not None else torch.empty((B, H, Tq), dtype=torch.float32, device=dev)
-    p = MemEfficientBwdParams()
-    p.Q, p.K, p.V, p.dO, p.LSE = Q.data_ptr(), K.data_ptr(), V.data_ptr(), dO.data_ptr(), LSE.data_ptr()
-    p.O = O.data_ptr() if O is not None else None
-    p.D, p.dQ, p.dK, p.dV = D.data_ptr(), dQ.data_ptr(), dK.data_ptr(), dV.data_ptr()
-    p.B, p.nh, p.T = B, H, Tq
-    p.scale, p.is_causal = scale, bool(causal)
-    for name, t in (("q", Q), ("k", K), ("v", V), ("do", dO), ("dq", dQ), ("dk", dK), ("dv", dV)):
-        _set3(p, name, t)
-    if O is not None:
-        _set3(p, "o", O)
-    p.lse_strideB, p.lse_strideH = LSE.stride(0), LSE.stride(1)
-    p.d_strideB, p.d_strideH = D.stride(0), D.stride(1)
-    p.dropout_p = dropout_p
-    p.dropout_mask = dropout_mask.data_ptr() if dropout_mask is not None else None
-    p.kv_len = Tk if Tk != Tq else 0
-    p.q_pos0, p.k_pos0, p.bh_pos0 = q_pos0, k_pos0, bh_pos0
     flags = 0
     if philox_seed is not None:
         flags |= FLAG_PHILOX_DROPOUT
-        p.dropout_seed, p.dropout_offset = philox_seed, philox_offset
     if prerounded:
         flags |= FLAG_OPERANDS_PREROUNDED
     if d_precomputed:
@@ -327,20 +278,17 @@ def attention_backward(Q, K, V, O, dO, LSE, scale: float, causal: bool, *, dropo
         flags |= FLAG_ROUND_IN_HBM
     if deterministic_dq:
         flags |= FLAG_DETERMINISTIC_DQ
-    p.flags = flags
-    ws = _workspace(bwd_workspace_bytes(p), Q, workspace)
-    if ws is not None:
-        p.workspace, p.workspace_bytes = ws[1], bwd_workspace_bytes(p)
-    mem_efficient_bwd_unified(p, stream)
-    return dQ, dK, dV, D
+    r = (_native or _torch_calls()).backward(
+        Q, K, V, O, dO, LSE, scale, causal, dropout_p, dropout_mask, philox_seed, philox_offset, q_pos0, k_pos0, bh_pos0,
+        flags, workspace, D, dQ, dK, dV, stream if stream is None else _stream_handle(stream))
+    if type(r) is int:
+        raise HKError(r, "hk_attn_backward")
+    return r
 
 
 def zero_dq(dQ, stream=None) -> None:
     """Zeroes a [B, H, T, 64] dQ on a stream of the caller's choice, for a backward with accum_dq."""
-    p = MemEfficientBwdParams()
-    p.dQ, (p.B, p.nh, p.T) = dQ.data_ptr(), dQ.shape[:3]
-    _set3(p, "dq", dQ)
-    _check(lib().hk_attn_zero_dq(C.byref(p), _stream_handle(stream)), "hk_attn_zero_dq")
+    _check((_native or _torch_calls()).zero(dQ, stream if stream is None else _stream_handle(stream)), "hk_attn_zero_dq")
 
 
 def round_tf32(x, out=None, stream=None):

@@ -1,0 +1,241 @@
+// hk_torch.cpp -- attention_forward / attention_backward over torch tensors, from native code: reads the tensors,
+// allocates the outputs that were not given, fills the argument block and calls the library.
+//
+// The two calls on a small problem are host-bound: filling the ctypes blocks, allocating through torch's Python API and
+// asking for the current stream took longer than the kernels run.  This module does the same work without Python
+// objects in between.  The library is the one attention.py loads (dlsym on its handle), so an instrumented build given
+// by HK_ATTENTION_LIB is used here too.
+#include <ATen/ATen.h>
+#include <Python.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/hk_attention.h"
+
+namespace {
+
+typedef int (*FwdFn)(const hk_attn_fwd_params*, void*);
+typedef int (*BwdFn)(const hk_attn_bwd_params*, void*);
+typedef int (*ZeroFn)(const hk_attn_bwd_params*, void*);
+typedef size_t (*FwdSizeFn)(const hk_attn_fwd_params*);
+typedef size_t (*BwdSizeFn)(const hk_attn_bwd_params*);
+struct Library {
+    FwdFn forward;
+    BwdFn backward;
+    ZeroFn zero_dq;
+    FwdSizeFn fwd_bytes;
+    BwdSizeFn bwd_bytes;
+} g_lib = {};
+
+// A tensor argument; nullptr for None or anything that is no tensor.
+const at::Tensor* tensor_or_null(PyObject* o) {
+    return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+}
+
+// strides of a [B, H, T, 64] view into the block's (B, M, H) triple; false with AssertionError set
+bool strides(const at::Tensor& t, int64_t* sB, int64_t* sM, int64_t* sH) {
+    if (t.dim() != 4 || t.size(3) != 64 || t.stride(3) != 1) {
+        PyErr_SetString(PyExc_AssertionError, "expected [B,H,T,64] with unit last stride");
+        return false;
+    }
+    *sB = t.stride(0);
+    *sM = t.stride(2);
+    *sH = t.stride(1);
+    return true;
+}
+
+bool need_tensors(std::initializer_list<const at::Tensor*> ts) {
+    for (const at::Tensor* t : ts)
+        if (!t) {
+            PyErr_SetString(PyExc_TypeError, "expected a tensor");
+            return false;
+        }
+    return true;
+}
+
+void* stream_of(PyObject* o) {
+    if (o == Py_None) return c10::cuda::getCurrentCUDAStream().stream();
+    return reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(o));
+}
+
+float* data(const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); }
+
+// workspace: 256-byte aligned start inside a tensor a caller brought; false with AssertionError set if `need` does not fit
+bool given_workspace(const at::Tensor* t, size_t need, void** ptr, size_t* bytes) {
+    if (!t) return true;
+    uint8_t* base = static_cast<uint8_t*>(t->data_ptr());
+    const size_t off = (256 - (reinterpret_cast<uintptr_t>(base) & 255u)) & 255u;
+    const size_t have = (size_t)t->numel();
+    if (need > 0 && have < off + need) {
+        PyErr_SetString(PyExc_AssertionError, "workspace too small");
+        return false;
+    }
+    *ptr = base + off;
+    *bytes = have > off ? have - off : 0;
+    return true;
+}
+
+}  // namespace
+
+// forward(Q, K, V, scale, causal, dropout_p, dropout_mask, seed, offset, q_pos0, k_pos0, bh_pos0, flags, workspace, out,
+//         lse, stream) -> (O, LSE), or the negative status of the call
+static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 17) {
+        PyErr_SetString(PyExc_TypeError, "forward: 17 arguments");
+        return nullptr;
+    }
+    const at::Tensor *Q = tensor_or_null(a[0]), *K = tensor_or_null(a[1]), *V = tensor_or_null(a[2]), *mask = tensor_or_null(a[6]),
+                     *ws = tensor_or_null(a[13]), *out = tensor_or_null(a[14]), *lse = tensor_or_null(a[15]);
+    if (!need_tensors({Q, K, V})) return nullptr;
+    hk_attn_fwd_params p = {};
+    if (!strides(*Q, &p.q_strideB, &p.q_strideM, &p.q_strideH) || !strides(*K, &p.k_strideB, &p.k_strideM, &p.k_strideH) ||
+        !strides(*V, &p.v_strideB, &p.v_strideM, &p.v_strideH))
+        return nullptr;
+    const int64_t B = Q->size(0), H = Q->size(1), Tq = Q->size(2), Tk = K->size(2);
+    at::Tensor O, L;
+    try {
+        const auto opt = Q->options().dtype(at::kFloat);
+        O = out ? *out : at::empty({B, H, Tq, 64}, opt);
+        L = lse ? *lse : at::empty({B, H, Tq}, opt);
+        if (!strides(O, &p.o_strideB, &p.o_strideM, &p.o_strideH)) return nullptr;
+        p.lse_strideB = L.stride(0);
+        p.lse_strideH = L.stride(1);
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    p.Q = data(*Q); p.K = data(*K); p.V = data(*V); p.O = data(O); p.LSE = data(L);
+    p.B = (int)B; p.nh = (int)H; p.T = Tq;
+    p.scale = (float)PyFloat_AsDouble(a[3]);
+    p.is_causal = PyObject_IsTrue(a[4]) != 0;
+    p.dropout_p = (float)PyFloat_AsDouble(a[5]);
+    p.dropout_mask = mask ? data(*mask) : nullptr;
+    p.kv_len = Tk != Tq ? Tk : 0;
+    p.dropout_seed = a[7] == Py_None ? 0 : PyLong_AsUnsignedLongLongMask(a[7]);
+    p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[8]);
+    p.q_pos0 = PyLong_AsLongLong(a[9]);
+    p.k_pos0 = PyLong_AsLongLong(a[10]);
+    p.bh_pos0 = (uint32_t)PyLong_AsUnsignedLongLongMask(a[11]);
+    p.flags = (uint32_t)PyLong_AsUnsignedLongLongMask(a[12]);
+    void* stream = stream_of(a[16]);
+    if (PyErr_Occurred()) return nullptr;
+    if (ws && !given_workspace(ws, g_lib.fwd_bytes(&p), &p.workspace, &p.workspace_bytes)) return nullptr;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_lib.forward(&p, stream);
+    Py_END_ALLOW_THREADS
+    if (rc != 0) return PyLong_FromLong(rc);
+    PyObject* res = PyTuple_New(2);
+    PyTuple_SET_ITEM(res, 0, THPVariable_Wrap(std::move(O)));
+    PyTuple_SET_ITEM(res, 1, THPVariable_Wrap(std::move(L)));
+    return res;
+}
+
+// backward(Q, K, V, O, dO, LSE, scale, causal, dropout_p, dropout_mask, seed, offset, q_pos0, k_pos0, bh_pos0, flags,
+//          workspace, D, dQ, dK, dV, stream) -> (dQ, dK, dV, D), or the negative status of the call
+static PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 22) {
+        PyErr_SetString(PyExc_TypeError, "backward: 22 arguments");
+        return nullptr;
+    }
+    const at::Tensor *Q = tensor_or_null(a[0]), *K = tensor_or_null(a[1]), *V = tensor_or_null(a[2]), *O = tensor_or_null(a[3]),
+                     *dO = tensor_or_null(a[4]), *LSE = tensor_or_null(a[5]), *mask = tensor_or_null(a[9]),
+                     *ws = tensor_or_null(a[16]);
+    const at::Tensor* given[4] = {tensor_or_null(a[18]), tensor_or_null(a[19]), tensor_or_null(a[20]), tensor_or_null(a[17])};
+    if (!need_tensors({Q, K, V, dO, LSE})) return nullptr;
+    hk_attn_bwd_params p = {};
+    if (!strides(*Q, &p.q_strideB, &p.q_strideM, &p.q_strideH) || !strides(*K, &p.k_strideB, &p.k_strideM, &p.k_strideH) ||
+        !strides(*V, &p.v_strideB, &p.v_strideM, &p.v_strideH) || !strides(*dO, &p.do_strideB, &p.do_strideM, &p.do_strideH) ||
+        (O && !strides(*O, &p.o_strideB, &p.o_strideM, &p.o_strideH)))
+        return nullptr;
+    const int64_t B = Q->size(0), H = Q->size(1), Tq = Q->size(2), Tk = K->size(2);
+    p.flags = (uint32_t)PyLong_AsUnsignedLongLongMask(a[15]);
+    p.B = (int)B; p.nh = (int)H; p.T = (int)Tq;
+    p.kv_len = Tk != Tq ? Tk : 0;
+    at::Tensor r[4], slabs;  // dQ, dK, dV, D
+    try {
+        const auto opt = Q->options().dtype(at::kFloat);
+        for (int i = 0; i < 4; ++i)
+            r[i] = given[i] ? *given[i] : i == 3 ? at::empty({B, H, Tq}, opt) : at::empty({B, H, i == 0 ? Tq : Tk, 64}, opt);
+        if (!strides(r[0], &p.dq_strideB, &p.dq_strideM, &p.dq_strideH) || !strides(r[1], &p.dk_strideB, &p.dk_strideM, &p.dk_strideH) ||
+            !strides(r[2], &p.dv_strideB, &p.dv_strideM, &p.dv_strideH))
+            return nullptr;
+        p.d_strideB = r[3].stride(0);
+        p.d_strideH = r[3].stride(1);
+        p.lse_strideB = LSE->stride(0);
+        p.lse_strideH = LSE->stride(1);
+        if (ws) {
+            if (!given_workspace(ws, g_lib.bwd_bytes(&p), &p.workspace, &p.workspace_bytes)) return nullptr;
+        } else if (p.flags & HK_FLAG_DETERMINISTIC_DQ) {  // the slabs of partial dQ are the only scratch there is
+            hk_attn_bwd_params q = p;
+            q.flags |= HK_FLAG_OPERANDS_PREROUNDED;
+            const size_t bytes = g_lib.bwd_bytes(&q);
+            slabs = at::empty({(int64_t)bytes + 256}, Q->options().dtype(at::kByte));
+            if (!given_workspace(&slabs, bytes, &p.workspace, &p.workspace_bytes)) return nullptr;
+        }
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+    p.Q = data(*Q); p.K = data(*K); p.V = data(*V); p.O = O ? data(*O) : nullptr; p.dO = data(*dO); p.LSE = data(*LSE);
+    p.dQ = data(r[0]); p.dK = data(r[1]); p.dV = data(r[2]); p.D = data(r[3]);
+    p.scale = (float)PyFloat_AsDouble(a[6]);
+    p.is_causal = PyObject_IsTrue(a[7]) != 0;
+    p.dropout_p = (float)PyFloat_AsDouble(a[8]);
+    p.dropout_mask = mask ? data(*mask) : nullptr;
+    p.dropout_seed = a[10] == Py_None ? 0 : PyLong_AsUnsignedLongLongMask(a[10]);
+    p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[11]);
+    p.q_pos0 = PyLong_AsLongLong(a[12]);
+    p.k_pos0 = PyLong_AsLongLong(a[13]);
+    p.bh_pos0 = (uint32_t)PyLong_AsUnsignedLongLongMask(a[14]);
+    void* stream = stream_of(a[21]);
+    if (PyErr_Occurred()) return nullptr;
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_lib.backward(&p, stream);
+    Py_END_ALLOW_THREADS
+    if (rc != 0) return PyLong_FromLong(rc);
+    PyObject* res = PyTuple_New(4);
+    for (int i = 0; i < 4; ++i) PyTuple_SET_ITEM(res, i, THPVariable_Wrap(std::move(r[i])));
+    return res;
+}
+
+// zero(x, stream) -> status: zeroes a [B, H, T, 64] view
+static PyObject* zero(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    const at::Tensor* x = n == 2 ? tensor_or_null(a[0]) : nullptr;
+    if (!need_tensors({x})) return nullptr;
+    hk_attn_bwd_params p = {};
+    if (!strides(*x, &p.dq_strideB, &p.dq_strideM, &p.dq_strideH)) return nullptr;
+    p.B = (int)x->size(0); p.nh = (int)x->size(1); p.T = (int)x->size(2);
+    p.dQ = data(*x);
+    void* stream = stream_of(a[1]);
+    if (PyErr_Occurred()) return nullptr;
+    return PyLong_FromLong(g_lib.zero_dq(&p, stream));
+}
+
+// bind(handle): the dlopen handle of libhk_attention.so
+static PyObject* bind(PyObject*, PyObject* h) {
+    void* so = reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(h));
+    if (PyErr_Occurred()) return nullptr;
+    g_lib.forward = reinterpret_cast<FwdFn>(dlsym(so, "hk_attn_forward_noscratch"));
+    g_lib.backward = reinterpret_cast<BwdFn>(dlsym(so, "hk_attn_backward_noscratch"));
+    g_lib.zero_dq = reinterpret_cast<ZeroFn>(dlsym(so, "hk_attn_zero_dq"));
+    g_lib.fwd_bytes = reinterpret_cast<FwdSizeFn>(dlsym(so, "hk_attn_fwd_workspace_bytes"));
+    g_lib.bwd_bytes = reinterpret_cast<BwdSizeFn>(dlsym(so, "hk_attn_bwd_workspace_bytes"));
+    if (!g_lib.forward || !g_lib.backward || !g_lib.zero_dq || !g_lib.fwd_bytes || !g_lib.bwd_bytes) {
+        PyErr_SetString(PyExc_ImportError, "libhk_attention.so lacks an entry point");
+        return nullptr;
+    }
+    Py_RETURN_NONE;
+}
+
+static PyMethodDef methods[] = {
+    {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward)), METH_FASTCALL, nullptr},
+    {"backward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(backward)), METH_FASTCALL, nullptr},
+    {"zero", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(zero)), METH_FASTCALL, nullptr},
+    {"bind", bind, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+static PyModuleDef module = {PyModuleDef_HEAD_INIT, "_hk_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+PyMODINIT_FUNC PyInit__hk_torch() { return PyModule_Create(&module); }

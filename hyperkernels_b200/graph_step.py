@@ -41,7 +41,6 @@ class GraphedAttentionStep:
         self.dV = torch.empty((B, H, Tk, 64), dtype=torch.float32, device=dev)
         self.LSE = torch.empty((B, H, T), dtype=torch.float32, device=dev)
         self.D = torch.empty((B, H, T), dtype=torch.float32, device=dev)
-        self._ws = torch.empty(2 * B * H * (T + Tk) * 256 + 1024, dtype=torch.uint8, device=dev)
         drop = {}
         if dropout_p > 0:
             if philox_seed is None:
@@ -54,11 +53,11 @@ class GraphedAttentionStep:
         def step():
             main = torch.cuda.current_stream(dev)
             zero_stream.wait_stream(main)
-            att.attention_forward(Q, K, V, scale, causal, workspace=self._ws, out=self.O, lse=self.LSE, **drop)
+            att.attention_forward(Q, K, V, scale, causal, out=self.O, lse=self.LSE, **drop)
             att.zero_dq(self.dQ, zero_stream)
             main.wait_stream(zero_stream)
-            att.attention_backward(Q, K, V, self.O, dO, self.LSE, scale, causal, workspace=self._ws, D=self.D,
-                                   dQ=self.dQ, dK=self.dK, dV=self.dV, reuse_fwd_rounded=True, accum_dq=True, **drop)
+            att.attention_backward(Q, K, V, self.O, dO, self.LSE, scale, causal, D=self.D,
+                                   dQ=self.dQ, dK=self.dK, dV=self.dV, accum_dq=True, **drop)
 
         n0 = att.launch_count()
         side = torch.cuda.Stream(device=dev)

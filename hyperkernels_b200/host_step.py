@@ -17,7 +17,7 @@ queues -- is captured in a CUDA graph the second time it is called with the same
 host tensors and replayed from then on, so the host issues one call per step.
 
 Everything on the device goes through the C ABI (``hk_attn_forward`` and
-``hk_attn_backward`` per chunk, with preallocated buffers and workspace); torch
+``hk_attn_backward`` per chunk, with preallocated buffers); torch
 is used for pinned host memory, streams and events only.
 """
 from __future__ import annotations
@@ -78,7 +78,6 @@ class HostAttentionStep:
                  for k in ("Q", "K", "V", "dO", "O", "dQ", "dK", "dV")}
             s["LSE"] = torch.empty(lshp, dtype=torch.float32, device=self.device)
             s["D"] = torch.empty(lshp, dtype=torch.float32, device=self.device)
-            s["ws"] = torch.empty(4 * self.cb * T * 256 + 512, dtype=torch.uint8, device=self.device)
             self.slots.append(s)
         self.s_in, self.s_cmp, self.s_out = (torch.cuda.Stream(device=self.device) for _ in range(3))
         self.ev_start = torch.cuda.Event()
@@ -132,7 +131,7 @@ class HostAttentionStep:
         for i in range(self.chunks):
             full = self.slots[i % n_slots]
             m = self.sizes[i]
-            d = {k: (v if k == "ws" else v[:m]) for k, v in full.items()}  # this chunk's part of the slot's buffers
+            d = {k: v[:m] for k, v in full.items()}  # this chunk's part of the slot's buffers
             sl = slice(self.starts[i], self.starts[i] + m)
             with torch.cuda.stream(self.s_in):
                 if i >= n_slots:  # the kernels of the chunk that used this slot have read its inputs
@@ -147,11 +146,11 @@ class HostAttentionStep:
                 if i >= n_slots:  # the results of the chunk that used this slot have left
                     self.s_cmp.wait_event(self.ev_out[i - n_slots])
                 drop = dict(self.drop, philox_offset=self.philox_offset, bh_pos0=self.starts[i]) if self.drop else {}
-                att.attention_forward(d["Q"], d["K"], d["V"], self.scale, self.causal, workspace=d["ws"], out=d["O"],
+                att.attention_forward(d["Q"], d["K"], d["V"], self.scale, self.causal, out=d["O"],
                                       lse=d["LSE"], stream=self.s_cmp, **drop)
                 att.attention_backward(d["Q"], d["K"], d["V"], d["O"], d["dO"], d["LSE"], self.scale, self.causal,
-                                       workspace=d["ws"], D=d["D"], dQ=d["dQ"], dK=d["dK"], dV=d["dV"],
-                                       reuse_fwd_rounded=True, stream=self.s_cmp, **drop)
+                                       D=d["D"], dQ=d["dQ"], dK=d["dK"], dV=d["dV"],
+                                       stream=self.s_cmp, **drop)
                 self.ev_cmp[i].record(self.s_cmp)
             with torch.cuda.stream(self.s_out):
                 self.s_out.wait_event(self.ev_cmp[i])
