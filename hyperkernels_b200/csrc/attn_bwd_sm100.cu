@@ -225,24 +225,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         }
     }
     if (threadIdx.x == 0) {
-        mbar_init(&sh.v_ready, NUM_COMPUTE);
+        // compute-warp barriers count one arrival per warp
+        mbar_init(&sh.v_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.qk_free, 1);
         mbar_init(&sh.dok_free, 1);
         mbar_init(&sh.s_full, 1);
         mbar_init(&sh.dp_full, 1);
         for (int g = 0; g < 4; ++g) {
-            mbar_init(&sh.pt_ready[g], TILE);
-            mbar_init(&sh.p_ready[g], TILE);
+            mbar_init(&sh.pt_ready[g], TILE / 32);
+            mbar_init(&sh.p_ready[g], TILE / 32);
         }
         mbar_init(&sh.dv_done, 1);
         mbar_init(&sh.dk_done, 1);
-        mbar_init(&sh.ds_ready, NUM_COMPUTE);
+        mbar_init(&sh.ds_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.dq_full, 1);
-        mbar_init(&sh.dq_empty, 256);   // column groups 2, 3 drain dQ
-        mbar_init(&sh.dq_staged, 256);
+        mbar_init(&sh.dq_empty, 8);   // column groups 2, 3 drain dQ
+        mbar_init(&sh.dq_staged, 8);
         mbar_init(&sh.dq_out, 1);
-        mbar_init(&sh.staged, 256);    // the threads that stage LSE and D
-        mbar_init(&sh.acc_staged, NUM_COMPUTE);
+        mbar_init(&sh.staged, 8);    // the threads that stage LSE and D
+        mbar_init(&sh.acc_staged, NUM_COMPUTE / 32);
         sh.abort_flag = 0;
         fence_mbar_init();
     }
@@ -517,14 +518,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             tmem_ld32(trow + COL_DQ + 32 * (part & 1), v);
             tmem_wait_ld();
             tc_fence_before_sync();
-            mbar_arrive(&sh.dq_empty);  // dQ is in registers: the next dQ = dS K may overwrite tensor memory
+            mbar_arrive_warp(&sh.dq_empty, lane);  // dQ is in registers: the next dQ = dS K may overwrite tensor memory
             uint8_t* srow = sdO + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
                 *reinterpret_cast<uint4*>(srow + ((c ^ (row & 7)) << 4)) =
                     make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
             fence_proxy_async_smem();
-            mbar_arrive(&sh.dq_staged);
+            mbar_arrive_warp(&sh.dq_staged, lane);
             return true;
         };
 
@@ -544,7 +545,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tmem_st16(trow + COL_V + 16 * part, rv);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive(&sh.v_ready);
+                mbar_arrive_warp(&sh.v_ready, lane);
             }
             HK_XSTAMP(tlx, 3);
         }
@@ -562,7 +563,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     sh.lse[it & 1][tid] = staged_val;
                 else
                     sh.dsum[it & 1][tid - TILE] = staged_val;
-                mbar_arrive(&sh.staged);
+                mbar_arrive_warp(&sh.staged, lane);
                 if (it + 1 < n_it) staged_val = fetch_lse_or_d(q0 + TILE);
             }
             // an mbarrier rather than bar.sync: its wait is bounded, so a CTA that is
@@ -670,7 +671,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tmem_st32(trow + COL_S + c0, rp);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive(&sh.pt_ready[part]);
+                mbar_arrive_warp(&sh.pt_ready[part], lane);
             }
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, it & 1, W_SFULL, 1000 + it));
             if (!ok) break;
@@ -713,7 +714,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             tmem_wait_st();
             stamp(a, tlc, it, 1, 13);
             tc_fence_before_sync();
-            mbar_arrive(&sh.p_ready[part]);  // this group's slices of dK += dS^T Q may go
+            mbar_arrive_warp(&sh.p_ready[part], lane);  // this group's slices of dK += dS^T Q may go
             stamp(a, tlc, it, 1, 5);
 
             // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns
@@ -744,7 +745,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 }
             }
             fence_proxy_async_smem();
-            mbar_arrive(&sh.ds_ready);
+            mbar_arrive_warp(&sh.ds_ready, lane);
             stamp(a, tlc, it, 1, 7);
         }
 
@@ -767,7 +768,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     make_float4(__uint_as_float(rs[4 * c]) * f, __uint_as_float(rs[4 * c + 1]) * f,
                                 __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
             fence_proxy_async_smem();
-            mbar_arrive(&sh.acc_staged);
+            mbar_arrive_warp(&sh.acc_staged, lane);
             HK_XSTAMP(tlx, 6);
         } else if (n_it == 0 && kv_ok && !a.accum_dkdv) {
             // no query sees this KV tile: its dK and dV rows are zero

@@ -170,7 +170,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // buffer is only refilled after every thread has handed over the P it held.
         for (int bf = 0; bf < 3; ++bf) {
             mbar_init(&sh.s_full[bf], 1);
-            mbar_init(&sh.p_full[bf], 128);
+            mbar_init(&sh.p_full[bf], 4);  // one arrival per warp of the tile
             mbar_init(&sh.o_full[bf], 1);
         }
         sh.abort_flag = 0;
@@ -226,73 +226,104 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // ------------------------------ MMA issuer ------------------------------
             // The whole warp runs this code with uniform control flow; only the tcgen05 instructions are predicated
             // on the elected lane (see umma_ss_tf32_lead).
+            //
+            // The tensor pipe takes instructions about as fast as it executes them and queues next to none, so every
+            // cycle this warp spends on something else than issuing leaves the pipe idle.  A wait costs some 150 cycles
+            // even when the barrier completed long ago; each barrier is therefore looked at (test_wait) while the MMAs
+            // before it are still being issued, and waited for only if that look came too early.
             if (n > 0) {
                 const uint32_t leader = elect_one_sync();
-                auto wait = [&](uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
+                auto wait = [&](bool seen, uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
+                    if (__all_sync(0xffffffffu, seen)) return true;
                     return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
                 };
                 const bool tlm = tl && leader;
                 constexpr uint32_t IDESC_S = make_idesc_tf32(TILE, TILE, false, false);
                 constexpr uint32_t IDESC_O = make_idesc_tf32(TILE, HEAD_DIM, false, true);
                 const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-                auto issue_qk = [&](int t, int s, int buf) {
-                    const uint32_t d = tmem + score_col(buf);
-#pragma unroll
-                    for (int kk = 0; kk < HEAD_DIM / 8; ++kk)
-                        umma_ss_tf32_lead(leader, d, kmajor_desc(q_addr + t * TILE_BYTES, kk, BOX_BYTES),
-                                     kmajor_desc(k_addr + s * TILE_BYTES, kk, BOX_BYTES), IDESC_S, kk > 0);
-                    umma_commit_lead(leader, &sh.s_full[buf]);
+                // products in issue order: step by step, tile 0 before tile 1 (a tile takes part while j < n_t)
+                struct Product {
+                    int j, t, buf;      // KV step, query tile, score buffer
+                    uint32_t par;       // parity of the score buffer's barriers
                 };
-                auto issue_pv = [&](int t, int s, int buf, bool first) {  // O_t += P V, P in score buffer buf
-                    const uint32_t p = tmem + score_col(buf);
+                const int total = n0 + n1;
+                auto advance = [&](Product& p) {
+                    if (p.t == 0 && p.j < n1) {
+                        p.t = 1;
+                    } else {
+                        ++p.j;
+                        p.t = (p.j < n0) ? 0 : 1;
+                    }
+                    if (++p.buf == 3) {
+                        p.buf = 0;
+                        p.par ^= 1u;
+                    }
+                };
+                auto issue_qk = [&](const Product& p, int kk0, int kk1) {
+                    const uint32_t d = tmem + score_col(p.buf);
+                    const int s = p.j % NST;
+#pragma unroll
+                    for (int kk = kk0; kk < kk1; ++kk)
+                        umma_ss_tf32_lead(leader, d, kmajor_desc(q_addr + p.t * TILE_BYTES, kk, BOX_BYTES),
+                                          kmajor_desc(k_addr + s * TILE_BYTES, kk, BOX_BYTES), IDESC_S, kk > 0);
+                };
+                auto commit_qk = [&](const Product& p) {
+                    umma_commit_lead(leader, &sh.s_full[p.buf]);
+                    if (p.t == 1 || p.j >= n1) umma_commit_lead(leader, &sh.k_empty[p.j % NST]);  // last one that reads it
+                };
+                auto issue_pv = [&](const Product& p) {  // O_t += P V, P in the product's score buffer
+                    const uint32_t pc = tmem + score_col(p.buf);
+                    const uint32_t acc0 = (p.j > 0 || a.continue_state) ? 1u : 0u;
 #pragma unroll
                     for (int kk = 0; kk < TILE / 8; ++kk)
-                        umma_ts_tf32_lead(leader, tmem + COL_O0 + t * HEAD_DIM, p + kk * 8,
-                                     mnmajor_desc(v_addr + s * TILE_BYTES, kk, BOX_BYTES), IDESC_O,
-                                     (!first || kk > 0) ? 1u : 0u);
-                    umma_commit_lead(leader, &sh.o_full[buf]);
+                        umma_ts_tf32_lead(leader, tmem + COL_O0 + p.t * HEAD_DIM, pc + kk * 8,
+                                          mnmajor_desc(v_addr + (p.j % NST) * TILE_BYTES, kk, BOX_BYTES), IDESC_O,
+                                          kk > 0 ? 1u : acc0);
+                    umma_commit_lead(leader, &sh.o_full[p.buf]);
+                    if (p.t == 1 || p.j >= n1) umma_commit_lead(leader, &sh.v_empty[p.j % NST]);
                 };
-                // products in issue order: step by step, tile 0 before tile 1 (a tile takes part while j < n_t)
-                const int total = n0 + n1;
-                auto advance = [&](int& j, int& t) {
-                    if (t == 0 && j < n1) {
-                        t = 1;
-                    } else {
-                        ++j;
-                        t = (j < n0) ? 0 : 1;
-                    }
-                };
-                int jq = 0, tq = (n0 > 0) ? 0 : 1, nq = 0;  // the next S = Q K^T to issue and its number
-                auto next_qk = [&]() -> bool {
-                    if (nq >= total) return true;
-                    const int s = jq % NST;
-                    if (tq == 0 || jq >= n0) {  // first product that reads this key tile
-                        if (!wait(&sh.k_full[s], (jq / NST) & 1, W_KFULL, jq)) return false;
-                        tc_fence_after_sync();
-                    }
-                    issue_qk(tq, s, nq % 3);
-                    if (tq == 1 || jq >= n1) umma_commit_lead(leader, &sh.k_empty[s]);  // last one that reads it
-                    ++nq;
-                    advance(jq, tq);
-                    return true;
-                };
-                bool ok = wait(&sh.q_full, 0, W_QFULL, 0);
-                for (int i = 0; ok && i < 3; ++i) ok = next_qk();
-                int j = 0, t = (n0 > 0) ? 0 : 1;
-                for (int q = 0; ok && q < total; ++q) {
-                    const int s = j % NST;
-                    stamp(a, tlm, j, 0, 3 * t);
-                    if (t == 0 || j >= n0) {
-                        if (!(ok = wait(&sh.v_full[s], (j / NST) & 1, W_VFULL, j))) break;
-                    }
-                    if (!(ok = wait(&sh.p_full[q % 3], (q / 3) & 1, W_PFULL, j))) break;
-                    stamp(a, tlm, j, 0, 1 + 3 * t);
+                auto new_k = [&](const Product& p) { return p.t == 0 || p.j >= n0; };  // first product to read its K / V tile
+                auto k_bar = [&](const Product& p) { return &sh.k_full[p.j % NST]; };
+                auto v_bar = [&](const Product& p) { return &sh.v_full[p.j % NST]; };
+                auto kv_par = [&](const Product& p) { return (uint32_t)(p.j / NST) & 1u; };
+                Product pq{0, (n0 > 0) ? 0 : 1, 0, 0u};  // the next S = Q K^T to issue
+                Product pv = pq;                         // the next P V to issue
+                int nq = 0;
+                bool ok = wait(false, &sh.q_full, 0, W_QFULL, 0);
+                for (; ok && nq < 3 && nq < total; ++nq) {
+                    if (new_k(pq) && !(ok = wait(false, k_bar(pq), kv_par(pq), W_KFULL, pq.j))) break;
                     tc_fence_after_sync();
-                    issue_pv(t, s, q % 3, j == 0 && !a.continue_state);
-                    if (t == 1 || j >= n1) umma_commit_lead(leader, &sh.v_empty[s]);
-                    ok = next_qk();
-                    stamp(a, tlm, j, 0, 2 + 3 * t);
-                    advance(j, t);
+                    issue_qk(pq, 0, HEAD_DIM / 8);
+                    commit_qk(pq);
+                    advance(pq);
+                }
+                bool seen_p = false, seen_v = false;
+                for (int q = 0; ok && q < total; ++q) {
+                    stamp(a, tlm, pv.j, 0, 3 * pv.t);
+                    if (new_k(pv) && !(ok = wait(seen_v, v_bar(pv), kv_par(pv), W_VFULL, pv.j))) break;
+                    if (!(ok = wait(seen_p, &sh.p_full[pv.buf], pv.par, W_PFULL, pv.j))) break;
+                    stamp(a, tlm, pv.j, 0, 1 + 3 * pv.t);
+                    tc_fence_after_sync();
+                    const bool more = nq < total;
+                    const bool seen_k = mbar_test_wait(k_bar(pq), kv_par(pq));
+                    Product nx = pv;
+                    issue_pv(pv);
+                    advance(nx);
+                    if (more) {
+                        if (new_k(pq) && !(ok = wait(seen_k, k_bar(pq), kv_par(pq), W_KFULL, pq.j))) break;
+                        tc_fence_after_sync();
+                        issue_qk(pq, 0, 6);
+                    }
+                    seen_v = mbar_test_wait(v_bar(nx), kv_par(nx));
+                    seen_p = mbar_test_wait(&sh.p_full[nx.buf], nx.par);
+                    if (more) {
+                        issue_qk(pq, 6, HEAD_DIM / 8);
+                        commit_qk(pq);
+                        ++nq;
+                        advance(pq);
+                    }
+                    stamp(a, tlm, pv.j, 0, 2 + 3 * pv.t);
+                    pv = nx;
                 }
             }
         }
@@ -475,7 +506,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             stamp(a, tls, j, 1 + t, 3);
             tmem_wait_st();
             tc_fence_before_sync();
-            mbar_arrive(&sh.p_full[q % 3]);
+            mbar_arrive_warp(&sh.p_full[q % 3], lane);
             q_prev = q;
             stamp(a, tls, j, 1 + t, 4);
         }
