@@ -8,32 +8,39 @@
 // O = alpha*O + P V with P rounded to TF32, finally O /= l (0 if l == 0) and
 // LSE = m + log l (-inf if l == 0).
 //
-// Blackwell structure: one CTA per 256 query rows = two 128-row tiles that take
-// turns on the tensor pipe, so that the softmax of one tile runs while the
-// MMAs of the other execute.
-//   warp 0        TMA producer: both Q tiles once, then K and V tiles through a
-//                 two-stage ring (128-byte-swizzled boxes of 128 rows x 32
-//                 floats, mbarrier tx; V with the 32-byte-chunk swizzle an
-//                 MN-major TF32 operand needs).
+// Blackwell structure: a CTA runs two streams of "products", 128 query rows against 128 keys each, which take turns on
+// the tensor pipe, so that the softmax of one runs while the MMAs of the other execute.  The streams are
+//   rows mode     two adjacent blocks of 128 query rows against the same key tiles (256 rows per CTA),
+//   row mode      one block of 128 rows, the second stream idle, or
+//   keys mode     the even and the odd key tiles of one block of 128 rows, merged at the end.
+// The last two have twice the CTAs, each shorter, and twice the loads: for problems whose row blocks are few.
+//   warp 0        TMA producer: Q once, then K and V tiles through one ring of five slots in the order the products
+//                 use them up, K0 K1 V0 K2 V1 ... (128-byte-swizzled boxes of 128 rows x 32 floats, mbarrier tx; V
+//                 with the 32-byte-chunk swizzle an MN-major TF32 operand needs).  Two stages of K and V each,
+//                 the previous layout, waited for the copy of the tile they had just released (9 % at 8 192 keys).
 //   warp 1        MMA issuer (the whole warp runs the issuing code, one elected lane issues).
-//                 S_t = Q_t K^T is 8 tcgen05.mma (M128 N128 K8, operands from
-//                 shared memory), O_t += P_t V is 16 (M128 N64 K8, A = P_t read
-//                 from tensor memory, B = V MN-major from shared memory).  The
-//                 (step, tile) products are numbered in the order (0,0) (0,1) (1,0)
-//                 (1,1) ...; product q keeps its S, then its P, in score buffer
-//                 q mod 3, and the issue order is S(0) S(1) S(2) | P V(0) S(3) |
-//                 P V(1) S(4) | ...: the scores of a tile's NEXT step are computed
-//                 while its softmax works on the current one (the tensor pipe
-//                 executes in issue order, so S(q+3) cannot overtake the P V(q)
-//                 that reads the same buffer).
-//   warps 4-7     softmax of tile 0, warps 8-11 softmax of tile 1: thread r owns
-//                 query row r (tensor-memory lane r), holds the 128 scores of a
-//                 step in registers (one tensor-memory read per score), writes P
-//                 back over S.  The running output is rescaled only when the
-//                 running maximum grew by more than 2^8 (the final O/l and LSE
-//                 use the same maximum, so the result is the same function).
+//                 S = Q K^T is 8 tcgen05.mma (M128 N128 K8, operands from shared memory), O_t += P V is 16
+//                 (M128 N64 K8, A = P from tensor memory, B = V MN-major from shared memory).  Product q keeps
+//                 its S, then its P, in score buffer q mod 3, and the issue order is S(0) S(1) S(2) | P V(0) S(3) |
+//                 P V(1) S(4) | ...: the scores of a stream's NEXT step are computed while its softmax works on the
+//                 current one (the tensor pipe executes in issue order, so S(q+3) cannot overtake the P V(q) that
+//                 reads the same buffer).
+//   warps 4-7     softmax of stream 0, warps 8-11 softmax of stream 1: thread r owns query row r (tensor-memory lane
+//                 r), holds the 128 scores of a step in registers (one tensor-memory read per score) and writes P back
+//                 over S.  (Two threads per row, sixteen warps: the exchange of the row maximum alone takes 300 cycles
+//                 of a step.)  The running output is rescaled only when the running maximum grew by more than 2^8 (the
+//                 final O/l and LSE use the same maximum, so the result is the same function).
 // Tensor memory: three score buffers (128 columns each), O_0, O_1 (64 columns each): 512 of 512 columns.
 // Warps 0-3 give most of their registers to the softmax warps (setmaxnreg 56 / 224).
+//
+// Key splits: a cluster of NS CTAs shares one block of query rows; split s takes a contiguous run of its key tiles, and at
+// the end every CTA combines a slice of the rows from the partial (O, m, l) the others left in their shared memory (keys
+// mode merges its two streams with the same code).  The host picks mode and splits (launch_attn_fwd).
+// CTA pairs (cta_group::2, half of every K and V tile per CTA) were built and measured: the MMAs and copies alone run at
+// 2 360 instead of 3 100 cycles per step, the whole kernel 4 % faster at H32 T8192, but every CTA spends ~4 000 cycles
+// more on set-up and hand-over between the two, 57 against 45 us at B8 H12 T1024.
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "attn_kernels.cuh"
@@ -43,134 +50,141 @@ namespace hk {
 
 namespace fwd {
 
-constexpr int NUM_THREADS = 384;
+constexpr int NUM_SOFTMAX = 256;
+constexpr int NUM_THREADS = 128 + NUM_SOFTMAX;
 constexpr int TMEM_COLS = 512;
 constexpr int COL_O0 = 256;  // O_t at COL_O0 + 64 t
 // score buffer b of three: columns 0, 128, 384
 __device__ __forceinline__ uint32_t score_col(int b) { return b == 2 ? 384u : (uint32_t)b * 128u; }
-constexpr int NST = 2;       // K/V ring depth
-constexpr float RESCALE_THRESHOLD = 8.f;  // log2 units
+constexpr int SLOTS = 5;                    // K / V ring
+constexpr float RESCALE_THRESHOLD = 8.f;    // log2 units
 
-struct __align__(8) Shared {
-    uint64_t q_full, k_full[NST], k_empty[NST], v_full[NST], v_empty[NST], s_full[3], p_full[3], o_full[3];
+struct __align__(16) Shared {
+    float m[2][TILE], l[2][TILE];  // [stream]: row maxima and sums for the combination
+    uint64_t q_full[2], kv_full[SLOTS], kv_empty[SLOTS], s_full[3], p_full[3], o_full[3];
     uint32_t tmem_base;
     int abort_flag;
 };
 
 constexpr int OFF_Q = 0;                          // two tiles
-constexpr int OFF_K = 2 * TILE_BYTES;             // NST stages
-constexpr int OFF_V = OFF_K + NST * TILE_BYTES;   // NST stages
-constexpr int OFF_SH = OFF_V + NST * TILE_BYTES;
+constexpr int OFF_KV = 2 * TILE_BYTES;            // ring
+constexpr int OFF_SH = OFF_KV + SLOTS * TILE_BYTES;
 constexpr int SMEM_BYTES = OFF_SH + sizeof(Shared);
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may opt in to");
 
-enum WaitId { W_QFULL = 101, W_KFULL, W_KEMPTY, W_VFULL, W_VEMPTY, W_SFULL, W_PFULL, W_OFULL };
-
-// Timeline slots (SM clock): role 0 = MMA issuer, 1 = softmax thread 0 of tile 0, 2 = of tile 1;
-// buffer[1 + (j * 3 + role) * 8 + ph]; buffer[0] = number of KV steps of the recorded CTA.
-#ifdef HK_TIMELINE
-__device__ __forceinline__ void stamp(const FwdArgs& a, bool on, int j, int role, int ph) {
-    if (on && j < 150) a.timeline[1 + (j * 3 + role) * 8 + ph] = clock64();
-}
-#else
-__device__ __forceinline__ void stamp(const FwdArgs&, bool, int, int, int) {}
-#endif
+enum WaitId { W_QFULL = 101, W_KFULL, W_KVEMPTY, W_VFULL, W_SFULL, W_PFULL, W_OFULL };
 
 // 384 threads x 168 registers at launch = 128 x 56 + 256 x 224 after the hand-over (setmaxnreg.inc can only take what
 // the launch-time pool of the CTA holds)
-static_assert(128 * 56 + 256 * 224 <= NUM_THREADS * 168, "register hand-over exceeds the CTA's pool");
+static_assert(128 * 56 + NUM_SOFTMAX * 224 <= NUM_THREADS * 168, "register hand-over exceeds the CTA's pool");
 __device__ __forceinline__ void reg_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n"); }
 __device__ __forceinline__ void reg_acquire() { asm volatile("setmaxnreg.inc.sync.aligned.u32 224;\n"); }
 
-// number of key tiles the 128-row query tile starting at local row q0 attends to
-__device__ __forceinline__ int kv_tiles_for(const FwdArgs& a, int q0) {
-    if (q0 >= a.Tq) return 0;
-    int kv_end = a.Tk;
-    if (a.causal) {
-        const int last_row = min(q0 + TILE, a.Tq) - 1;
-        const long long lim = (long long)a.q_pos0 + last_row - a.k_pos0 + 1;
-        kv_end = (int)max(0ll, min((long long)a.Tk, lim));
+// Ring sequence: K0 K1 V0 K2 V1 K3 V2 ...: K(0) is entry 0, K(j) entry 2 j - 1, V(j) entry 2 j + 2 (so the entry before the
+// last V is skipped).
+struct RingPos {
+    uint32_t slot, phase;
+    __device__ __forceinline__ void advance(uint32_t by) {
+        slot += by;
+        if (slot >= SLOTS) {
+            slot -= SLOTS;
+            phase ^= 1u;
+        }
     }
-    return (kv_end + TILE - 1) / TILE;
+};
+
+// number of key tiles the query rows q0 .. q0 + TILE - 1 attend to
+__host__ __device__ inline int kv_tiles_for(int q0, int Tq, int Tk, int causal, int q_pos0, int k_pos0) {
+    if (q0 >= Tq) return 0;
+    long long kv_end = Tk;
+    if (causal) {
+        const int last_row = (q0 + TILE < Tq ? q0 + TILE : Tq) - 1;
+        const long long lim = (long long)q_pos0 + last_row - k_pos0 + 1;
+        kv_end = lim < 0 ? 0 : lim < kv_end ? lim : kv_end;
+    }
+    return (int)((kv_end + TILE - 1) / TILE);
 }
 
 }  // namespace fwd
 
+template <int DROP>  // 0 none, 1 dense mask, 2 Philox
 __global__ void __launch_bounds__(fwd::NUM_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const FwdArgs a) {
     using namespace fwd;
     extern __shared__ __align__(1024) uint8_t smem[];
-    // schedule trace (timeline_block < 0): {start ns, end ns, SM id, key tiles} of each of the first 1024 CTAs
-#ifdef HK_TIMELINE
-    const bool trace = a.timeline != nullptr && a.timeline_block < 0 && blockIdx.x < 1024 && threadIdx.x == 0;
-#else
-    constexpr bool trace = false;
-#endif
-    if (trace) {
-        a.timeline[4 * blockIdx.x] = (long long)globaltimer_ns();
-        a.timeline[4 * blockIdx.x + 2] = smid();
-    }
-    if ((smem_u32(smem) & 1023u) != 0) {  // never expected; refuse to run on a misplaced buffer
-        if (threadIdx.x == 0 && atomicCAS(&a.status->code, 0, 199) == 0) a.status->block = blockIdx.x;
-        return;
-    }
     uint8_t* sQ = smem + OFF_Q;
-    uint8_t* sK = smem + OFF_K;
-    uint8_t* sV = smem + OFF_V;
+    uint8_t* sKV = smem + OFF_KV;
     Shared& sh = *reinterpret_cast<Shared*>(smem + OFF_SH);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = (int)uniform(threadIdx.x >> 5);  // uniform for the compiler too: the issuing warp depends on it
     const int lane = threadIdx.x & 31;
+    const int ns = a.n_splits;  // cluster size
+    const int split = ns > 1 ? (int)cluster_ctarank() : 0;
 
     // heavy (late) query blocks first: under the causal mask they have the most key tiles
-    const int bh = blockIdx.x % a.BH;
-    const int qb = a.n_qtiles - 1 - (int)(blockIdx.x / a.BH);  // n_qtiles counts 256-row blocks here
+    const int work = blockIdx.x / ns;
+    const int bh = work % a.BH;
+    const int qb = a.n_qblocks - 1 - work / a.BH;
     const int b = bh / a.H;
     const int h = bh - b * a.H;
-    const int q0 = qb * 2 * TILE;
-    const int n0 = kv_tiles_for(a, q0);
-    const int n1 = kv_tiles_for(a, q0 + TILE);
-    const int n = max(n0, n1);
+    // rows mode: stream t = query rows q0 + 128 t ..; keys mode: both streams = rows q0 .., stream t = key tiles 2 j + t.
+    // q_end: end of the block's rows
+    // jb: this split's first key tile; n_t: steps of stream t; nk: key tiles this split loads, jb + 0 .. jb + nk - 1, one
+    // per step (rows) or per product (keys)
+    const bool keys = a.mode == FWD_KEYS;
+    const int block_rows = a.mode == FWD_ROWS ? 2 * TILE : TILE;
+    const int q0 = qb * block_rows, q_end = min(a.Tq, q0 + block_rows);
+    const int all0 = kv_tiles_for(q0, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+    const int all1 = keys ? all0 : a.mode == FWD_ROW ? 0 : kv_tiles_for(q0 + TILE, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+    const int all = max(all0, all1);
+    const int per = (all + ns - 1) / ns;  // split 0 is never empty while any key is seen
+    const int jb = min(all, split * per), je = min(all, jb + per);
+    const int nk = je - jb;
+    const int n0 = keys ? (nk + 1) / 2 : max(0, min(je, all0) - jb);
+    const int n1 = keys ? nk / 2 : max(0, min(je, all1) - jb);
 
-    // The producer initialises the barriers its copies complete on and issues the first loads at once (Q, and the
-    // first NST key/value tiles, which wait for no consumer): the rest of the set-up -- the other barriers, the
-    // tensor-memory allocation -- runs under their latency.  The other warps meet these barriers only after the
-    // __syncthreads below.
+    auto row0_of = [&](int t) { return q0 + (keys ? 0 : t * TILE); };  // first row of stream t
+    auto load_q = [&](int t) {
+        mbar_arrive_expect_tx(&sh.q_full[t], TILE_BYTES);
+        tma_load_4d(sQ + t * TILE_BYTES, &mapQ, &sh.q_full[t], 0, row0_of(t), h, b);
+        tma_load_4d(sQ + t * TILE_BYTES + BOX_BYTES, &mapQ, &sh.q_full[t], HALF_D, row0_of(t), h, b);
+    };
+    auto load_kv = [&](int i) {  // entry i of the ring sequence
+        const bool v = i > 0 && (i & 1) == 0;
+        const int tile = v ? (i - 2) / 2 : (i + 1) / 2;
+        const CUtensorMap* map = v ? &mapV : &mapK;
+        const int s = i % SLOTS;
+        mbar_arrive_expect_tx(&sh.kv_full[s], TILE_BYTES);
+        tma_load_4d(sKV + s * TILE_BYTES, map, &sh.kv_full[s], 0, (jb + tile) * TILE, h, b);
+        tma_load_4d(sKV + s * TILE_BYTES + BOX_BYTES, map, &sh.kv_full[s], HALF_D, (jb + tile) * TILE, h, b);
+    };
+    auto in_ring = [&](int i) { return i < 2 * nk - 1 || i == 2 * nk; };
+
+    // The producer initialises the barriers its copies complete on and issues the first loads at once (they wait for no
+    // consumer): the rest of the set-up -- the other barriers, the tensor-memory allocation -- runs under their latency.
+    // The other warps meet these barriers only after the __syncthreads below.
     if (warp == 0 && lane == 0) {
-        mbar_init(&sh.q_full, 1);
-        for (int s = 0; s < NST; ++s) {
-            mbar_init(&sh.k_full[s], 1);
-            mbar_init(&sh.v_full[s], 1);
-        }
+        for (int i = 0; i < 2; ++i) mbar_init(&sh.q_full[i], 1);
+        for (int s = 0; s < SLOTS; ++s) mbar_init(&sh.kv_full[s], 1);
         fence_mbar_init();
-        if (n > 0) {
-            mbar_arrive_expect_tx(&sh.q_full, 2 * TILE_BYTES);
-            for (int t = 0; t < 2; ++t) {
-                tma_load_4d(sQ + t * TILE_BYTES, &mapQ, &sh.q_full, 0, q0 + t * TILE, h, b);
-                tma_load_4d(sQ + t * TILE_BYTES + BOX_BYTES, &mapQ, &sh.q_full, HALF_D, q0 + t * TILE, h, b);
-            }
-            for (int j = 0; j < n && j < NST; ++j) {
-                mbar_arrive_expect_tx(&sh.k_full[j], TILE_BYTES);
-                tma_load_4d(sK + j * TILE_BYTES, &mapK, &sh.k_full[j], 0, j * TILE, h, b);
-                tma_load_4d(sK + j * TILE_BYTES + BOX_BYTES, &mapK, &sh.k_full[j], HALF_D, j * TILE, h, b);
-                mbar_arrive_expect_tx(&sh.v_full[j], TILE_BYTES);
-                tma_load_4d(sV + j * TILE_BYTES, &mapV, &sh.v_full[j], 0, j * TILE, h, b);
-                tma_load_4d(sV + j * TILE_BYTES + BOX_BYTES, &mapV, &sh.v_full[j], HALF_D, j * TILE, h, b);
-            }
+        if (nk > 0) {
+            if (n0 > 0) load_q(0);
+            load_kv(0);
+            if (n1 > 0 && !keys) load_q(1);
+#pragma unroll 1
+            for (int i = 1; i < SLOTS; ++i)
+                if (in_ring(i)) load_kv(i);
         }
     }
     if (threadIdx.x == 64) {  // an idle warp takes the rest of the barriers
-        for (int s = 0; s < NST; ++s) {
-            mbar_init(&sh.k_empty[s], 1);
-            mbar_init(&sh.v_empty[s], 1);
-        }
-        // The score barriers belong to the score BUFFER, not to the tile: the warps of a tile may be a whole step
+        for (int s = 0; s < SLOTS; ++s) mbar_init(&sh.kv_empty[s], 1);
+        // The score barriers belong to the score BUFFER, not to the stream: the warps of a stream may be a whole step
         // apart (the scores of the next step are there before the slowest warp has finished this one), and a
-        // buffer is only refilled after every thread has handed over the P it held.
+        // buffer is only refilled after every warp has handed over the P it held.
         for (int bf = 0; bf < 3; ++bf) {
             mbar_init(&sh.s_full[bf], 1);
-            mbar_init(&sh.p_full[bf], 4);  // one arrival per warp of the tile
+            mbar_init(&sh.p_full[bf], 4);  // one arrival per softmax warp of the stream
             mbar_init(&sh.o_full[bf], 1);
         }
         sh.abort_flag = 0;
@@ -183,44 +197,36 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = sh.tmem_base;
+    const uint32_t tmem = uniform(sh.tmem_base);
     WaitCtx wc{&sh.abort_flag, a.status};
-#ifdef HK_TIMELINE
-    const bool tl = a.timeline != nullptr && (int)blockIdx.x == a.timeline_block;
-#else
-    constexpr bool tl = false;
-#endif
-    if (tl && threadIdx.x == 0) a.timeline[0] = n;
+    // all threads of the cluster (of the CTA, when it is alone)
+    auto barrier_all = [&] {
+        if (ns > 1) {
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+    };
+    const bool combine = ns > 1 || keys;  // the results of several streams or splits are merged at the end
 
     if (warp < 4) {
         reg_release();
         if (warp == 0) {
             // ------------------------------ TMA producer ------------------------------
-            if (lane == 0 && n > 0) {
-                // Q and the first NST key/value tiles were issued before the set-up barrier
-                int issued = min(n, NST);
-                for (int j = NST; j < n; ++j) {
-                    const int s = j % NST;
-                    const uint32_t par = ((j / NST) - 1) & 1;
-                    if (j >= NST && !mbar_wait(wc, &sh.k_empty[s], par, W_KEMPTY, j)) break;
-                    mbar_arrive_expect_tx(&sh.k_full[s], TILE_BYTES);
-                    tma_load_4d(sK + s * TILE_BYTES, &mapK, &sh.k_full[s], 0, j * TILE, h, b);
-                    tma_load_4d(sK + s * TILE_BYTES + BOX_BYTES, &mapK, &sh.k_full[s], HALF_D, j * TILE, h, b);
-                    if (j >= NST && !mbar_wait(wc, &sh.v_empty[s], par, W_VEMPTY, j)) {
-                        for (int i = 0; i < 100000 && !mbar_try_wait(&sh.k_full[s], (j / NST) & 1); ++i) {}
-                        break;
-                    }
-                    mbar_arrive_expect_tx(&sh.v_full[s], TILE_BYTES);
-                    tma_load_4d(sV + s * TILE_BYTES, &mapV, &sh.v_full[s], 0, j * TILE, h, b);
-                    tma_load_4d(sV + s * TILE_BYTES + BOX_BYTES, &mapV, &sh.v_full[s], HALF_D, j * TILE, h, b);
-                    issued = j + 1;
+            if (lane == 0) {
+                bool tok = true;
+                for (int i = SLOTS; tok && i <= 2 * nk; ++i) {
+                    if (!in_ring(i)) continue;
+                    if (!(tok = mbar_wait(wc, &sh.kv_empty[i % SLOTS], (i / SLOTS - 1) & 1, W_KVEMPTY, i))) break;
+                    load_kv(i);
                 }
-                // Do not leave the CTA while bulk copies into its shared memory are in flight.
-                for (int i = 0; i < 100000 && !mbar_try_wait(&sh.q_full, 0); ++i) {}
-                for (int j = max(0, issued - NST); j < issued; ++j) {
-                    for (int i = 0; i < 100000 && !mbar_try_wait(&sh.k_full[j % NST], (j / NST) & 1); ++i) {}
-                    for (int i = 0; i < 100000 && !mbar_try_wait(&sh.v_full[j % NST], (j / NST) & 1); ++i) {}
-                }
+                // Every copy has landed once the softmax warps have seen the last product complete (they wait for it, and
+                // the barrier below waits for them).  Only a CTA that gave up may have some in flight still: give them
+                // time to land before it leaves.
+                if (!tok)
+                    for (const unsigned long long t0 = globaltimer_ns(); globaltimer_ns() - t0 < 100000ull;) {}
             }
         } else if (warp == 1) {
             // ------------------------------ MMA issuer ------------------------------
@@ -231,139 +237,136 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // cycle this warp spends on something else than issuing leaves the pipe idle.  A wait costs some 150 cycles
             // even when the barrier completed long ago; each barrier is therefore looked at (test_wait) while the MMAs
             // before it are still being issued, and waited for only if that look came too early.
-            if (n > 0) {
+            if (nk > 0) {
                 const uint32_t leader = elect_one_sync();
                 auto wait = [&](bool seen, uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
                     if (__all_sync(0xffffffffu, seen)) return true;
                     return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
                 };
-                const bool tlm = tl && leader;
                 constexpr uint32_t IDESC_S = make_idesc_tf32(TILE, TILE, false, false);
                 constexpr uint32_t IDESC_O = make_idesc_tf32(TILE, HEAD_DIM, false, true);
-                const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-                // products in issue order: step by step, tile 0 before tile 1 (a tile takes part while j < n_t)
+                // products in issue order: step by step, stream 0 before stream 1 (a stream takes part while j < n_t)
                 struct Product {
-                    int j, t, buf;      // KV step, query tile, score buffer
-                    uint32_t par;       // parity of the score buffer's barriers
+                    int j, t, buf;   // step, stream, score buffer
+                    uint32_t par;    // parity of the score buffer's barriers
+                    RingPos k, v;    // its key and value tile
+                    bool first;      // key tile 0
                 };
                 const int total = n0 + n1;
                 auto advance = [&](Product& p) {
-                    if (p.t == 0 && p.j < n1) {
-                        p.t = 1;
-                    } else {
-                        ++p.j;
-                        p.t = (p.j < n0) ? 0 : 1;
+                    const bool next_step = p.t == 1 || p.j >= n1;
+                    if (next_step) ++p.j;
+                    p.t = (next_step && p.j < n0) ? 0 : 1;
+                    if (next_step || keys) {
+                        p.k.advance(p.first ? 1 : 2);
+                        p.v.advance(2);
+                        p.first = false;
                     }
                     if (++p.buf == 3) {
                         p.buf = 0;
                         p.par ^= 1u;
                     }
                 };
-                auto issue_qk = [&](const Product& p, int kk0, int kk1) {
-                    const uint32_t d = tmem + score_col(p.buf);
-                    const int s = p.j % NST;
-#pragma unroll
-                    for (int kk = kk0; kk < kk1; ++kk)
-                        umma_ss_tf32_lead(leader, d, kmajor_desc(q_addr + p.t * TILE_BYTES, kk, BOX_BYTES),
-                                          kmajor_desc(k_addr + s * TILE_BYTES, kk, BOX_BYTES), IDESC_S, kk > 0);
+                // first and last product that reads its K / V tile
+                auto new_kv = [&](const Product& p) { return keys || p.t == 0 || p.j >= n0; };
+                auto last_kv = [&](const Product& p) { return keys || p.t == 1 || p.j >= n1; };
+                const Desc q_desc = kmajor_desc(smem_u32(sQ), 0, BOX_BYTES), k_desc = kmajor_desc(smem_u32(sKV), 0, BOX_BYTES),
+                           v_desc = mnmajor_desc(smem_u32(sKV), 0, BOX_BYTES);
+                auto issue_qk = [&](const Product& p, int box) {  // 32 of the 64 d's
+                    umma_ss4<KMAJOR_STEP, KMAJOR_STEP>(leader, tmem + score_col(p.buf),
+                                                       q_desc + ((keys ? 0 : p.t * TILE_BYTES) + box * BOX_BYTES),
+                                                       k_desc + (p.k.slot * TILE_BYTES + box * BOX_BYTES), IDESC_S, box);
                 };
                 auto commit_qk = [&](const Product& p) {
                     umma_commit_lead(leader, &sh.s_full[p.buf]);
-                    if (p.t == 1 || p.j >= n1) umma_commit_lead(leader, &sh.k_empty[p.j % NST]);  // last one that reads it
+                    if (last_kv(p)) umma_commit_lead(leader, &sh.kv_empty[p.k.slot]);
                 };
-                auto issue_pv = [&](const Product& p) {  // O_t += P V, P in the product's score buffer
-                    const uint32_t pc = tmem + score_col(p.buf);
-                    const uint32_t acc0 = (p.j > 0 || a.continue_state) ? 1u : 0u;
+                auto issue_pv = [&](const Product& p, bool acc_first) {  // O_t += P V, P in the product's score buffer
+                    const uint32_t pc = tmem + score_col(p.buf), d = tmem + COL_O0 + p.t * HEAD_DIM;
+                    const Desc vd = v_desc + p.v.slot * TILE_BYTES;
+                    umma_ts4<MNMAJOR_STEP>(leader, d, pc, vd, IDESC_O, (p.j > 0 || (acc_first && !(keys && p.t == 1))) ? 1u : 0u);
 #pragma unroll
-                    for (int kk = 0; kk < TILE / 8; ++kk)
-                        umma_ts_tf32_lead(leader, tmem + COL_O0 + p.t * HEAD_DIM, pc + kk * 8,
-                                          mnmajor_desc(v_addr + (p.j % NST) * TILE_BYTES, kk, BOX_BYTES), IDESC_O,
-                                          kk > 0 ? 1u : acc0);
+                    for (int g = 1; g < 4; ++g) umma_ts4<MNMAJOR_STEP>(leader, d, pc + 32 * g, vd + 4096 * g, IDESC_O, 1u);
                     umma_commit_lead(leader, &sh.o_full[p.buf]);
-                    if (p.t == 1 || p.j >= n1) umma_commit_lead(leader, &sh.v_empty[p.j % NST]);
+                    if (last_kv(p)) umma_commit_lead(leader, &sh.kv_empty[p.v.slot]);
                 };
-                auto new_k = [&](const Product& p) { return p.t == 0 || p.j >= n0; };  // first product to read its K / V tile
-                auto k_bar = [&](const Product& p) { return &sh.k_full[p.j % NST]; };
-                auto v_bar = [&](const Product& p) { return &sh.v_full[p.j % NST]; };
-                auto kv_par = [&](const Product& p) { return (uint32_t)(p.j / NST) & 1u; };
-                Product pq{0, (n0 > 0) ? 0 : 1, 0, 0u};  // the next S = Q K^T to issue
-                Product pv = pq;                         // the next P V to issue
+                const bool state_in = a.continue_state && split == 0;
+                Product pq{0, (n0 > 0) ? 0 : 1, 0, 0u, {0u, 0u}, {2u, 0u}, true};  // the next S = Q K^T to issue
+                Product pv = pq;                                                   // the next P V to issue
                 int nq = 0;
-                bool ok = wait(false, &sh.q_full, 0, W_QFULL, 0);
+                bool ok = true;
                 for (; ok && nq < 3 && nq < total; ++nq) {
-                    if (new_k(pq) && !(ok = wait(false, k_bar(pq), kv_par(pq), W_KFULL, pq.j))) break;
+                    if (pq.j == 0 && !(ok = wait(false, &sh.q_full[keys ? 0 : pq.t], 0, W_QFULL, pq.t))) break;
+                    if (new_kv(pq) && !(ok = wait(false, &sh.kv_full[pq.k.slot], pq.k.phase, W_KFULL, pq.j))) break;
                     tc_fence_after_sync();
-                    issue_qk(pq, 0, HEAD_DIM / 8);
+                    issue_qk(pq, 0);
+                    issue_qk(pq, 1);
                     commit_qk(pq);
                     advance(pq);
                 }
                 bool seen_p = false, seen_v = false;
                 for (int q = 0; ok && q < total; ++q) {
-                    stamp(a, tlm, pv.j, 0, 3 * pv.t);
-                    if (new_k(pv) && !(ok = wait(seen_v, v_bar(pv), kv_par(pv), W_VFULL, pv.j))) break;
+                    if (new_kv(pv) && !(ok = wait(seen_v, &sh.kv_full[pv.v.slot], pv.v.phase, W_VFULL, pv.j))) break;
                     if (!(ok = wait(seen_p, &sh.p_full[pv.buf], pv.par, W_PFULL, pv.j))) break;
-                    stamp(a, tlm, pv.j, 0, 1 + 3 * pv.t);
                     tc_fence_after_sync();
                     const bool more = nq < total;
-                    const bool seen_k = mbar_test_wait(k_bar(pq), kv_par(pq));
-                    Product nx = pv;
-                    issue_pv(pv);
-                    advance(nx);
+                    const bool seen_k = mbar_test_wait(&sh.kv_full[pq.k.slot], pq.k.phase);
+                    issue_pv(pv, state_in);
+                    advance(pv);
                     if (more) {
-                        if (new_k(pq) && !(ok = wait(seen_k, k_bar(pq), kv_par(pq), W_KFULL, pq.j))) break;
+                        if (new_kv(pq) && !(ok = wait(seen_k, &sh.kv_full[pq.k.slot], pq.k.phase, W_KFULL, pq.j))) break;
                         tc_fence_after_sync();
-                        issue_qk(pq, 0, 6);
+                        issue_qk(pq, 0);
                     }
-                    seen_v = mbar_test_wait(v_bar(nx), kv_par(nx));
-                    seen_p = mbar_test_wait(&sh.p_full[nx.buf], nx.par);
+                    seen_v = mbar_test_wait(&sh.kv_full[pv.v.slot], pv.v.phase);
+                    seen_p = mbar_test_wait(&sh.p_full[pv.buf], pv.par);
                     if (more) {
-                        issue_qk(pq, 6, HEAD_DIM / 8);
+                        issue_qk(pq, 1);
                         commit_qk(pq);
                         ++nq;
                         advance(pq);
                     }
-                    stamp(a, tlm, pv.j, 0, 2 + 3 * pv.t);
-                    pv = nx;
                 }
             }
         }
         // teardown of the control warps (kept inside this branch: the two register regimes never
         // share code after the hand-over)
+        if (combine) barrier_all();  // partial results staged
         tc_fence_before_sync();
-        __syncthreads();
+        barrier_all();
         if (warp == 1) {
-            __syncwarp();
             tc_fence_after_sync();
             tmem_dealloc(tmem, TMEM_COLS);
         }
     } else {
         // ------------------------------ softmax ------------------------------
         reg_acquire();
-        const int t = (warp - 4) >> 2;                   // which of the two query tiles
+        const int t = (warp - 4) >> 2;                   // stream
         const int quarter = warp & 3;
-        const int row = quarter * 32 + lane;             // row inside the query tile = tensor-memory lane
-        const int qrow = q0 + t * TILE + row;            // row inside this (b,h)
-        const bool row_ok = qrow < a.Tq;
+        const int row = quarter * 32 + lane;             // row inside the product = tensor-memory lane
+        const int qrow = row0_of(t) + row;               // row inside this (b,h)
+        const bool row_ok = qrow < q_end;
+        const bool warp_live = row0_of(t) + quarter * 32 < q_end;  // any row of this warp exists
         const int nt = t == 0 ? n0 : n1;
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
         const uint32_t tO = trow + COL_O0 + t * HEAD_DIM;
-        const bool tls = tl && row == 0;
         // last key index (local to this call's K) this row may see
         long long lim_ll = a.Tk - 1;
         if (a.causal) lim_ll = min(lim_ll, (long long)a.q_pos0 + qrow - a.k_pos0);
         const int kv_lim = row_ok ? (int)max(-1ll, lim_ll) : -1;
-        const float c = a.scale_log2e;
-        const float worst = (c >= 0.f) ? -INFINITY : INFINITY;  // raw score that can never win the max
-
+        const float cs = a.scale_log2e;
+        const float worst = (cs >= 0.f) ? -INFINITY : INFINITY;  // raw score that can never win the max
         const bool scaled = a.drop_scaled != 0;
+        const bool state_in = a.continue_state && split == 0 && !(keys && t == 1);
+
         float m = -INFINITY;  // running max actually used as exponent reference, log2 units
         float l = 0.f;
         bool ok = true;
         uint32_t r[128];
-        if (a.continue_state && nt > 0) {
+        if (state_in && nt > 0) {
             // The result over the keys seen so far is the starting state: reference LSE, normaliser 1 and the running
             // output O itself (a row that has seen no key starts from nothing).  The output accumulator is written
-            // before this thread's first arrival on p_full, which the first P V of the tile waits for.
+            // before this warp's first arrival on p_full, which the first P V of the stream waits for.
             const float lse0 = row_ok ? a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] : -INFINITY;
             const bool have = lse0 > -INFINITY;
             m = have ? lse0 * LOG2E : -INFINITY;
@@ -381,140 +384,141 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             tmem_wait_st();
         }
 
-        int q_prev = 0;  // number of this tile's previous product
+        // a product's number in the issue order picks its score buffer
+        auto product = [&](int j) { return min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0); };
+        int q_prev = 0;  // number of this stream's previous product
         for (int j = 0; j < nt; ++j) {
-            stamp(a, tls, j, 1 + t, 0);
-            // this product's number in the issue order picks its score buffer
-            const int q = min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0);
-            const uint32_t tS = trow + score_col(q % 3);
+            const int q = product(j);
+            const int buf = q % 3;
+            const uint32_t tS = trow + score_col(buf);
             // the vote keeps the warp converged for the .sync.aligned tensor-memory accesses below
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full[q % 3], (q / 3) & 1, W_SFULL, j));
+            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full[buf], (q / 3) & 1, W_SFULL, j));
             if (!ok) break;
-            stamp(a, tls, j, 1 + t, 1);
-            tc_fence_after_sync();
-            tmem_ld32p(tS, r);
-            tmem_ld32p(tS + 32, r + 32);
-            tmem_ld32p(tS + 64, r + 64);
-            tmem_ld32p(tS + 96, r + 96);
-            const int kv0 = j * TILE;
-            const int lim_local = kv_lim - kv0;  // columns 0..lim_local are visible
-            tmem_wait_ld();
-            stamp(a, tls, j, 1 + t, 2);
-            if (lim_local < TILE - 1) {
+            if (warp_live) {
+                tc_fence_after_sync();
+                tmem_ld32p(tS, r);
+                tmem_ld32p(tS + 32, r + 32);
+                tmem_ld32p(tS + 64, r + 64);
+                tmem_ld32p(tS + 96, r + 96);
+                const int kv0 = (keys ? jb + 2 * j + t : jb + j) * TILE;
+                const int lim_local = kv_lim - kv0;  // columns 0..lim_local are visible
+                tmem_wait_ld();
+                if (lim_local < TILE - 1) {
 #pragma unroll
-                for (int i = 0; i < 128; ++i)
-                    if (i > lim_local) r[i] = __float_as_uint(worst);
-            }
-            // row max of the raw scores (min if the scale is negative), four chains
-            float mx0 = __uint_as_float(r[0]), mx1 = __uint_as_float(r[1]), mx2 = __uint_as_float(r[2]),
-                  mx3 = __uint_as_float(r[3]);
-            if (c >= 0.f) {
+                    for (int i = 0; i < 128; ++i)
+                        if (i > lim_local) r[i] = __float_as_uint(worst);
+                }
+                // row max of the raw scores (min if the scale is negative), four chains
+                float mx0 = __uint_as_float(r[0]), mx1 = __uint_as_float(r[1]), mx2 = __uint_as_float(r[2]),
+                      mx3 = __uint_as_float(r[3]);
+                if (cs >= 0.f) {
 #pragma unroll
-                for (int i = 4; i < 128; i += 4) {
-                    mx0 = fmaxf(mx0, __uint_as_float(r[i]));
-                    mx1 = fmaxf(mx1, __uint_as_float(r[i + 1]));
-                    mx2 = fmaxf(mx2, __uint_as_float(r[i + 2]));
-                    mx3 = fmaxf(mx3, __uint_as_float(r[i + 3]));
-                }
-                mx0 = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-            } else {
+                    for (int i = 4; i < 124; i += 8) {
+                        mx0 = fmax3(mx0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                        mx1 = fmax3(mx1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                        mx2 = fmax3(mx2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
+                        mx3 = fmax3(mx3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
+                    }
+                    mx0 = fmax3(mx0, __uint_as_float(r[124]), __uint_as_float(r[125]));
+                    mx1 = fmax3(mx1, __uint_as_float(r[126]), __uint_as_float(r[127]));
+                    mx0 = fmax3(fmaxf(mx0, mx1), mx2, mx3);
+                } else {
 #pragma unroll
-                for (int i = 4; i < 128; i += 4) {
-                    mx0 = fminf(mx0, __uint_as_float(r[i]));
-                    mx1 = fminf(mx1, __uint_as_float(r[i + 1]));
-                    mx2 = fminf(mx2, __uint_as_float(r[i + 2]));
-                    mx3 = fminf(mx3, __uint_as_float(r[i + 3]));
+                    for (int i = 4; i < 128; i += 4) {
+                        mx0 = fminf(mx0, __uint_as_float(r[i]));
+                        mx1 = fminf(mx1, __uint_as_float(r[i + 1]));
+                        mx2 = fminf(mx2, __uint_as_float(r[i + 2]));
+                        mx3 = fminf(mx3, __uint_as_float(r[i + 3]));
+                    }
+                    mx0 = fminf(fminf(mx0, mx1), fminf(mx2, mx3));
                 }
-                mx0 = fminf(fminf(mx0, mx1), fminf(mx2, mx3));
-            }
-            const float m_cand = mx0 * c;  // -inf when nothing is visible
-            // raise the reference only when it pays: a stale m makes p at most 2^8 larger, which fp32 absorbs
-            const bool raise = (m == -INFINITY) ? (m_cand > -INFINITY) : (m_cand > m + RESCALE_THRESHOLD);
-            const float m_new = raise ? m_cand : m;
-            const float alpha = raise ? ((m == -INFINITY) ? 0.f : ex2_approx(m - m_cand)) : 1.f;
-            if ((j > 0 || a.continue_state) && __any_sync(0xffffffffu, raise)) {
-                // rescale the running output, once the P V of the previous step has completed
-                if (j > 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, j));
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                }
+                const float m_cand = mx0 * cs;  // -inf when nothing is visible
+                // raise the reference only when it pays: a stale m makes p at most 2^8 larger, which fp32 absorbs
+                const bool raise = (m == -INFINITY) ? (m_cand > -INFINITY) : (m_cand > m + RESCALE_THRESHOLD);
+                const float m_new = raise ? m_cand : m;
+                const float alpha = raise ? ((m == -INFINITY) ? 0.f : ex2_approx(m - m_cand)) : 1.f;
+                if ((j > 0 || state_in) && __any_sync(0xffffffffu, raise)) {
+                    // rescale the running output, once the P V of the previous step has completed
+                    if (j > 0) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, j));
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                    }
 #pragma unroll 1
-                for (int cc = 0; cc < 2; ++cc) {
-                    uint32_t o[32];
-                    tmem_ld32(tO + cc * 32, o);
-                    tmem_wait_ld();
+                    for (int cc = 0; cc < 2; ++cc) {
+                        uint32_t o[32];
+                        tmem_ld32(tO + cc * 32, o);
+                        tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    tmem_st32(tO + cc * 32, o);
-                }
-            }
-            const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-            if (a.dropout_mode == 0) {
-                // two scores per FMA and per add (fma.rn.f32x2 / add.rn.f32x2: the same roundings as the scalar forms)
-                const float2 c2 = make_float2(c, c), nm2 = make_float2(neg_m, neg_m);
-                float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < 128; i += 4) {
-                    const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
-                    const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), c2, nm2);
-                    const float2 p01 = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
-                    const float2 p23 = make_float2(ex2_approx(t23.x), ex2_approx(t23.y));
-                    s01 = __fadd2_rn(s01, p01);
-                    s23 = __fadd2_rn(s23, p23);
-                    r[i] = tf32_round_bits_mma(__float_as_uint(p01.x));
-                    r[i + 1] = tf32_round_bits_mma(__float_as_uint(p01.y));
-                    r[i + 2] = tf32_round_bits_mma(__float_as_uint(p23.x));
-                    r[i + 3] = tf32_round_bits_mma(__float_as_uint(p23.y));
-                }
-                s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
-            } else if (a.dropout_mode == 2) {
-                // one Philox call per eight keys of this row
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    const uint32_t kpos = (uint32_t)(a.k_pos0 + kv0 + g * 8);
-                    const hk_philox4_t w = hk_philox_row8(a.seed, a.offset, a.bh_pos0 + (uint32_t)bh, (uint32_t)(a.q_pos0 + qrow), kpos >> 3);
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        float p = ex2_approx(fmaf(__uint_as_float(r[g * 8 + u]), c, neg_m));
-                        const uint32_t half = (u & 1) ? (w.v[u >> 1] >> 16) : (w.v[u >> 1] & 0xFFFFu);
-                        if (scaled) { if (u & 1) s3 += p; else s2 += p; }  // the normaliser ignores the mask
-                        if (half < a.drop_thr) p = 0.f;
-                        if (u & 1) s1 += p; else s0 += p;
-                        r[g * 8 + u] = tf32_round_bits_mma(__float_as_uint(p));
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st32(tO + cc * 32, o);
                     }
                 }
-            } else {
-                const float* mrow = a.mask + ((size_t)bh * a.Tq + (row_ok ? qrow : 0)) * (size_t)a.Tk + kv0;
+                const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+                if constexpr (DROP == 0) {
+                    // two scores per FMA and per add (fma.rn.f32x2 / add.rn.f32x2: the same roundings as the scalar forms)
+                    const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
+                    float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 128; ++i) {
-                    float p = ex2_approx(fmaf(__uint_as_float(r[i]), c, neg_m));
-                    if (scaled) s2 += (i <= lim_local) ? p : 0.f;
-                    p = (i <= lim_local) ? p * __ldg(mrow + i) : 0.f;
-                    s0 += p;
-                    r[i] = tf32_round_bits_mma(__float_as_uint(p));
+                    for (int i = 0; i < 128; i += 4) {
+                        const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
+                        const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), c2, nm2);
+                        const float2 p01 = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
+                        const float2 p23 = make_float2(ex2_approx(t23.x), ex2_approx(t23.y));
+                        s01 = __fadd2_rn(s01, p01);
+                        s23 = __fadd2_rn(s23, p23);
+                        r[i] = tf32_round_bits_mma(__float_as_uint(p01.x));
+                        r[i + 1] = tf32_round_bits_mma(__float_as_uint(p01.y));
+                        r[i + 2] = tf32_round_bits_mma(__float_as_uint(p23.x));
+                        r[i + 3] = tf32_round_bits_mma(__float_as_uint(p23.y));
+                    }
+                    s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
+                } else if constexpr (DROP == 2) {
+                    // one Philox call per eight keys of this row
+#pragma unroll
+                    for (int g = 0; g < 16; ++g) {
+                        const uint32_t kpos = (uint32_t)(a.k_pos0 + kv0 + g * 8);
+                        const hk_philox4_t w = hk_philox_row8(a.seed, a.offset, a.bh_pos0 + (uint32_t)bh, (uint32_t)(a.q_pos0 + qrow), kpos >> 3);
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            float p = ex2_approx(fmaf(__uint_as_float(r[g * 8 + u]), cs, neg_m));
+                            const uint32_t half = (u & 1) ? (w.v[u >> 1] >> 16) : (w.v[u >> 1] & 0xFFFFu);
+                            if (scaled) { if (u & 1) s3 += p; else s2 += p; }  // the normaliser ignores the mask
+                            if (half < a.drop_thr) p = 0.f;
+                            if (u & 1) s1 += p; else s0 += p;
+                            r[g * 8 + u] = tf32_round_bits_mma(__float_as_uint(p));
+                        }
+                    }
+                } else {
+                    const float* mrow = a.mask + ((size_t)bh * a.Tq + (row_ok ? qrow : 0)) * (size_t)a.Tk + kv0;
+#pragma unroll
+                    for (int i = 0; i < 128; ++i) {
+                        float p = ex2_approx(fmaf(__uint_as_float(r[i]), cs, neg_m));
+                        if (scaled) s2 += (i <= lim_local) ? p : 0.f;
+                        p = (i <= lim_local) ? p * __ldg(mrow + i) : 0.f;
+                        s0 += p;
+                        r[i] = tf32_round_bits_mma(__float_as_uint(p));
+                    }
                 }
+                tmem_st32p(tS, r);
+                tmem_st32p(tS + 32, r + 32);
+                tmem_st32p(tS + 64, r + 64);
+                tmem_st32p(tS + 96, r + 96);
+                // inverted dropout: s2, s3 hold the sums over all visible keys, s0, s1 the kept ones
+                l = l * alpha + ((scaled && DROP != 0) ? (s2 + s3) : ((s0 + s1) + (s2 + s3)));
+                m = m_new;
+                tmem_wait_st();
+                tc_fence_before_sync();
             }
-            tmem_st32p(tS, r);
-            tmem_st32p(tS + 32, r + 32);
-            tmem_st32p(tS + 64, r + 64);
-            tmem_st32p(tS + 96, r + 96);
-            // inverted dropout: s2, s3 hold the sums over all visible keys, s0, s1 the kept ones
-            l = l * alpha + ((scaled && a.dropout_mode != 0) ? (s2 + s3) : ((s0 + s1) + (s2 + s3)));
-            m = m_new;
-            stamp(a, tls, j, 1 + t, 3);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive_warp(&sh.p_full[q % 3], lane);
+            mbar_arrive_warp(&sh.p_full[buf], lane);
             q_prev = q;
-            stamp(a, tls, j, 1 + t, 4);
         }
 
         // epilogue: O / l and LSE
         if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, nt));
         tc_fence_after_sync();
-        const float inv_l = (l > 0.f) ? a.keep_scale / l : 0.f;
+        const float inv_l = combine ? 1.f : (l > 0.f) ? a.keep_scale / l : 0.f;
         if (ok && nt > 0) {
             tmem_ld32p(tO, r);
             tmem_ld32p(tO + 32, r + 32);
@@ -523,66 +527,179 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
             for (int i = 0; i < 64; ++i) r[i] = 0u;
         }
-        // O leaves through shared memory and a TMA bulk store (a thread-per-row store would touch 32 lines per
-        // instruction).  The tile's own Q buffer is dead -- o_full covered its last S = Q K^T -- and takes the
-        // two 32-column boxes of a 128-byte-swizzled TMA tile: 16-byte chunk c of row r at position c ^ (r & 7).
-        // Rows past the end of the sequence are clipped by the copy.
-        // (a tile that had no key tile to wait for must still let the load of its Q land before reusing the buffer)
-        if (nt == 0 && n > 0) __all_sync(0xffffffffu, mbar_wait(wc, &sh.q_full, 0, W_QFULL, 0));
+        // O leaves through shared memory (a thread-per-row store would touch 32 lines per instruction).  The stream's own Q
+        // buffer is dead -- o_full covered its last S = Q K^T, and in keys mode, where the streams share Q, every S: the
+        // last one is issued before the last two P V -- and takes the two 32-column boxes of a 128-byte-swizzled TMA tile:
+        // 16-byte chunk i of row r at position i ^ (r & 7).
         {
             uint8_t* srow = sQ + t * TILE_BYTES + row * 128;
 #pragma unroll
-            for (int i = 0; i < 64; i += 4) {
-                float4 v;
-                v.x = __uint_as_float(r[i]) * inv_l;
-                v.y = __uint_as_float(r[i + 1]) * inv_l;
-                v.z = __uint_as_float(r[i + 2]) * inv_l;
-                v.w = __uint_as_float(r[i + 3]) * inv_l;
-                const int c = (i >> 2) & 7;
-                *reinterpret_cast<float4*>(srow + (i >> 5) * BOX_BYTES + ((c ^ (row & 7)) << 4)) = v;
-            }
-            fence_proxy_async_smem();
+            for (int ch = 0; ch < 16; ++ch)
+                *reinterpret_cast<float4*>(srow + (ch >> 3) * BOX_BYTES + (((ch & 7) ^ (row & 7)) << 4)) =
+                    make_float4(__uint_as_float(r[4 * ch]) * inv_l, __uint_as_float(r[4 * ch + 1]) * inv_l,
+                                __uint_as_float(r[4 * ch + 2]) * inv_l, __uint_as_float(r[4 * ch + 3]) * inv_l);
         }
-        // a tile that saw no key of this call leaves a continued result untouched
-        const bool keep_old = a.continue_state && nt == 0;
-        if (row_ok && !keep_old)
-            a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
-        // the 128 threads of this query tile (every one gets here, whatever `ok` is), then one of them stores
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
-        if (row == 0 && q0 + t * TILE < a.Tq && !keep_old) {
-            tma_store_4d(&mapO, sQ + t * TILE_BYTES, 0, q0 + t * TILE, h, b);
-            tma_store_4d(&mapO, sQ + t * TILE_BYTES + BOX_BYTES, HALF_D, q0 + t * TILE, h, b);
-            bulk_commit_group();
-            bulk_wait_group_all();
+        // a block none of whose rows sees a key of this call leaves a continued result untouched
+        const bool keep_old = a.continue_state && (t == 0 ? all0 : all1) == 0;
+        if (!combine) {
+            fence_proxy_async_smem();
+            if (row_ok && !keep_old)
+                a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
+            // the 128 threads of this stream (every one gets here, whatever `ok` is), then one of them stores; rows past
+            // the end of the sequence are clipped by the copy
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
+            if (row == 0 && row_ok && !keep_old) {
+                tma_store_4d(&mapO, sQ + t * TILE_BYTES, 0, qrow, h, b);
+                tma_store_4d(&mapO, sQ + t * TILE_BYTES + BOX_BYTES, HALF_D, qrow, h, b);
+                bulk_commit_group();
+                bulk_wait_group_read_all();  // the copies have read their source; they complete on their own
+            }
+        } else {
+            // Combine: O = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M) over the splits and, in keys mode, the two
+            // streams.  Each CTA takes an equal slice of the rows it shares with its counterparts, 16 threads per row.
+            sh.m[t][row] = m;
+            sh.l[t][row] = l;
+            barrier_all();
+            const int rows = block_rows / ns, streams = keys ? 2 : 1;
+#pragma unroll 1
+            for (int i = threadIdx.x - 128; i < rows * 16; i += NUM_SOFTMAX) {
+                const int rr = split * rows + (i >> 4), ch = i & 15;
+                const int tt = rr / TILE, r1 = rr % TILE;
+                const int qr = row0_of(tt) + r1;
+                if (qr >= q_end || (a.continue_state && (tt == 0 ? all0 : all1) == 0)) continue;
+                const uint8_t* src = sQ + tt * TILE_BYTES + (ch >> 3) * BOX_BYTES + r1 * 128 + (((ch & 7) ^ (r1 & 7)) << 4);
+                float M = -INFINITY, L = 0.f;
+                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                auto fold = [&](float ms, float ls, const float4& v) {
+                    const float Mn = fmaxf(M, ms);
+                    const float wa = M == -INFINITY ? 0.f : ex2_approx(M - Mn), w = ms == -INFINITY ? 0.f : ex2_approx(ms - Mn);
+                    L = L * wa + w * ls;
+                    acc.x = acc.x * wa + w * v.x; acc.y = acc.y * wa + w * v.y;
+                    acc.z = acc.z * wa + w * v.z; acc.w = acc.w * wa + w * v.w;
+                    M = Mn;
+                };
+                for (int u = 0; u < streams; ++u) {
+                    if (ns == 1) {
+                        fold(sh.m[tt + u][r1], sh.l[tt + u][r1], *reinterpret_cast<const float4*>(src + u * TILE_BYTES));
+                    } else {
+                        for (int s0 = 0; s0 < ns; s0 += 2) {
+                            float ms[2], ls[2];
+                            float4 v[2];
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                ms[s] = ld_cluster_f(mapa(&sh.m[tt + u][r1], s0 + s));
+                                ls[s] = ld_cluster_f(mapa(&sh.l[tt + u][r1], s0 + s));
+                                v[s] = ld_cluster_f4(mapa(src + u * TILE_BYTES, s0 + s));
+                            }
+                            fold(ms[0], ls[0], v[0]);
+                            fold(ms[1], ls[1], v[1]);
+                        }
+                    }
+                }
+                const float f = (L > 0.f) ? a.keep_scale / L : 0.f;
+                reinterpret_cast<float4*>(a.O + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH + (int64_t)qr * a.o_sM)[ch] =
+                    make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
+                if (ch == 0)
+                    a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qr] = (L > 0.f) ? (M + log2f(L)) * LN2 : -INFINITY;
+            }
         }
         tc_fence_before_sync();
-        __syncthreads();  // pairs with the control warps' barrier before tensor memory is freed
-    }
-    if (trace) {
-        a.timeline[4 * blockIdx.x + 1] = (long long)globaltimer_ns();
-        a.timeline[4 * blockIdx.x + 3] = n;
+        barrier_all();  // pairs with the control warps' barrier before tensor memory is freed
     }
 }
 
+// Per-device launch data: the large shared-memory opt-in and how many clusters of each size run at once.
+namespace {
+struct FwdDevice {
+    std::once_flag once;
+    cudaError_t rc = cudaSuccess;
+    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs
+};
+typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
+
+cudaLaunchConfig_t fwd_config(unsigned blocks, int ns, cudaStream_t stream, cudaLaunchAttribute* attr) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ns;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(fwd::NUM_THREADS);
+    cfg.dynamicSmemBytes = fwd::SMEM_BYTES;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = ns > 1 ? 1 : 0;
+    return cfg;
+}
+}  // namespace
+
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                    const FwdArgs& a, cudaStream_t stream) {
-    // the opt-in to large dynamic shared memory is per device: once per device, safe from any number of host threads
-    static std::once_flag attr_once[HK_MAX_DEVICES];
-    static cudaError_t attr_rc[HK_MAX_DEVICES];
+                    FwdArgs a, cudaStream_t stream) {
+    static FwdDevice devices[HK_MAX_DEVICES];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HK_ERR_CUDA;
     if (dev < 0 || dev >= HK_MAX_DEVICES) return HK_ERR_UNSUPPORTED;
-    std::call_once(attr_once[dev], [dev] {
-        attr_rc[dev] = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM_BYTES);
+    static const FwdKernel kernels[3] = {attn_fwd_kernel<0>, attn_fwd_kernel<1>, attn_fwd_kernel<2>};
+    FwdDevice& d = devices[dev];
+    std::call_once(d.once, [&d] {
+        for (FwdKernel k : kernels)
+            if (d.rc == cudaSuccess)
+                d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM_BYTES);
+        for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
+            cudaLaunchAttribute attr[1];
+            const cudaLaunchConfig_t cfg = fwd_config(8u << i, 1 << i, nullptr, attr);
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kernels[0], &cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+        }
     });
-    if (attr_rc[dev] != cudaSuccess) return HK_ERR_CUDA;
-    const long long nblocks = (long long)a.n_qtiles * a.BH;
+    if (d.rc != cudaSuccess) return HK_ERR_CUDA;
+    // Mode and splits by an estimate of the makespan: the mean load of a slot plus half of the longest cluster, but at
+    // least that cluster.  A CTA costs ~3.5 us and ~2.1 us per step of two products (1.3 with one stream, 2.3 in keys
+    // mode), ~2 us more when it merges streams and ~3 us more when it combines splits.  Rows mode loads a key tile once
+    // for two products and is the fastest where it fills the chip; row mode where it does not; keys mode and splits
+    // when even those leave most SMs idle (512 queries of 32 heads against 8 192 keys: 64 CTAs of 64 steps on 148 SMs).
+    // Those two sum in another order, and the choice depends on batch x heads: they are left out for sequences of
+    // training length, so that a batch cut into calls gives the bits of the single call.
+    const bool may_split = a.Tk > 4096 || a.Tk >= 2 * (long long)a.Tq;
+    double best_cost = 0;
+    long long blocks = 0;
+    for (int mode = FWD_ROWS; mode <= (may_split ? FWD_KEYS : FWD_ROW); ++mode) {
+        const int rows = mode == FWD_ROWS ? 2 * TILE : TILE;
+        const int nb = (a.Tq + rows - 1) / rows;
+        double sum = 0, longest = 0;  // steps of one (batch, head) slice, of its longest block
+        const int sampled = std::min(nb, 64);  // the work per block is linear in its position: long sequences are sampled
+        for (int i = 0; i < sampled; ++i) {
+            const long long blk = sampled == nb ? i : (long long)i * (nb - 1) / (sampled - 1);
+            const int last = (int)(std::min<long long>(a.Tq, (blk + 1) * rows) - 1);  // its tile sees the most keys of the block
+            const int tiles = fwd::kv_tiles_for(last / TILE * TILE, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+            const double st = mode == FWD_KEYS ? 0.5 * tiles : tiles;
+            sum += st;
+            longest = std::max(longest, st);
+        }
+        sum *= (double)nb / sampled;
+        for (int i = 0; i < (may_split ? 4 : 1); ++i) {
+            const double fixed = 3.5 + (mode == FWD_KEYS ? 2.0 : 0.0) + (i ? 3.0 : 0.0);
+            const double step = mode == FWD_ROWS ? 2.1 : mode == FWD_ROW ? 1.3 : 2.3;
+            const double one = fixed + step * std::ceil(longest / (1 << i));
+            const double mean = a.BH * (nb * fixed + step * sum / (1 << i)) / d.slots[i];
+            const double cost = std::max(one, mean + 0.5 * one);
+            if ((mode == FWD_ROWS && i == 0) || cost < 0.95 * best_cost) {
+                best_cost = cost;
+                a.mode = mode;
+                a.n_splits = 1 << i;
+                a.n_qblocks = nb;
+                blocks = (long long)nb * a.BH;
+            }
+        }
+    }
+    const long long nblocks = blocks * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);
-    attn_fwd_kernel<<<(unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream>>>(mq, mk, mv, mo, a);
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = fwd_config((unsigned)nblocks, a.n_splits, stream, attr);
+    const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernels[a.dropout_mode], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
-    return check_launch();
+    return rc == cudaSuccess ? HK_OK : check_launch();
 }
 
 }  // namespace hk

@@ -4,6 +4,9 @@
 
 namespace hk {
 
+// what the two streams of a forward CTA are (attn_fwd_sm100.cu)
+enum FwdMode { FWD_ROWS = 0, FWD_ROW = 1, FWD_KEYS = 2 };
+
 struct FwdArgs {
     float* O;
     float* LSE;
@@ -11,7 +14,7 @@ struct FwdArgs {
     int64_t o_sB, o_sM, o_sH, lse_sB, lse_sH;
     int H, BH;
     int Tq, Tk;
-    int n_qtiles;
+    int n_qblocks, n_splits, mode;  // how the work is cut: set by launch_attn_fwd
     int q_pos0, k_pos0;
     float scale_log2e;
     int causal;
@@ -23,13 +26,11 @@ struct FwdArgs {
     uint32_t bh_pos0;  // added to the local (batch, head) index in the Philox counter
     uint64_t seed, offset;
     DeviceStatus* status;
-    long long* timeline;  // per-phase SM clock stamps of one CTA; only builds with -DHK_TIMELINE read it
-    int timeline_block;
 };
 
 // mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                    const FwdArgs& a, cudaStream_t stream);
+                    FwdArgs a, cudaStream_t stream);
 
 struct BwdArgs {
     const float* LSE;

@@ -205,7 +205,6 @@ int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_s
     a.o_sB = p->o_strideB; a.o_sM = p->o_strideM; a.o_sH = p->o_strideH;
     a.lse_sB = p->lse_strideB; a.lse_sH = p->lse_strideH;
     a.H = H; a.BH = BH; a.Tq = (int)Tq; a.Tk = (int)Tk;
-    a.n_qtiles = (int)((Tq + 2 * TILE - 1) / (2 * TILE));  // the forward takes two 128-row tiles per CTA
     a.q_pos0 = (int)p->q_pos0; a.k_pos0 = (int)p->k_pos0;
     a.scale_log2e = p->scale * LOG2E;
     a.causal = p->is_causal ? 1 : 0;
@@ -218,8 +217,6 @@ int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_s
     a.seed = p->dropout_seed; a.offset = p->dropout_offset; a.bh_pos0 = p->bh_pos0;
     a.status = device_status_ptr();
     if (!a.status) return HK_ERR_CUDA;
-    a.timeline = g_timeline.load();
-    a.timeline_block = g_timeline_block.load();
     CUtensorMap mo;
     if ((rc = make_tile_map(&mo, p->O, HEAD_DIM, B, H, Tq, p->o_strideB, p->o_strideM, p->o_strideH, TILE))) return rc;
     return launch_attn_fwd(mq, mk, mv, mo, a, stream);
