@@ -81,10 +81,10 @@ struct __align__(16) Shared {
     uint64_t v_ready;       // V is in tensor memory (and its landing buffer is free)
     uint64_t qk_free, dok_free;  // S^T(i) / dP^T(i) complete: the K-major Q / dO tile may be refilled
     uint64_t s_full, dp_full;
-    // per column group (32 query columns = four K = 8 slices of dV and dK): the warps of a group arrive together, the
-    // groups one after the other (the schedulers favour the older warps), and each group's slices go as soon as it is in
-    uint64_t pt_ready[4];   // P^T of the group is in tensor memory: its slices of dV += P^T dO may go
-    uint64_t p_ready[4];    // dS^T of the group is in tensor memory: its slices of dK += dS^T Q may go
+    // One barrier for all four column groups: with one each (so that a group's slices could go as soon as it was in) the
+    // issuing warp spent more on the six extra waits per tile than the early start gained (4 - 8 % of the kernel).
+    uint64_t pt_ready;      // P^T is in tensor memory: dV += P^T dO may go
+    uint64_t p_ready;       // dS^T is in tensor memory: dK += dS^T Q may go
     uint64_t dv_done, dk_done;   // dV(i) / dK(i) complete: the MN-major dO / Q tile is free
     uint64_t ds_ready, dq_full, dq_empty, staged;
     uint64_t acc_staged;    // dV, dK of the CTA are staged for the bulk store
@@ -167,7 +167,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     uint8_t* sdS = smem + OFF_DS;  // box b at sdS + b * BOX_BYTES
     Shared& sh = *reinterpret_cast<Shared*>(smem + OFF_SH);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = (int)uniform(threadIdx.x >> 5);  // uniform for the compiler too: see uniform()
     const int lane = threadIdx.x & 31;
 
     // early KV tiles first: under the causal mask they see the most query tiles
@@ -231,10 +231,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.dok_free, 1);
         mbar_init(&sh.s_full, 1);
         mbar_init(&sh.dp_full, 1);
-        for (int g = 0; g < 4; ++g) {
-            mbar_init(&sh.pt_ready[g], TILE / 32);
-            mbar_init(&sh.p_ready[g], TILE / 32);
-        }
+        mbar_init(&sh.pt_ready, NUM_COMPUTE / 32);
+        mbar_init(&sh.p_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.dv_done, 1);
         mbar_init(&sh.dk_done, 1);
         mbar_init(&sh.ds_ready, NUM_COMPUTE / 32);
@@ -254,7 +252,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = sh.tmem_base;
+    const uint32_t tmem = uniform(sh.tmem_base);
     WaitCtx wc{&sh.abort_flag, a.status};
 #ifdef HK_TIMELINE
     const bool tl = a.timeline != nullptr && (int)blockIdx.x == a.timeline_block;  // never in trace mode
@@ -366,34 +364,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 stamp(a, tlm, it, 0, 0);
                 if (!(ok = wait(&sh.dom_full, par, W_QMFULL, it))) break;
                 stamp(a, tlm, it, 0, 1);
-                for (int g = 0; ok && g < 4; ++g) {  // dV += P^T dO, group by group
-                    if (!(ok = wait(&sh.pt_ready[g], par, W_PREADY, 4 * it + g))) break;
-                    tc_fence_after_sync();
+                // dV += P^T dO
+                if (!(ok = wait(&sh.pt_ready, par, W_PREADY, it))) break;
+                tc_fence_after_sync();
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4) {
-                        const int kk = 4 * g + k4;
-                        umma_ts_tf32_lead(leader, tmem + COL_DV, tmem + COL_S + kk * 8, mnmajor_desc(dom_addr, kk, BOX_BYTES),
-                                          IDESC_TS, (it > 0 || kk > 0) ? 1u : 0u);
-                    }
-                }
-                if (!ok) break;
+                for (int kk = 0; kk < TILE / 8; ++kk)
+                    umma_ts_tf32_lead(leader, tmem + COL_DV, tmem + COL_S + kk * 8, mnmajor_desc(dom_addr, kk, BOX_BYTES), IDESC_TS,
+                                      (it > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_lead(leader, &sh.dv_done);  // MN-major dO consumed: two of the dS boxes may be staged over it
                 stamp(a, tlm, it, 0, 2);
                 // next tile's S^T: P^T of this tile was consumed by the MMAs just issued
                 if (it + 1 < n_it && !(ok = issue_st(it + 1))) break;
                 stamp(a, tlm, it, 0, 3);
                 if (!(ok = wait(&sh.qm_full, par, W_QMFULL, 1000 + it))) break;
-                for (int g = 0; ok && g < 4; ++g) {  // dK += dS^T Q, group by group
-                    if (!(ok = wait(&sh.p_ready[g], par, W_PREADY, 1000 + 4 * it + g))) break;
-                    tc_fence_after_sync();
+                // dK += dS^T Q
+                if (!(ok = wait(&sh.p_ready, par, W_PREADY, 1000 + it))) break;
+                tc_fence_after_sync();
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4) {
-                        const int kk = 4 * g + k4;
-                        umma_ts_tf32_lead(leader, tmem + COL_DK, tmem + COL_DP + kk * 8, mnmajor_desc(qm_addr, kk, BOX_BYTES),
-                                          IDESC_TS, (it > 0 || kk > 0) ? 1u : 0u);
-                    }
-                }
-                if (!ok) break;
+                for (int kk = 0; kk < TILE / 8; ++kk)
+                    umma_ts_tf32_lead(leader, tmem + COL_DK, tmem + COL_DP + kk * 8, mnmajor_desc(qm_addr, kk, BOX_BYTES), IDESC_TS,
+                                      (it > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_lead(leader, &sh.dk_done);  // MN-major Q consumed
                 // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
                 if (it + 1 < n_it && !(ok = issue_dp(it + 1))) break;
@@ -671,7 +661,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tmem_st32(trow + COL_S + c0, rp);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive_warp(&sh.pt_ready[part], lane);
+                mbar_arrive_warp(&sh.pt_ready, lane);
             }
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, it & 1, W_SFULL, 1000 + it));
             if (!ok) break;
@@ -714,7 +704,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             tmem_wait_st();
             stamp(a, tlc, it, 1, 13);
             tc_fence_before_sync();
-            mbar_arrive_warp(&sh.p_ready[part], lane);  // this group's slices of dK += dS^T Q may go
+            mbar_arrive_warp(&sh.p_ready, lane);
             stamp(a, tlc, it, 1, 5);
 
             // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns

@@ -423,16 +423,15 @@ __device__ __forceinline__ void umma_ts_tf32_lead(uint32_t leader, uint32_t d_tm
 }
 
 // Runs of four MMAs over consecutive K = 8 slices, the form the attention kernels issue.  The tensor pipe executes an
-// M128 N64 K8 instruction in 35 cycles and queues next to none, so the issuing warp must not need more per instruction:
-// written slice by slice with 64-bit descriptors it took 57 - 75.  Here a slice costs a 32-bit addition per operand (the
-// descriptors of a tile's slices differ in the address field only, and shared memory is smaller than that field's range).
-// The warp index and every address must be warp-uniform for the compiler too (see uniform()): otherwise each operand is
-// moved from vector to uniform registers, instruction by instruction.
-struct Desc {  // the two words of a shared-memory descriptor
-    uint32_t lo, hi;
-    __device__ __forceinline__ Desc(uint64_t d) : lo((uint32_t)d), hi((uint32_t)(d >> 32)) {}
-    __device__ __forceinline__ Desc(uint32_t l, uint32_t h) : lo(l), hi(h) {}
-    __device__ __forceinline__ Desc operator+(uint32_t bytes) const { return Desc(lo + (bytes >> 4), hi); }
+// M128 N64 K8 instruction in 35 cycles and queues next to none, so the issuing warp must not need more per instruction.
+// The descriptors of a tile's slices differ in the address field only (shared memory is smaller than that field's range,
+// so no carry leaves it): one addition per slice.  The warp index and every address must be warp-uniform for the compiler
+// too (see uniform()): otherwise each operand is moved from vector to uniform registers, instruction by instruction --
+// 57 - 75 cycles per MMA.  (All four instructions in one asm statement with 32-bit additions: no faster.)
+struct Desc {  // a shared-memory descriptor that can be moved by bytes
+    uint64_t d;
+    __device__ __forceinline__ Desc(uint64_t x) : d(x) {}
+    __device__ __forceinline__ Desc operator+(uint32_t bytes) const { return Desc(d + (bytes >> 4)); }
 };
 __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 
@@ -442,66 +441,15 @@ constexpr int MNMAJOR_STEP = 1024 >> 4;  // slice to slice of an MN-major tile
 // D[tmem] (+)= A[tmem] * B[smem], four slices: A columns a, a + 8, ...; `acc` = 0: the first one overwrites D
 template <int BSTEP>
 __device__ __forceinline__ void umma_ts4(uint32_t leader, uint32_t d, uint32_t a, Desc b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t;\n"
-        ".reg .b32 a1, a2, a3, l1, l2, l3;\n"
-        ".reg .b64 b0, b1, b2, b3;\n"
-        "setp.ne.b32 q, %6, 0;\n"
-        "setp.ne.b32 p, %5, 0;\n"
-        "setp.eq.b32 t, 0, 0;\n"
-        "add.u32 a1, %1, 8;\n"
-        "add.u32 a2, %1, 16;\n"
-        "add.u32 a3, %1, 24;\n"
-        "add.u32 l1, %2, %7;\n"
-        "add.u32 l2, %2, %8;\n"
-        "add.u32 l3, %2, %9;\n"
-        "mov.b64 b0, {%2, %3};\n"
-        "mov.b64 b1, {l1, %3};\n"
-        "mov.b64 b2, {l2, %3};\n"
-        "mov.b64 b3, {l3, %3};\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], b0, %4, p;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [a1], b1, %4, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [a2], b2, %4, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [a3], b3, %4, t;\n"
-        "}\n"
-        ::"r"(d), "r"(a), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(acc), "r"(leader), "n"(BSTEP), "n"(2 * BSTEP), "n"(3 * BSTEP)
-        : "memory");
+#pragma unroll
+    for (int k = 0; k < 4; ++k) umma_ts_tf32_lead(leader, d, a + 8 * k, b.d + BSTEP * k, idesc, k > 0 ? 1u : acc);
 }
 
 // D[tmem] (+)= A[smem] * B[smem], four slices
 template <int ASTEP, int BSTEP>
 __device__ __forceinline__ void umma_ss4(uint32_t leader, uint32_t d, Desc a, Desc b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t;\n"
-        ".reg .b32 k1, k2, k3, l1, l2, l3;\n"
-        ".reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n"
-        "setp.ne.b32 q, %7, 0;\n"
-        "setp.ne.b32 p, %6, 0;\n"
-        "setp.eq.b32 t, 0, 0;\n"
-        "add.u32 k1, %1, %8;\n"
-        "add.u32 k2, %1, %9;\n"
-        "add.u32 k3, %1, %10;\n"
-        "add.u32 l1, %3, %11;\n"
-        "add.u32 l2, %3, %12;\n"
-        "add.u32 l3, %3, %13;\n"
-        "mov.b64 a0, {%1, %2};\n"
-        "mov.b64 a1, {k1, %2};\n"
-        "mov.b64 a2, {k2, %2};\n"
-        "mov.b64 a3, {k3, %2};\n"
-        "mov.b64 b0, {%3, %4};\n"
-        "mov.b64 b1, {l1, %4};\n"
-        "mov.b64 b2, {l2, %4};\n"
-        "mov.b64 b3, {l3, %4};\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], a0, b0, %5, p;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], a1, b1, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], a2, b2, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], a3, b3, %5, t;\n"
-        "}\n"
-        ::"r"(d), "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(acc), "r"(leader), "n"(ASTEP), "n"(2 * ASTEP),
-        "n"(3 * ASTEP), "n"(BSTEP), "n"(2 * BSTEP), "n"(3 * BSTEP)
-        : "memory");
+#pragma unroll
+    for (int k = 0; k < 4; ++k) umma_ss_tf32_lead(leader, d, a.d + ASTEP * k, b.d + BSTEP * k, idesc, k > 0 ? 1u : acc);
 }
 
 __device__ __forceinline__ void umma_commit_lead(uint32_t leader, uint64_t* bar) {
