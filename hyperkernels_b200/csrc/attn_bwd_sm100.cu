@@ -128,6 +128,7 @@ enum WaitId {
 
 }  // namespace bwd
 
+template <int DROP>  // 0 none, 1 dense mask, 2 Philox
 __global__ void __launch_bounds__(bwd::NUM_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapdO,
@@ -579,7 +580,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
             // dropout keep bits of this thread's 32 (query, key) pairs
             uint32_t keep = 0xffffffffu;
-            if (a.dropout_mode == 2) {
+            if constexpr (DROP == 2) {
                 // One Philox call covers the eight keys kpos & ~7 .. of one query row, i.e. the key rows of eight
                 // adjacent lanes (k_pos0 and kv0 are multiples of 8, so row & 7 == lane & 7).  Lane j of such a
                 // group evaluates the query columns 8m + j (m = 0..3) and keeps 8 bits per call; the group then
@@ -599,7 +600,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     const uint32_t other = __shfl_sync(0xffffffffu, mine, (lane & ~7) | j);  // lane j's columns 8m + j
                     keep |= ((other >> j8) & 0x01010101u) << j;                              // its bit for MY key row
                 }
-            } else if (a.dropout_mode == 1) {
+            } else if constexpr (DROP == 1) {
                 keep = 0u;
                 if (kv_ok) {
 #pragma unroll 4
@@ -618,7 +619,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 keep &= vis;
             }
             // pairs whose p is zero: hidden ones, and dropped ones unless the dropout is the inverted kind
-            const uint32_t live = a.drop_scaled ? vis : keep;
+            const uint32_t live = DROP != 0 && a.drop_scaled ? vis : keep;
             tmem_wait_ld();
             stamp(a, tlc, it, 1, 9);
 
@@ -650,7 +651,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // keeps its p for dS below): dV += P^T dO and, behind it, the next tile's S^T run while dS is computed,
             // and the store has drained by the time its first reader starts.  rp is free until dP^T is loaded.
             {
-                const bool dropped_some = a.drop_scaled && keep != 0xffffffffu;
+                const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
 #pragma unroll
                 for (int i = 0; i < 32; ++i) rp[i] = tf32_round_bits_mma(rs[i]);
                 if (dropped_some) {
@@ -675,7 +676,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // dS = p * (dP*scale - D*scale), two elements per packed instruction
             {
                 const float4* ds4 = reinterpret_cast<const float4*>(sh.dsum[it & 1] + c0);
-                const bool dropped_some = a.drop_scaled && keep != 0xffffffffu;
+                const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
                 if (dropped_some) {
                     // inverted dropout: a dropped pair keeps the -D term of dS but contributes neither dP (zeroed
                     // here) nor to dV (its P^T entry was stored as zero above)
@@ -798,6 +799,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 }
 
 int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream) {
+    typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
+                           CUtensorMap, CUtensorMap, BwdArgs);
+    static const Kernel kernels[3] = {attn_bwd_kernel<0>, attn_bwd_kernel<1>, attn_bwd_kernel<2>};
     // the opt-in to large dynamic shared memory is per device: once per device, safe from any number of host threads
     static std::once_flag attr_once[HK_MAX_DEVICES];
     static cudaError_t attr_rc[HK_MAX_DEVICES];
@@ -805,14 +809,16 @@ int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream) {
     if (cudaGetDevice(&dev) != cudaSuccess) return HK_ERR_CUDA;
     if (dev < 0 || dev >= HK_MAX_DEVICES) return HK_ERR_UNSUPPORTED;
     std::call_once(attr_once[dev], [dev] {
-        attr_rc[dev] = cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);
+        for (Kernel k : kernels)
+            if (attr_rc[dev] == cudaSuccess)
+                attr_rc[dev] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);
     });
     if (attr_rc[dev] != cudaSuccess) return HK_ERR_CUDA;
     const long long nblocks = (long long)a.n_kvtiles * a.BH;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_BWD, true, stream);
-    attn_bwd_kernel<<<(unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream>>>(m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
-                                                                                       m.dO_mn, m.dQ, m.dK, m.dV, a);
+    kernels[a.dropout_mode]<<<(unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream>>>(m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
+                                                                                              m.dO_mn, m.dQ, m.dK, m.dV, a);
     timing_mark(TIMED_BWD, false, stream);
     count_launch();
     return check_launch();

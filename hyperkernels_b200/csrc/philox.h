@@ -78,16 +78,18 @@ HK_HD hk_philox4_t hk_philox_row8(uint64_t seed, uint64_t offset, uint32_t bh, u
                             (uint32_t)(seed >> 32) ^ (uint32_t)(offset >> 32));
 }
 
+/* Is key u (0..7) of one Philox call kept?  half >= thr, compared in the upper 16 bits (thr < 2^16). */
+HK_HD int hk_philox_keep1(hk_philox4_t r, int u, uint32_t thr) {
+    return ((u & 1) ? r.v[u >> 1] : r.v[u >> 1] << 16) >= (thr << 16);
+}
+
 /* Keep bits of the eight keys of one Philox call: bit u <=> key 8*kj8+u is kept. */
 HK_HD uint32_t hk_philox_keep8(hk_philox4_t r, uint32_t thr) {
     uint32_t m = 0;
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-    for (int w = 0; w < 4; ++w) {
-        m |= ((r.v[w] & 0xFFFFu) >= thr ? 1u : 0u) << (2 * w);
-        m |= ((r.v[w] >> 16) >= thr ? 1u : 0u) << (2 * w + 1);
-    }
+    for (int u = 0; u < 8; ++u) m |= hk_philox_keep1(r, u, thr) ? 1u << u : 0u;
     return m;
 }
 
