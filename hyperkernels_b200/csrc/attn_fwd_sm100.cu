@@ -672,7 +672,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
     // Mode and splits by an estimate of the makespan: the mean load of a slot plus half of the longest cluster, but at
-    // least that cluster.  A CTA costs ~3.5 us and ~2.1 us per step of two products (1.3 with one stream, 2.3 in keys
+    // least that cluster.  A CTA costs ~3.5 us and ~2.1 us per step of two products (1.5 with one stream, 2.3 in keys
     // mode), ~2 us more when it merges streams and ~3 us more when it combines splits.  Rows mode loads a key tile once
     // for two products and is the fastest where it fills the chip; row mode where it does not; keys mode and splits
     // when even those leave most SMs idle (512 queries of 32 heads against 8 192 keys: 64 CTAs of 64 steps on 148 SMs).
@@ -697,7 +697,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
         sum *= (double)nb / sampled;
         for (int i = 0; i < (may_split ? 4 : 1); ++i) {
             const double fixed = 3.5 + (mode == FWD_KEYS ? 2.0 : 0.0) + (i ? 3.0 : 0.0);
-            const double step = mode == FWD_ROWS ? 2.1 : mode == FWD_ROW ? 1.3 : 2.3;
+            const double step = mode == FWD_ROWS ? 2.1 : mode == FWD_ROW ? 1.5 : 2.3;
             const double one = fixed + step * std::ceil(longest / (1 << i));
             const double mean = a.BH * (nb * fixed + step * sum / (1 << i)) / d.slots[i];
             const double cost = std::max(one, mean + 0.5 * one);

@@ -32,6 +32,22 @@ struct FwdArgs {
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                     FwdArgs a, cudaStream_t stream);
 
+// A few query rows against many keys (attn_decode.cu): no dropout, no starting state.
+constexpr int DECODE_MAX_Q = 2;
+struct DecodeArgs {
+    View4 Q, K, V;
+    float* O;
+    float* LSE;
+    int64_t o_sB, o_sM, o_sH, lse_sB, lse_sH;
+    int H, BH;
+    int Tq, Tk;
+    int q_pos0, k_pos0;
+    float scale_log2e;
+    int causal;
+    int n_splits;  // set by launch_attn_decode
+};
+int launch_attn_decode(DecodeArgs a, cudaStream_t stream);
+
 struct BwdArgs {
     const float* LSE;
     const float* D;

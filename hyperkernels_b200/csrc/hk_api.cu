@@ -194,6 +194,23 @@ int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_s
     if (check_scratch && !scratch_ok(p->workspace, p->workspace_bytes, hk_attn_fwd_workspace_bytes(p))) return HK_ERR_WORKSPACE;
 
     const int B = p->B, H = p->nh, BH = B * H;
+    // A few query rows: the tensor-core kernel would work on 128 rows whatever there are, this one is bound by reading K
+    // and V.  Up to two rows: its arithmetic per key grows with them (B8 H12, 2 047 keys: four rows 31 us, eight 54, 29 with
+    // the tensor cores); below 128 keys there is nothing to split.
+    if (Tq <= DECODE_MAX_Q && Tk >= 128 && mode == 0 && !(p->flags & HK_FLAG_CONTINUE_SOFTMAX_STATE)) {
+        DecodeArgs d{};
+        d.Q = View4{p->Q, p->q_strideB, p->q_strideM, p->q_strideH};
+        d.K = View4{p->K, p->k_strideB, p->k_strideM, p->k_strideH};
+        d.V = View4{p->V, p->v_strideB, p->v_strideM, p->v_strideH};
+        d.O = p->O; d.LSE = p->LSE;
+        d.o_sB = p->o_strideB; d.o_sM = p->o_strideM; d.o_sH = p->o_strideH;
+        d.lse_sB = p->lse_strideB; d.lse_sH = p->lse_strideH;
+        d.H = H; d.BH = BH; d.Tq = (int)Tq; d.Tk = (int)Tk;
+        d.q_pos0 = (int)p->q_pos0; d.k_pos0 = (int)p->k_pos0;
+        d.scale_log2e = p->scale * LOG2E;
+        d.causal = p->is_causal ? 1 : 0;
+        return launch_attn_decode(d, stream);
+    }
     CUtensorMap mq, mk, mv;
     if ((rc = make_tile_map(&mq, p->Q, HEAD_DIM, B, H, Tq, p->q_strideB, p->q_strideM, p->q_strideH, TILE, false, true))) return rc;
     if ((rc = make_tile_map(&mk, p->K, HEAD_DIM, B, H, Tk, p->k_strideB, p->k_strideM, p->k_strideH, TILE, false, true))) return rc;

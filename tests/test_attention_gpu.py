@@ -840,3 +840,19 @@ def test_bounded_wait_reports_timeout_and_context_survives():
     ok_status()
     O_ref, _ = ol.attn_forward_mt(host(Q), host(K), host(V), SCALE, 1)
     gate("O", host(O), O_ref)
+
+
+@pytest.mark.parametrize("Tq,Tk,causal", [(1, 128, 1), (2, 129, 1), (1, 1000, 0), (2, 2047, 1), (3, 300, 1), (1, 4100, 1)])
+def test_few_queries_against_a_cache(Tq, Tk, causal):
+    """One or two query rows run in the decode kernel, three in the tensor-core one: run boundaries of the key splits,
+    keys that only the last row sees, rows that see no key (k_pos0 beyond them)."""
+    B, H = 2, 3
+    q = normal((B, H, Tq, 64), 930)
+    k, v = normal((B, H, Tk, 64), 931), normal((B, H, Tk, 64), 932)
+    for q_pos0, k_pos0 in ((Tk - Tq, 0), (Tk // 2, 0), (5, 6)) if causal else ((0, 0),):
+        O_ref, L_ref = ol.attn_forward_mt(q, k, v, SCALE, causal, q_pos0=q_pos0, k_pos0=k_pos0)
+        O, LSE = hk.attention_forward(dev(q), dev(k), dev(v), SCALE, causal, q_pos0=q_pos0, k_pos0=k_pos0)
+        ok_status()
+        gate("O", host(O), O_ref)
+        L, seen = host(LSE), np.isfinite(L_ref)
+        assert np.array_equal(np.isfinite(L), seen) and (not seen.any() or np.abs(L[seen] - L_ref[seen]).max() <= 2e-3)
