@@ -155,10 +155,10 @@ class HostAttentionStep:
             with torch.cuda.stream(self.s_out):
                 self.s_out.wait_event(self.ev_cmp[i])
                 hO[sl].copy_(d["O"], non_blocking=True)
-                hLSE[sl].copy_(d["LSE"], non_blocking=True)
                 hdQ[sl].copy_(d["dQ"], non_blocking=True)
                 hdK[sl].copy_(d["dK"], non_blocking=True)
                 hdV[sl].copy_(d["dV"], non_blocking=True)
+                hLSE[sl].copy_(d["LSE"], non_blocking=True)
                 self.ev_out[i].record(self.s_out)
         cur.wait_event(self.ev_out[self.chunks - 1])
         cur.wait_event(self.ev_cmp[self.chunks - 1])
