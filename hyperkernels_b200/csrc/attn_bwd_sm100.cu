@@ -108,19 +108,6 @@ constexpr int OFF_SH = 7 * TILE_BYTES;
 constexpr int SMEM_BYTES = OFF_SH + sizeof(Shared);
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may opt in to");
 
-// Timeline slots (SM clock): role r in {0: MMA issuer, 1: compute thread 0}, iteration it, phase ph:
-// buffer[1 + (it * 2 + r) * 8 + ph]; buffer[0] = number of iterations of the recorded CTA.
-#ifdef HK_TIMELINE
-// fixed-cost stamps of the recorded CTA: buffer[3900 + k]
-#define HK_XSTAMP(on, k) do { if (on) a.timeline[3900 + (k)] = clock64(); } while (0)
-__device__ __forceinline__ void stamp(const BwdArgs& a, bool on, int it, int role, int ph) {
-    if (on && it < 80) a.timeline[1 + (it * 3 + role) * 16 + ph] = clock64();
-}
-#else
-__device__ __forceinline__ void stamp(const BwdArgs&, bool, int, int, int) {}
-#define HK_XSTAMP(on, k)
-#endif
-
 enum WaitId {
     W_KVFULL = 201, W_QKFULL, W_QKEMPTY, W_QMFULL, W_QMFREE, W_SFULL, W_PREADY, W_BDONE, W_DSREADY, W_DQFULL, W_DQEMPTY,
     W_STAGED, W_DQSTAGED, W_ACCSTAGED, W_VREADY, W_DVDONE, W_DQOUT
@@ -138,22 +125,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const BwdArgs a) {
     using namespace bwd;
     extern __shared__ __align__(1024) uint8_t smem[];
-    // schedule trace (timeline_block < 0): {start ns, end ns, SM id, query tiles} of each of the first 1024 CTAs
-#ifdef HK_TIMELINE
-    const bool trace = a.timeline != nullptr && a.timeline_block < 0 && blockIdx.x < 1024 && threadIdx.x == 0;
-#else
-    constexpr bool trace = false;
-#endif
-    if (trace) {
-        a.timeline[4 * blockIdx.x] = (long long)globaltimer_ns();
-        a.timeline[4 * blockIdx.x + 2] = clock64();
-    }
-#ifdef HK_TIMELINE
-    const bool tlx = a.timeline != nullptr && (int)blockIdx.x == a.timeline_block && threadIdx.x == 0;
-#else
-    constexpr bool tlx = false;
-#endif
-    HK_XSTAMP(tlx, 0);
     if ((smem_u32(smem) & 1023u) != 0) {  // never expected; refuse to run on a misplaced buffer
         if (threadIdx.x == 0 && atomicCAS(&a.status->code, 0, 299) == 0) a.status->block = blockIdx.x;
         return;
@@ -255,13 +226,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     tc_fence_after_sync();
     const uint32_t tmem = uniform(sh.tmem_base);
     WaitCtx wc{&sh.abort_flag, a.status};
-#ifdef HK_TIMELINE
-    const bool tl = a.timeline != nullptr && (int)blockIdx.x == a.timeline_block;  // never in trace mode
-#else
-    constexpr bool tl = false;
-#endif
-    if (tl && threadIdx.x == 0) a.timeline[0] = n_it;
-    HK_XSTAMP(tlx, 1);
 
     if (warp == W_LOAD) {
         // ------------------------------ TMA producer ------------------------------
@@ -328,7 +292,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             auto wait = [&](uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
                 return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
             };
-            const bool tlm = tl && leader;
             constexpr uint32_t IDESC_ST = make_idesc_tf32(TILE, TILE, false, false);     // K-major x K-major, N = 128
             constexpr uint32_t IDESC_TS = make_idesc_tf32(TILE, HEAD_DIM, false, true);  // tmem A, MN-major B, N = 64
             constexpr uint32_t IDESC_DQ = make_idesc_tf32(TILE, HEAD_DIM, true, true);   // MN-major A and B, N = 64
@@ -362,9 +325,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             bool ok = issue_st(0) && issue_dp(0);
             for (int it = 0; ok && it < n_it; ++it) {
                 const uint32_t par = it & 1;
-                stamp(a, tlm, it, 0, 0);
                 if (!(ok = wait(&sh.dom_full, par, W_QMFULL, it))) break;
-                stamp(a, tlm, it, 0, 1);
                 // dV += P^T dO
                 if (!(ok = wait(&sh.pt_ready, par, W_PREADY, it))) break;
                 tc_fence_after_sync();
@@ -373,10 +334,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     umma_ts_tf32_lead(leader, tmem + COL_DV, tmem + COL_S + kk * 8, mnmajor_desc(dom_addr, kk, BOX_BYTES), IDESC_TS,
                                       (it > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_lead(leader, &sh.dv_done);  // MN-major dO consumed: two of the dS boxes may be staged over it
-                stamp(a, tlm, it, 0, 2);
                 // next tile's S^T: P^T of this tile was consumed by the MMAs just issued
                 if (it + 1 < n_it && !(ok = issue_st(it + 1))) break;
-                stamp(a, tlm, it, 0, 3);
                 if (!(ok = wait(&sh.qm_full, par, W_QMFULL, 1000 + it))) break;
                 // dK += dS^T Q
                 if (!(ok = wait(&sh.p_ready, par, W_PREADY, 1000 + it))) break;
@@ -388,40 +347,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 umma_commit_lead(leader, &sh.dk_done);  // MN-major Q consumed
                 // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
                 if (it + 1 < n_it && !(ok = issue_dp(it + 1))) break;
-                stamp(a, tlm, it, 0, 4);
                 // dQ = dS K once dS is staged (shortly after dS^T was stored) and the previous dQ has left tensor memory
                 if (!(ok = wait(&sh.ds_ready, par, W_DSREADY, it))) break;
                 if (it > 0 && !(ok = wait(&sh.dq_empty, (it - 1) & 1, W_DQEMPTY, it))) break;
                 if (it == 0 && !(ok = wait(&sh.km_full, 0, W_KVFULL, 2))) break;
-                stamp(a, tlm, it, 0, 5);
                 tc_fence_after_sync();
 #pragma unroll
                 for (int kk = 0; kk < TILE / 8; ++kk)
                     umma_ss_tf32_lead(leader, tmem + COL_DQ, mnmajor_desc(ds_addr, kk, BOX_BYTES),
                                       mnmajor_desc(km_addr, kk, BOX_BYTES), IDESC_DQ, kk > 0);
                 umma_commit_lead(leader, &sh.dq_full);  // also: the dS staging area is free again
-                stamp(a, tlm, it, 0, 6);
-                stamp(a, tlm, it, 0, 7);
             }
         }
     } else if (warp == W_STORE) {
-#ifdef HK_TIMELINE
-        // completion monitor (development builds): when each product of a tile is done
-        if (lane == 1 && tl) {
-            bool mok = true;
-            for (int it = 0; mok && it < n_it; ++it) {
-                if ((mok = mbar_wait(wc, &sh.dv_done, it & 1, 990, it))) stamp(a, true, it, 2, 0);
-                if (mok && it + 1 < n_it && (mok = mbar_wait(wc, &sh.s_full, (it + 1) & 1, 991, it))) stamp(a, true, it, 2, 1);
-                if (mok && (mok = mbar_wait(wc, &sh.dk_done, it & 1, 992, it))) stamp(a, true, it, 2, 2);
-                if (mok && it + 1 < n_it && (mok = mbar_wait(wc, &sh.dp_full, (it + 1) & 1, 993, it))) stamp(a, true, it, 2, 3);
-                if (mok && (mok = mbar_wait(wc, &sh.dq_full, it & 1, 994, it))) stamp(a, true, it, 2, 4);
-            }
-        }
-#endif
         // ------------------------------ store warp ------------------------------
         // Everything that leaves the CTA: the staged dQ tiles (bulk reductions) and, at the end, dV and dK (bulk
         // stores).  A thread of its own, so that a reduction is issued the moment its tile is staged.
         if (lane == 0 && n_it > 0) {
+            pdl_wait();
             tma_prefetch_desc(&mapdK);
             tma_prefetch_desc(&mapdV);
             tma_prefetch_desc(&mapdQ);
@@ -464,7 +407,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             }
             // the copies have read their shared-memory sources; they complete on their own
             bulk_wait_group_read_all();
-            HK_XSTAMP(tl, 8);
         }
     } else {
         // ------------------------------ compute ------------------------------
@@ -480,10 +422,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const float* d_bh = a.D + (int64_t)b * a.d_sB + (int64_t)h * a.d_sH;
         bool ok = true;
         uint32_t rs[32], rp[32];
-#ifndef HK_TL_TID
-#define HK_TL_TID 0  // compute thread whose phases a -DHK_TIMELINE build records
-#endif
-        const bool tlc = tl && tid == HK_TL_TID;
         // -LSE * log2e (threads 0..127; -inf past the end and for a fully dropped row, so that every p is 0) or
         // -D * scale (threads 128..255) of query row q0 + (tid & 127): negated, so that both enter as FMA addends
         auto fetch_lse_or_d = [&](int q0) -> float {
@@ -495,6 +433,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             }
             return (q < a.Tq) ? -__ldg(d_bh + q) * a.scale : 0.f;
         };
+        pdl_wait();  // D, and the zeroed dQ the store warp adds to
         float staged_val = (tid < 2 * TILE && n_it > 0) ? fetch_lse_or_d(it0 * TILE) : 0.f;
 
         // dQ of query tile j out of tensor memory into the K-major dO tile (column groups 2 and 3 only: this thread's
@@ -524,7 +463,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // columns, read from the 128-byte-swizzled landing buffer (16-byte chunk c of row r at position c ^ (r & 7))
         if (n_it > 0) {
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.v_full, 0, W_KVFULL, 3));
-            HK_XSTAMP(tlx, 2);
             if (ok) {
                 uint32_t rv[16];
                 const uint8_t* vrow = sV + (part >> 1) * BOX_BYTES + row * 128;
@@ -538,12 +476,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tc_fence_before_sync();
                 mbar_arrive_warp(&sh.v_ready, lane);
             }
-            HK_XSTAMP(tlx, 3);
         }
 
         for (int it = 0; ok && it < n_it; ++it) {
             const int q0 = (it0 + it) * TILE;
-            stamp(a, tlc, it, 1, 0);
             // stage LSE (threads 0..127) and D (threads 128..255) of this query tile into buffer it & 1.
             // The buffer was last read two tiles ago; every compute thread passed that tile's ds_ready
             // arrival long before this thread could get here (it has since waited on dq_full or s_full
@@ -561,14 +497,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // winding down after a failed wait cannot strand warps at a barrier
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.staged, it & 1, W_STAGED, it));
             if (!ok) break;
-            stamp(a, tlc, it, 1, 1);
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, it & 1, W_SFULL, it));
             if (!ok) break;
-            stamp(a, tlc, it, 1, 2);
             tc_fence_after_sync();
 
             tmem_ld32(trow + COL_S + c0, rs);
-            stamp(a, tlc, it, 1, 8);
 
             // first query column (local to the tile) this key row is visible to
             int cmin = 0;
@@ -621,7 +554,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // pairs whose p is zero: hidden ones, and dropped ones unless the dropout is the inverted kind
             const uint32_t live = DROP != 0 && a.drop_scaled ? vis : keep;
             tmem_wait_ld();
-            stamp(a, tlc, it, 1, 9);
 
             // p = exp2(s*scale*log2e - LSE*log2e) needs S^T only: dP^T is still being computed.  Two scores per
             // packed FMA (fma.rn.f32x2 gives the same bits as two scalar FMAs).
@@ -646,7 +578,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                         if (!((live >> i) & 1u)) rs[i] = 0u;
                 }
             }
-            stamp(a, tlc, it, 1, 10);
             // P^T goes to tensor memory at once (rounded; a pair dropped by inverted dropout counts as zero in dV but
             // keeps its p for dS below): dV += P^T dO and, behind it, the next tile's S^T run while dS is computed,
             // and the store has drained by the time its first reader starts.  rp is free until dP^T is loaded.
@@ -666,12 +597,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             }
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, it & 1, W_SFULL, 1000 + it));
             if (!ok) break;
-            stamp(a, tlc, it, 1, 11);
             tc_fence_after_sync();
             if (it > 0 && part >= 2 && !(ok = drain_dq(it - 1, rp))) break;  // rp is free until dP^T is loaded
             tmem_ld32(trow + COL_DP + c0, rp);
             tmem_wait_ld();
-            stamp(a, tlc, it, 1, 3);
 
             // dS = p * (dP*scale - D*scale), two elements per packed instruction
             {
@@ -699,14 +628,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     }
                 }
             }
-            stamp(a, tlc, it, 1, 4);
             tmem_st32(trow + COL_DP + c0, rp);
-            stamp(a, tlc, it, 1, 12);
             tmem_wait_st();
-            stamp(a, tlc, it, 1, 13);
             tc_fence_before_sync();
             mbar_arrive_warp(&sh.p_ready, lane);
-            stamp(a, tlc, it, 1, 5);
 
             // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns
             // 32*part..32*part+31, one 128-byte row per key row, 32-byte chunks XOR-swizzled with (row & 3).  Boxes 0, 1
@@ -720,7 +645,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, it & 1, W_DVDONE, it));
             }
             if (!ok) break;
-            stamp(a, tlc, it, 1, 6);
             {
                 // Rows r and r + 4 share a 32-byte chunk position; they store its two halves in opposite order so
                 // that the eight lanes of a quarter-warp hit eight different 16-byte bank groups.
@@ -737,16 +661,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             }
             fence_proxy_async_smem();
             mbar_arrive_warp(&sh.ds_ready, lane);
-            stamp(a, tlc, it, 1, 7);
         }
 
         // dV and dK of this KV tile are complete once dK of the last query tile is (dV precedes it on the tensor
         // pipe).  Column groups 0,1 put dV (times 1/(1-p) for inverted dropout) into the MN-major Q tile and groups
         // 2,3 dK into the K-major K tile, both dead by then, as the boxes of a 128-byte-swizzled TMA tile: 16-byte
         // chunk c of row r at position c ^ (r & 7).
-        HK_XSTAMP(tlx, 4);
         if (ok && n_it > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dk_done, (n_it - 1) & 1, W_BDONE, n_it));
-        HK_XSTAMP(tlx, 5);
         if (ok && n_it > 0) {
             tc_fence_after_sync();
             tmem_ld32(trow + ((part < 2) ? COL_DV + part * 32 : COL_DK + (part - 2) * 32), rs);
@@ -760,7 +681,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                                 __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
             fence_proxy_async_smem();
             mbar_arrive_warp(&sh.acc_staged, lane);
-            HK_XSTAMP(tlx, 6);
         } else if (n_it == 0 && kv_ok && !a.accum_dkdv) {
             // no query sees this KV tile: its dK and dV rows are zero
             float* out_row = (part < 2)
@@ -777,7 +697,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (ok && n_it > 0 && part >= 2) {
             if (n_it > 1) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_out, (n_it - 2) & 1, W_DQOUT, n_it - 2));
             if (ok) ok = drain_dq(n_it - 1, rs);
-            HK_XSTAMP(tl && tid == 256, 9);
         }
 
     }
@@ -785,20 +704,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     // ------------------------------ teardown ------------------------------
     tc_fence_before_sync();
     __syncthreads();
-    HK_XSTAMP(tlx, 7);
     if (warp == W_MMA) {
         __syncwarp();
         tc_fence_after_sync();
         tmem_dealloc(tmem, TMEM_COLS);
     }
-    if (trace) {
-        a.timeline[4 * blockIdx.x + 1] = (long long)globaltimer_ns();
-        a.timeline[4 * blockIdx.x + 2] = smid() | ((clock64() - a.timeline[4 * blockIdx.x + 2]) << 10);  // SM id, SM cycles
-        a.timeline[4 * blockIdx.x + 3] = n_it;
-    }
 }
 
-int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream) {
+int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, bool after_prepass, cudaStream_t stream) {
     typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
                            CUtensorMap, CUtensorMap, BwdArgs);
     static const Kernel kernels[3] = {attn_bwd_kernel<0>, attn_bwd_kernel<1>, attn_bwd_kernel<2>};
@@ -817,11 +730,12 @@ int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream) {
     const long long nblocks = (long long)a.n_kvtiles * a.BH;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_BWD, true, stream);
-    kernels[a.dropout_mode]<<<(unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream>>>(m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
-                                                                                              m.dO_mn, m.dQ, m.dK, m.dV, a);
+    LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, 1, after_prepass);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
+                                              m.dK, m.dV, a);
     timing_mark(TIMED_BWD, false, stream);
     count_launch();
-    return check_launch();
+    return rc == cudaSuccess ? HK_OK : check_launch();
 }
 
 }  // namespace hk

@@ -54,4 +54,29 @@ enum TimedKernel { TIMED_FWD = 0, TIMED_BWD = 1, TIMED_KINDS = 2 };
 void timing_mark(int kind, bool begin, cudaStream_t stream);
 int check_launch();  // cudaGetLastError -> hk_status
 
+// Launch attributes of this library's kernels: cluster size (1: none) and programmatic dependent launch (sm100_ptx.cuh).
+struct LaunchConfig {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    LaunchConfig(unsigned blocks, unsigned threads, size_t smem, cudaStream_t stream, int cluster, bool dependent) {
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        if (cluster > 1) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+            attr[cfg.numAttrs].val.clusterDim.x = cluster;
+            attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+            ++cfg.numAttrs;
+        }
+        if (dependent) {
+            attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+            ++cfg.numAttrs;
+        }
+    }
+    LaunchConfig(const LaunchConfig&) = delete;
+};
+
 }  // namespace hk

@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(WARPS * 32, (NQ == 1 ? 24 : 16) / WARPS) attn_
     const int ns = a.n_splits, split = ns > 1 ? (int)cluster_ctarank() : 0;
     const int bh = blockIdx.x / ns, b = bh / a.H, h = bh - b * a.H;
 
+    pdl_wait();
+    pdl_trigger();
     // keys any row of the call may see, and this CTA's run of them
     long long n_ll = a.Tk;
     if (a.causal) n_ll = max(0ll, min(n_ll, (long long)a.q_pos0 + a.Tq - a.k_pos0));
@@ -180,19 +182,9 @@ int launch_attn_decode(DecodeArgs a, cudaStream_t stream) {
     while (a.n_splits > 1 && (long long)a.n_splits * warps * batch > a.Tk) a.n_splits /= 2;
     const long long blocks = (long long)a.BH * a.n_splits;
     if (blocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.n_splits;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(warps * 32);
-    cfg.dynamicSmemBytes = warps * sizeof(dec::Partial);
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = a.n_splits > 1 ? 1 : 0;
+    LaunchConfig lc((unsigned)blocks, warps * 32, warps * sizeof(dec::Partial), stream, a.n_splits, true);
     timing_mark(TIMED_FWD, true, stream);
-    const cudaError_t rc = cudaLaunchKernelEx(&cfg, k, a);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, k, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();

@@ -168,6 +168,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         for (int i = 0; i < 2; ++i) mbar_init(&sh.q_full[i], 1);
         for (int s = 0; s < SLOTS; ++s) mbar_init(&sh.kv_full[s], 1);
         fence_mbar_init();
+        pdl_wait();  // whatever made Q, K, V
+        pdl_trigger();
         if (nk > 0) {
             if (n0 > 0) load_q(0);
             load_kv(0);
@@ -341,6 +343,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     } else {
         // ------------------------------ softmax ------------------------------
         reg_acquire();
+        pdl_wait();  // these warps write the outputs, which an earlier kernel may still be using
         const int t = (warp - 4) >> 2;                   // stream
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;             // row inside the product = tensor-memory lane
@@ -636,19 +639,6 @@ struct FwdDevice {
 };
 typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
 
-cudaLaunchConfig_t fwd_config(unsigned blocks, int ns, cudaStream_t stream, cudaLaunchAttribute* attr) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ns;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(fwd::NUM_THREADS);
-    cfg.dynamicSmemBytes = fwd::SMEM_BYTES;
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = ns > 1 ? 1 : 0;
-    return cfg;
-}
 }  // namespace
 
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
@@ -664,10 +654,9 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
             if (d.rc == cudaSuccess)
                 d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM_BYTES);
         for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
-            cudaLaunchAttribute attr[1];
-            const cudaLaunchConfig_t cfg = fwd_config(8u << i, 1 << i, nullptr, attr);
+            LaunchConfig lc(8u << i, fwd::NUM_THREADS, fwd::SMEM_BYTES, nullptr, 1 << i, false);
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernels[0], &cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+            if (cudaOccupancyMaxActiveClusters(&n, kernels[0], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
         }
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
@@ -713,9 +702,8 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     const long long nblocks = blocks * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);
-    cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = fwd_config((unsigned)nblocks, a.n_splits, stream, attr);
-    const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernels[a.dropout_mode], mq, mk, mv, mo, a);
+    LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();

@@ -74,8 +74,6 @@ struct BwdArgs {
     uint32_t bh_pos0;  // added to the local (batch, head) index in the Philox counter
     uint64_t seed, offset;
     DeviceStatus* status;
-    long long* timeline;  // per-phase SM clock stamps of one CTA; only builds with -DHK_TIMELINE read it
-    int timeline_block;
 };
 
 // K-major maps (16-byte-chunk swizzle) of Q, K, V, dO and MN-major maps
@@ -86,7 +84,9 @@ struct BwdMaps {
     CUtensorMap q, k, v, dO, q_mn, k_mn, dO_mn, dQ, dK, dV;
 };
 
-int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, cudaStream_t stream);
+// after_prepass: the launch before it in the stream is this call's D pre-pass, the only kernel whose results it waits for
+// itself (Q, K, V and dO are complete when the pre-pass lets it start)
+int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, bool after_prepass, cudaStream_t stream);
 
 // What hk_attn_forward / hk_attn_backward run.  check_scratch: ask for the workspace the C ABI documents; without it the
 // forward takes none and `workspace` of a deterministic backward holds the slabs of partial dQ alone.

@@ -60,6 +60,8 @@ constexpr int ROWS_PER_BLOCK = 64;  // 256 threads: 16 lanes per row, four rows 
 // kernels_test.cu:562).  HBM-bound: a lane issues the eight loads of its four rows before it uses the first.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) precompute_D_kernel(const DJob j, uint32_t nrows) {
+    pdl_wait();     // O comes from the forward
+    pdl_trigger();  // the backward sets itself up and loads its first tiles meanwhile
     const int sub = threadIdx.x & 15;
     const uint32_t row0 = blockIdx.x * ROWS_PER_BLOCK + (threadIdx.x >> 4);
     float4 g[4], o[4];
@@ -92,7 +94,8 @@ int launch_precompute_D(const DJob& job, cudaStream_t stream) {
         j.D += b * j.d_sB;
         if (j.dQ_zero) j.dQ_zero += b * j.dq_sB;
         const uint32_t nrows = (uint32_t)std::min(step, B - b) * j.H * j.T;
-        precompute_D_kernel<<<(nrows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 256, 0, stream>>>(j, nrows);
+        LaunchConfig lc((nrows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK, 256, 0, stream, 1, true);
+        if (cudaLaunchKernelEx(&lc.cfg, precompute_D_kernel, j, nrows) != cudaSuccess) return check_launch();
         count_launch();
     }
     return check_launch();

@@ -110,10 +110,6 @@ int make_tile_map(CUtensorMap* map, const float* ptr, int inner, int B, int H, i
     return r == CUDA_SUCCESS ? HK_OK : HK_ERR_CUDA;
 }
 
-// ---- optional phase timeline of one CTA (performance debugging) ------------------
-static std::atomic<long long*> g_timeline{nullptr};
-static std::atomic<int> g_timeline_block{0};
-
 // ---- validation helpers -------------------------------------------------------
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 static inline bool stride_ok(int64_t s) { return s >= 0 && (s % 4) == 0; }
@@ -341,9 +337,7 @@ int attn_backward(const hk_attn_bwd_params& pr, cudaStream_t stream, bool check_
     a.seed = p->dropout_seed; a.offset = p->dropout_offset; a.bh_pos0 = p->bh_pos0;
     a.status = device_status_ptr();
     if (!a.status) return HK_ERR_CUDA;
-    a.timeline = g_timeline.load();
-    a.timeline_block = g_timeline_block.load();
-    if ((rc = launch_attn_bwd(m, a, stream))) return rc;
+    if ((rc = launch_attn_bwd(m, a, !d_given, stream))) return rc;
     if (det_dq) {
         DqReduceJob r{};
         r.slabs = dq_slabs; r.dQ = p->dQ;
@@ -542,15 +536,5 @@ int hk_attn_round_tf32(const float* src, float* dst, int64_t rows, void* stream_
     if (!aligned16(src) || !aligned16(dst)) return HK_ERR_MISALIGNED;
     return launch_round_tf32(src, dst, rows, static_cast<cudaStream_t>(stream_));
 }
-
-#ifdef HK_TIMELINE
-// Development builds only: CTA `block` of every forward/backward launch writes SM-clock stamps of its pipeline
-// phases into device_buffer (4096 int64; slot layout in attn_*_sm100.cu); block = -1: every CTA b < 1024 writes
-// {start ns, end ns, SM id, tiles} to slots 4b..4b+3.  nullptr turns it off.
-void hk_attn_debug_timeline(long long* device_buffer, int block) {
-    g_timeline_block.store(block);
-    g_timeline.store(device_buffer);
-}
-#endif
 
 }  // extern "C"

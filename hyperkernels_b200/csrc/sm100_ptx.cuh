@@ -471,6 +471,16 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------------
+// A kernel launched with the attribute may start once every CTA of the one before it in the stream has triggered (or
+// ended): its set-up then runs beside the predecessor's last CTAs.  pdl_wait returns when the predecessor is complete and
+// its writes are visible; nothing the predecessor may have written is read, and nothing at all written, before it.  A
+// kernel triggers only after its own pdl_wait, so that what precedes IT is complete too when its successor starts.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // thread-block clusters
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
