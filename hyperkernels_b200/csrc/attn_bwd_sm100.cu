@@ -523,7 +523,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 uint32_t mine = 0u;  // bit 8m + u: query column c0 + 8m + j8, key row (row & ~7) + u
 #pragma unroll
                 for (int mI = 0; mI < 4; ++mI) {
-                    const hk_philox4_t w = hk_philox_row8(a.seed, a.offset, a.bh_pos0 + (uint32_t)bh,
+                    const hk_philox4_t w = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
                                                           (uint32_t)(a.q_pos0 + q0 + c0 + 8 * mI + j8), kgrp);
                     mine |= hk_philox_keep8(w, a.drop_thr) << (8 * mI);
                 }

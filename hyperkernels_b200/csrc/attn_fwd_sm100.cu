@@ -494,7 +494,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
                             for (int g = 4 * q4; g < 4 * q4 + 4; ++g) {
                                 const uint32_t kpos = (uint32_t)(a.k_pos0 + kv0 + g * 8);
-                                const hk_philox4_t w = hk_philox_row8(a.seed, a.offset, a.bh_pos0 + (uint32_t)bh,
+                                const hk_philox4_t w = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
                                                                       (uint32_t)(a.q_pos0 + qrow), kpos >> 3);
 #pragma unroll
                                 for (int u = 0; u < 8; u += 2) {

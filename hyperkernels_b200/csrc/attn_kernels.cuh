@@ -1,6 +1,7 @@
 // attn_kernels.cuh -- argument blocks and launchers of the two tensor-core kernels.
 #pragma once
 #include "attn_common.cuh"
+#include "philox.h"
 
 namespace hk {
 
@@ -24,7 +25,8 @@ struct FwdArgs {
     float keep_scale;  // 1/(1-p) when drop_scaled, else 1
     uint32_t drop_thr;
     uint32_t bh_pos0;  // added to the local (batch, head) index in the Philox counter
-    uint64_t seed, offset;
+    hk_philox_keys_t philox_keys;
+    uint32_t philox_offset;
     DeviceStatus* status;
 };
 
@@ -72,7 +74,8 @@ struct BwdArgs {
     float dv_scale;    // factor of the dV accumulator: 1/(1-p) when drop_scaled, else 1
     uint32_t drop_thr;
     uint32_t bh_pos0;  // added to the local (batch, head) index in the Philox counter
-    uint64_t seed, offset;
+    hk_philox_keys_t philox_keys;
+    uint32_t philox_offset;
     DeviceStatus* status;
 };
 

@@ -227,7 +227,9 @@ int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_s
     a.continue_state = (p->flags & HK_FLAG_CONTINUE_SOFTMAX_STATE) ? 1 : 0;
     if (a.continue_state && a.drop_scaled) return HK_ERR_UNSUPPORTED;
     a.drop_thr = hk_philox_threshold(p->dropout_p);
-    a.seed = p->dropout_seed; a.offset = p->dropout_offset; a.bh_pos0 = p->bh_pos0;
+    a.philox_keys = hk_philox_keys(p->dropout_seed, p->dropout_offset);
+    a.philox_offset = (uint32_t)p->dropout_offset;
+    a.bh_pos0 = p->bh_pos0;
     a.status = device_status_ptr();
     if (!a.status) return HK_ERR_CUDA;
     CUtensorMap mo;
@@ -334,7 +336,9 @@ int attn_backward(const hk_attn_bwd_params& pr, cudaStream_t stream, bool check_
     a.dv_scale = keep_scale_of(p->dropout_p, mode, p->flags);
     a.dp_scale = p->scale * a.dv_scale;
     a.drop_thr = hk_philox_threshold(p->dropout_p);
-    a.seed = p->dropout_seed; a.offset = p->dropout_offset; a.bh_pos0 = p->bh_pos0;
+    a.philox_keys = hk_philox_keys(p->dropout_seed, p->dropout_offset);
+    a.philox_offset = (uint32_t)p->dropout_offset;
+    a.bh_pos0 = p->bh_pos0;
     a.status = device_status_ptr();
     if (!a.status) return HK_ERR_CUDA;
     if ((rc = launch_attn_bwd(m, a, !d_given, stream))) return rc;

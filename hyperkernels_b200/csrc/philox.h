@@ -64,6 +64,34 @@ HK_HD hk_philox4_t hk_philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint3
     return out;
 }
 
+/* The key of every round, which the kernels take from their argument block: 20 additions per call less. */
+typedef struct { uint32_t k0[10], k1[10]; } hk_philox_keys_t;
+HK_HD hk_philox_keys_t hk_philox_keys(uint64_t seed, uint64_t offset) {
+    hk_philox_keys_t k;
+    for (int r = 0; r < 10; ++r) {
+        k.k0[r] = (uint32_t)seed + (uint32_t)r * HK_PHILOX_W0;
+        k.k1[r] = ((uint32_t)(seed >> 32) ^ (uint32_t)(offset >> 32)) + (uint32_t)r * HK_PHILOX_W1;
+    }
+    return k;
+}
+#if defined(__CUDACC__)
+__device__ __forceinline__ hk_philox4_t hk_philox_row8_keys(const hk_philox_keys_t& k, uint32_t offset, uint32_t bh, uint32_t qi,
+                                                            uint32_t kj8) {
+    uint32_t c0 = kj8, c1 = qi, c2 = bh, c3 = offset;
+#pragma unroll
+    for (int r = 0; r < 10; ++r) {
+        uint32_t hi0, lo0, hi1, lo1;
+        hk_mulhilo32(HK_PHILOX_M0, c0, &hi0, &lo0);
+        hk_mulhilo32(HK_PHILOX_M1, c2, &hi1, &lo1);
+        const uint32_t n0 = hi1 ^ c1 ^ k.k0[r], n2 = hi0 ^ c3 ^ k.k1[r];
+        c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
+    }
+    hk_philox4_t out;
+    out.v[0] = c0; out.v[1] = c1; out.v[2] = c2; out.v[3] = c3;
+    return out;
+}
+#endif
+
 /* floor(p * 2^16), in [0, 65535]; p in [0,1). */
 HK_HD uint32_t hk_philox_threshold(float p) {
     double t = (double)p * 65536.0;
