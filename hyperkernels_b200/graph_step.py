@@ -35,12 +35,12 @@ class GraphedAttentionStep:
         Tk = K.shape[2]
         dev = Q.device
         self.Q, self.K, self.V, self.dO = Q, K, V, dO
-        self.O = torch.empty((B, H, T, 64), dtype=torch.float32, device=dev)
-        self.dQ = torch.empty((B, H, T, 64), dtype=torch.float32, device=dev)
-        self.dK = torch.empty((B, H, Tk, 64), dtype=torch.float32, device=dev)
-        self.dV = torch.empty((B, H, Tk, 64), dtype=torch.float32, device=dev)
-        self.LSE = torch.empty((B, H, T), dtype=torch.float32, device=dev)
-        self.D = torch.empty((B, H, T), dtype=torch.float32, device=dev)
+        # one allocation for everything the step writes
+        rows_q, rows_k = B * H * T, B * H * Tk
+        flat = torch.empty(2 * (rows_q + rows_k) * 64 + 2 * rows_q, dtype=torch.float32, device=dev)
+        self.O, self.dQ, self.dK, self.dV, self.LSE, self.D = (
+            x.view(shape) for x, shape in zip(flat.split([rows_q * 64] * 2 + [rows_k * 64] * 2 + [rows_q] * 2),
+                                              [(B, H, T, 64)] * 2 + [(B, H, Tk, 64)] * 2 + [(B, H, T)] * 2))
         drop = {}
         if dropout_p > 0:
             if philox_seed is None:
