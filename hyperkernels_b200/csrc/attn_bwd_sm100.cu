@@ -32,18 +32,17 @@
 // of them into shared memory twice, once per swizzle.
 //
 // Tensor-pipe order per query tile i:
-//     dV(i) | S^T(i+1) | dK(i) | dP^T(i+1) | dQ(i)
+//     dV(i) | S^T(i+1) | dK(i) | dQ(i) | dP^T(i+1)
 // dV(i) starts as soon as P^T(i) is in tensor memory, i.e. before the compute
 // warps have formed dS(i); dK(i) follows when dS^T(i) is there, dQ(i) when dS(i)
 // is staged in shared memory.
 // S^T(i+1) only needs the P^T columns back, i.e. dV(i); issuing it before dK(i)
 // lets the compute warps start the exponentials of tile i+1 -- the longest
-// stretch of scalar work -- while dK(i), dP^T(i+1) and dQ(i) execute.  Two of the
+// stretch of scalar work -- while dK(i), dQ(i) and dP^T(i+1) execute.  Two of the
 // four 32-column boxes of dS(i) go over the MN-major dO tile as soon as dV(i) has
-// consumed it; the other two have a buffer of their own, through which the
-// drained dQ(i-1) first leaves by bulk reduction.  No staging touches the K-major
-// Q and dO tiles, so their prefetch for tile i+1 starts as soon as S^T(i) and
-// dP^T(i) are done.  Measured tensor-pipe time of the 72 instructions of a tile:
+// consumed it, so that tile can be loaded for i+1 only when dQ(i) is done, and
+// dV(i+1) waits for it: with dQ(i) in front of dP^T(i+1) half of that load is
+// hidden (B4 H16 T2048 433 -> 388 us, H32 T8192 1 670 -> 1 500, against dQ last).  Measured tensor-pipe time of the 72 instructions of a tile:
 // about 3 050 cycles (M128 N128 K8: 74 cycles, M128 N64 K8: 36 from tensor
 // memory, 52 from shared memory).
 //
@@ -345,8 +344,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     umma_ts_tf32_lead(leader, tmem + COL_DK, tmem + COL_DP + kk * 8, mnmajor_desc(qm_addr, kk, BOX_BYTES), IDESC_TS,
                                       (it > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_lead(leader, &sh.dk_done);  // MN-major Q consumed
-                // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
-                if (it + 1 < n_it && !(ok = issue_dp(it + 1))) break;
                 // dQ = dS K once dS is staged (shortly after dS^T was stored) and the previous dQ has left tensor memory
                 if (!(ok = wait(&sh.ds_ready, par, W_DSREADY, it))) break;
                 if (it > 0 && !(ok = wait(&sh.dq_empty, (it - 1) & 1, W_DQEMPTY, it))) break;
@@ -357,6 +354,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     umma_ss_tf32_lead(leader, tmem + COL_DQ, mnmajor_desc(ds_addr, kk, BOX_BYTES),
                                       mnmajor_desc(km_addr, kk, BOX_BYTES), IDESC_DQ, kk > 0);
                 umma_commit_lead(leader, &sh.dq_full);  // also: the dS staging area is free again
+                // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
+                if (it + 1 < n_it && !(ok = issue_dp(it + 1))) break;
             }
         }
     } else if (warp == W_STORE) {
