@@ -856,3 +856,27 @@ def test_few_queries_against_a_cache(Tq, Tk, causal):
         gate("O", host(O), O_ref)
         L, seen = host(LSE), np.isfinite(L_ref)
         assert np.array_equal(np.isfinite(L), seen) and (not seen.any() or np.abs(L[seen] - L_ref[seen]).max() <= 2e-3)
+
+
+@pytest.mark.parametrize("BH,Tq,Tk,causal", [
+    (1, 3, 641, 0), (12, 3, 640, 1), (6, 129, 650, 0), (12, 129, 640, 1), (16, 257, 1000, 0), (24, 3, 700, 1),
+    (24, 257, 1000, 1), (48, 3, 4200, 0), (24, 3, 8193, 1)])
+def test_key_splits_of_short_query_blocks(BH, Tq, Tk, causal):
+    """Few queries against many keys: 2, 4, 8 key splits of one and of two blocks of 128 rows, and the even / odd key tiles
+    of one block, each plain, with the Philox mask and continued from the state of the first keys."""
+    q, k, v = normal((1, BH, Tq, 64), 940), normal((1, BH, Tk, 64), 941), normal((1, BH, Tk, 64), 942)
+    pos, cut = (Tk - Tq if causal else 0), 136  # the second part starts inside a key tile
+    tq, tk, tv = dev(q), dev(k), dev(v)
+    mask = ol.dropout_mask(BH, Tq, Tk, 0.25, 99, 7, q_pos0=pos)
+    for kw, m in (({}, None), (dict(dropout_p=0.25, philox_seed=99, philox_offset=7), mask)):
+        O_ref, L_ref = ol.attn_forward_mt(q, k, v, SCALE, causal, m, q_pos0=pos)
+        O, LSE = hk.attention_forward(tq, tk, tv, SCALE, bool(causal), q_pos0=pos, **kw)
+        ok_status()
+        gate("O", host(O), O_ref)
+        lse_check(host(LSE), L_ref)
+        O, LSE = hk.attention_forward(tq, tk[:, :, :cut], tv[:, :, :cut], SCALE, bool(causal), q_pos0=pos, **kw)
+        hk.attention_forward(tq, tk[:, :, cut:], tv[:, :, cut:], SCALE, bool(causal), q_pos0=pos, k_pos0=cut, out=O, lse=LSE,
+                             continue_state=True, **kw)
+        ok_status()
+        gate("O", host(O), O_ref)
+        lse_check(host(LSE), L_ref)
