@@ -8,7 +8,15 @@ step, which at these sizes is an order of magnitude more than the kernels.  The
 (batch, head) slices of the problem are independent, so this helper cuts the
 batch into chunks and runs three queues: chunk i+1 travels to the device while
 the kernels work on chunk i and the results of chunk i-1 travel back (the two
-copy directions use different DMA engines and the link is full duplex).  The
+copy directions use different DMA engines and the link is full duplex).  What
+bounds it is the link: 101 MB each way take 1.84 ms alone and 2.2 ms in both
+directions at B8 H12 T1024, to which the first chunk's way in and the last one's
+way out add.  So a chunk's forward starts when Q, K and V have arrived, beside
+the copy of dO, and its O leaves beside the backward as soon as dO is there, when
+the next chunk's Q sets out: copies that start together in the two directions
+share the link best.  2.51 against 2.71 ms with one dependency each way per chunk,
+6.4 against 7.3 at B2 H16 T8192; O leaving as soon as it is written, the forward
+waiting for dO, or LSE between O and the gradients: 2.60-2.88.  The
 chunks are runs of consecutive (batch, head) slices, so a single-batch problem
 with many heads is pipelined too; small problems (under 2 MB per tensor and
 chunk) are not cut, the extra launches would cost more than the overlap gains.
@@ -47,7 +55,7 @@ class HostAttentionStep:
         n = B * H  # independent slices; a chunk is a run of them, handed to the kernels as a batch of one-head items
         # chunk sizes in slices: by default up to eight equal chunks of at least 2 MB per tensor (every copy costs a fixed
         # ~10 us on its engine; schedules with small chunks at both ends and large ones in the middle measured slower
-        # than equal chunks: 2.92-3.02 against 2.61 ms at B8 H12 T1024)
+        # than equal chunks: both directions run at the same rate, so the largest chunk adds its time once)
         if chunks is None:
             c = next(c for c in (8, 4, 2, 1) if n % c == 0 and (c == 1 or n // c * T * 256 >= (2 << 20)))
             sizes = [n // c] * c
@@ -82,6 +90,8 @@ class HostAttentionStep:
         self.s_in, self.s_cmp, self.s_out = (torch.cuda.Stream(device=self.device) for _ in range(3))
         self.ev_start = torch.cuda.Event()
         self.ev_in = [torch.cuda.Event() for _ in range(chunks)]
+        self.ev_qkv = [torch.cuda.Event() for _ in range(chunks)]
+        self.ev_fwd = [torch.cuda.Event() for _ in range(chunks)]
         self.ev_cmp = [torch.cuda.Event() for _ in range(chunks)]
         self.ev_out = [torch.cuda.Event() for _ in range(chunks)]
         self.use_graph = bool(graph)
@@ -139,22 +149,26 @@ class HostAttentionStep:
                 d["Q"].copy_(hQ[sl], non_blocking=True)
                 d["K"].copy_(hK[sl], non_blocking=True)
                 d["V"].copy_(hV[sl], non_blocking=True)
+                self.ev_qkv[i].record(self.s_in)  # the forward can start
                 d["dO"].copy_(hdO[sl], non_blocking=True)
                 self.ev_in[i].record(self.s_in)
             with torch.cuda.stream(self.s_cmp):
-                self.s_cmp.wait_event(self.ev_in[i])
+                self.s_cmp.wait_event(self.ev_qkv[i])
                 if i >= n_slots:  # the results of the chunk that used this slot have left
                     self.s_cmp.wait_event(self.ev_out[i - n_slots])
                 drop = dict(self.drop, philox_offset=self.philox_offset, bh_pos0=self.starts[i]) if self.drop else {}
                 att.attention_forward(d["Q"], d["K"], d["V"], self.scale, self.causal, out=d["O"],
                                       lse=d["LSE"], stream=self.s_cmp, **drop)
+                self.s_cmp.wait_event(self.ev_in[i])
+                self.ev_fwd[i].record(self.s_cmp)  # the forward is done and dO has arrived: O leaves
                 att.attention_backward(d["Q"], d["K"], d["V"], d["O"], d["dO"], d["LSE"], self.scale, self.causal,
                                        D=d["D"], dQ=d["dQ"], dK=d["dK"], dV=d["dV"],
                                        stream=self.s_cmp, **drop)
                 self.ev_cmp[i].record(self.s_cmp)
             with torch.cuda.stream(self.s_out):
-                self.s_out.wait_event(self.ev_cmp[i])
+                self.s_out.wait_event(self.ev_fwd[i])
                 hO[sl].copy_(d["O"], non_blocking=True)
+                self.s_out.wait_event(self.ev_cmp[i])
                 hdQ[sl].copy_(d["dQ"], non_blocking=True)
                 hdK[sl].copy_(d["dK"], non_blocking=True)
                 hdV[sl].copy_(d["dV"], non_blocking=True)
