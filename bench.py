@@ -349,8 +349,7 @@ def run_ours(args, cfg, rank, local_rank, world):
     assert hk.last_device_status() == 0, "a bounded wait inside a kernel gave up"
 
     # the same steps issued launch by launch: forward call and backward call timed separately (bwd = everything
-    # hk_attn_backward launches: D pre-pass with dO rounding and dQ zeroing + the main kernel; fwd = the rounding
-    # pre-pass of Q, K, V + the main kernel), and the library's own events round the two tensor-core kernels
+    # hk_attn_backward launches: D pre-pass with dQ zeroing + the main kernel), and the library's own events round the two tensor-core kernels
     n_e = max(args.steps, 10)
     L.hk_attn_kernel_timing_enable(1)
     fwd_s = timed_samples(prob.forward, n_e, flush, stream, torch)
@@ -439,7 +438,7 @@ def run_ours(args, cfg, rank, local_rank, world):
             "config": {"workload": cfg["name"] + (" per GPU" if world > 1 and args.scaling == "weak" else ""),
                        "config_id": args.config,
                        "l2": "256 MiB buffer written before every timed sample (untimed)",
-                       "step": "hk_attn_forward + hk_attn_backward with every launch they make (operand rounding to TF32: in shared memory inside the kernels for 512 <= N <= 2048 causal / 1024 otherwise, else one HBM pre-pass per step; D pre-pass with dO rounding and dQ zeroing; the two main kernels), captured in a CUDA graph and replayed",
+                       "step": "hk_attn_forward + hk_attn_backward with every launch they make (operand rounding to TF32 by the TMA loads; dQ zeroing; D pre-pass; the two main kernels), captured in a CUDA graph and replayed",
                        "launches_per_step": launches_per_step,
                        "timing": f"median of {len(samples)} samples ({args.steps} steps x {inner} replays), one CUDA-event pair per replay",
                        "partition": "batch x head across GPUs, no collective"},
@@ -447,7 +446,7 @@ def run_ours(args, cfg, rank, local_rank, world):
             "pct_of_tf32_peak": total / world / (ms * 1e-3) / 1e12 / peaks["tf32_tflops"],
             "fwd_tflops": f_fwd / (ms_fwd_call * 1e-3) / 1e12, "bwd_tflops": f_bwd / (ms_bwd_call * 1e-3) / 1e12,
             "call_ms": {"hk_attn_forward": ms_fwd_call, "hk_attn_backward": ms_bwd_call,
-                        "note": "every launch of the call: fwd = Q/K/V rounding pre-pass (if the config takes the HBM path) + forward kernel; bwd = D pre-pass (dO rounding, dQ zeroing) + backward kernel"},
+                        "note": "every launch of the call: fwd = forward kernel; bwd = D pre-pass (with dQ zeroing) + backward kernel"},
             "kernel_ms": {"fwd_kernel": k_fwd, "bwd_kernel": k_bwd,
                           "fwd_kernel_tflops": f_fwd / (k_fwd * 1e-3) / 1e12 if k_fwd else None,
                           "bwd_kernel_tflops": achieved},
