@@ -46,6 +46,11 @@
 // about 3 050 cycles (M128 N128 K8: 74 cycles, M128 N64 K8: 36 from tensor
 // memory, 52 from shared memory).
 //
+// Splits: where few KV tiles have many query tiles (cross-attention of a long sequence to a short one), a cluster of 2, 4
+// or 8 CTAs shares the query tiles of a KV tile; at the end each adds up a slice of the rows of dV and dK from the partial
+// sums the others left in their shared memory (launch_attn_bwd picks the number).  B1 H4, 5 000 queries,
+// 200 keys: 107 -> 25 us; B1 H1, 16 384 and 4 096: 330 -> 100; B4 H6, 777 and 333: 26.5 -> 24.6.
+//
 //   warps 0-15  compute: four threads per key row (tensor-memory lane), each
 //               owning 32 of the 128 query columns, all held in registers so
 //               that S^T and dP^T are read from tensor memory exactly once
@@ -53,6 +58,8 @@
 //   warp 17     MMA issuer (the whole warp runs the issuing code, one elected lane
 //               issues)
 //   warp 18     TMA reductions of dQ (per query tile) and stores of dK, dV (at the end)
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "attn_kernels.cuh"
@@ -114,7 +121,9 @@ enum WaitId {
 
 }  // namespace bwd
 
-template <int DROP>  // 0 none, 1 dense mask, 2 Philox
+// DROP: 0 none, 1 dense mask, 2 Philox.  SPLIT: a cluster shares the query tiles of a KV tile (an instantiation of its own:
+// the set-up and the registers it needs cost the plain kernel 1 - 3 %).
+template <int DROP, bool SPLIT>
 __global__ void __launch_bounds__(bwd::NUM_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapdO,
@@ -142,8 +151,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int lane = threadIdx.x & 31;
 
     // early KV tiles first: under the causal mask they see the most query tiles
-    const int bh = blockIdx.x % a.BH;
-    const int kt = (int)(blockIdx.x / a.BH);
+    const int ns = SPLIT ? a.n_splits : 1;  // cluster size
+    const int split = SPLIT ? (int)cluster_ctarank() : 0;
+    const int item = (int)blockIdx.x / ns;
+    const int bh = item % a.BH;
+    const int kt = item / a.BH;
     const int b = bh / a.H;
     const int h = bh - b * a.H;
     const int kv0 = kt * TILE;
@@ -155,7 +167,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const long long first_q = (long long)kv0 + a.k_pos0 - a.q_pos0;  // smallest local q that sees key kv0
         if (first_q > 0) it0 = (int)min((long long)n_qtiles, first_q / TILE);
     }
-    const int n_it = n_qtiles - it0;
+    // With splits each CTA of the cluster takes a contiguous run of the query tiles.
+    const int n_all = n_qtiles - it0, run = (n_all + ns - 1) / ns;
+    if (SPLIT) it0 += split * run;
+    const int n_it = SPLIT ? max(0, min(run, n_all - split * run)) : n_all;
 
     // The load warp initialises the barriers its copies complete on and issues the loads of the first tile at once:
     // the other warps meet those barriers only after the __syncthreads below, and ~1 000 cycles of set-up (the other
@@ -390,7 +405,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // dK and S^T): stored -- added, if the caller accumulates -- with bulk copies; a thread-per-row store would
             // be 32 lines per instruction
             if (tok && (tok = mbar_wait(wc, &sh.acc_staged, 0, W_ACCSTAGED, 0))) {
-                if (a.accum_dkdv) {
+                if (SPLIT) {
+                    // added up over the cluster, below
+                } else if (a.accum_dkdv) {
                     tma_reduce_add_4d(&mapdV, sQm, 0, kv0, h, b);
                     tma_reduce_add_4d(&mapdV, sQm + BOX_BYTES, HALF_D, kv0, h, b);
                     tma_reduce_add_4d(&mapdK, sK, 0, kv0, h, b);
@@ -680,7 +697,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                                 __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
             fence_proxy_async_smem();
             mbar_arrive_warp(&sh.acc_staged, lane);
-        } else if (n_it == 0 && kv_ok && !a.accum_dkdv) {
+        } else if (n_it == 0 && !SPLIT && kv_ok && !a.accum_dkdv) {
             // no query sees this KV tile: its dK and dV rows are zero
             float* out_row = (part < 2)
                                  ? a.dV + (int64_t)b * a.dv_sB + (int64_t)h * a.dv_sH + (int64_t)kvrow * a.dv_sM + part * 32
@@ -700,6 +717,47 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
     }
 
+    if constexpr (SPLIT) {
+        // dV and dK of the KV tile: the sum over the splits, always in the same order, from what each left in its shared
+        // memory; each CTA adds up an equal slice of the rows, 32 threads per row (16 for dV, 16 for dK).
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (warp < W_LOAD) {
+            // (rows of this thread) x (splits) = 8: all loads first, their latency is that of the other SM's memory
+            const int live = (n_all + run - 1) / max(run, 1);  // the splits that had query tiles
+            const int ch = lane & 15;
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int row = split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
+                const uint8_t* src = (lane < 16 ? sQm : sK) + (ch >> 3) * BOX_BYTES + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+                v[u] = u % ns < live ? ld_cluster_f4(mapa(src, u % ns)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
+                if ((u + 1) % ns != 0) continue;
+                const int64_t kvrow = kv0 + split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
+                if (kvrow < a.Tk) {
+                    float* dst = lane < 16 ? a.dV + (int64_t)b * a.dv_sB + (int64_t)h * a.dv_sH + kvrow * a.dv_sM
+                                           : a.dK + (int64_t)b * a.dk_sB + (int64_t)h * a.dk_sH + kvrow * a.dk_sM;
+                    float4* out = reinterpret_cast<float4*>(dst) + ch;
+                    if (a.accum_dkdv) {
+                        const float4 old = *out;
+                        acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
+                    }
+                    *out = acc;
+                }
+                acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        __syncwarp();
+        cluster_arrive();  // the others have read this CTA's shared memory
+        cluster_wait();
+    }
+
     // ------------------------------ teardown ------------------------------
     tc_fence_before_sync();
     __syncthreads();
@@ -710,27 +768,59 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
 }
 
-int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, bool after_prepass, cudaStream_t stream) {
+// Per-device launch data: the large shared-memory opt-in and how many clusters of each size run at once.
+namespace {
+struct BwdDevice {
+    std::once_flag once;
+    cudaError_t rc = cudaSuccess;
+    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs
+};
+}  // namespace
+
+int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream) {
     typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
                            CUtensorMap, CUtensorMap, BwdArgs);
-    static const Kernel kernels[3] = {attn_bwd_kernel<0>, attn_bwd_kernel<1>, attn_bwd_kernel<2>};
-    // the opt-in to large dynamic shared memory is per device: once per device, safe from any number of host threads
-    static std::once_flag attr_once[HK_MAX_DEVICES];
-    static cudaError_t attr_rc[HK_MAX_DEVICES];
+    static const Kernel kernels[6] = {attn_bwd_kernel<0, false>, attn_bwd_kernel<1, false>, attn_bwd_kernel<2, false>,
+                                      attn_bwd_kernel<0, true>,  attn_bwd_kernel<1, true>,  attn_bwd_kernel<2, true>};
+    static BwdDevice devices[HK_MAX_DEVICES];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HK_ERR_CUDA;
     if (dev < 0 || dev >= HK_MAX_DEVICES) return HK_ERR_UNSUPPORTED;
-    std::call_once(attr_once[dev], [dev] {
+    BwdDevice& d = devices[dev];
+    std::call_once(d.once, [&d] {
         for (Kernel k : kernels)
-            if (attr_rc[dev] == cudaSuccess)
-                attr_rc[dev] = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);
+            if (d.rc == cudaSuccess)
+                d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);
+        for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
+            LaunchConfig lc(8u << i, bwd::NUM_THREADS, bwd::SMEM_BYTES, nullptr, 1 << i, false);
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kernels[3], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+        }
     });
-    if (attr_rc[dev] != cudaSuccess) return HK_ERR_CUDA;
-    const long long nblocks = (long long)a.n_kvtiles * a.BH;
+    if (d.rc != cudaSuccess) return HK_ERR_CUDA;
+    const long long tiles = (long long)a.n_kvtiles * a.BH;
+    // Splits by the same estimate of the makespan as the forward's: a CTA costs ~8 us and ~2.5 us per query tile, ~3 us
+    // more when it adds dV and dK up over a cluster.  They pay where few KV tiles have many query tiles (cross-attention of
+    // a long sequence to a short one).  The sum is taken in another order and the choice depends on batch x heads, so
+    // sequences of training length do without: a batch cut into calls gives the bits of the single call.
+    a.n_splits = 1;
+    if (a.Tq >= 2 * (long long)a.Tk) {
+        const double n_q = (a.Tq + TILE - 1) / TILE;
+        double best_cost = 0;
+        for (int i = 0; i < 4; ++i) {
+            const double one = 8.0 + (i ? 3.0 : 0.0) + 2.5 * std::ceil(n_q / (1 << i));
+            const double cost = one * std::max(1.0, tiles / (double)d.slots[i] + (tiles > d.slots[i] ? 0.5 : 0.0));
+            if (i == 0 || cost < 0.95 * best_cost) {
+                best_cost = cost;
+                a.n_splits = 1 << i;
+            }
+        }
+    }
+    const long long nblocks = tiles * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_BWD, true, stream);
-    LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, 1, after_prepass);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
+    LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
                                               m.dK, m.dV, a);
     timing_mark(TIMED_BWD, false, stream);
     count_launch();

@@ -62,6 +62,7 @@ struct BwdArgs {
     int H, BH;
     int Tq, Tk;
     int n_kvtiles;
+    int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; set by launch_attn_bwd
     int q_pos0, k_pos0;
     float scale, scale_log2e;
     int causal;
@@ -89,7 +90,7 @@ struct BwdMaps {
 
 // after_prepass: the launch before it in the stream is this call's D pre-pass, the only kernel whose results it waits for
 // itself (Q, K, V and dO are complete when the pre-pass lets it start)
-int launch_attn_bwd(const BwdMaps& m, const BwdArgs& a, bool after_prepass, cudaStream_t stream);
+int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream);
 
 // What hk_attn_forward / hk_attn_backward run.  check_scratch: ask for the workspace the C ABI documents; without it the
 // forward takes none and `workspace` of a deterministic backward holds the slabs of partial dQ alone.

@@ -880,3 +880,25 @@ def test_key_splits_of_short_query_blocks(BH, Tq, Tk, causal):
         ok_status()
         gate("O", host(O), O_ref)
         lse_check(host(LSE), L_ref)
+
+
+@pytest.mark.parametrize("BH,Tq,Tk,causal", [(1, 257, 128, 0), (8, 1024, 129, 0), (1, 4000, 40, 0), (24, 777, 333, 0), (2, 1281, 300, 1)])
+def test_query_splits_of_few_key_tiles(BH, Tq, Tk, causal):
+    """Many queries against few keys: 2, 4, 8 CTAs share the query tiles of a KV tile, splits without a tile of their own,
+    key tiles (causal, k_pos0) that few or no queries see; plain, with the Philox mask, into accumulated dK and dV."""
+    q, k, v, g = normal((1, BH, Tq, 64), 950), normal((1, BH, Tk, 64), 951), normal((1, BH, Tk, 64), 952), normal((1, BH, Tq, 64), 953)
+    k_pos0 = Tq - 200 if causal else 0
+    mask = ol.dropout_mask(BH, Tq, Tk, 0.25, 99, 7, k_pos0=k_pos0 // 8 * 8)
+    for kw, m in (({}, None), (dict(dropout_p=0.25, philox_seed=99, philox_offset=7), mask)):
+        kp = k_pos0 // 8 * 8
+        O_ref, L_ref = ol.attn_forward_mt(q, k, v, SCALE, causal, m, k_pos0=kp)
+        _, dQ_ref, dK_ref, dV_ref = ol.attn_backward_mt(q, k, v, O_ref, g, L_ref, SCALE, causal, m, k_pos0=kp)
+        args = (dev(q), dev(k), dev(v), dev(O_ref), dev(g), dev(L_ref), SCALE, bool(causal))
+        dQ, dK, dV, _ = hk.attention_backward(*args, k_pos0=kp, **kw)
+        ok_status()
+        for name, got, ref in (("dQ", dQ, dQ_ref), ("dK", dK, dK_ref), ("dV", dV, dV_ref)):
+            gate(name, host(got), ref)
+        dK2, dV2 = dK.clone(), dV.clone()
+        hk.attention_backward(*args, k_pos0=kp, dK=dK2, dV=dV2, accum_dkdv=True, **kw)
+        ok_status()
+        assert torch.equal(dK2, dK + dK) and torch.equal(dV2, dV + dV)
