@@ -18,8 +18,8 @@ share the link best.  2.51 against 2.71 ms with one dependency each way per chun
 6.4 against 7.3 at B2 H16 T8192; O leaving as soon as it is written, the forward
 waiting for dO, or LSE between O and the gradients: 2.60-2.88.  The
 chunks are runs of consecutive (batch, head) slices, so a single-batch problem
-with many heads is pipelined too; small problems (under 2 MB per tensor and
-chunk) are not cut, the extra launches would cost more than the overlap gains.
+with many heads is pipelined too; small problems are cut into fewer or not at
+all, the extra copies would cost more than the overlap gains.
 The whole step -- every copy, every launch, the dependencies between the three
 queues -- is captured in a CUDA graph the second time it is called with the same
 host tensors and replayed from then on, so the host issues one call per step.
@@ -53,11 +53,13 @@ class HostAttentionStep:
         self.torch = torch
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
         n = B * H  # independent slices; a chunk is a run of them, handed to the kernels as a batch of one-head items
-        # chunk sizes in slices: by default up to eight equal chunks of at least 2 MB per tensor (every copy costs a fixed
-        # ~10 us on its engine; schedules with small chunks at both ends and large ones in the middle measured slower
-        # than equal chunks: both directions run at the same rate, so the largest chunk adds its time once)
+        # chunk sizes in slices: by default two, four or eight equal chunks of at least 0.75, 1.25 and 2 MB per tensor.
+        # Every copy costs a fixed 4 - 10 us on its engine, so a chunk must be worth its nine (3.0 MB per tensor: 482 us
+        # in one chunk, 443 in two, 461 in four; 7.0 MB: 1 040, 900, 863; 9.4 MB: 1 095 in four, 1 190 in eight); small
+        # chunks at both ends and large ones in the middle do not pay: both directions run at the same rate, so the
+        # largest chunk adds its time once.
         if chunks is None:
-            c = next(c for c in (8, 4, 2, 1) if n % c == 0 and (c == 1 or n // c * T * 256 >= (2 << 20)))
+            c = next(c for c, mb in ((8, 2), (4, 1.25), (2, 0.75), (1, 0)) if n % c == 0 and n // c * T * 256 >= mb * 2**20)
             sizes = [n // c] * c
         elif isinstance(chunks, int):
             if chunks <= 0 or n % chunks != 0:
@@ -159,8 +161,12 @@ class HostAttentionStep:
                 drop = dict(self.drop, philox_offset=self.philox_offset, bh_pos0=self.starts[i]) if self.drop else {}
                 att.attention_forward(d["Q"], d["K"], d["V"], self.scale, self.causal, out=d["O"],
                                       lse=d["LSE"], stream=self.s_cmp, **drop)
+                # the last chunk's O (and LSE) leaves as soon as the forward is done: no copy comes in beside it
+                if i + 1 == self.chunks:
+                    self.ev_fwd[i].record(self.s_cmp)
                 self.s_cmp.wait_event(self.ev_in[i])
-                self.ev_fwd[i].record(self.s_cmp)  # the forward is done and dO has arrived: O leaves
+                if i + 1 < self.chunks:
+                    self.ev_fwd[i].record(self.s_cmp)  # the forward is done and dO has arrived: O leaves
                 att.attention_backward(d["Q"], d["K"], d["V"], d["O"], d["dO"], d["LSE"], self.scale, self.causal,
                                        D=d["D"], dQ=d["dQ"], dK=d["dK"], dV=d["dV"],
                                        stream=self.s_cmp, **drop)
@@ -168,11 +174,14 @@ class HostAttentionStep:
             with torch.cuda.stream(self.s_out):
                 self.s_out.wait_event(self.ev_fwd[i])
                 hO[sl].copy_(d["O"], non_blocking=True)
+                if i + 1 == self.chunks:
+                    hLSE[sl].copy_(d["LSE"], non_blocking=True)
                 self.s_out.wait_event(self.ev_cmp[i])
                 hdQ[sl].copy_(d["dQ"], non_blocking=True)
                 hdK[sl].copy_(d["dK"], non_blocking=True)
                 hdV[sl].copy_(d["dV"], non_blocking=True)
-                hLSE[sl].copy_(d["LSE"], non_blocking=True)
+                if i + 1 < self.chunks:
+                    hLSE[sl].copy_(d["LSE"], non_blocking=True)
                 self.ev_out[i].record(self.s_out)
         cur.wait_event(self.ev_out[self.chunks - 1])
         cur.wait_event(self.ev_cmp[self.chunks - 1])
