@@ -9,6 +9,7 @@
 #include <Python.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/hk_attention.h"
@@ -59,6 +60,24 @@ void* stream_of(PyObject* o) {
     return reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(o));
 }
 
+// Runs an entry point's body.  A C++ exception thrown anywhere in it (no device, no memory, a tensor without strides or
+// data) becomes the Python exception torch raises for it; left to itself it would end the process.
+template <class F>
+PyObject* guarded(F&& body) {
+    try {
+        return body();
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+
+// The interpreter is free for other threads while this lives; it is taken back on every way out.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 float* data(const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); }
 
 // workspace: 256-byte aligned start inside a tensor a caller brought; false with AssertionError set if `need` does not fit
@@ -80,7 +99,7 @@ bool given_workspace(const at::Tensor* t, size_t need, void** ptr, size_t* bytes
 
 // forward(Q, K, V, scale, causal, dropout_p, dropout_mask, seed, offset, q_pos0, k_pos0, bh_pos0, flags, workspace, out,
 //         lse, stream) -> (O, LSE), or the negative status of the call
-static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+static PyObject* forward_body(PyObject* const* a, Py_ssize_t n) {
     if (n != 17) {
         PyErr_SetString(PyExc_TypeError, "forward: 17 arguments");
         return nullptr;
@@ -93,18 +112,12 @@ static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         !strides(*V, &p.v_strideB, &p.v_strideM, &p.v_strideH))
         return nullptr;
     const int64_t B = Q->size(0), H = Q->size(1), Tq = Q->size(2), Tk = K->size(2);
-    at::Tensor O, L;
-    try {
-        const auto opt = Q->options().dtype(at::kFloat);
-        O = out ? *out : at::empty({B, H, Tq, 64}, opt);
-        L = lse ? *lse : at::empty({B, H, Tq}, opt);
-        if (!strides(O, &p.o_strideB, &p.o_strideM, &p.o_strideH)) return nullptr;
-        p.lse_strideB = L.stride(0);
-        p.lse_strideH = L.stride(1);
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-        return nullptr;
-    }
+    const auto opt = Q->options().dtype(at::kFloat);
+    at::Tensor O = out ? *out : at::empty({B, H, Tq, 64}, opt);
+    at::Tensor L = lse ? *lse : at::empty({B, H, Tq}, opt);
+    if (!strides(O, &p.o_strideB, &p.o_strideM, &p.o_strideH)) return nullptr;
+    p.lse_strideB = L.stride(0);
+    p.lse_strideH = L.stride(1);
     p.Q = data(*Q); p.K = data(*K); p.V = data(*V); p.O = data(O); p.LSE = data(L);
     p.B = (int)B; p.nh = (int)H; p.T = Tq;
     p.scale = (float)PyFloat_AsDouble(a[3]);
@@ -122,11 +135,13 @@ static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     if (ws && !given_workspace(ws, g_lib.fwd_bytes(&p), &p.workspace, &p.workspace_bytes)) return nullptr;
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = g_lib.forward(&p, stream);
-    Py_END_ALLOW_THREADS
+    {
+        NoGil nogil;
+        rc = g_lib.forward(&p, stream);
+    }
     if (rc != 0) return PyLong_FromLong(rc);
     PyObject* res = PyTuple_New(2);
+    if (!res) return nullptr;
     PyTuple_SET_ITEM(res, 0, THPVariable_Wrap(std::move(O)));
     PyTuple_SET_ITEM(res, 1, THPVariable_Wrap(std::move(L)));
     return res;
@@ -134,7 +149,7 @@ static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // backward(Q, K, V, O, dO, LSE, scale, causal, dropout_p, dropout_mask, seed, offset, q_pos0, k_pos0, bh_pos0, flags,
 //          workspace, D, dQ, dK, dV, stream) -> (dQ, dK, dV, D), or the negative status of the call
-static PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
     if (n != 22) {
         PyErr_SetString(PyExc_TypeError, "backward: 22 arguments");
         return nullptr;
@@ -154,29 +169,24 @@ static PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.B = (int)B; p.nh = (int)H; p.T = (int)Tq;
     p.kv_len = Tk != Tq ? Tk : 0;
     at::Tensor r[4], slabs;  // dQ, dK, dV, D
-    try {
-        const auto opt = Q->options().dtype(at::kFloat);
-        for (int i = 0; i < 4; ++i)
-            r[i] = given[i] ? *given[i] : i == 3 ? at::empty({B, H, Tq}, opt) : at::empty({B, H, i == 0 ? Tq : Tk, 64}, opt);
-        if (!strides(r[0], &p.dq_strideB, &p.dq_strideM, &p.dq_strideH) || !strides(r[1], &p.dk_strideB, &p.dk_strideM, &p.dk_strideH) ||
-            !strides(r[2], &p.dv_strideB, &p.dv_strideM, &p.dv_strideH))
-            return nullptr;
-        p.d_strideB = r[3].stride(0);
-        p.d_strideH = r[3].stride(1);
-        p.lse_strideB = LSE->stride(0);
-        p.lse_strideH = LSE->stride(1);
-        if (ws) {
-            if (!given_workspace(ws, g_lib.bwd_bytes(&p), &p.workspace, &p.workspace_bytes)) return nullptr;
-        } else if (p.flags & HK_FLAG_DETERMINISTIC_DQ) {  // the slabs of partial dQ are the only scratch there is
-            hk_attn_bwd_params q = p;
-            q.flags |= HK_FLAG_OPERANDS_PREROUNDED;
-            const size_t bytes = g_lib.bwd_bytes(&q);
-            slabs = at::empty({(int64_t)bytes + 256}, Q->options().dtype(at::kByte));
-            if (!given_workspace(&slabs, bytes, &p.workspace, &p.workspace_bytes)) return nullptr;
-        }
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    const auto opt = Q->options().dtype(at::kFloat);
+    for (int i = 0; i < 4; ++i)
+        r[i] = given[i] ? *given[i] : i == 3 ? at::empty({B, H, Tq}, opt) : at::empty({B, H, i == 0 ? Tq : Tk, 64}, opt);
+    if (!strides(r[0], &p.dq_strideB, &p.dq_strideM, &p.dq_strideH) || !strides(r[1], &p.dk_strideB, &p.dk_strideM, &p.dk_strideH) ||
+        !strides(r[2], &p.dv_strideB, &p.dv_strideM, &p.dv_strideH))
         return nullptr;
+    p.d_strideB = r[3].stride(0);
+    p.d_strideH = r[3].stride(1);
+    p.lse_strideB = LSE->stride(0);
+    p.lse_strideH = LSE->stride(1);
+    if (ws) {
+        if (!given_workspace(ws, g_lib.bwd_bytes(&p), &p.workspace, &p.workspace_bytes)) return nullptr;
+    } else if (p.flags & HK_FLAG_DETERMINISTIC_DQ) {  // the slabs of partial dQ are the only scratch there is
+        hk_attn_bwd_params q = p;
+        q.flags |= HK_FLAG_OPERANDS_PREROUNDED;
+        const size_t bytes = g_lib.bwd_bytes(&q);
+        slabs = at::empty({(int64_t)bytes + 256}, Q->options().dtype(at::kByte));
+        if (!given_workspace(&slabs, bytes, &p.workspace, &p.workspace_bytes)) return nullptr;
     }
     p.Q = data(*Q); p.K = data(*K); p.V = data(*V); p.O = O ? data(*O) : nullptr; p.dO = data(*dO); p.LSE = data(*LSE);
     p.dQ = data(r[0]); p.dK = data(r[1]); p.dV = data(r[2]); p.D = data(r[3]);
@@ -192,17 +202,19 @@ static PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     void* stream = stream_of(a[21]);
     if (PyErr_Occurred()) return nullptr;
     int rc;
-    Py_BEGIN_ALLOW_THREADS
-    rc = g_lib.backward(&p, stream);
-    Py_END_ALLOW_THREADS
+    {
+        NoGil nogil;
+        rc = g_lib.backward(&p, stream);
+    }
     if (rc != 0) return PyLong_FromLong(rc);
     PyObject* res = PyTuple_New(4);
+    if (!res) return nullptr;
     for (int i = 0; i < 4; ++i) PyTuple_SET_ITEM(res, i, THPVariable_Wrap(std::move(r[i])));
     return res;
 }
 
 // zero(x, stream) -> status: zeroes a [B, H, T, 64] view
-static PyObject* zero(PyObject*, PyObject* const* a, Py_ssize_t n) {
+static PyObject* zero_body(PyObject* const* a, Py_ssize_t n) {
     const at::Tensor* x = n == 2 ? tensor_or_null(a[0]) : nullptr;
     if (!need_tensors({x})) return nullptr;
     hk_attn_bwd_params p = {};
@@ -213,6 +225,10 @@ static PyObject* zero(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     return PyLong_FromLong(g_lib.zero_dq(&p, stream));
 }
+
+static PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) { return guarded([&] { return forward_body(a, n); }); }
+static PyObject* backward(PyObject*, PyObject* const* a, Py_ssize_t n) { return guarded([&] { return backward_body(a, n); }); }
+static PyObject* zero(PyObject*, PyObject* const* a, Py_ssize_t n) { return guarded([&] { return zero_body(a, n); }); }
 
 // bind(handle): the dlopen handle of libhk_attention.so
 static PyObject* bind(PyObject*, PyObject* h) {

@@ -1,0 +1,49 @@
+"""CPU tests of the calls on torch tensors (csrc/hk_torch.cpp): what they refuse, and that nothing they meet ends the
+process.  No call here gets as far as a launch."""
+import os
+import subprocess
+import sys
+
+import pytest
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+# (what throws, the call): each in a process of its own, which an exception that escapes the native code would end
+THROWS = {
+    "forward: the current stream of a machine without a device": "hk.attention_forward(x, x, x, 0.125, True)",
+    "backward: the same": "hk.attention_backward(x, x, x, x, x, l, 0.125, True)",
+    "zero_dq: the same": "att.zero_dq(x)",
+    "forward: a tensor without data": "vmap(lambda y: hk.attention_forward(x, y, x, 0.125, True, stream=0))(x[None])",
+    "backward: the same ": "vmap(lambda y: hk.attention_backward(x, x, x, x, y, l, 0.125, True, stream=0))(x[None])",
+    "zero_dq: the same ": "vmap(lambda y: att.zero_dq(y, 0))(x[None])",
+    "forward: no memory for the result": "hk.attention_forward(x.expand(1 << 24, 1 << 24, 64, 64), x, x, 0.125, True, stream=0)",
+    "backward: the same  ": "hk.attention_backward(x.expand(1 << 24, 1 << 24, 64, 64), x, x, x, x, l, 0.125, True, stream=0)",
+    "forward: a result without the dimensions": "hk.attention_forward(x, x, x, 0.125, True, lse=l[0, 0], stream=0)",
+}
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host tensors: a kernel must not get them")
+@pytest.mark.parametrize("what", THROWS)
+def test_exceptions_of_the_native_calls_reach_the_caller(what):
+    code = f"""
+import torch, hyperkernels_b200 as hk, hyperkernels_b200.attention as att
+from torch.func import vmap
+x, l = torch.zeros(1, 1, 64, 64), torch.zeros(1, 1, 64)
+try:
+    {THROWS[what]}
+except (RuntimeError, IndexError) as e:
+    print("caught", not isinstance(e, hk.HKError))
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "caught True", (r.returncode, r.stdout, r.stderr[-400:])
+
+
+@pytest.mark.gpu
+def test_no_memory_for_the_result_is_torchs_own_error():
+    """torch.OutOfMemoryError, which programs catch to free memory and try again, not a bare RuntimeError."""
+    import hyperkernels_b200 as hk
+
+    x = torch.zeros(1, 1, 64, 64, device="cuda")
+    with pytest.raises(torch.OutOfMemoryError):
+        hk.attention_forward(x.expand(1 << 20, 1 << 10, 64, 64), x, x, 0.125, True)
