@@ -29,9 +29,26 @@ struct Library {
     BwdSizeFn bwd_bytes;
 } g_lib = {};
 
-// A tensor argument; nullptr for None or anything that is no tensor.
-const at::Tensor* tensor_or_null(PyObject* o) {
-    return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
+// A tensor argument; None, where it may be left out, gives nullptr.  Anything else is refused: a mask or an output buffer
+// of another kind must not pass for one that was not given.  False with TypeError set.
+struct TensorArg {
+    PyObject* object;
+    const char* name;
+    bool optional;
+    const at::Tensor** tensor;
+};
+bool tensors(std::initializer_list<TensorArg> args) {
+    for (const TensorArg& x : args) {
+        *x.tensor = nullptr;
+        if (THPVariable_Check(x.object)) {
+            *x.tensor = &THPVariable_Unpack(x.object);
+        } else if (!x.optional || x.object != Py_None) {
+            PyErr_Format(PyExc_TypeError, "%s: expected a tensor%s, not %s", x.name, x.optional ? " or None" : "",
+                         Py_TYPE(x.object)->tp_name);
+            return false;
+        }
+    }
+    return true;
 }
 
 // strides of a [B, H, T, 64] view into the block's (B, M, H) triple; false with AssertionError set
@@ -43,15 +60,6 @@ bool strides(const at::Tensor& t, int64_t* sB, int64_t* sM, int64_t* sH) {
     *sB = t.stride(0);
     *sM = t.stride(2);
     *sH = t.stride(1);
-    return true;
-}
-
-bool need_tensors(std::initializer_list<const at::Tensor*> ts) {
-    for (const at::Tensor* t : ts)
-        if (!t) {
-            PyErr_SetString(PyExc_TypeError, "expected a tensor");
-            return false;
-        }
     return true;
 }
 
@@ -104,9 +112,10 @@ static PyObject* forward_body(PyObject* const* a, Py_ssize_t n) {
         PyErr_SetString(PyExc_TypeError, "forward: 17 arguments");
         return nullptr;
     }
-    const at::Tensor *Q = tensor_or_null(a[0]), *K = tensor_or_null(a[1]), *V = tensor_or_null(a[2]), *mask = tensor_or_null(a[6]),
-                     *ws = tensor_or_null(a[13]), *out = tensor_or_null(a[14]), *lse = tensor_or_null(a[15]);
-    if (!need_tensors({Q, K, V})) return nullptr;
+    const at::Tensor *Q, *K, *V, *mask, *ws, *out, *lse;
+    if (!tensors({{a[0], "Q", false, &Q}, {a[1], "K", false, &K}, {a[2], "V", false, &V}, {a[6], "dropout_mask", true, &mask},
+                  {a[13], "workspace", true, &ws}, {a[14], "out", true, &out}, {a[15], "lse", true, &lse}}))
+        return nullptr;
     hk_attn_fwd_params p = {};
     if (!strides(*Q, &p.q_strideB, &p.q_strideM, &p.q_strideH) || !strides(*K, &p.k_strideB, &p.k_strideM, &p.k_strideH) ||
         !strides(*V, &p.v_strideB, &p.v_strideM, &p.v_strideH))
@@ -154,11 +163,11 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
         PyErr_SetString(PyExc_TypeError, "backward: 22 arguments");
         return nullptr;
     }
-    const at::Tensor *Q = tensor_or_null(a[0]), *K = tensor_or_null(a[1]), *V = tensor_or_null(a[2]), *O = tensor_or_null(a[3]),
-                     *dO = tensor_or_null(a[4]), *LSE = tensor_or_null(a[5]), *mask = tensor_or_null(a[9]),
-                     *ws = tensor_or_null(a[16]);
-    const at::Tensor* given[4] = {tensor_or_null(a[18]), tensor_or_null(a[19]), tensor_or_null(a[20]), tensor_or_null(a[17])};
-    if (!need_tensors({Q, K, V, dO, LSE})) return nullptr;
+    const at::Tensor *Q, *K, *V, *O, *dO, *LSE, *mask, *ws, *given[4];  // given: dQ, dK, dV, D
+    if (!tensors({{a[0], "Q", false, &Q}, {a[1], "K", false, &K}, {a[2], "V", false, &V}, {a[3], "O", true, &O}, {a[4], "dO", false, &dO},
+                  {a[5], "LSE", false, &LSE}, {a[9], "dropout_mask", true, &mask}, {a[16], "workspace", true, &ws},
+                  {a[17], "D", true, &given[3]}, {a[18], "dQ", true, &given[0]}, {a[19], "dK", true, &given[1]}, {a[20], "dV", true, &given[2]}}))
+        return nullptr;
     hk_attn_bwd_params p = {};
     if (!strides(*Q, &p.q_strideB, &p.q_strideM, &p.q_strideH) || !strides(*K, &p.k_strideB, &p.k_strideM, &p.k_strideH) ||
         !strides(*V, &p.v_strideB, &p.v_strideM, &p.v_strideH) || !strides(*dO, &p.do_strideB, &p.do_strideM, &p.do_strideH) ||
@@ -215,8 +224,12 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
 
 // zero(x, stream) -> status: zeroes a [B, H, T, 64] view
 static PyObject* zero_body(PyObject* const* a, Py_ssize_t n) {
-    const at::Tensor* x = n == 2 ? tensor_or_null(a[0]) : nullptr;
-    if (!need_tensors({x})) return nullptr;
+    if (n != 2) {
+        PyErr_SetString(PyExc_TypeError, "zero: 2 arguments");
+        return nullptr;
+    }
+    const at::Tensor* x;
+    if (!tensors({{a[0], "dQ", false, &x}})) return nullptr;
     hk_attn_bwd_params p = {};
     if (!strides(*x, &p.dq_strideB, &p.dq_strideM, &p.dq_strideH)) return nullptr;
     p.B = (int)x->size(0); p.nh = (int)x->size(1); p.T = (int)x->size(2);

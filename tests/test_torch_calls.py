@@ -39,6 +39,41 @@ except (RuntimeError, IndexError) as e:
     assert r.returncode == 0 and r.stdout.strip() == "caught True", (r.returncode, r.stdout, r.stderr[-400:])
 
 
+FORWARD_TENSORS = ["Q", "K", "V", "dropout_mask", "workspace", "out", "lse"]
+BACKWARD_TENSORS = ["Q", "K", "V", "O", "dO", "LSE", "dropout_mask", "workspace", "D", "dQ", "dK", "dV"]
+
+
+@pytest.mark.parametrize("call,name", [("forward", n) for n in FORWARD_TENSORS] + [("backward", n) for n in BACKWARD_TENSORS])
+@pytest.mark.parametrize("kind", ["numpy array", "list", "address", "False"])
+def test_what_is_no_tensor_is_refused(call, name, kind):
+    """A mask that is no tensor must not run without dropout, a buffer that is none must not be left unwritten."""
+    import numpy as np
+
+    import hyperkernels_b200 as hk
+
+    x, l = torch.zeros(1, 1, 64, 64), torch.zeros(1, 1, 64)
+    wrong = {"numpy array": np.ones((1, 64, 64), np.float32), "list": [1.0], "address": 4096, "False": False}[kind]
+    args = dict(Q=x, K=x, V=x) if call == "forward" else dict(Q=x, K=x, V=x, O=x, dO=x, LSE=l)
+    args.update(scale=0.125, causal=True, dropout_p=0.1)
+    args[name] = wrong
+    with pytest.raises(TypeError, match=f"^{name}: expected a tensor"):
+        (hk.attention_forward if call == "forward" else hk.attention_backward)(**args)
+
+
+@pytest.mark.parametrize("name", ["Q", "K", "V", "dO", "LSE"])
+def test_none_is_refused_where_a_tensor_is_needed(name):
+    import hyperkernels_b200 as hk
+    import hyperkernels_b200.attention as att
+
+    x, l = torch.zeros(1, 1, 64, 64), torch.zeros(1, 1, 64)
+    args = dict(Q=x, K=x, V=x, O=x, dO=x, LSE=l, scale=0.125, causal=True)
+    args[name] = None
+    with pytest.raises(TypeError, match=f"^{name}: expected a tensor"):
+        hk.attention_backward(**args)
+    with pytest.raises(TypeError, match="^dQ: expected a tensor"):
+        att.zero_dq(None)
+
+
 @pytest.mark.gpu
 def test_no_memory_for_the_result_is_torchs_own_error():
     """torch.OutOfMemoryError, which programs catch to free memory and try again, not a bare RuntimeError."""
