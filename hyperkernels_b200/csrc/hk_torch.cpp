@@ -134,8 +134,10 @@ static PyObject* forward_body(PyObject* const* a, Py_ssize_t n) {
     p.dropout_p = (float)PyFloat_AsDouble(a[5]);
     p.dropout_mask = mask ? data(*mask) : nullptr;
     p.kv_len = Tk != Tq ? Tk : 0;
-    p.dropout_seed = a[7] == Py_None ? 0 : PyLong_AsUnsignedLongLongMask(a[7]);
-    p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[8]);
+    if (a[7] != Py_None) {  // the offset counts only beside a seed
+        p.dropout_seed = PyLong_AsUnsignedLongLongMask(a[7]);
+        p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[8]);
+    }
     p.q_pos0 = PyLong_AsLongLong(a[9]);
     p.k_pos0 = PyLong_AsLongLong(a[10]);
     p.bh_pos0 = (uint32_t)PyLong_AsUnsignedLongLongMask(a[11]);
@@ -203,8 +205,10 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
     p.is_causal = PyObject_IsTrue(a[7]) != 0;
     p.dropout_p = (float)PyFloat_AsDouble(a[8]);
     p.dropout_mask = mask ? data(*mask) : nullptr;
-    p.dropout_seed = a[10] == Py_None ? 0 : PyLong_AsUnsignedLongLongMask(a[10]);
-    p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[11]);
+    if (a[10] != Py_None) {  // the offset counts only beside a seed
+        p.dropout_seed = PyLong_AsUnsignedLongLongMask(a[10]);
+        p.dropout_offset = PyLong_AsUnsignedLongLongMask(a[11]);
+    }
     p.q_pos0 = PyLong_AsLongLong(a[12]);
     p.k_pos0 = PyLong_AsLongLong(a[13]);
     p.bh_pos0 = (uint32_t)PyLong_AsUnsignedLongLongMask(a[14]);

@@ -74,6 +74,20 @@ def test_none_is_refused_where_a_tensor_is_needed(name):
         att.zero_dq(None)
 
 
+def test_an_offset_without_a_seed_is_not_read():
+    """philox_offset=None beside philox_seed=None, as a caller that forwards its own defaults passes them."""
+    import hyperkernels_b200 as hk
+
+    x, l = torch.zeros(1, 1, 64, 64), torch.zeros(1, 1, 64)
+    # dropout_p = 1 is refused by the library, behind all reading of arguments and in front of any launch
+    for call in (lambda **kw: hk.attention_forward(x, x, x, 0.125, True, dropout_p=1.0, stream=0, **kw),
+                 lambda **kw: hk.attention_backward(x, x, x, x, x, l, 0.125, True, dropout_p=1.0, stream=0, **kw)):
+        with pytest.raises(hk.HKError, match="dropout"):
+            call(philox_offset=None)
+        with pytest.raises(TypeError):
+            call(philox_seed=1, philox_offset=None)
+
+
 @pytest.mark.gpu
 def test_no_memory_for_the_result_is_torchs_own_error():
     """torch.OutOfMemoryError, which programs catch to free memory and try again, not a bare RuntimeError."""
