@@ -475,6 +475,12 @@ int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* stream) {
 }
 
 int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream) {
+    if (!p || !p->dQ) return HK_ERR_NULL_POINTER;
+    if (p->B <= 0 || p->nh <= 0 || p->T <= 0) return HK_ERR_BAD_SHAPE;
+    // the rows are written 16 bytes at a time; the stride of a dimension of one is not used
+    if (!aligned16(p->dQ) || (p->B > 1 && !stride_ok(p->dq_strideB)) || (p->nh > 1 && !stride_ok(p->dq_strideH)) ||
+        (p->T > 1 && !stride_ok(p->dq_strideM)))
+        return HK_ERR_MISALIGNED;
     return launch_zero_rows(p->dQ, p->dq_strideB, p->dq_strideM, p->dq_strideH, p->B, p->nh, p->T, static_cast<cudaStream_t>(stream));
 }
 

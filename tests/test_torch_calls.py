@@ -88,6 +88,25 @@ def test_an_offset_without_a_seed_is_not_read():
             call(philox_seed=1, philox_offset=None)
 
 
+@pytest.mark.parametrize("status,address,dims,strides", [
+    (-1, 0, (1, 1, 64), (4096, 4096, 64)), (-2, 4096, (1, 1, 0), (4096, 4096, 64)), (-2, 4096, (0, 1, 64), (4096, 4096, 64)),
+    (-2, 4096, (1, 0, 64), (4096, 4096, 64)), (-3, 4100, (1, 1, 64), (4096, 4096, 64)), (-3, 4096, (1, 1, 64), (4096, 4096, 66)),
+    (-3, 4096, (2, 1, 64), (4097, 4096, 64)), (-3, 4096, (1, 2, 64), (4096, 4098, 64))])
+def test_zero_dq_refuses_what_its_kernel_cannot_write(status, address, dims, strides):
+    """No rows (a division by zero on the host), no memory, or rows that are not on 16 bytes (a fault on the device).
+    In a process of its own: the unchecked call ended it."""
+    code = f"""
+import ctypes as C, hyperkernels_b200 as hk
+p = hk.MemEfficientBwdParams()
+p.dQ = {address} or None
+p.B, p.nh, p.T = {dims}
+p.dq_strideB, p.dq_strideH, p.dq_strideM = {strides}
+print(hk.lib().hk_attn_zero_dq(C.byref(p), None))
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == str(status), (r.returncode, r.stdout, r.stderr[-400:])
+
+
 @pytest.mark.gpu
 def test_no_memory_for_the_result_is_torchs_own_error():
     """torch.OutOfMemoryError, which programs catch to free memory and try again, not a bare RuntimeError."""
