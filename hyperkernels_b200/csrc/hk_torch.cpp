@@ -7,6 +7,7 @@
 // by HK_ATTENTION_LIB is used here too.
 #include <ATen/ATen.h>
 #include <Python.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
@@ -179,6 +180,8 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
     p.flags = (uint32_t)PyLong_AsUnsignedLongLongMask(a[15]);
     p.B = (int)B; p.nh = (int)H; p.T = (int)Tq;
     p.kv_len = Tk != Tq ? Tk : 0;
+    void* stream = stream_of(a[21]);
+    if (PyErr_Occurred()) return nullptr;
     at::Tensor r[4], slabs;  // dQ, dK, dV, D
     const auto opt = Q->options().dtype(at::kFloat);
     for (int i = 0; i < 4; ++i)
@@ -196,6 +199,11 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
         hk_attn_bwd_params q = p;
         q.flags |= HK_FLAG_OPERANDS_PREROUNDED;
         const size_t bytes = g_lib.bwd_bytes(&q);
+        // They are given back when this call returns, long before the kernels are done with them: they have to come from
+        // the pool of the stream the kernels run on, where the next user of the memory is behind these.
+        c10::cuda::OptionalCUDAStreamGuard guard;
+        if (a[21] != Py_None && Q->is_cuda())
+            guard.reset_stream(c10::cuda::getStreamFromExternal(static_cast<cudaStream_t>(stream), Q->device().index()));
         slabs = at::empty({(int64_t)bytes + 256}, Q->options().dtype(at::kByte));
         if (!given_workspace(&slabs, bytes, &p.workspace, &p.workspace_bytes)) return nullptr;
     }
@@ -212,7 +220,6 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
     p.q_pos0 = PyLong_AsLongLong(a[12]);
     p.k_pos0 = PyLong_AsLongLong(a[13]);
     p.bh_pos0 = (uint32_t)PyLong_AsUnsignedLongLongMask(a[14]);
-    void* stream = stream_of(a[21]);
     if (PyErr_Occurred()) return nullptr;
     int rc;
     {

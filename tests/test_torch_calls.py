@@ -115,3 +115,29 @@ def test_no_memory_for_the_result_is_torchs_own_error():
     x = torch.zeros(1, 1, 64, 64, device="cuda")
     with pytest.raises(torch.OutOfMemoryError):
         hk.attention_forward(x.expand(1 << 20, 1 << 10, 64, 64), x, x, 0.125, True)
+
+
+@pytest.mark.gpu
+def test_slabs_of_a_backward_on_another_stream_are_not_handed_on():
+    """The slabs of the deterministic dQ are given back when the call returns.  Called with a stream that is not the
+    current one and still busy, the kernels write them later: a tensor made meanwhile must not get that memory."""
+    import hyperkernels_b200 as hk
+
+    B, H, T = 1, 8, 1000
+    g = torch.Generator(device="cuda").manual_seed(5)
+    Q, K, V, dO = (torch.randn((B, H, T, 64), generator=g, device="cuda") for _ in range(4))
+    O, LSE = hk.attention_forward(Q, K, V, 0.125, True)
+    want = hk.attention_backward(Q, K, V, O, dO, LSE, 0.125, True, deterministic_dq=True)
+    dQ, dK, dV = (torch.empty_like(Q) for _ in range(3))
+    D = torch.empty_like(LSE)
+    slab_floats = (T + 127) // 128 * B * H * T * 64 + 64
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # about 0.1 s
+    hk.attention_backward(Q, K, V, O, dO, LSE, 0.125, True, deterministic_dq=True, dQ=dQ, dK=dK, dV=dV, D=D, stream=side)
+    others = [torch.full((slab_floats,), 7.0, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+    assert all(bool((t == 7.0).all()) for t in others)
+    assert torch.equal(dQ, want[0]) and torch.equal(dK, want[1]) and torch.equal(dV, want[2])
