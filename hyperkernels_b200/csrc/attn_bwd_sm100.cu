@@ -773,7 +773,7 @@ namespace {
 struct BwdDevice {
     std::once_flag once;
     cudaError_t rc = cudaSuccess;
-    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs
+    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
 }  // namespace
 
@@ -788,6 +788,7 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     if (dev < 0 || dev >= HK_MAX_DEVICES) return HK_ERR_UNSUPPORTED;
     BwdDevice& d = devices[dev];
     std::call_once(d.once, [&d] {
+        d.slots[0] = sm_count();
         for (Kernel k : kernels)
             if (d.rc == cudaSuccess)
                 d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);

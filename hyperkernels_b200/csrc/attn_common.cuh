@@ -47,6 +47,7 @@ int make_tile_map(CUtensorMap* map, const float* ptr, int inner, int B, int H, i
 
 DeviceStatus* device_status_ptr();  // per-device status word (allocated as a __device__ symbol)
 void count_launch(int n = 1);
+int sm_count();  // SMs of the current device, asked for once per device; a B200's 148 where it does not answer
 
 // Optional per-kernel timing (hk_attn_kernel_timing_enable): CUDA events recorded on
 // the launching stream around the two tensor-core kernels.

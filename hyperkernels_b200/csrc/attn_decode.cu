@@ -175,7 +175,8 @@ int launch_attn_decode(DecodeArgs a, cudaStream_t stream) {
     static const Kernel kernels[2][3] = {{attn_decode_kernel<1, 4>, attn_decode_kernel<1, 8>, attn_decode_kernel<1, 16>},
                                          {attn_decode_kernel<2, 4>, attn_decode_kernel<2, 8>, attn_decode_kernel<2, 16>}};
     int w = 0, warps = 4;
-    for (; w < 2 && (long long)a.BH * 8 * warps < 148 * 16; ++w) warps *= 2;
+    const int sms = sm_count();
+    for (; w < 2 && (long long)a.BH * 8 * warps < sms * 16; ++w) warps *= 2;
     const Kernel k = kernels[a.Tq - 1][w];
     const int batch = 2 * dec::UNROLL;
     a.n_splits = 8;

@@ -635,7 +635,7 @@ namespace {
 struct FwdDevice {
     std::once_flag once;
     cudaError_t rc = cudaSuccess;
-    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs
+    int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
 typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
 
@@ -650,6 +650,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     static const FwdKernel kernels[3] = {attn_fwd_kernel<0>, attn_fwd_kernel<1>, attn_fwd_kernel<2>};
     FwdDevice& d = devices[dev];
     std::call_once(d.once, [&d] {
+        d.slots[0] = sm_count();
         for (FwdKernel k : kernels)
             if (d.rc == cudaSuccess)
                 d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM_BYTES);

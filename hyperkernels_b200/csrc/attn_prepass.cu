@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(256) round_tf32_kernel(const float* src, float
 int launch_round_tf32(const float* src, float* dst, int64_t rows, cudaStream_t stream) {
     const long long nvec = (long long)rows * 16;  // 16 float4 per 64-float row
     if (nvec == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((nvec + 255) / 256, 148 * 8);
+    const int blocks = (int)std::min<long long>((nvec + 255) / 256, sm_count() * 8);
     round_tf32_kernel<<<blocks, 256, 0, stream>>>(src, dst, nvec);
     count_launch();
     return check_launch();
@@ -150,7 +150,7 @@ static void launch_D_hd(const DJob& j, cudaStream_t stream) {
     constexpr int NV = HD / 4;
     constexpr int LANES = NV >= 32 ? 32 : NV >= 16 ? 16 : NV >= 8 ? 8 : 4;
     const long long nrows = (long long)j.BH * j.T;
-    const int blocks = (int)std::min<long long>((nrows * LANES + 255) / 256, 148 * 8);
+    const int blocks = (int)std::min<long long>((nrows * LANES + 255) / 256, sm_count() * 8);
     precompute_D_hd_kernel<HD><<<blocks, 256, 0, stream>>>(j);
 }
 
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256) merge_partial_kernel(float* O_acc, float*
 int launch_merge_partial(float* O_acc, float* LSE_acc, const float* O_part, const float* LSE_part, long long rows,
                          cudaStream_t stream) {
     if (rows == 0) return HK_OK;
-    const int blocks = (int)std::min<long long>((rows * 16 + 255) / 256, 148 * 8);
+    const int blocks = (int)std::min<long long>((rows * 16 + 255) / 256, sm_count() * 8);
     merge_partial_kernel<<<blocks, 256, 0, stream>>>(O_acc, LSE_acc, O_part, LSE_part, rows);
     count_launch();
     return check_launch();

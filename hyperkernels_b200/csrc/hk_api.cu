@@ -36,6 +36,16 @@ namespace hk {
 static std::atomic<uint64_t> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
+int sm_count() {
+    static std::atomic<int> cache[HK_MAX_DEVICES];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= HK_MAX_DEVICES) return 148;
+    if ((n = cache[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    cache[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 // ---- optional kernel timing -----------------------------------------------------
 static std::atomic<int> g_timing_on{0};
 static std::mutex g_timing_mu;
