@@ -775,13 +775,13 @@ struct BwdDevice {
     cudaError_t rc = cudaSuccess;
     int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
-}  // namespace
+typedef void (*BwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
+                          CUtensorMap, CUtensorMap, BwdArgs);
+const BwdKernel bwd_kernels[6] = {attn_bwd_kernel<0, false>, attn_bwd_kernel<1, false>, attn_bwd_kernel<2, false>,
+                                  attn_bwd_kernel<0, true>,  attn_bwd_kernel<1, true>,  attn_bwd_kernel<2, true>};
 
-int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream) {
-    typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
-                           CUtensorMap, CUtensorMap, BwdArgs);
-    static const Kernel kernels[6] = {attn_bwd_kernel<0, false>, attn_bwd_kernel<1, false>, attn_bwd_kernel<2, false>,
-                                      attn_bwd_kernel<0, true>,  attn_bwd_kernel<1, true>,  attn_bwd_kernel<2, true>};
+// of the current device; set up by the first call on it
+int bwd_device(BwdDevice** out) {
     static BwdDevice devices[HK_MAX_DEVICES];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HK_ERR_CUDA;
@@ -789,39 +789,61 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     BwdDevice& d = devices[dev];
     std::call_once(d.once, [&d] {
         d.slots[0] = sm_count();
-        for (Kernel k : kernels)
+        for (BwdKernel k : bwd_kernels)
             if (d.rc == cudaSuccess)
                 d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::SMEM_BYTES);
         for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
             LaunchConfig lc(8u << i, bwd::NUM_THREADS, bwd::SMEM_BYTES, nullptr, 1 << i, false);
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernels[3], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+            if (cudaOccupancyMaxActiveClusters(&n, bwd_kernels[3], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
         }
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
-    const long long tiles = (long long)a.n_kvtiles * a.BH;
+    *out = &d;
+    return HK_OK;
+}
+
+}  // namespace
+
+int attn_bwd_slots(const int** slots) {
+    BwdDevice* d = nullptr;
+    const int rc = bwd_device(&d);
+    if (rc == HK_OK) *slots = d->slots;
+    return rc;
+}
+
+int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]) {
     // Splits by the same estimate of the makespan as the forward's: a CTA costs ~8 us and ~2.5 us per query tile, ~3 us
     // more when it adds dV and dK up over a cluster.  They pay where few KV tiles have many query tiles (cross-attention of
     // a long sequence to a short one).  The sum is taken in another order and the choice depends on batch x heads, so
     // sequences of training length do without: a batch cut into calls gives the bits of the single call.
-    a.n_splits = 1;
-    if (a.Tq >= 2 * (long long)a.Tk) {
-        const double n_q = (a.Tq + TILE - 1) / TILE;
+    int n_splits = 1;
+    if (Tq >= 2 * (long long)Tk) {
+        const double n_q = (Tq + TILE - 1) / TILE;
         double best_cost = 0;
         for (int i = 0; i < 4; ++i) {
             const double one = 8.0 + (i ? 3.0 : 0.0) + 2.5 * std::ceil(n_q / (1 << i));
-            const double cost = one * std::max(1.0, tiles / (double)d.slots[i] + (tiles > d.slots[i] ? 0.5 : 0.0));
+            const double cost = one * std::max(1.0, tiles / (double)slots[i] + (tiles > slots[i] ? 0.5 : 0.0));
             if (i == 0 || cost < 0.95 * best_cost) {
                 best_cost = cost;
-                a.n_splits = 1 << i;
+                n_splits = 1 << i;
             }
         }
     }
+    return n_splits;
+}
+
+int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream) {
+    BwdDevice* d = nullptr;
+    const int device_rc = bwd_device(&d);
+    if (device_rc != HK_OK) return device_rc;
+    const long long tiles = (long long)a.n_kvtiles * a.BH;
+    a.n_splits = plan_attn_bwd(tiles, a.Tq, a.Tk, d->slots);
     const long long nblocks = tiles * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_BWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
                                               m.dK, m.dV, a);
     timing_mark(TIMED_BWD, false, stream);
     count_launch();

@@ -170,17 +170,21 @@ __global__ void __launch_bounds__(WARPS * 32, (NQ == 1 ? 24 : 16) / WARPS) attn_
 
 // CTAs per slice: up to eight (the portable cluster size), each warp with at least one batch of rows.  Warps per CTA:
 // four, more where the slices are so few that eight CTAs each do not put ~16 warps on every SM.
+DecodePlan plan_attn_decode(int BH, int Tk, int sms) {
+    DecodePlan p{4, 8};
+    for (int w = 0; w < 2 && (long long)BH * 8 * p.warps < sms * 16; ++w) p.warps *= 2;
+    while (p.n_splits > 1 && (long long)p.n_splits * p.warps * 2 * dec::UNROLL > Tk) p.n_splits /= 2;
+    return p;
+}
+
 int launch_attn_decode(DecodeArgs a, cudaStream_t stream) {
     typedef void (*Kernel)(DecodeArgs);
     static const Kernel kernels[2][3] = {{attn_decode_kernel<1, 4>, attn_decode_kernel<1, 8>, attn_decode_kernel<1, 16>},
                                          {attn_decode_kernel<2, 4>, attn_decode_kernel<2, 8>, attn_decode_kernel<2, 16>}};
-    int w = 0, warps = 4;
-    const int sms = sm_count();
-    for (; w < 2 && (long long)a.BH * 8 * warps < sms * 16; ++w) warps *= 2;
-    const Kernel k = kernels[a.Tq - 1][w];
-    const int batch = 2 * dec::UNROLL;
-    a.n_splits = 8;
-    while (a.n_splits > 1 && (long long)a.n_splits * warps * batch > a.Tk) a.n_splits /= 2;
+    const DecodePlan plan = plan_attn_decode(a.BH, a.Tk, sm_count());
+    const int warps = plan.warps;
+    const Kernel k = kernels[a.Tq - 1][warps == 4 ? 0 : warps == 8 ? 1 : 2];
+    a.n_splits = plan.n_splits;
     const long long blocks = (long long)a.BH * a.n_splits;
     if (blocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     LaunchConfig lc((unsigned)blocks, warps * 32, warps * sizeof(dec::Partial), stream, a.n_splits, true);

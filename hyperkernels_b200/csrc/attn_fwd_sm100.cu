@@ -638,29 +638,41 @@ struct FwdDevice {
     int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
 typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
+const FwdKernel fwd_kernels[3] = {attn_fwd_kernel<0>, attn_fwd_kernel<1>, attn_fwd_kernel<2>};
 
-}  // namespace
-
-int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                    FwdArgs a, cudaStream_t stream) {
+// of the current device; set up by the first call on it
+int fwd_device(FwdDevice** out) {
     static FwdDevice devices[HK_MAX_DEVICES];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HK_ERR_CUDA;
     if (dev < 0 || dev >= HK_MAX_DEVICES) return HK_ERR_UNSUPPORTED;
-    static const FwdKernel kernels[3] = {attn_fwd_kernel<0>, attn_fwd_kernel<1>, attn_fwd_kernel<2>};
     FwdDevice& d = devices[dev];
     std::call_once(d.once, [&d] {
         d.slots[0] = sm_count();
-        for (FwdKernel k : kernels)
+        for (FwdKernel k : fwd_kernels)
             if (d.rc == cudaSuccess)
                 d.rc = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM_BYTES);
         for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
             LaunchConfig lc(8u << i, fwd::NUM_THREADS, fwd::SMEM_BYTES, nullptr, 1 << i, false);
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernels[0], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+            if (cudaOccupancyMaxActiveClusters(&n, fwd_kernels[0], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
         }
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
+    *out = &d;
+    return HK_OK;
+}
+
+}  // namespace
+
+int attn_fwd_slots(const int** slots) {
+    FwdDevice* d = nullptr;
+    const int rc = fwd_device(&d);
+    if (rc == HK_OK) *slots = d->slots;
+    return rc;
+}
+
+FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]) {
     // Mode and splits by an estimate of the makespan: the mean load of a slot plus half of the longest cluster, but at
     // least that cluster.  A CTA costs ~3.5 us and ~2.1 us per step of two products (1.5 with one stream, 2.3 in keys
     // mode), ~2 us more when it merges streams and ~3 us more when it combines splits.  Rows mode loads a key tile once
@@ -668,18 +680,18 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     // when even those leave most SMs idle (512 queries of 32 heads against 8 192 keys: 64 CTAs of 64 steps on 148 SMs).
     // Those two sum in another order, and the choice depends on batch x heads: they are left out for sequences of
     // training length, so that a batch cut into calls gives the bits of the single call.
-    const bool may_split = a.Tk > 4096 || a.Tk >= 2 * (long long)a.Tq;
+    const bool may_split = Tk > 4096 || Tk >= 2 * (long long)Tq;
+    FwdPlan plan{};
     double best_cost = 0;
-    long long blocks = 0;
     for (int mode = FWD_ROWS; mode <= (may_split ? FWD_KEYS : FWD_ROW); ++mode) {
         const int rows = mode == FWD_ROWS ? 2 * TILE : TILE;
-        const int nb = (a.Tq + rows - 1) / rows;
+        const int nb = (Tq + rows - 1) / rows;
         double sum = 0, longest = 0;  // steps of one (batch, head) slice, of its longest block
         const int sampled = std::min(nb, 64);  // the work per block is linear in its position: long sequences are sampled
         for (int i = 0; i < sampled; ++i) {
             const long long blk = sampled == nb ? i : (long long)i * (nb - 1) / (sampled - 1);
-            const int last = (int)(std::min<long long>(a.Tq, (blk + 1) * rows) - 1);  // its tile sees the most keys of the block
-            const int tiles = fwd::kv_tiles_for(last / TILE * TILE, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+            const int last = (int)(std::min<long long>(Tq, (blk + 1) * rows) - 1);  // its tile sees the most keys of the block
+            const int tiles = fwd::kv_tiles_for(last / TILE * TILE, Tq, Tk, causal, q_pos0, k_pos0);
             const double st = mode == FWD_KEYS ? 0.5 * tiles : tiles;
             sum += st;
             longest = std::max(longest, st);
@@ -689,22 +701,31 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
             const double fixed = 3.5 + (mode == FWD_KEYS ? 2.0 : 0.0) + (i ? 3.0 : 0.0);
             const double step = mode == FWD_ROWS ? 2.1 : mode == FWD_ROW ? 1.5 : 2.3;
             const double one = fixed + step * std::ceil(longest / (1 << i));
-            const double mean = a.BH * (nb * fixed + step * sum / (1 << i)) / d.slots[i];
+            const double mean = BH * (nb * fixed + step * sum / (1 << i)) / slots[i];
             const double cost = std::max(one, mean + 0.5 * one);
             if ((mode == FWD_ROWS && i == 0) || cost < 0.95 * best_cost) {
                 best_cost = cost;
-                a.mode = mode;
-                a.n_splits = 1 << i;
-                a.n_qblocks = nb;
-                blocks = (long long)nb * a.BH;
+                plan = {mode, 1 << i, nb};
             }
         }
     }
-    const long long nblocks = blocks * a.n_splits;
+    return plan;
+}
+
+int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
+                    FwdArgs a, cudaStream_t stream) {
+    FwdDevice* d = nullptr;
+    const int device_rc = fwd_device(&d);
+    if (device_rc != HK_OK) return device_rc;
+    const FwdPlan plan = plan_attn_fwd(a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, d->slots);
+    a.mode = plan.mode;
+    a.n_splits = plan.n_splits;
+    a.n_qblocks = plan.n_qblocks;
+    const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, kernels[a.dropout_mode], mq, mk, mv, mo, a);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();

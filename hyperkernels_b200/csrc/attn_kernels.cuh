@@ -30,6 +30,13 @@ struct FwdArgs {
     DeviceStatus* status;
 };
 
+// How a forward's work is cut, from sizes and the resident clusters of 1, 2, 4, 8 CTAs (slots) alone.
+struct FwdPlan {
+    int mode, n_splits, n_qblocks;
+};
+FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]);
+int attn_fwd_slots(const int** slots);  // of the current device; status
+
 // mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                     FwdArgs a, cudaStream_t stream);
@@ -48,6 +55,10 @@ struct DecodeArgs {
     int causal;
     int n_splits;  // set by launch_attn_decode
 };
+struct DecodePlan {
+    int warps, n_splits;
+};
+DecodePlan plan_attn_decode(int BH, int Tk, int sms);
 int launch_attn_decode(DecodeArgs a, cudaStream_t stream);
 
 struct BwdArgs {
@@ -88,6 +99,10 @@ struct BwdMaps {
     CUtensorMap q, k, v, dO, q_mn, k_mn, dO_mn, dQ, dK, dV;
 };
 
+// CTAs that share the query tiles of each of `tiles` KV tiles
+int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]);
+int attn_bwd_slots(const int** slots);
+
 // after_prepass: the launch before it in the stream is this call's D pre-pass, the only kernel whose results it waits for
 // itself (Q, K, V and dO are complete when the pre-pass lets it start)
 int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream);
@@ -99,6 +114,11 @@ int attn_backward(const hk_attn_bwd_params& p, cudaStream_t stream, bool check_s
 // the same for callers in this package, by name (dlsym)
 extern "C" int hk_attn_forward_noscratch(const hk_attn_fwd_params* p, void* stream);
 extern "C" int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* stream);
+// How the call of this block would be cut, for tests: nothing is launched and no pointer is read.  slots: resident clusters
+// of 1, 2, 4, 8 CTAs, or null for those of the current device.  Forward: plan = {FwdMode, or -1 for the decode kernel; CTAs
+// that share a block of rows (decode: a slice); warps of a CTA}.  Backward: plan = {CTAs that share a KV tile}.
+extern "C" int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* plan);
+extern "C" int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slots, int* plan);
 // zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ
 extern "C" int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream);
 

@@ -171,6 +171,13 @@ static int validate_dropout(float p, const float* mask, uint32_t flags, int64_t 
     return HK_OK;
 }
 
+// A few query rows: the tensor-core kernel would work on 128 rows whatever there are, the decode kernel is bound by reading
+// K and V.  Up to two rows: its arithmetic per key grows with them (B8 H12, 2 047 keys: four rows 31 us, eight 54, 29 with
+// the tensor cores); below 128 keys there is nothing to split.
+static bool decodes(int64_t Tq, int64_t Tk, int dropout_mode, uint32_t flags) {
+    return Tq <= DECODE_MAX_Q && Tk >= 128 && dropout_mode == 0 && !(flags & HK_FLAG_CONTINUE_SOFTMAX_STATE);
+}
+
 int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_scratch) {
     const hk_attn_fwd_params* p = &pr;
     if (!p->Q || !p->K || !p->V || !p->O || !p->LSE) return HK_ERR_NULL_POINTER;
@@ -200,10 +207,7 @@ int attn_forward(const hk_attn_fwd_params& pr, cudaStream_t stream, bool check_s
     if (check_scratch && !scratch_ok(p->workspace, p->workspace_bytes, hk_attn_fwd_workspace_bytes(p))) return HK_ERR_WORKSPACE;
 
     const int B = p->B, H = p->nh, BH = B * H;
-    // A few query rows: the tensor-core kernel would work on 128 rows whatever there are, this one is bound by reading K
-    // and V.  Up to two rows: its arithmetic per key grows with them (B8 H12, 2 047 keys: four rows 31 us, eight 54, 29 with
-    // the tensor cores); below 128 keys there is nothing to split.
-    if (Tq <= DECODE_MAX_Q && Tk >= 128 && mode == 0 && !(p->flags & HK_FLAG_CONTINUE_SOFTMAX_STATE)) {
+    if (decodes(Tq, Tk, mode, p->flags)) {
         DecodeArgs d{};
         d.Q = View4{p->Q, p->q_strideB, p->q_strideM, p->q_strideH};
         d.K = View4{p->K, p->k_strideB, p->k_strideM, p->k_strideH};
@@ -482,6 +486,29 @@ int hk_attn_forward_noscratch(const hk_attn_fwd_params* p, void* stream) {
 
 int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* stream) {
     return attn_backward(*p, static_cast<cudaStream_t>(stream), false);
+}
+
+int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* plan) {
+    const int64_t Tk = p->kv_len > 0 ? p->kv_len : p->T;
+    int mode = 0, rc = validate_dropout(p->dropout_p, p->dropout_mask, p->flags, p->k_pos0, &mode);
+    if (rc != HK_OK) return rc;
+    if (decodes(p->T, Tk, mode, p->flags)) {
+        const DecodePlan d = plan_attn_decode(p->B * p->nh, (int)Tk, slots ? slots[0] : sm_count());
+        plan[0] = -1; plan[1] = d.n_splits; plan[2] = d.warps;
+        return HK_OK;
+    }
+    if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
+    const FwdPlan f = plan_attn_fwd(p->B * p->nh, (int)p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, slots);
+    plan[0] = f.mode; plan[1] = f.n_splits; plan[2] = 12;
+    return HK_OK;
+}
+
+int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slots, int* plan) {
+    const int64_t Tk = p->kv_len > 0 ? p->kv_len : p->T;
+    int rc = HK_OK;
+    if (!slots && (rc = attn_bwd_slots(&slots))) return rc;
+    plan[0] = plan_attn_bwd((Tk + TILE - 1) / TILE * p->B * p->nh, p->T, (int)Tk, slots);
+    return HK_OK;
 }
 
 int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream) {

@@ -1,0 +1,130 @@
+"""How a call's work is cut over CTAs (mode, key splits, query splits) and what that may change: the choice from sizes
+(CPU), and on the GPU every mode and number of splits with every kind of dropout, against the oracle."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import hyperkernels_b200 as hk
+import oracle_lib as ol
+
+SCALE = 0.125
+ROWS, ROW, KEYS, DECODE = 0, 1, 2, -1
+B200 = (C.c_int * 4)(148, 74, 33, 15)  # resident clusters of 1, 2, 4, 8 CTAs, one CTA per SM
+
+
+def forward_plan(BH, Tq, Tk, causal=False, q_pos0=0, k_pos0=0, flags=0, dropout_p=0.0, slots=None):
+    """(mode, CTAs per block of rows or decoded slice); slots=None: those of the current device"""
+    p = hk.MemEfficientFwdParams()
+    p.B, p.nh, p.T, p.kv_len, p.is_causal = 1, BH, Tq, Tk, bool(causal)
+    p.q_pos0, p.k_pos0, p.flags, p.dropout_p = q_pos0, k_pos0, flags, dropout_p
+    out = (C.c_int * 3)()
+    assert hk.lib().hk_attn_forward_plan(C.byref(p), slots, out) == 0
+    return out[0], out[1]
+
+
+def backward_splits(BH, Tq, Tk, slots=None):
+    p = hk.MemEfficientBwdParams()
+    p.B, p.nh, p.T, p.kv_len = 1, BH, Tq, Tk
+    out = (C.c_int * 1)()
+    assert hk.lib().hk_attn_backward_plan(C.byref(p), slots, out) == 0
+    return out[0]
+
+
+# ---- the choice -----------------------------------------------------------------------------------------------------
+def test_decode_kernel_for_one_or_two_rows():
+    plan = lambda Tq, Tk, **kw: forward_plan(4, Tq, Tk, slots=B200, **kw)[0]  # noqa: E731
+    assert plan(1, 128) == plan(2, 128) == plan(1, 5000, causal=True) == DECODE
+    assert DECODE not in (plan(3, 128), plan(1, 127), plan(1, 500, flags=hk.FLAG_CONTINUE_SOFTMAX_STATE),
+                          plan(1, 500, flags=hk.FLAG_PHILOX_DROPOUT, dropout_p=0.1))
+
+
+# ---- every cut, with every mask -------------------------------------------------------------------------------------
+def _dev(x):
+    return torch.from_numpy(np.ascontiguousarray(x)).cuda()
+
+
+def _normal(shape, seed):
+    return np.random.default_rng(seed).standard_normal(shape).astype(np.float32)
+
+
+P, SEED, OFFSET = 0.25, 99, 7
+MASKS = ["none", "philox", "dense", "philox inverted", "dense inverted"]
+
+
+def _mask(kind, BH, Tq, Tk, q_pos0=0, k_pos0=0):
+    """(keyword arguments of the calls, the oracle's mask); p = 1/4 is exact in 16 bits, so both kinds drop with it"""
+    if kind == "none":
+        return {}, None
+    mask = ol.dropout_mask(BH, Tq, Tk, P, SEED, OFFSET, q_pos0=q_pos0, k_pos0=k_pos0)
+    kw = dict(dropout_mask=_dev(mask)) if kind.startswith("dense") else dict(philox_seed=SEED, philox_offset=OFFSET)
+    return dict(kw, dropout_p=P, dropout_scaled=kind.endswith("inverted")), mask
+
+
+def _oracle_forward(kind, mask, q, k, v, causal, **pos):
+    if kind.endswith("inverted"):
+        return ol.attn_forward_scaled(q, k, v, SCALE, causal, mask, P, **pos)
+    return ol.attn_forward_mt(q, k, v, SCALE, causal, mask, **pos)
+
+
+def _oracle_backward(kind, mask, q, k, v, O, g, L, causal, **pos):
+    if kind.endswith("inverted"):
+        return ol.attn_backward_scaled(q, k, v, O, g, L, SCALE, causal, mask, P, **pos)
+    return ol.attn_backward_mt(q, k, v, O, g, L, SCALE, causal, mask, **pos)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", MASKS)
+@pytest.mark.parametrize("mode,splits,BH,Tq,Tk,causal", [
+    (ROWS, 1, 64, 129, 400, 0), (ROWS, 2, 16, 257, 1000, 0), (ROWS, 4, 12, 129, 640, 1), (ROWS, 8, 6, 129, 650, 0),
+    (ROW, 1, 24, 3, 600, 1), (ROW, 2, 24, 3, 700, 1), (ROW, 4, 12, 3, 640, 1), (ROW, 8, 1, 3, 641, 0),
+    (KEYS, 1, 24, 257, 1000, 1), (KEYS, 2, 48, 3, 4200, 0), (KEYS, 4, 24, 3, 8193, 1), (KEYS, 8, 3, 385, 8193, 1)])
+def test_every_forward_cut_with_every_mask(mode, splits, BH, Tq, Tk, causal, kind):
+    from test_attention_gpu import gate, host, lse_check, ok_status
+
+    q, k, v = _normal((1, BH, Tq, 64), 960), _normal((1, BH, Tk, 64), 961), _normal((1, BH, Tk, 64), 962)
+    pos = Tk - Tq if causal else 0
+    kw, mask = _mask(kind, BH, Tq, Tk, q_pos0=pos)
+    assert forward_plan(BH, Tq, Tk, causal, pos) == (mode, splits)
+    O_ref, L_ref = _oracle_forward(kind, mask, q, k, v, causal, q_pos0=pos)
+    O, LSE = hk.attention_forward(_dev(q), _dev(k), _dev(v), SCALE, bool(causal), q_pos0=pos, **kw)
+    ok_status()
+    gate("O", host(O), O_ref)
+    lse_check(host(LSE), L_ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", MASKS)
+@pytest.mark.parametrize("splits,BH,Tq,Tk,causal", [
+    (1, 48, 257, 40, 0), (2, 24, 777, 333, 0), (4, 8, 1024, 129, 0), (4, 1, 257, 128, 0), (8, 1, 4000, 40, 0), (8, 2, 1281, 300, 1)])
+def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
+    """Beside the default call: dQ through slabs (the same bits on every run, dK and dV those of the default call) and
+    results added to what the buffers hold."""
+    from test_attention_gpu import gate, host, ok_status
+
+    q, g = _normal((1, BH, Tq, 64), 970), _normal((1, BH, Tq, 64), 971)
+    k, v = _normal((1, BH, Tk, 64), 972), _normal((1, BH, Tk, 64), 973)
+    pos = dict(k_pos0=(Tq - 200) // 8 * 8 if causal else 0)
+    kw, mask = _mask(kind, BH, Tq, Tk, **pos)
+    assert backward_splits(BH, Tq, Tk) == splits
+    O_ref, L_ref = _oracle_forward(kind, mask, q, k, v, causal, **pos)
+    _, *refs = _oracle_backward(kind, mask, q, k, v, O_ref, g, L_ref, causal, **pos)
+    args = (_dev(q), _dev(k), _dev(v), _dev(O_ref), _dev(g), _dev(L_ref), SCALE, bool(causal))
+    call = lambda **more: hk.attention_backward(*args, **pos, **kw, **more)  # noqa: E731
+    plain = call()[:3]
+    ok_status()
+    for name, got, ref in zip(("dQ", "dK", "dV"), plain, refs):
+        gate(name, host(got), ref)
+    slabs, again = call(deterministic_dq=True)[:3], call(deterministic_dq=True)[:3]
+    ok_status()
+    gate("dQ", host(slabs[0]), refs[0])
+    assert all(torch.equal(a, b) for a, b in zip(slabs, again))
+    assert torch.equal(slabs[1], plain[1]) and torch.equal(slabs[2], plain[2])
+    base = [_dev(_normal(r.shape, 974 + i)) for i, r in enumerate(refs)]
+    sums = [b.clone() for b in base]
+    call(deterministic_dq=True, accum_dq=True, accum_dkdv=True, dQ=sums[0], dK=sums[1], dV=sums[2])
+    ok_status()
+    for s, b, x in zip(sums, base, slabs):
+        # fp32 sums of at most ceil(Tk / 128) + 1 terms in another order
+        assert float((s - (b + x)).abs().max()) <= 4 * 2.0 ** -23 * float(x.abs().max() + b.abs().max())
