@@ -230,7 +230,10 @@ def attention_forward(Q, K, V, scale: float, causal: bool, *, dropout_p: float =
                       philox_seed: Optional[int] = None, philox_offset: int = 0, q_pos0: int = 0, k_pos0: int = 0,
                       bh_pos0: int = 0, prerounded: bool = False, dropout_scaled: bool = False, continue_state: bool = False,
                       round_in_hbm: bool = False, workspace=None, out=None, lse=None, stream=None):
-    """O, LSE = fused attention forward of [B,H,Tq,64] Q against [B,H,Tk,64] K, V (fp32 CUDA tensors)."""
+    """O, LSE = fused attention forward of [B,H,Tq,64] Q against [B,H,Tk,64] K, V (fp32 CUDA tensors).
+
+    With Tk <= 4096 and Tk < 2 Tq a (batch, head) slice gives the same bits in any batch; otherwise (long sequences,
+    chunks against a cache, decoding) they may change with B * H, by the rounding of sums in another order."""
     flags = 0
     if philox_seed is not None:
         flags |= FLAG_PHILOX_DROPOUT
@@ -257,7 +260,10 @@ def attention_backward(Q, K, V, O, dO, LSE, scale: float, causal: bool, *, dropo
                        accum_dq: bool = False, reuse_fwd_rounded: bool = False, dropout_scaled: bool = False,
                        round_in_hbm: bool = False, deterministic_dq: bool = False, workspace=None, dQ=None, dK=None, dV=None,
                        stream=None):
-    """dQ, dK, dV, D = fused attention backward (fp32 CUDA tensors, [B,H,T,64])."""
+    """dQ, dK, dV, D = fused attention backward (fp32 CUDA tensors, [B,H,T,64]).
+
+    With Tq < 2 Tk a (batch, head) slice gives the same dK and dV in any batch (dQ: deterministic_dq); otherwise they may
+    change with B * H, by the rounding of sums in another order."""
     flags = 0
     if philox_seed is not None:
         flags |= FLAG_PHILOX_DROPOUT

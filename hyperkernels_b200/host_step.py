@@ -42,6 +42,10 @@ class HostAttentionStep:
     [B, H, T, 64] (LSE: [B, H, T]).  The call enqueues everything and returns; the caller's current stream waits for
     the last result copy, so a ``torch.cuda.synchronize()`` (or an event on that stream) marks completion.
 
+    The chunks are calls of their own.  Up to T = 4 096 they give O, LSE, dK and dV of a single call over the whole batch
+    bit for bit (dQ up to the order of its additions); for longer sequences the forward may share a slice's keys among
+    CTAs by a number that depends on how many slices a call has, and the results agree within rounding.
+
     With Philox dropout every chunk passes the index of its first (batch, head) slice (``bh_pos0``) with the same
     seed and offset, so the keep-mask of a chunked step is the one a single call over the whole batch draws.
     """

@@ -23,6 +23,14 @@
  *     the reference's pointer arithmetic allows) is refused with
  *     HK_ERR_UNSUPPORTED when that dimension is larger than 1: the TMA tensor
  *     maps the kernels read through cannot express it.
+ *   - Bits: the same call gives the same O, LSE, D, dK, dV on every run (dQ:
+ *     HK_FLAG_DETERMINISTIC_DQ).  At training lengths -- forward with
+ *     kv_len <= 4096 and kv_len < 2 T, backward with T < 2 kv_len -- a (batch,
+ *     head) slice also gives them whatever other slices are in the call, so a
+ *     batch may be cut into several calls.  Outside these the keys (backward:
+ *     the queries) of a slice may be shared by several CTAs, by a number that
+ *     depends on B * nh: the same slice in another batch then differs by the
+ *     rounding of sums in another order, a decoding step (T <= 2) included.
  *   - Re-entrant: no call keeps state between calls except per-device caches
  *     that are filled once under a lock, so any number of host threads may
  *     drive any number of devices and streams.  Device ordinals 0..63.

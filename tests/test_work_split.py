@@ -1,6 +1,7 @@
 """How a call's work is cut over CTAs (mode, key splits, query splits) and what that may change: the choice from sizes
 (CPU), and on the GPU every mode and number of splits with every kind of dropout, against the oracle."""
 import ctypes as C
+import random
 
 import numpy as np
 import pytest
@@ -33,6 +34,32 @@ def backward_splits(BH, Tq, Tk, slots=None):
 
 
 # ---- the choice -----------------------------------------------------------------------------------------------------
+def test_training_lengths_are_never_split():
+    """kv_len <= 4 096 and < 2 T forward, T < 2 kv_len backward: every slice is summed in one order, whatever the batch."""
+    rnd = random.Random(1)
+    modes = set()
+    for _ in range(3000):
+        Tk = int(2 ** rnd.uniform(0, 12))
+        Tq = max(Tk // 2 + 1, int(2 ** rnd.uniform(0, 13)))
+        BH, causal = int(2 ** rnd.uniform(0, 11)), rnd.random() < 0.5
+        mode, splits = forward_plan(BH, Tq, Tk, causal, rnd.choice([0, 0, 300]), rnd.choice([0, 0, 128]), slots=B200)
+        assert mode in (ROWS, ROW) and splits == 1, (BH, Tq, Tk, causal)
+        modes.add(mode)
+        Tq = max(1, int(rnd.uniform(0.01, 2.0) * Tk) - 1)
+        assert backward_splits(BH, Tq, Tk, slots=B200) == 1, (BH, Tq, Tk)
+    assert modes == {ROWS, ROW}
+    assert forward_plan(1, 4096, 4096, True, slots=B200)[1] == 1 and forward_plan(1, 2048, 4095, slots=B200)[1] == 1
+    assert backward_splits(1, 1023, 512, slots=B200) == 1
+
+
+def test_the_batch_decides_outside_training_lengths():
+    """The other side of the same lines: a slice alone and the same slice among others are cut differently."""
+    assert forward_plan(1, 8192, 8192, True, slots=B200) != forward_plan(32, 8192, 8192, True, slots=B200)
+    assert forward_plan(1, 512, 1024, slots=B200)[1] > 1 and forward_plan(64, 512, 1024, slots=B200)[1] == 1
+    assert backward_splits(1, 1024, 512, slots=B200) > 1 and backward_splits(64, 1024, 512, slots=B200) == 1
+    assert forward_plan(1, 1, 300, True, slots=B200) != forward_plan(192, 1, 3000, True, slots=B200)
+
+
 def test_decode_kernel_for_one_or_two_rows():
     plan = lambda Tq, Tk, **kw: forward_plan(4, Tq, Tk, slots=B200, **kw)[0]  # noqa: E731
     assert plan(1, 128) == plan(2, 128) == plan(1, 5000, causal=True) == DECODE
@@ -128,3 +155,48 @@ def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
     for s, b, x in zip(sums, base, slabs):
         # fp32 sums of at most ceil(Tk / 128) + 1 terms in another order
         assert float((s - (b + x)).abs().max()) <= 4 * 2.0 ** -23 * float(x.abs().max() + b.abs().max())
+
+
+# ---- what the cut may change ----------------------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.parametrize("Tq,Tk,causal,q_pos0", [(4096, 4096, 1, 0), (2048, 4095, 0, 0), (65, 129, 1, 64), (1023, 512, 0, 0), (1500, 1500, 1, 0)])
+def test_a_slice_keeps_its_bits_in_any_batch_at_training_lengths(Tq, Tk, causal, q_pos0):
+    """Up to the lines themselves: O, LSE, dK and dV of a slice alone and of the same slice among 40, of which the forward
+    runs one in row, the other in rows mode."""
+    BH = 40
+    assert forward_plan(1, Tq, Tk, causal, q_pos0)[0] == ROW and forward_plan(BH, Tq, Tk, causal, q_pos0)[0] == (ROW if Tq <= 128 else ROWS)
+    gen = torch.Generator(device="cuda").manual_seed(77)
+    Q, dO = (torch.randn((1, BH, Tq, 64), generator=gen, device="cuda") for _ in range(2))
+    K, V = (torch.randn((1, BH, Tk, 64), generator=gen, device="cuda") for _ in range(2))
+    for kw in ({}, dict(dropout_p=0.1, philox_seed=3)):
+        O, LSE = hk.attention_forward(Q, K, V, SCALE, causal, q_pos0=q_pos0, **kw)
+        _, dK, dV, _ = hk.attention_backward(Q, K, V, O, dO, LSE, SCALE, causal, q_pos0=q_pos0, **kw)
+        for i in (0, 23):
+            s = slice(i, i + 1)
+            one = dict(kw, bh_pos0=i) if kw else {}
+            o, l = hk.attention_forward(Q[:, s], K[:, s], V[:, s], SCALE, causal, q_pos0=q_pos0, **one)
+            _, dk, dv, _ = hk.attention_backward(Q[:, s], K[:, s], V[:, s], o, dO[:, s], l, SCALE, causal, q_pos0=q_pos0, **one)
+            assert torch.equal(o, O[:, s]) and torch.equal(l, LSE[:, s])
+            assert torch.equal(dk, dK[:, s]) and torch.equal(dv, dV[:, s])
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+
+
+@pytest.mark.gpu
+def test_a_chunked_host_step_beyond_them_agrees_within_rounding():
+    """One long sequence, its heads one by one or in one call: the forward is cut differently, so a probability is rounded
+    to TF32 (2^-11 of itself) relative to another maximum on either side."""
+    B, H, T = 1, 4, 6000
+    assert forward_plan(1, T, T, True) != forward_plan(H, T, T, True)
+    gen = torch.Generator(device="cuda").manual_seed(78)
+    Q, K, V, dO = (torch.randn((B, H, T, 64), generator=gen, device="cuda") for _ in range(4))
+    O, LSE = hk.attention_forward(Q, K, V, SCALE, True)
+    want = (O, LSE) + hk.attention_backward(Q, K, V, O, dO, LSE, SCALE, True)[:3]
+    hin = [x.cpu().pin_memory() for x in (Q, K, V, dO)]
+    hout = [torch.full(x.shape, float("nan")).pin_memory() for x in want]
+    hk.HostAttentionStep(B, H, T, SCALE, True, chunks=H).step(*hin, *hout)
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+    for got, ref in zip(hout, want):
+        ref = ref.cpu().double()
+        assert float((got.double() - ref).norm() / ref.norm()) <= 2.0 ** -10
