@@ -39,7 +39,7 @@ EncodeTiledFn get_encode_tiled();
 // mn_major = false: 128-byte swizzle of 16-byte chunks (K-major MMA operand);
 // mn_major = true:  128-byte swizzle of 32-byte chunks (MN-major TF32 operand).
 // operand = true: the map of an MMA operand.  Its element type is TFLOAT32, with which a load rounds every fp32 value to
-// TF32 (to nearest, ties to even: checked bit for bit over random patterns, ties and denormals) on its way into shared
+// TF32 (to nearest, ties to even: tests/test_operand_rounding.py reads every map out bit for bit) on its way into shared
 // memory.  The tensor core itself truncates, so without this the operands would have to be rounded by a pass over HBM
 // (18 us at B8 H12 T1024 forward, 115 us for a 2047-key decoding step of 192 heads) or over shared memory (17 us).
 int make_tile_map(CUtensorMap* map, const float* ptr, int inner, int B, int H, int64_t T, int64_t sB, int64_t sM,
