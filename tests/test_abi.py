@@ -72,9 +72,9 @@ def test_forward_argument_validation():
     p = _fwd_block(); p.dropout_p = 0.1; p.dropout_mask = 0x1000; p.flags |= hk.FLAG_PHILOX_DROPOUT
     assert L.hk_attn_forward(C.byref(p), None) == -4          # both mask sources
     p = _fwd_block(); p.flags = hk.FLAG_ROUND_IN_HBM
-    assert L.hk_attn_forward(C.byref(p), None) == -5          # workspace missing (the HBM pre-pass needs one)
+    assert L.hk_attn_forward(C.byref(p), None) == -5          # workspace missing (asked for with this flag)
     p = _fwd_block(); p.flags = 0; p.T = 4096
-    assert L.hk_attn_forward(C.byref(p), None) == -5          # long sequences are always rounded by the pre-pass
+    assert L.hk_attn_forward(C.byref(p), None) == -5          # and beyond 2 048 queries
     p = _fwd_block(); p.dropout_p = 0.1; p.flags |= hk.FLAG_PHILOX_DROPOUT; p.k_pos0 = 2
     assert L.hk_attn_forward(C.byref(p), None) == -6          # unsupported Philox alignment
 
@@ -129,7 +129,7 @@ def test_workspace_sizes():
     assert hk.fwd_workspace_bytes(p) == 2 * 3 * 256 * (100 + 2 * 40)
     p.flags = hk.FLAG_OPERANDS_PREROUNDED
     assert hk.fwd_workspace_bytes(p) == 0
-    # short sequences are rounded in shared memory: the forward needs no scratch at all
+    # by size: none is asked for between 512 and 2 048 queries (1 024 without the causal mask)
     p.flags = 0; p.kv_len = 0
     for T, causal, inside in ((100, False, False), (511, True, False), (512, False, True), (1024, False, True),
                               (1025, False, False), (2048, True, True), (2049, True, False)):

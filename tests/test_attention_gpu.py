@@ -264,8 +264,7 @@ def test_strided_bthd_layout_prerounded():
 def test_packed_qkv_layout():
     """Packed [B, T, 3, H, 64] storage (the output of a fused QKV projection): Q, K, V are views into one buffer,
     addressed through the reference block's stride triplets (fused_attn_forward_kernel_tc_sm89.cu:24-28); the
-    gradients go into a buffer of the same packing.  Arbitrary fp32 inputs: the rounding pre-pass reads the strided
-    views."""
+    gradients go into a buffer of the same packing.  Arbitrary fp32 inputs, rounded as the loads read the strided views."""
     B, H, T = 2, 4, 333
     qkv = normal((B, T, 3, H, 64), 35)
     dO = normal((B, H, T, 64), 36)
@@ -455,7 +454,7 @@ def test_backward_with_precomputed_D_and_accumulation():
 
 
 def test_backward_reuses_forward_rounded_operands():
-    """Same workspace for forward and backward: the backward skips re-rounding Q, K, V."""
+    """Same workspace for forward and backward, with the flag that says so: accepted, and the results are those without."""
     B, H, T = 2, 3, 300
     Q, K, V, dO = (normal((B, H, T, 64), 90 + s) for s in range(4))
     O_ref, L_ref = ol.attn_forward_mt(Q, K, V, SCALE, 1)
@@ -545,11 +544,9 @@ def test_batch_head_slices_reproduce_the_whole_call_under_dropout():
 @pytest.mark.parametrize("causal", [0, 1])
 @pytest.mark.parametrize("B,H,T", [(2, 3, 640), (1, 2, 556), (1, 1, 1024)])
 def test_rounding_in_shared_memory_equals_the_hbm_prepass(B, H, T, causal):
-    """Short sequences have their operands rounded to TF32 in shared memory after the TMA landing (forward: Q, K, V;
-    backward: K, V), long ones -- and every call with HK_FLAG_ROUND_IN_HBM -- by the HBM pre-pass into the workspace.
-    Same rounding function, same kernels: O, LSE, dK, dV must be identical bit for bit, dQ up to the order of its
-    atomic additions.  Also with the workspace handed from the forward to the backward (the forward leaves the rounded
-    Q there; HK_FLAG_REUSE_FWD_ROUNDED)."""
+    """HK_FLAG_ROUND_IN_HBM, a workspace and HK_FLAG_REUSE_FWD_ROUNDED come from versions that rounded the operands in a
+    pass over HBM or in shared memory; the loads round them now, and these change nothing: O, LSE, dK, dV identical bit
+    for bit, dQ up to the order of its additions."""
     Q, K, V, dO = (dev(normal((B, H, T, 64), 900 + s)) for s in range(4))
     O_h, L_h = hk.attention_forward(Q, K, V, SCALE, causal, round_in_hbm=True)
     O_s, L_s = hk.attention_forward(Q, K, V, SCALE, causal)
@@ -564,7 +561,7 @@ def test_rounding_in_shared_memory_equals_the_hbm_prepass(B, H, T, causal):
     p = hk.MemEfficientBwdParams()
     p.B, p.nh, p.T = B, H, T
     ws = torch.empty(hk.bwd_workspace_bytes(p) + 256, dtype=torch.uint8, device="cuda")
-    ws.fill_(0x7F)  # nothing may be taken from a workspace the forward has not written
+    ws.fill_(0x7F)  # nothing may be taken from the workspace
     O_w, L_w = hk.attention_forward(Q, K, V, SCALE, causal, workspace=ws)
     g_w = hk.attention_backward(Q, K, V, O_w, dO, L_w, SCALE, causal, workspace=ws, reuse_fwd_rounded=True)
     ok_status()
@@ -575,9 +572,8 @@ def test_rounding_in_shared_memory_equals_the_hbm_prepass(B, H, T, causal):
 
 @pytest.mark.parametrize("Tq,Tk,q_pos0", [(640, 896, 256), (512, 1024, 0), (700, 300, 0)])
 def test_workspace_handed_from_forward_to_backward_with_unequal_lengths(Tq, Tk, q_pos0):
-    """The forward writes the rounded K/V tiles it loads into the workspace, each tile by the first query block that
-    loads it; key tiles no query sees are never written, and the backward must not read them.  Poisoned workspace,
-    causal mask with a query offset, more keys than any query sees, fewer keys than queries."""
+    """A workspace full of NaN patterns, handed from the forward to the backward, is not read: causal mask with a query
+    offset, more keys than any query sees, fewer keys than queries."""
     B, H = 1, 2
     Q, dO = dev(normal((B, H, Tq, 64), 910)), dev(normal((B, H, Tq, 64), 911))
     K, V = dev(normal((B, H, Tk, 64), 912)), dev(normal((B, H, Tk, 64), 913))
@@ -595,16 +591,12 @@ def test_workspace_handed_from_forward_to_backward_with_unequal_lengths(Tq, Tk, 
     assert float((g_w[0] - g_h[0]).abs().max()) <= 1e-4
 
 
-def test_random_shapes_the_two_rounding_paths_and_the_workspace_hand_over_agree():
-    """Seeded random shapes (ragged lengths, unequal query/key lengths, position offsets, Philox dropout) around the
-    window in which the operands are rounded in shared memory: that path, the HBM pre-pass and the forward-to-backward
-    workspace hand-over must give identical O, LSE, dK, dV (dQ up to the order of its atomic additions)."""
+def random_shapes():
+    """24 seeded problems: ragged lengths, unequal query/key lengths, position offsets, Philox dropout."""
     import random
 
     rnd = random.Random(2024)
-    g = torch.Generator(device="cuda").manual_seed(11)
-    same = lambda a, b: torch.equal(torch.nan_to_num(a, nan=0.0, neginf=-1e30), torch.nan_to_num(b, nan=0.0, neginf=-1e30))
-    for case in range(24):
+    for _ in range(24):
         B, H = rnd.choice([(1, 1), (1, 3), (2, 2), (3, 5)])
         causal = rnd.random() < 0.6
         Tq = rnd.choice([512, 513, 600, 700, 1000, 1024, 1100, 1536, 2047, 2048, 300])
@@ -612,6 +604,27 @@ def test_random_shapes_the_two_rounding_paths_and_the_workspace_hand_over_agree(
         kw = dict(q_pos0=rnd.choice([0, 0, 128, 616]) if causal else 0, k_pos0=rnd.choice([0, 0, 64, 128]) if causal else 0)
         if rnd.random() < 0.3:
             kw.update(dropout_p=0.2, philox_seed=rnd.randrange(1 << 30), philox_offset=8 * rnd.randrange(100))
+        yield B, H, Tq, Tk, causal, kw
+
+
+@pytest.mark.parametrize("case", range(24))
+def test_random_shapes_against_the_oracle(case):
+    B, H, Tq, Tk, causal, kw = list(random_shapes())[case]
+    Q, dO = normal((B, H, Tq, 64), 1000 + case), normal((B, H, Tq, 64), 1100 + case)
+    K, V = normal((B, H, Tk, 64), 1200 + case), normal((B, H, Tk, 64), 1300 + case)
+    pos = {k: kw.pop(k) for k in ("q_pos0", "k_pos0")}
+    mask = None
+    if kw:
+        mask = ol.dropout_mask(B * H, Tq, Tk, kw["dropout_p"], kw["philox_seed"], kw["philox_offset"], **pos)
+    run_fwd_bwd_check(Q, K, V, dO, causal, mask=mask, fwd_kw=kw, bwd_kw=kw, **pos)
+
+
+def test_random_shapes_the_two_rounding_paths_and_the_workspace_hand_over_agree():
+    """The random shapes (their values are held against the oracle above) with HK_FLAG_ROUND_IN_HBM, with a workspace and
+    with HK_FLAG_REUSE_FWD_ROUNDED, which change nothing: identical O, LSE, dK, dV (dQ up to the order of its additions)."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    same = lambda a, b: torch.equal(torch.nan_to_num(a, nan=0.0, neginf=-1e30), torch.nan_to_num(b, nan=0.0, neginf=-1e30))
+    for case, (B, H, Tq, Tk, causal, kw) in enumerate(random_shapes()):
         Q, dO = (torch.randn((B, H, Tq, 64), generator=g, device="cuda") for _ in range(2))
         K, V = (torch.randn((B, H, Tk, 64), generator=g, device="cuda") for _ in range(2))
         O1, L1 = hk.attention_forward(Q, K, V, SCALE, causal, round_in_hbm=True, **kw)
@@ -710,7 +723,7 @@ def test_graphed_step_replays_the_direct_calls():
     B, H, T = 2, 3, 320
     tQ, tK, tV, tdO = (dev(normal((B, H, T, 64), 90 + s)) for s in range(4))
     gs = hk.GraphedAttentionStep(tQ, tK, tV, tdO, SCALE, True)
-    assert gs.launches_per_replay == 4  # rounding pre-pass, forward, D pre-pass, backward (T < 512: rounded in HBM)
+    assert gs.launches_per_replay == 4  # forward, dQ zeroing beside it, D pre-pass, backward
     for seed in (0, 1):
         if seed:
             for t_, s in zip((tQ, tK, tV, tdO), range(4)):

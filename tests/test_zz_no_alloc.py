@@ -4,9 +4,8 @@ where cudaMalloc would stall the device).  The file name sorts last on purpose: 
 stops at the first failure has then already run every other test.
 
 The entry point must give what hk_attn_forward gives for the same block (it runs the same
-kernels on the same rounded operands, so the results are required to be identical, which is
-inside the tolerance every other forward test uses), on two calls in a row that share the
-built-in scratch, and must refuse problems that do not fit in it.
+kernel, so the results are required to be identical), on calls in a row, must allocate nothing,
+and must refuse problems beyond its documented size limit.
 """
 import ctypes as C
 
@@ -49,10 +48,10 @@ def test_static_scratch_forward_matches_workspace_forward():
         assert rc == 0, (call, L.hk_status_string(rc))
         if call > 0:
             # nothing was allocated or freed by the call (the first call on a device may make the driver load the
-            # module that holds the array, which is when the 24 MiB become resident: it is exempt)
+            # module: it is exempt)
             assert free_after == free_before, (call, free_before, free_after)
         assert hk.last_device_status() == 0
-        # same kernels, same rounded operands: identical results (tolerance of the other tests: 5e-3 / 1e-3)
+        # same kernel: identical results (tolerance of the other tests: 5e-3 / 1e-3)
         assert torch.equal(O, O_ref) and torch.equal(LSE, LSE_ref), call
         assert float((O - O_ref).abs().max()) <= 5e-3
 
@@ -61,7 +60,7 @@ def test_static_scratch_rejects_oversized_problem():
     L = hk.lib()
     L.hk_attn_forward_static_scratch.argtypes = [C.POINTER(hk.MemEfficientFwdParams), C.c_void_p]
     t = torch.zeros(64, device="cuda")
-    B, H, T = 8, 12, 1024  # 3 * 96 * 1024 * 256 B = 72 MiB of rounded copies > 24 MiB
+    B, H, T = 8, 12, 1024  # 3 * 96 * 1024 * 256 B = 72 MiB > 24 MiB
     p = hk.MemEfficientFwdParams()
     p.Q = p.K = p.V = p.O = p.LSE = t.data_ptr()
     p.B, p.nh, p.T, p.scale = B, H, T, 0.125
