@@ -54,10 +54,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
 
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)));
-}
-
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -144,12 +140,6 @@ __device__ __forceinline__ bool mbar_wait(const WaitCtx& ctx, uint64_t* bar, uin
     return mbar_wait_slow(ctx, bar, parity, wait_id, aux);
 }
 
-__device__ __forceinline__ int smid() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(r));
-    return (int)r;
-}
-
 // ---------------------------------------------------------------------------
 // TMA: tiled bulk-tensor load, global -> shared, completion on an mbarrier
 // ---------------------------------------------------------------------------
@@ -167,13 +157,6 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2),
         "r"(c3)
         : "memory");
-}
-
-// Requests the tile into L2 only (no shared-memory destination, no completion to wait for).
-__device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
 }
 
 // 4-D tile reduction, shared -> global: global[tile] += shared tile (fp32 add performed by the
@@ -198,10 +181,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all committed bulk groups of this thread have finished READING shared memory
 __device__ __forceinline__ void bulk_wait_group_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all but the latest committed bulk group of this thread have finished reading shared memory
-__device__ __forceinline__ void bulk_wait_group_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-// all committed bulk groups of this thread are complete
-__device__ __forceinline__ void bulk_wait_group_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // tensor memory
@@ -266,38 +245,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
 }
 
 // 16 consecutive columns of this warp's 32 lanes
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-
-// 16 lanes x 64 consecutive columns in the accumulator-fragment shape (16x256b, eight times): thread t of the warp
-// receives, for each group j of eight columns, r[4j], r[4j+1] = lane (t >> 2), columns 8j + 2(t & 3) + {0, 1} and
-// r[4j+2], r[4j+3] = lane (t >> 2) + 8, same columns -- four threads hold 32 consecutive bytes of a row, so that
-// what they write to global memory falls into whole sectors.  taddr names the first of the 16 lanes.
-__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
         : "memory");
 }
 
@@ -531,15 +484,5 @@ __device__ __forceinline__ uint32_t tf32_round_bits(uint32_t bits) { return (bit
 // Same value as seen by the tensor core, which drops the low 13 bits itself:
 // for operands written by a kernel straight into tensor or shared memory.
 __device__ __forceinline__ uint32_t tf32_round_bits_mma(uint32_t bits) { return bits + 0x1000u; }
-
-__device__ __forceinline__ void red_add_v2(float* gptr, uint32_t a, uint32_t b) {
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gptr), "f"(__uint_as_float(a)), "f"(__uint_as_float(b))
-                 : "memory");
-}
-
-__device__ __forceinline__ void red_add_v4(float* gptr, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(gptr), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
-}
 
 }  // namespace hk
