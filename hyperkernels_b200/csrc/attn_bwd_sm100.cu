@@ -48,7 +48,7 @@
 //
 // Splits: where few KV tiles have many query tiles (cross-attention of a long sequence to a short one), a cluster of 2, 4
 // or 8 CTAs shares the query tiles of a KV tile; at the end each adds up a slice of the rows of dV and dK from the partial
-// sums the others left in their shared memory (launch_attn_bwd picks the number).  B1 H4, 5 000 queries,
+// sums the others left in their shared memory (plan_attn_bwd picks the number).  B1 H4, 5 000 queries,
 // 200 keys: 107 -> 25 us; B1 H1, 16 384 and 4 096: 330 -> 100; B4 H6, 777 and 333: 26.5 -> 24.6.
 //
 //   warps 0-15  compute: four threads per key row (tensor-memory lane), each

@@ -35,7 +35,7 @@
 //
 // Key splits: a cluster of NS CTAs shares one block of query rows; split s takes a contiguous run of its key tiles, and at
 // the end every CTA combines a slice of the rows from the partial (O, m, l) the others left in their shared memory (keys
-// mode merges its two streams with the same code).  The host picks mode and splits (launch_attn_fwd).
+// mode merges its two streams with the same code).  The host picks mode and splits (plan_attn_fwd).
 // CTA pairs (cta_group::2, half of every K and V tile per CTA) were built and measured: the MMAs and copies alone run at
 // 2 360 instead of 3 100 cycles per step, the whole kernel 4 % faster at H32 T8192, but every CTA spends ~4 000 cycles
 // more on set-up and hand-over between the two, 57 against 45 us at B8 H12 T1024.
@@ -479,9 +479,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
                 } else if constexpr (DROP == 2) {
                     // One Philox call per eight keys of this row, four calls in flight; none for 32 keys that no row of
-                    // the warp sees (on the diagonal three in eight).  What bounds dropout is this integer arithmetic:
-                    // H25 B32 T1024 takes 477 us with, 170 without it (all sixteen calls interleaved: 530; one at a
-                    // time: 780; the calls in front of the wait for S: 570 - 640; wide 32 x 32 multiplications: + 15 %).
+                    // the warp sees (on the diagonal three in eight).  This integer arithmetic is what dropout costs:
+                    // H25 B32 T1024 takes 545 us with, 340 without it in one run (in another, where it took 477 - 495 with
+                    // it, all sixteen calls interleaved: 530; one at a time: 780; the calls in front of the wait for S:
+                    // 570 - 640; wide 32 x 32 multiplications: + 15 %).
                     const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
                     float2 sk = make_float2(0.f, 0.f), sa = make_float2(0.f, 0.f);  // kept terms, all terms
                     const int warp_lim = __reduce_max_sync(0xffffffffu, lim_local);

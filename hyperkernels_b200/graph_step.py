@@ -1,11 +1,12 @@
 """Forward + backward captured once in a CUDA graph and replayed.
 
 A training step of the attention path is four launches (dQ zeroing, forward, D
-pre-pass, backward).  At small sizes
-the gaps between dependent launches are a large part of the step (B=2, H=4,
-T=256: 0.064 ms issued launch by launch, 0.033 ms replayed from a graph); at
-B=8, H=12, T=1024 the graph saves about 2 %.  Zeroing dQ depends on nothing, so it is a
-branch of its own beside the forward: its stores (25 MB at B=8, H=12, T=1024) leave the
+pre-pass, backward).  A replay takes the host 3.3 us instead of 18 for the two
+calls, which it has for other work; the device is no faster for it where the
+host keeps ahead (B=8, H=12, T=1024: 172 us replayed, 169 by calls; B=2, H=4,
+T=256: 25.0 and 22.3), since the launches of a call are dependent launches
+already and the zeroing is one of its own here.  Zeroing dQ depends on nothing, so it is a
+branch beside the forward: its stores (25 MB at B=8, H=12, T=1024) leave the
 D pre-pass and fill SMs the forward's last wave leaves idle.  Capture goes through
 ``hk_attn_forward`` and ``hk_attn_backward`` on a side stream after one eager warm-up step (which sets
 the kernels' attributes and resolves the library's device symbols -- neither is

@@ -9,9 +9,9 @@ step, which at these sizes is an order of magnitude more than the kernels.  The
 batch into chunks and runs three queues: chunk i+1 travels to the device while
 the kernels work on chunk i and the results of chunk i-1 travel back (the two
 copy directions use different DMA engines and the link is full duplex).  What
-bounds it is the link: 101 MB each way take 1.84 ms alone and 2.2 ms in both
-directions at B8 H12 T1024, to which the first chunk's way in and the last one's
-way out add.  So a chunk's forward starts when Q, K and V have arrived, beside
+bounds it is the link: at B8 H12 T1024 101 MB take 1.8 ms one way alone, 2.03 - 2.09
+in both directions at once and 2.2 - 2.35 cut into the step's 64 copies, to which the
+first chunk's way in and the last one's way out add.  So a chunk's forward starts when Q, K and V have arrived, beside
 the copy of dO, and its O leaves beside the backward as soon as dO is there, when
 the next chunk's Q sets out: copies that start together in the two directions
 share the link best.  2.51 against 2.71 ms with one dependency each way per chunk,
