@@ -202,8 +202,13 @@ static PyObject* backward_body(PyObject* const* a, Py_ssize_t n) {
         // They are given back when this call returns, long before the kernels are done with them: they have to come from
         // the pool of the stream the kernels run on, where the next user of the memory is behind these.
         c10::cuda::OptionalCUDAStreamGuard guard;
-        if (a[21] != Py_None && Q->is_cuda())
-            guard.reset_stream(c10::cuda::getStreamFromExternal(static_cast<cudaStream_t>(stream), Q->device().index()));
+        if (a[21] != Py_None && Q->is_cuda()) {
+            const cudaStream_t s = static_cast<cudaStream_t>(stream);
+            const auto device = Q->device().index();
+            // 0 and cudaStreamLegacy are the default stream, which torch does not know by a handle
+            guard.reset_stream(s == nullptr || s == cudaStreamLegacy ? c10::cuda::getDefaultCUDAStream(device)
+                                                                     : c10::cuda::getStreamFromExternal(s, device));
+        }
         slabs = at::empty({(int64_t)bytes + 256}, Q->options().dtype(at::kByte));
         if (!given_workspace(&slabs, bytes, &p.workspace, &p.workspace_bytes)) return nullptr;
     }

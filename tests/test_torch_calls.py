@@ -141,3 +141,20 @@ def test_slabs_of_a_backward_on_another_stream_are_not_handed_on():
     assert hk.last_device_status() == 0
     assert all(bool((t == 7.0).all()) for t in others)
     assert torch.equal(dQ, want[0]) and torch.equal(dK, want[1]) and torch.equal(dV, want[2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("handle", [0, 1, 2])
+def test_slabs_under_the_streams_that_have_no_object(handle):
+    """0, cudaStreamLegacy and cudaStreamPerThread, as numbers."""
+    import hyperkernels_b200 as hk
+
+    g = torch.Generator(device="cuda").manual_seed(6)
+    Q, K, V, dO = (torch.randn((1, 2, 300, 64), generator=g, device="cuda") for _ in range(4))
+    O, LSE = hk.attention_forward(Q, K, V, 0.125, True)
+    want = hk.attention_backward(Q, K, V, O, dO, LSE, 0.125, True, deterministic_dq=True)
+    torch.cuda.synchronize()
+    got = hk.attention_backward(Q, K, V, O, dO, LSE, 0.125, True, deterministic_dq=True, stream=handle)
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
