@@ -289,13 +289,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 load_dom(q1);
             }
             // Do not leave the CTA while bulk copies into its shared memory are in flight.
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.k_full, 0); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.v_full, 0); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.km_full, 0); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.q_full, (issued_q - 1) & 1); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.do_full, (issued_do - 1) & 1); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.qm_full, (issued_qm - 1) & 1); ++i) {}
-            for (int i = 0; i < 100000 && !mbar_try_wait(&sh.dom_full, (issued_dom - 1) & 1); ++i) {}
+            auto drain = [](uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+                for (int i = 0; i < 100000 && !mbar_try_wait(bar, parity); ++i) {}
+            };
+            drain(&sh.k_full, 0);
+            drain(&sh.v_full, 0);
+            drain(&sh.km_full, 0);
+            drain(&sh.q_full, (issued_q - 1) & 1);
+            drain(&sh.do_full, (issued_do - 1) & 1);
+            drain(&sh.qm_full, (issued_qm - 1) & 1);
+            drain(&sh.dom_full, (issued_dom - 1) & 1);
         }
     } else if (warp == W_MMA) {
         // ------------------------------ MMA issuer ------------------------------
