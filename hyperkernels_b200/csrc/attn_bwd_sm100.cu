@@ -58,6 +58,7 @@
 //   warp 17     MMA issuer (the whole warp runs the issuing code, one elected lane
 //               issues)
 //   warp 18     TMA reductions of dQ (per query tile) and stores of dK, dV (at the end)
+//   warp 19     LSE and D of the query rows into shared memory
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -70,8 +71,8 @@ namespace hk {
 namespace bwd {
 
 constexpr int NUM_COMPUTE = 512;
-constexpr int NUM_THREADS = NUM_COMPUTE + 96;  // 16 compute warps, 3 control warps
-constexpr int W_LOAD = 16, W_MMA = 17, W_STORE = 18;
+constexpr int NUM_THREADS = NUM_COMPUTE + 128;  // 16 compute warps, 4 control warps
+constexpr int W_LOAD = 16, W_MMA = 17, W_STORE = 18, W_ROWS = 19;
 constexpr int TMEM_COLS = 512;
 constexpr int COL_S = 0;     // S^T, then P^T
 constexpr int COL_DP = 128;  // dP^T, then dS^T
@@ -81,19 +82,20 @@ constexpr int COL_DQ = 384;
 constexpr int COL_V = 448;   // V of this KV tile, A operand of dP^T
 
 struct __align__(16) Shared {
-    float lse[2][TILE];   // -LSE * log2e of the query tile (-inf for rows past the end), double-buffered
-    float dsum[2][TILE];  // -D * scale of the query tile
+    float lse[TILE];   // -LSE * log2e of the query tile; -inf for a row that saw no key or is past the end
+    float dsum[TILE];  // -D * scale of the query tile
     uint64_t k_full, v_full, km_full, q_full, do_full, qm_full, dom_full;  // TMA loads
     uint64_t v_ready;       // V is in tensor memory (and its landing buffer is free)
     uint64_t qk_free, dok_free;  // S^T(i) / dP^T(i) complete: the K-major Q / dO tile may be refilled
-    uint64_t s_full, dp_full;
+    uint64_t s_full;        // S^T is complete and the query tile's LSE and D are staged
+    uint64_t dp_full;
     // One barrier for all four column groups: with one each (so that a group's slices could go as soon as it was in) the
     // issuing warp spent more on the six extra waits per tile than the early start gained (4 - 8 % of the kernel).
     uint64_t pt_ready;      // P^T is in tensor memory: dV += P^T dO may go
     uint64_t p_ready;       // dS^T is in tensor memory: dK += dS^T Q may go
     uint64_t dv_done, dk_done;   // dV(i) / dK(i) complete: the MN-major dO / Q tile is free
-    uint64_t ds_ready, dq_full, dq_empty, staged;
-    uint64_t acc_staged;    // dV, dK of the CTA are staged for the bulk store
+    uint64_t ds_ready, dq_full, dq_empty;
+    uint64_t dv_staged, dk_staged;  // dV / dK of the CTA is staged for the bulk store
     uint64_t dq_staged;     // dQ of a query tile is staged (in the K-major dO tile) for the bulk reduction
     uint64_t dq_out;        // the bulk reduction has read the staged dQ tile: the K-major dO tile may be refilled
     uint32_t tmem_base;
@@ -102,9 +104,9 @@ struct __align__(16) Shared {
 
 constexpr int OFF_KK = 0;                // K, K-major swizzle   (S^T = K Q^T); dK staging at the end
 constexpr int OFF_KM = TILE_BYTES;       // K, MN-major swizzle  (dQ = dS K)
-constexpr int OFF_QK = 2 * TILE_BYTES;   // Q, K-major           (S^T); staging of the last dQ
+constexpr int OFF_QK = 2 * TILE_BYTES;   // Q, K-major           (S^T); dV staging at the end
 constexpr int OFF_DOK = 3 * TILE_BYTES;  // dO, K-major          (dP^T)
-constexpr int OFF_QM = 4 * TILE_BYTES;   // Q, MN-major          (dK += dS^T Q); dV staging at the end
+constexpr int OFF_QM = 4 * TILE_BYTES;   // Q, MN-major          (dK += dS^T Q)
 constexpr int OFF_DS = 5 * TILE_BYTES;   // dS boxes 0, 1 ([128 kv][32 q] each); first of all the landing buffer of V
 constexpr int OFF_DOM = 6 * TILE_BYTES;  // dO, MN-major         (dV += P^T dO); dS boxes 2, 3 once dV is done
 static_assert(OFF_DOM == OFF_DS + 2 * BOX_BYTES, "the four dS boxes are one descriptor: equally spaced");
@@ -116,7 +118,7 @@ static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may opt in to");
 
 enum WaitId {
     W_KVFULL = 201, W_QKFULL, W_QKEMPTY, W_QMFULL, W_QMFREE, W_SFULL, W_PREADY, W_BDONE, W_DSREADY, W_DQFULL, W_DQEMPTY,
-    W_STAGED, W_DQSTAGED, W_ACCSTAGED, W_VREADY, W_DVDONE, W_DQOUT
+    W_ROWSFREE, W_DQSTAGED, W_ACCSTAGED, W_VREADY, W_DVDONE, W_DQOUT
 };
 
 }  // namespace bwd
@@ -215,7 +217,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.v_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.qk_free, 1);
         mbar_init(&sh.dok_free, 1);
-        mbar_init(&sh.s_full, 1);
+        mbar_init(&sh.s_full, 2);     // the commit of S^T and the warp that stages LSE and D
         mbar_init(&sh.dp_full, 1);
         mbar_init(&sh.pt_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.p_ready, NUM_COMPUTE / 32);
@@ -226,8 +228,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.dq_empty, 8);   // column groups 2, 3 drain dQ
         mbar_init(&sh.dq_staged, 8);
         mbar_init(&sh.dq_out, 1);
-        mbar_init(&sh.staged, 8);    // the threads that stage LSE and D
-        mbar_init(&sh.acc_staged, NUM_COMPUTE / 32);
+        mbar_init(&sh.dv_staged, 8);  // column groups 0, 1
+        mbar_init(&sh.dk_staged, 8);  // column groups 2, 3
         sh.abort_flag = 0;
         fence_mbar_init();
     }
@@ -405,70 +407,87 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             };
             bool tok = true;
             for (int j = 0; tok && j + 1 < n_it; ++j) tok = reduce_dq(j);  // the last tile's dQ follows dV and dK
-            // dV and dK, staged by the compute warps in the MN-major Q tile and the K-major K tile (dead after the last
-            // dK and S^T): stored -- added, if the caller accumulates -- with bulk copies; a thread-per-row store would
-            // be 32 lines per instruction
-            if (tok && (tok = mbar_wait(wc, &sh.acc_staged, 0, W_ACCSTAGED, 0))) {
-                if (SPLIT) {
-                    // added up over the cluster, below
-                } else if (a.accum_dkdv) {
-                    tma_reduce_add_4d(&mapdV, sQm, 0, kv0, h, b);
-                    tma_reduce_add_4d(&mapdV, sQm + BOX_BYTES, HALF_D, kv0, h, b);
-                    tma_reduce_add_4d(&mapdK, sK, 0, kv0, h, b);
-                    tma_reduce_add_4d(&mapdK, sK + BOX_BYTES, HALF_D, kv0, h, b);
-                } else {
-                    tma_store_4d(&mapdV, sQm, 0, kv0, h, b);
-                    tma_store_4d(&mapdV, sQm + BOX_BYTES, HALF_D, kv0, h, b);
-                    tma_store_4d(&mapdK, sK, 0, kv0, h, b);
-                    tma_store_4d(&mapdK, sK + BOX_BYTES, HALF_D, kv0, h, b);
+            // dV and dK, staged by the compute warps in the K-major Q and K tiles (dead after the last S^T): stored --
+            // added, if the caller accumulates -- with bulk copies, each as soon as it is staged; a thread-per-row store
+            // would be 32 lines per instruction.  Over a cluster they are added up below.
+            auto store_acc = [&](uint64_t* bar, const CUtensorMap* map, const uint8_t* src) -> bool {
+                if (!mbar_wait(wc, bar, 0, W_ACCSTAGED, 0)) return false;
+                if (!SPLIT) {
+                    if (a.accum_dkdv) {
+                        tma_reduce_add_4d(map, src, 0, kv0, h, b);
+                        tma_reduce_add_4d(map, src + BOX_BYTES, HALF_D, kv0, h, b);
+                    } else {
+                        tma_store_4d(map, src, 0, kv0, h, b);
+                        tma_store_4d(map, src + BOX_BYTES, HALF_D, kv0, h, b);
+                    }
+                    bulk_commit_group();
                 }
-                bulk_commit_group();
-                tok = reduce_dq(n_it - 1);
-            }
+                return true;
+            };
+            if (tok && store_acc(&sh.dv_staged, &mapdV, sQ) && store_acc(&sh.dk_staged, &mapdK, sK))
+                reduce_dq(n_it - 1);
             // the copies have read their shared-memory sources; they complete on their own
             bulk_wait_group_read_all();
+        }
+    } else if (warp == W_ROWS) {
+        // ------------------------------ LSE and D of the query rows ------------------------------
+        // A lane takes rows lane, lane + 32, .. of each query tile; they are fetched a tile ahead and written, negated and
+        // scaled so that both enter the arithmetic as FMA addends, once the compute warps are through with the previous
+        // tile's (they are when dS^T is stored).  A warp of its own: eight compute warps that did this beside their work,
+        // and sixteen that waited for it, were ~400 cycles per tile longer at it.
+        if (n_it > 0) {
+            const float* lse_bh = a.LSE + (int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH;
+            const float* d_bh = a.D + (int64_t)b * a.d_sB + (int64_t)h * a.d_sH;
+            float l[TILE / 32], d[TILE / 32];
+            auto fetch = [&](int q0) {
+#pragma unroll
+                for (int u = 0; u < TILE / 32; ++u) {
+                    const int q = q0 + 32 * u + lane;
+                    l[u] = q < a.Tq ? __ldg(lse_bh + q) : -INFINITY;
+                    d[u] = q < a.Tq ? __ldg(d_bh + q) : 0.f;
+                }
+            };
+            pdl_wait();  // D
+            fetch(it0 * TILE);
+            for (int it = 0; it < n_it; ++it) {
+                if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(wc, &sh.p_ready, (it - 1) & 1, W_ROWSFREE, it))) break;
+#pragma unroll
+                for (int u = 0; u < TILE / 32; ++u) {
+                    sh.lse[32 * u + lane] = (l[u] == -INFINITY) ? -INFINITY : -l[u] * LOG2E;
+                    sh.dsum[32 * u + lane] = -d[u] * a.scale;
+                }
+                mbar_arrive_warp(&sh.s_full, lane);
+                if (it + 1 < n_it) fetch((it0 + it + 1) * TILE);
+            }
         }
     } else {
         // ------------------------------ compute ------------------------------
         const int quarter = warp & 3;
         const int part = warp >> 2;             // which 32 of the 128 query columns this thread owns
         const int row = quarter * 32 + lane;    // key row inside the tile = tensor-memory lane
-        const int tid = threadIdx.x;            // 0..511: the compute warps come first
         const int c0 = part * 32;
         const int kvrow = kv0 + row;
         const bool kv_ok = kvrow < a.Tk;
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-        const float* lse_bh = a.LSE + (int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH;
-        const float* d_bh = a.D + (int64_t)b * a.d_sB + (int64_t)h * a.d_sH;
         bool ok = true;
         uint32_t rs[32], rp[32];
-        // -LSE * log2e (threads 0..127; -inf past the end and for a fully dropped row, so that every p is 0) or
-        // -D * scale (threads 128..255) of query row q0 + (tid & 127): negated, so that both enter as FMA addends
-        auto fetch_lse_or_d = [&](int q0) -> float {
-            const int q = q0 + (tid & 127);
-            if (tid < TILE) {
-                if (q >= a.Tq) return -INFINITY;
-                const float l = __ldg(lse_bh + q);
-                return (l == -INFINITY) ? -INFINITY : -l * LOG2E;
-            }
-            return (q < a.Tq) ? -__ldg(d_bh + q) * a.scale : 0.f;
-        };
-        pdl_wait();  // D, and the zeroed dQ the store warp adds to
-        float staged_val = (tid < 2 * TILE && n_it > 0) ? fetch_lse_or_d(it0 * TILE) : 0.f;
+        if (n_it == 0) pdl_wait();  // the rows written below; with query tiles the barriers order everything
 
         // dQ of query tile j out of tensor memory into the K-major dO tile (column groups 2 and 3 only: this thread's
         // query row `row`, 32 columns), in the layout of a 128-byte-swizzled TMA box: 16-byte chunk c of row r at
-        // position c ^ (r & 7).  Called between the two halves of the NEXT tile's compute, when dP^T of that tile is
-        // done: its operand, the K-major dO tile, is then dead until the tile after it is prefetched, long enough for
-        // the bulk reduction, which keeps its source for ~1 600 cycles.  Groups 2, 3 run behind groups 0, 1 (the
-        // schedulers favour the older warps), late enough for dQ(j) to be complete when they get here.
-        auto drain_dq = [&](int j, uint32_t (&v)[32]) -> bool {
+        // position c ^ (r & 7).  Done in the middle of the NEXT tile, in two parts: read while dP^T of that tile is still
+        // being computed, stored when it is done: its operand, the K-major dO tile, is then dead until the tile after it
+        // is prefetched, long enough for the bulk reduction, which keeps its source for ~1 600 cycles.
+        auto read_dq = [&](int j, uint32_t (&v)[32]) -> bool {
             if (!__all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_full, j & 1, W_DQFULL, j))) return false;
             tc_fence_after_sync();
             tmem_ld32(trow + COL_DQ + 32 * (part & 1), v);
             tmem_wait_ld();
             tc_fence_before_sync();
             mbar_arrive_warp(&sh.dq_empty, lane);  // dQ is in registers: the next dQ = dS K may overwrite tensor memory
+            return true;
+        };
+        auto stage_dq = [&](const uint32_t (&v)[32]) {
             uint8_t* srow = sdO + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
@@ -476,7 +495,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
             fence_proxy_async_smem();
             mbar_arrive_warp(&sh.dq_staged, lane);
-            return true;
         };
 
         // V of this KV tile into tensor memory (A operand of dP^T = V dO^T): this thread's key row, 16 of the 64
@@ -500,23 +518,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
         for (int it = 0; ok && it < n_it; ++it) {
             const int q0 = (it0 + it) * TILE;
-            // stage LSE (threads 0..127) and D (threads 128..255) of this query tile into buffer it & 1.
-            // The buffer was last read two tiles ago; every compute thread passed that tile's ds_ready
-            // arrival long before this thread could get here (it has since waited on dq_full or s_full
-            // of the previous tile, which follow it).
-            // The value was fetched from global memory one tile ahead, so that its latency is not paid here.
-            if (tid < 2 * TILE) {
-                if (tid < TILE)
-                    sh.lse[it & 1][tid] = staged_val;
-                else
-                    sh.dsum[it & 1][tid - TILE] = staged_val;
-                mbar_arrive_warp(&sh.staged, lane);
-                if (it + 1 < n_it) staged_val = fetch_lse_or_d(q0 + TILE);
-            }
-            // an mbarrier rather than bar.sync: its wait is bounded, so a CTA that is
-            // winding down after a failed wait cannot strand warps at a barrier
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.staged, it & 1, W_STAGED, it));
-            if (!ok) break;
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, it & 1, W_SFULL, it));
             if (!ok) break;
             tc_fence_after_sync();
@@ -578,7 +579,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // p = exp2(s*scale*log2e - LSE*log2e) needs S^T only: dP^T is still being computed.  Two scores per
             // packed FMA (fma.rn.f32x2 gives the same bits as two scalar FMAs).
             {
-                const float4* lse4 = reinterpret_cast<const float4*>(sh.lse[it & 1] + c0);
+                const float4* lse4 = reinterpret_cast<const float4*>(sh.lse + c0);
                 const float2 c2 = make_float2(a.scale_log2e, a.scale_log2e);
 #pragma unroll
                 for (int g = 0; g < 8; ++g) {
@@ -615,16 +616,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tc_fence_before_sync();
                 mbar_arrive_warp(&sh.pt_ready, lane);
             }
+            if (it > 0 && part >= 2 && !(ok = read_dq(it - 1, rp))) break;  // rp is free until dP^T is loaded
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, it & 1, W_SFULL, 1000 + it));
             if (!ok) break;
             tc_fence_after_sync();
-            if (it > 0 && part >= 2 && !(ok = drain_dq(it - 1, rp))) break;  // rp is free until dP^T is loaded
+            if (it > 0 && part >= 2) stage_dq(rp);
             tmem_ld32(trow + COL_DP + c0, rp);
             tmem_wait_ld();
 
             // dS = p * (dP*scale - D*scale), two elements per packed instruction
             {
-                const float4* ds4 = reinterpret_cast<const float4*>(sh.dsum[it & 1] + c0);
+                const float4* ds4 = reinterpret_cast<const float4*>(sh.dsum + c0);
                 const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
                 if (dropped_some) {
                     // inverted dropout: a dropped pair keeps the -D term of dS but contributes neither dP (zeroed
@@ -683,24 +685,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mbar_arrive_warp(&sh.ds_ready, lane);
         }
 
-        // dV and dK of this KV tile are complete once dK of the last query tile is (dV precedes it on the tensor
-        // pipe).  Column groups 0,1 put dV (times 1/(1-p) for inverted dropout) into the MN-major Q tile and groups
-        // 2,3 dK into the K-major K tile, both dead by then, as the boxes of a 128-byte-swizzled TMA tile: 16-byte
-        // chunk c of row r at position c ^ (r & 7).
-        if (ok && n_it > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dk_done, (n_it - 1) & 1, W_BDONE, n_it));
+        // The accumulators: column groups 0, 1 put dV (times 1/(1-p) for inverted dropout), complete before the last dS
+        // was formed, into the K-major Q tile and groups 2, 3 put dK into the K-major K tile -- both dead after the last
+        // S^T -- as the boxes of a 128-byte-swizzled TMA tile: 16-byte chunk c of row r at position c ^ (r & 7).
+        if (ok && n_it > 0)
+            ok = __all_sync(0xffffffffu, mbar_wait(wc, (part < 2) ? &sh.dv_done : &sh.dk_done, (n_it - 1) & 1, W_BDONE, n_it));
         if (ok && n_it > 0) {
             tc_fence_after_sync();
             tmem_ld32(trow + ((part < 2) ? COL_DV + part * 32 : COL_DK + (part - 2) * 32), rs);
             tmem_wait_ld();
             const float f = (part < 2) ? a.dv_scale : 1.f;
-            uint8_t* srow = ((part < 2) ? sQm : sK) + (part & 1) * BOX_BYTES + row * 128;
+            uint8_t* srow = ((part < 2) ? sQ : sK) + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
                 *reinterpret_cast<float4*>(srow + ((c ^ (row & 7)) << 4)) =
                     make_float4(__uint_as_float(rs[4 * c]) * f, __uint_as_float(rs[4 * c + 1]) * f,
                                 __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
             fence_proxy_async_smem();
-            mbar_arrive_warp(&sh.acc_staged, lane);
+            mbar_arrive_warp((part < 2) ? &sh.dv_staged : &sh.dk_staged, lane);
         } else if (n_it == 0 && !SPLIT && kv_ok && !a.accum_dkdv) {
             // no query sees this KV tile: its dK and dV rows are zero
             float* out_row = (part < 2)
@@ -716,7 +718,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // CTA and held up the bulk stores of dV and dK behind it.)
         if (ok && n_it > 0 && part >= 2) {
             if (n_it > 1) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_out, (n_it - 2) & 1, W_DQOUT, n_it - 2));
-            if (ok) ok = drain_dq(n_it - 1, rs);
+            if (ok) ok = read_dq(n_it - 1, rs);
+            if (ok) stage_dq(rs);
         }
 
     }
@@ -735,7 +738,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int row = split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
-                const uint8_t* src = (lane < 16 ? sQm : sK) + (ch >> 3) * BOX_BYTES + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+                const uint8_t* src = (lane < 16 ? sQ : sK) + (ch >> 3) * BOX_BYTES + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
                 v[u] = u % ns < live ? ld_cluster_f4(mapa(src, u % ns)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
