@@ -64,6 +64,7 @@
 #include <mutex>
 
 #include "attn_kernels.cuh"
+#include "attn_prepass.cuh"
 #include "philox.h"
 
 namespace hk {
@@ -80,6 +81,19 @@ constexpr int COL_DV = 256;
 constexpr int COL_DK = 320;
 constexpr int COL_DQ = 384;
 constexpr int COL_V = 448;   // V of this KV tile, A operand of dP^T
+
+// The KV tile of a work item and the query tiles it loops over.
+struct Item {
+    int b, h, bh, kt;
+    int it0, n_it;  // first query tile (with splits: of this CTA) and number of them, 0 with splits alone; -1: there is no item
+    int live;       // splits that have query tiles
+    int pad;
+    __device__ __forceinline__ int kv0() const { return kt * TILE; }
+};
+
+// Work items beyond the first that may be known at a time: the load warp can be two items ahead of the store warp and asks
+// for one more, into a buffer that every warp has read.
+constexpr int ITEMS = 4;
 
 struct __align__(16) Shared {
     float lse[TILE];   // -LSE * log2e of the query tile; -inf for a row that saw no key or is past the end
@@ -98,15 +112,20 @@ struct __align__(16) Shared {
     uint64_t dv_staged, dk_staged;  // dV / dK of the CTA is staged for the bulk store
     uint64_t dq_staged;     // dQ of a query tile is staged (in the K-major dO tile) for the bulk reduction
     uint64_t dq_out;        // the bulk reduction has read the staged dQ tile: the K-major dO tile may be refilled
+    uint64_t dv_out, dk_out;  // the bulk store has read the staged dV / dK: the MN-major K / Q tile may be refilled
+    uint64_t item_full[ITEMS], item_empty[ITEMS];
+    Item item[ITEMS];       // the items taken over, decoded
+    uint4 answer;           // to a request for one
+    uint64_t answered;
     uint32_t tmem_base;
-    int abort_flag;
+    Abort abort;
 };
 
-constexpr int OFF_KK = 0;                // K, K-major swizzle   (S^T = K Q^T); dK staging at the end
-constexpr int OFF_KM = TILE_BYTES;       // K, MN-major swizzle  (dQ = dS K)
-constexpr int OFF_QK = 2 * TILE_BYTES;   // Q, K-major           (S^T); dV staging at the end
-constexpr int OFF_DOK = 3 * TILE_BYTES;  // dO, K-major          (dP^T)
-constexpr int OFF_QM = 4 * TILE_BYTES;   // Q, MN-major          (dK += dS^T Q)
+constexpr int OFF_KK = 0;                // K, K-major swizzle   (S^T = K Q^T)
+constexpr int OFF_KM = TILE_BYTES;       // K, MN-major swizzle  (dQ = dS K); staging of dV between items
+constexpr int OFF_QK = 2 * TILE_BYTES;   // Q, K-major           (S^T); staging of the last dV
+constexpr int OFF_DOK = 3 * TILE_BYTES;  // dO, K-major          (dP^T); staging of dQ
+constexpr int OFF_QM = 4 * TILE_BYTES;   // Q, MN-major          (dK += dS^T Q); staging of dK
 constexpr int OFF_DS = 5 * TILE_BYTES;   // dS boxes 0, 1 ([128 kv][32 q] each); first of all the landing buffer of V
 constexpr int OFF_DOM = 6 * TILE_BYTES;  // dO, MN-major         (dV += P^T dO); dS boxes 2, 3 once dV is done
 static_assert(OFF_DOM == OFF_DS + 2 * BOX_BYTES, "the four dS boxes are one descriptor: equally spaced");
@@ -118,9 +137,36 @@ static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may opt in to");
 
 enum WaitId {
     W_KVFULL = 201, W_QKFULL, W_QKEMPTY, W_QMFULL, W_QMFREE, W_SFULL, W_PREADY, W_BDONE, W_DSREADY, W_DQFULL, W_DQEMPTY,
-    W_ROWSFREE, W_DQSTAGED, W_ACCSTAGED, W_VREADY, W_DVDONE, W_DQOUT
+    W_ROWSFREE, W_DQSTAGED, W_ACCSTAGED, W_ACCOUT, W_VREADY, W_DVDONE, W_DQOUT, W_ITEM
 };
 
+}  // namespace bwd
+
+namespace bwd {
+__device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split, int ns) {
+    Item x;
+    // early KV tiles first: under the causal mask they see the most query tiles
+    x.bh = item % a.BH;
+    x.kt = item / a.BH;
+    x.b = x.bh / a.H;
+    x.h = x.bh - x.b * a.H;
+    const int n_qtiles = (a.Tq + TILE - 1) / TILE;
+    // first query tile with a row at or below the diagonal of this KV tile
+    x.it0 = 0;
+    if (a.causal) {
+        const long long first_q = (long long)x.kv0() + a.k_pos0 - a.q_pos0;  // smallest local q that sees key kv0
+        if (first_q > 0) x.it0 = (int)min((long long)n_qtiles, first_q / TILE);
+    }
+    x.n_it = n_qtiles - x.it0;
+    x.live = 1;
+    if (ns > 1) {  // each CTA of the cluster takes a contiguous run of the query tiles
+        const int run = (x.n_it + ns - 1) / ns, n_all = x.n_it;
+        x.it0 += split * run;
+        x.n_it = max(0, min(run, n_all - split * run));
+        x.live = (n_all + run - 1) / max(run, 1);
+    }
+    return x;
+}
 }  // namespace bwd
 
 // DROP: 0 none, 1 dense mask, 2 Philox.  SPLIT: a cluster shares the query tiles of a KV tile (an instantiation of its own:
@@ -132,7 +178,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const __grid_constant__ CUtensorMap mapQm, const __grid_constant__ CUtensorMap mapKm,
                 const __grid_constant__ CUtensorMap mapdOm, const __grid_constant__ CUtensorMap mapdQ,
                 const __grid_constant__ CUtensorMap mapdK, const __grid_constant__ CUtensorMap mapdV,
-                const BwdArgs a) {
+                const __grid_constant__ BwdArgs a) {
     using namespace bwd;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {  // never expected; refuse to run on a misplaced buffer
@@ -152,27 +198,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int warp = (int)uniform(threadIdx.x >> 5);  // uniform for the compiler too: see uniform()
     const int lane = threadIdx.x & 31;
 
-    // early KV tiles first: under the causal mask they see the most query tiles
     const int ns = SPLIT ? a.n_splits : 1;  // cluster size
     const int split = SPLIT ? (int)cluster_ctarank() : 0;
-    const int item = (int)blockIdx.x / ns;
-    const int bh = item % a.BH;
-    const int kt = item / a.BH;
-    const int b = bh / a.H;
-    const int h = bh - b * a.H;
-    const int kv0 = kt * TILE;
-    const int n_qtiles = (a.Tq + TILE - 1) / TILE;
+    const Item first = make_item(a, (int)blockIdx.x / ns, split, ns);
 
-    // first query tile with a row at or below the diagonal of this KV tile
-    int it0 = 0;
-    if (a.causal) {
-        const long long first_q = (long long)kv0 + a.k_pos0 - a.q_pos0;  // smallest local q that sees key kv0
-        if (first_q > 0) it0 = (int)min((long long)n_qtiles, first_q / TILE);
-    }
-    // With splits each CTA of the cluster takes a contiguous run of the query tiles.
-    const int n_all = n_qtiles - it0, run = (n_all + ns - 1) / ns;
-    if (SPLIT) it0 += split * run;
-    const int n_it = SPLIT ? max(0, min(run, n_all - split * run)) : n_all;
+    auto load_tile = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row, const Item& x) {
+        mbar_arrive_expect_tx(bar, TILE_BYTES);
+        tma_load_tile(dst, map, bar, row, x.h, x.b);
+    };
+    // everything an item starts with, in the order its first products need it: K, Q (S^T), V, dO (dP^T), MN-major dO (dV),
+    // Q (dK), K (dQ)
+    auto load_all = [&](const Item& x) {
+        load_tile(sK, &mapK, &sh.k_full, x.kv0(), x);
+        load_tile(sQ, &mapQ, &sh.q_full, x.it0 * TILE, x);
+        load_tile(sV, &mapV, &sh.v_full, x.kv0(), x);
+        load_tile(sdO, &mapdO, &sh.do_full, x.it0 * TILE, x);
+        load_tile(sdOm, &mapdOm, &sh.dom_full, x.it0 * TILE, x);
+        load_tile(sQm, &mapQm, &sh.qm_full, x.it0 * TILE, x);
+        load_tile(sKm, &mapKm, &sh.km_full, x.kv0(), x);
+    };
 
     // The load warp initialises the barriers its copies complete on and issues the loads of the first tile at once:
     // the other warps meet those barriers only after the __syncthreads below, and ~1 000 cycles of set-up (the other
@@ -185,36 +229,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.do_full, 1);
         mbar_init(&sh.qm_full, 1);
         mbar_init(&sh.dom_full, 1);
-        fence_mbar_init();
-        if (n_it > 0) {
-            // in the order the first products need them: K, Q (S^T), V, dO (dP^T), MN-major dO (dV), Q (dK), K (dQ)
-            const int q0 = it0 * TILE;
-            mbar_arrive_expect_tx(&sh.k_full, TILE_BYTES);
-            tma_load_4d(sK, &mapK, &sh.k_full, 0, kv0, h, b);
-            tma_load_4d(sK + BOX_BYTES, &mapK, &sh.k_full, HALF_D, kv0, h, b);
-            mbar_arrive_expect_tx(&sh.q_full, TILE_BYTES);
-            tma_load_4d(sQ, &mapQ, &sh.q_full, 0, q0, h, b);
-            tma_load_4d(sQ + BOX_BYTES, &mapQ, &sh.q_full, HALF_D, q0, h, b);
-            mbar_arrive_expect_tx(&sh.v_full, TILE_BYTES);
-            tma_load_4d(sV, &mapV, &sh.v_full, 0, kv0, h, b);
-            tma_load_4d(sV + BOX_BYTES, &mapV, &sh.v_full, HALF_D, kv0, h, b);
-            mbar_arrive_expect_tx(&sh.do_full, TILE_BYTES);
-            tma_load_4d(sdO, &mapdO, &sh.do_full, 0, q0, h, b);
-            tma_load_4d(sdO + BOX_BYTES, &mapdO, &sh.do_full, HALF_D, q0, h, b);
-            mbar_arrive_expect_tx(&sh.dom_full, TILE_BYTES);
-            tma_load_4d(sdOm, &mapdOm, &sh.dom_full, 0, q0, h, b);
-            tma_load_4d(sdOm + BOX_BYTES, &mapdOm, &sh.dom_full, HALF_D, q0, h, b);
-            mbar_arrive_expect_tx(&sh.qm_full, TILE_BYTES);
-            tma_load_4d(sQm, &mapQm, &sh.qm_full, 0, q0, h, b);
-            tma_load_4d(sQm + BOX_BYTES, &mapQm, &sh.qm_full, HALF_D, q0, h, b);
-            mbar_arrive_expect_tx(&sh.km_full, TILE_BYTES);
-            tma_load_4d(sKm, &mapKm, &sh.km_full, 0, kv0, h, b);
-            tma_load_4d(sKm + BOX_BYTES, &mapKm, &sh.km_full, HALF_D, kv0, h, b);
+        for (int i = 0; i < ITEMS; ++i) {
+            mbar_init(&sh.item_full[i], 1);
+            mbar_init(&sh.item_empty[i], NUM_THREADS / 32 - 1);  // every warp but the load warp
         }
+        mbar_init(&sh.answered, 1);
+        fence_mbar_init();
+        if (first.n_it > 0) load_all(first);
     }
     if (threadIdx.x == 0) {
         // compute-warp barriers count one arrival per warp
-        mbar_init(&sh.v_ready, NUM_COMPUTE / 32);
+        mbar_init(&sh.v_ready, 8);    // column groups 2, 3 copy V
         mbar_init(&sh.qk_free, 1);
         mbar_init(&sh.dok_free, 1);
         mbar_init(&sh.s_full, 2);     // the commit of S^T and the warp that stages LSE and D
@@ -230,7 +255,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.dq_out, 1);
         mbar_init(&sh.dv_staged, 8);  // column groups 0, 1
         mbar_init(&sh.dk_staged, 8);  // column groups 2, 3
-        sh.abort_flag = 0;
+        mbar_init(&sh.dv_out, 1);
+        mbar_init(&sh.dk_out, 1);
+        sh.abort.id = 0;
         fence_mbar_init();
     }
     if (warp == W_MMA) {
@@ -240,192 +267,262 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = uniform(sh.tmem_base);
-    WaitCtx wc{&sh.abort_flag, a.status};
+    // The CTA holds all 512 columns of tensor memory, so its allocation starts at address 0: with the base a constant, so is
+    // every operand of the MMAs, and none has to be moved to a uniform register.
+    constexpr uint32_t tmem = 0;
+    if (sh.tmem_base != tmem) {  // never expected
+        sh.abort.id = 298;
+    }
+    WaitNote wc{&sh.abort};
 
+    // Work items.  A CTA starts with the one of its blockIdx and then, until none is left, takes over those of CTAs that have
+    // not started yet (cluster launch control), so that the loads and the first S^T of the next KV tile run under the last
+    // products and the stores of this one.  One CTA per item spent ~13 000 cycles on set-up, first loads, first tile and last
+    // stores beside ~5 000 per query tile; B8 H12 T1024 (768 items of 1 .. 8 tiles) 104 -> 93 us, B32 H25 T1024 995 -> 895.
+    // The load warp asks, decodes the answer and puts the item into a ring that every warp reads in its own time.
+    struct Items {
+        Item x;    // the current one
+        int n;     // items read from the ring
+    };
+    // Goes on to the next item; false if there is none (or a wait gave up).  All lanes of a warp, or one thread alone (`solo`).
+    auto next_item = [&](Items& s, bool solo) -> bool {
+        if (SPLIT) return false;
+        const int buf = s.n % ITEMS;
+        bool ok = mbar_wait(wc, &sh.item_full[buf], (s.n / ITEMS) & 1, W_ITEM, s.n);
+        if (!solo) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
+        s.x = sh.item[buf];
+        ++s.n;
+        if (!solo) __syncwarp();
+        if (solo || lane == 0) mbar_arrive(&sh.item_empty[buf]);
+        return s.x.n_it >= 0;
+    };
     if (warp == W_LOAD) {
         // ------------------------------ TMA producer ------------------------------
-        if (lane == 0 && n_it > 0) {
-            // the loads of the first tile were issued before the set-up barrier
-            int issued_q = 1, issued_do = 1, issued_qm = 1, issued_dom = 1;
-            auto load_q = [&](int q0) {
-                mbar_arrive_expect_tx(&sh.q_full, TILE_BYTES);
-                tma_load_4d(sQ, &mapQ, &sh.q_full, 0, q0, h, b);
-                tma_load_4d(sQ + BOX_BYTES, &mapQ, &sh.q_full, HALF_D, q0, h, b);
-                ++issued_q;
+        if (lane == 0 && first.n_it > 0) {
+            Item cur = first;
+            int published = 0;
+            int items = 0;  // whose accumulators have left
+            bool tok = true, more = !SPLIT;
+            // on to the next item: publishes what the request brought, if one was made
+            auto next = [&]() -> bool {
+                const int buf = published % ITEMS;
+                if (!more) return false;
+                int id = -1;
+                if (a.take_over) {
+                    if (!(tok = mbar_wait(wc, &sh.answered, published & 1, W_ITEM, published))) return false;
+                    id = clc_read(&sh.answer);
+                    fence_proxy_async_smem();  // the answer's buffer is next written by the async proxy
+                }
+                if (published >= ITEMS && !(tok = mbar_wait(wc, &sh.item_empty[buf], (published / ITEMS - 1) & 1, W_ITEM, 1000 + published)))
+                    return false;
+                more = id >= 0;
+                if (more) {
+                    cur = make_item(a, id, 0, 1);
+                    sh.item[buf] = cur;
+                } else {
+                    sh.item[buf].n_it = -1;
+                }
+                mbar_arrive(&sh.item_full[buf]);
+                ++published;
+                return more;
             };
-            auto load_do = [&](int q0) {
-                mbar_arrive_expect_tx(&sh.do_full, TILE_BYTES);
-                tma_load_4d(sdO, &mapdO, &sh.do_full, 0, q0, h, b);
-                tma_load_4d(sdO + BOX_BYTES, &mapdO, &sh.do_full, HALF_D, q0, h, b);
-                ++issued_do;
-            };
-            auto load_qm = [&](int q0) {
-                mbar_arrive_expect_tx(&sh.qm_full, TILE_BYTES);
-                tma_load_4d(sQm, &mapQm, &sh.qm_full, 0, q0, h, b);
-                tma_load_4d(sQm + BOX_BYTES, &mapQm, &sh.qm_full, HALF_D, q0, h, b);
-                ++issued_qm;
-            };
-            auto load_dom = [&](int q0) {
-                mbar_arrive_expect_tx(&sh.dom_full, TILE_BYTES);
-                tma_load_4d(sdOm, &mapdOm, &sh.dom_full, 0, q0, h, b);
-                tma_load_4d(sdOm + BOX_BYTES, &mapdOm, &sh.dom_full, HALF_D, q0, h, b);
-                ++issued_dom;
-            };
-            bool tok = true;
-            for (int it = 0; it + 1 < n_it; ++it) {
-                const int q1 = (it0 + it + 1) * TILE;
-                // K-major Q: free as soon as S^T(it) is done
-                if (!(tok = mbar_wait(wc, &sh.qk_free, it & 1, W_QKEMPTY, it))) break;
-                load_q(q1);
-                // K-major dO: dQ(it-1) passes through the tile once dP^T(it) is done; free when the reduction has read it
-                if (it == 0) {
-                    if (!(tok = mbar_wait(wc, &sh.dok_free, 0, W_QKEMPTY, 1000))) break;
-                } else if (!(tok = mbar_wait(wc, &sh.dq_out, (it - 1) & 1, W_DQOUT, it - 1))) break;
-                load_do(q1);
-                // MN-major Q: free once dK(it) is done
-                if (!(tok = mbar_wait(wc, &sh.dk_done, it & 1, W_QMFREE, it))) break;
-                load_qm(q1);
-                // MN-major dO doubles as staging area of two dS boxes: free once dQ(it) is done
-                if (!(tok = mbar_wait(wc, &sh.dq_full, it & 1, W_QMFREE, 1000 + it))) break;
-                load_dom(q1);
+            // The query tiles of all items in a row: iteration n of the loop loads K-major Q (and K) of tile n and the rest of
+            // tile n - 1, each as soon as its buffer is free, in the order in which that happens.  The K-major Q tile is
+            // free first (S^T runs a tile ahead); behind the others its load came late for S^T.
+            struct Tile {
+                Item x;
+                int it;
+            } t1, t2{first, -1};  // tile n - 1, tile n
+            for (int n = 0;; ++n) {
+                t1 = t2;
+                if (++t2.it >= cur.n_it && next()) t2.it = 0;
+                if (!tok) break;
+                t2.x = cur;
+                const bool have = t2.it < cur.n_it;
+                // Asked for a tile before it is needed: at the start of a long item it would be taken from a CTA that is
+                // through sooner (training step at B2 H16 T2000, reproducible: 190 instead of 183 us).
+                if (!SPLIT && a.take_over && t2.it + 1 == cur.n_it) {
+                    mbar_arrive_expect_tx(&sh.answered, sizeof(uint4));
+                    clc_try_cancel(&sh.answer, &sh.answered);
+                }
+                if (have && n > 0) {  // (tile 0: issued before the set-up barrier)
+                    // free as soon as S^T(n - 1) is done
+                    if (!(tok = mbar_wait(wc, &sh.qk_free, (n - 1) & 1, W_QKEMPTY, n))) break;
+                    if (t2.it == 0) load_tile(sK, &mapK, &sh.k_full, t2.x.kv0(), t2.x);
+                    load_tile(sQ, &mapQ, &sh.q_full, (t2.x.it0 + t2.it) * TILE, t2.x);
+                }
+                const int g = n - 2;  // the tile before tile n - 1
+                const int q1 = (t1.x.it0 + t1.it) * TILE;
+                if (n > 1) {
+                    auto free = [&](uint64_t* bar, int phase, int id) { return tok = mbar_wait(wc, bar, phase & 1, id, n); };
+                    // K-major dO: dQ(g-1) passes through the tile once dP^T(g) is done; free when the reduction has read it
+                    if (!(g == 0 ? free(&sh.dok_free, 0, W_QKEMPTY) : free(&sh.dq_out, g - 1, W_DQOUT))) break;
+                    load_tile(sdO, &mapdO, &sh.do_full, q1, t1.x);
+                    if (t1.it > 0) {
+                        // MN-major Q: free once dK(g) is done
+                        if (!free(&sh.dk_done, g, W_QMFREE)) break;
+                        load_tile(sQm, &mapQm, &sh.qm_full, q1, t1.x);
+                    }
+                    // MN-major dO doubles as staging area of two dS boxes: free once dQ(g) is done; so is that of the other
+                    // two, where V of the next item lands
+                    if (!free(&sh.dq_full, g, W_QMFREE)) break;
+                    if (t1.it == 0) load_tile(sV, &mapV, &sh.v_full, t1.x.kv0(), t1.x);
+                    load_tile(sdOm, &mapdOm, &sh.dom_full, q1, t1.x);
+                    if (t1.it == 0) {
+                        // dK leaves through the MN-major Q tile, dV through the MN-major K tile
+                        if (!free(&sh.dk_out, items, W_ACCOUT)) break;
+                        load_tile(sQm, &mapQm, &sh.qm_full, q1, t1.x);
+                        if (!free(&sh.dv_out, items, W_ACCOUT)) break;
+                        load_tile(sKm, &mapKm, &sh.km_full, t1.x.kv0(), t1.x);
+                        ++items;
+                    }
+                }
+                if (!have) break;
             }
-            // Do not leave the CTA while bulk copies into its shared memory are in flight.
-            auto drain = [](uint64_t* bar, uint32_t parity) {
-#pragma unroll 1
-                for (int i = 0; i < 100000 && !mbar_try_wait(bar, parity); ++i) {}
-            };
-            drain(&sh.k_full, 0);
-            drain(&sh.v_full, 0);
-            drain(&sh.km_full, 0);
-            drain(&sh.q_full, (issued_q - 1) & 1);
-            drain(&sh.do_full, (issued_do - 1) & 1);
-            drain(&sh.qm_full, (issued_qm - 1) & 1);
-            drain(&sh.dom_full, (issued_dom - 1) & 1);
         }
     } else if (warp == W_MMA) {
         // ------------------------------ MMA issuer ------------------------------
         // The whole warp runs this code with uniform control flow; only the tcgen05 instructions are predicated on
         // the elected lane (see umma_ss_tf32_lead).
-        if (n_it > 0) {
-            const uint32_t leader = elect_one_sync();
-            auto wait = [&](uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
-                return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
-            };
-            constexpr uint32_t IDESC_ST = make_idesc_tf32(TILE, TILE, false, false);     // K-major x K-major, N = 128
-            constexpr uint32_t IDESC_TS = make_idesc_tf32(TILE, HEAD_DIM, false, true);  // tmem A, MN-major B, N = 64
-            constexpr uint32_t IDESC_DQ = make_idesc_tf32(TILE, HEAD_DIM, true, true);   // MN-major A and B, N = 64
-            const uint32_t k_addr = smem_u32(sK), q_addr = smem_u32(sQ), do_addr = smem_u32(sdO), qm_addr = smem_u32(sQm),
-                           dom_addr = smem_u32(sdOm), km_addr = smem_u32(sKm), ds_addr = smem_u32(sdS);
-            // S^T of query tile `it` (local index) as soon as K and Q have landed; the exponentials need nothing else
-            auto issue_st = [&](int it) -> bool {
-                if (it == 0 && !wait(&sh.k_full, 0, W_KVFULL, 0)) return false;
-                if (!wait(&sh.q_full, it & 1, W_QKFULL, it)) return false;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = 0; kk < HEAD_DIM / 8; ++kk)  // S^T = K Q^T
-                    umma_ss_tf32_lead(leader, tmem + COL_S, kmajor_desc(k_addr, kk, BOX_BYTES), kmajor_desc(q_addr, kk, BOX_BYTES),
-                                 IDESC_ST, kk > 0);
-                umma_commit_lead(leader, &sh.s_full);
-                umma_commit_lead(leader, &sh.qk_free);
-                return true;
-            };
-            // dP^T = V dO^T, V from tensor memory
-            auto issue_dp = [&](int it) -> bool {
-                if (it == 0 && !wait(&sh.v_ready, 0, W_VREADY, 0)) return false;
-                if (!wait(&sh.do_full, it & 1, W_QKFULL, 1000 + it)) return false;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = 0; kk < HEAD_DIM / 8; ++kk)
-                    umma_ts_tf32_lead(leader, tmem + COL_DP, tmem + COL_V + kk * 8, kmajor_desc(do_addr, kk, BOX_BYTES), IDESC_ST, kk > 0);
-                umma_commit_lead(leader, &sh.dp_full);
-                umma_commit_lead(leader, &sh.dok_free);
-                return true;
-            };
-            bool ok = issue_st(0) && issue_dp(0);
-            for (int it = 0; ok && it < n_it; ++it) {
-                const uint32_t par = it & 1;
-                if (!(ok = wait(&sh.dom_full, par, W_QMFULL, it))) break;
-                // dV += P^T dO
-                if (!(ok = wait(&sh.pt_ready, par, W_PREADY, it))) break;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = 0; kk < TILE / 8; ++kk)
-                    umma_ts_tf32_lead(leader, tmem + COL_DV, tmem + COL_S + kk * 8, mnmajor_desc(dom_addr, kk, BOX_BYTES), IDESC_TS,
-                                      (it > 0 || kk > 0) ? 1u : 0u);
-                umma_commit_lead(leader, &sh.dv_done);  // MN-major dO consumed: two of the dS boxes may be staged over it
-                // next tile's S^T: P^T of this tile was consumed by the MMAs just issued
-                if (it + 1 < n_it && !(ok = issue_st(it + 1))) break;
-                if (!(ok = wait(&sh.qm_full, par, W_QMFULL, 1000 + it))) break;
-                // dK += dS^T Q
-                if (!(ok = wait(&sh.p_ready, par, W_PREADY, 1000 + it))) break;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = 0; kk < TILE / 8; ++kk)
-                    umma_ts_tf32_lead(leader, tmem + COL_DK, tmem + COL_DP + kk * 8, mnmajor_desc(qm_addr, kk, BOX_BYTES), IDESC_TS,
-                                      (it > 0 || kk > 0) ? 1u : 0u);
-                umma_commit_lead(leader, &sh.dk_done);  // MN-major Q consumed
-                // dQ = dS K once dS is staged (shortly after dS^T was stored) and the previous dQ has left tensor memory
-                if (!(ok = wait(&sh.ds_ready, par, W_DSREADY, it))) break;
-                if (it > 0 && !(ok = wait(&sh.dq_empty, (it - 1) & 1, W_DQEMPTY, it))) break;
-                if (it == 0 && !(ok = wait(&sh.km_full, 0, W_KVFULL, 2))) break;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = 0; kk < TILE / 8; ++kk)
-                    umma_ss_tf32_lead(leader, tmem + COL_DQ, mnmajor_desc(ds_addr, kk, BOX_BYTES),
-                                      mnmajor_desc(km_addr, kk, BOX_BYTES), IDESC_DQ, kk > 0);
-                umma_commit_lead(leader, &sh.dq_full);  // also: the dS staging area is free again
-                // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
-                if (it + 1 < n_it && !(ok = issue_dp(it + 1))) break;
+        const uint32_t leader = elect_one_sync();
+        auto wait = [&](uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
+            return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
+        };
+        constexpr uint32_t IDESC_ST = make_idesc_tf32(TILE, TILE, false, false);     // K-major x K-major, N = 128
+        constexpr uint32_t IDESC_TS = make_idesc_tf32(TILE, HEAD_DIM, false, true);  // tmem A, MN-major B, N = 64
+        constexpr uint32_t IDESC_DQ = make_idesc_tf32(TILE, HEAD_DIM, true, true);   // MN-major A and B, N = 64
+        const Desc k_desc = kmajor_desc(smem_u32(sK), 0, BOX_BYTES), q_desc = kmajor_desc(smem_u32(sQ), 0, BOX_BYTES),
+                       do_desc = kmajor_desc(smem_u32(sdO), 0, BOX_BYTES), qm_desc = mnmajor_desc(smem_u32(sQm), 0, BOX_BYTES),
+                       dom_desc = mnmajor_desc(smem_u32(sdOm), 0, BOX_BYTES), km_desc = mnmajor_desc(smem_u32(sKm), 0, BOX_BYTES),
+                       ds_desc = mnmajor_desc(smem_u32(sdS), 0, BOX_BYTES);
+        // S^T of query tile `g` as soon as K (of item `item`, at its first tile) and Q have landed; the exponentials need
+        // nothing else
+        auto issue_st = [&](int g, bool first_tile, int item) -> bool {
+            if (first_tile && !wait(&sh.k_full, item & 1, W_KVFULL, 0)) return false;
+            if (!wait(&sh.q_full, g & 1, W_QKFULL, g)) return false;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t o = 0; o < 2; ++o)  // S^T = K Q^T
+                umma_ss4<KMAJOR_STEP, KMAJOR_STEP>(leader, tmem + COL_S, k_desc + o * BOX_BYTES, q_desc + o * BOX_BYTES, IDESC_ST, o);
+            umma_commit_lead(leader, &sh.s_full);
+            umma_commit_lead(leader, &sh.qk_free);
+            return true;
+        };
+        // dP^T = V dO^T, V from tensor memory
+        auto issue_dp = [&](int g, bool first_tile, int item) -> bool {
+            if (first_tile && !wait(&sh.v_ready, item & 1, W_VREADY, 0)) return false;
+            if (!wait(&sh.do_full, g & 1, W_QKFULL, 1000 + g)) return false;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t o = 0; o < 2; ++o)
+                umma_ts4<KMAJOR_STEP>(leader, tmem + COL_DP, tmem + COL_V + o * 32, do_desc + o * BOX_BYTES, IDESC_ST, o);
+            umma_commit_lead(leader, &sh.dp_full);
+            umma_commit_lead(leader, &sh.dok_free);
+            return true;
+        };
+        Items s{first, 0};
+        int n_it = first.n_it;
+        bool ok = n_it > 0 && issue_st(0, true, 0) && issue_dp(0, true, 0);
+        int it = 0, item = 0;  // query tile of the item, item
+        for (int g = 0; ok; ++g) {
+            const uint32_t par = g & 1;
+            if (!(ok = wait(&sh.dom_full, par, W_QMFULL, g))) break;
+            // dV += P^T dO
+            if (!(ok = wait(&sh.pt_ready, par, W_PREADY, g))) break;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t o = 0; o < 4; ++o)
+                umma_ts4<MNMAJOR_STEP>(leader, tmem + COL_DV, tmem + COL_S + o * 32, dom_desc + o * 4096, IDESC_TS, (it > 0 || o > 0) ? 1u : 0u);
+            umma_commit_lead(leader, &sh.dv_done);  // MN-major dO consumed: two of the dS boxes may be staged over it
+            // next tile's S^T: P^T of this tile was consumed by the MMAs just issued
+            const bool last = it + 1 == n_it;
+            const bool more = !last || next_item(s, false);
+            if (more && !(ok = issue_st(g + 1, last, item + 1))) break;
+            if (!(ok = wait(&sh.qm_full, par, W_QMFULL, 1000 + g))) break;
+            // dK += dS^T Q
+            if (!(ok = wait(&sh.p_ready, par, W_PREADY, 1000 + g))) break;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t o = 0; o < 4; ++o)
+                umma_ts4<MNMAJOR_STEP>(leader, tmem + COL_DK, tmem + COL_DP + o * 32, qm_desc + o * 4096, IDESC_TS, (it > 0 || o > 0) ? 1u : 0u);
+            umma_commit_lead(leader, &sh.dk_done);  // MN-major Q consumed
+            // dQ = dS K once dS is staged (shortly after dS^T was stored) and the previous dQ has left tensor memory
+            if (!(ok = wait(&sh.ds_ready, par, W_DSREADY, g))) break;
+            if (g > 0 && !(ok = wait(&sh.dq_empty, (g - 1) & 1, W_DQEMPTY, g))) break;
+            if (it == 0 && !(ok = wait(&sh.km_full, item & 1, W_KVFULL, 2))) break;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (uint32_t o = 0; o < 4; ++o)
+                umma_ss4<MNMAJOR_STEP, MNMAJOR_STEP>(leader, tmem + COL_DQ, ds_desc + o * 4096, km_desc + o * 4096, IDESC_DQ, o);
+            umma_commit_lead(leader, &sh.dq_full);  // also: the dS staging area is free again
+            if (!more) break;
+            // next tile's dP^T: dS^T of this tile was consumed by the MMAs just issued
+            if (!(ok = issue_dp(g + 1, last, item + 1))) break;
+            ++it;
+            if (last) {
+                it = 0;
+                ++item;
+                n_it = (int)uniform(s.x.n_it);
             }
         }
     } else if (warp == W_STORE) {
         // ------------------------------ store warp ------------------------------
-        // Everything that leaves the CTA: the staged dQ tiles (bulk reductions) and, at the end, dV and dK (bulk
+        // Everything that leaves the CTA: the staged dQ tiles (bulk reductions) and, at the end of an item, dK and dV (bulk
         // stores).  A thread of its own, so that a reduction is issued the moment its tile is staged.
-        if (lane == 0 && n_it > 0) {
+        if (lane == 0) {
             pdl_wait();
             tma_prefetch_desc(&mapdK);
             tma_prefetch_desc(&mapdV);
             tma_prefetch_desc(&mapdQ);
-            // dQ of query tile j, staged in the K-major dO tile: add it to global memory; once the reduction has read
+            Items s{first, 0};
+            int g = 0, items = 0;
+            bool tok = first.n_it > 0;
+            // dQ of the next query tile, staged in the K-major dO tile: add it to global memory; once the reduction has read
             // the tile, hand it back to the load warp
-            auto reduce_dq = [&](int j) -> bool {
-                if (!mbar_wait(wc, &sh.dq_staged, j & 1, W_DQSTAGED, j)) return false;
-                const int q = (it0 + j) * TILE;
+            auto reduce_dq = [&](int it) -> bool {
+                if (!mbar_wait(wc, &sh.dq_staged, g & 1, W_DQSTAGED, g)) return false;
+                const int q = (s.x.it0 + it) * TILE;
                 if (a.det_dq) {  // this KV tile's slab of partial dQ; reduce_dq_slabs adds the slabs in a fixed order
-                    tma_store_4d(&mapdQ, sdO, 0, q, h, kt * a.B + b);
-                    tma_store_4d(&mapdQ, sdO + BOX_BYTES, HALF_D, q, h, kt * a.B + b);
+                    tma_store_tile(&mapdQ, sdO, q, s.x.h, s.x.kt * a.B + s.x.b);
                 } else {
-                    tma_reduce_add_4d(&mapdQ, sdO, 0, q, h, b);
-                    tma_reduce_add_4d(&mapdQ, sdO + BOX_BYTES, HALF_D, q, h, b);
+                    tma_reduce_add_tile(&mapdQ, sdO, q, s.x.h, s.x.b);
                 }
                 bulk_commit_group();
                 bulk_wait_group_read_all();
                 mbar_arrive(&sh.dq_out);
+                ++g;
                 return true;
             };
-            bool tok = true;
-            for (int j = 0; tok && j + 1 < n_it; ++j) tok = reduce_dq(j);  // the last tile's dQ follows dV and dK
-            // dV and dK, staged by the compute warps in the K-major Q and K tiles (dead after the last S^T): stored --
-            // added, if the caller accumulates -- with bulk copies, each as soon as it is staged; a thread-per-row store
-            // would be 32 lines per instruction.  Over a cluster they are added up below.
-            auto store_acc = [&](uint64_t* bar, const CUtensorMap* map, const uint8_t* src) -> bool {
-                if (!mbar_wait(wc, bar, 0, W_ACCSTAGED, 0)) return false;
-                if (!SPLIT) {
-                    if (a.accum_dkdv) {
-                        tma_reduce_add_4d(map, src, 0, kv0, h, b);
-                        tma_reduce_add_4d(map, src + BOX_BYTES, HALF_D, kv0, h, b);
-                    } else {
-                        tma_store_4d(map, src, 0, kv0, h, b);
-                        tma_store_4d(map, src + BOX_BYTES, HALF_D, kv0, h, b);
-                    }
-                    bulk_commit_group();
+            // dK and dV, staged by the compute warps (see there): stored -- added, if the caller accumulates -- with bulk
+            // copies, each as soon as it is staged; a thread-per-row store would be 32 lines per instruction.  Over a cluster
+            // they are added up below.
+            auto store_acc = [&](bool v, bool more) -> bool {
+                if (!mbar_wait(wc, v ? &sh.dv_staged : &sh.dk_staged, items & 1, W_ACCSTAGED, items)) return false;
+                if (SPLIT) return true;
+                const CUtensorMap* map = v ? &mapdV : &mapdK;
+                const uint8_t* src = !v ? sQm : more ? sKm : sQ;
+                if (a.accum_dkdv)
+                    tma_reduce_add_tile(map, src, s.x.kv0(), s.x.h, s.x.b);
+                else
+                    tma_store_tile(map, src, s.x.kv0(), s.x.h, s.x.b);
+                bulk_commit_group();
+                if (more) {  // the load warp waits for the tile
+                    bulk_wait_group_read_all();
+                    mbar_arrive(v ? &sh.dv_out : &sh.dk_out);
                 }
                 return true;
             };
-            if (tok && store_acc(&sh.dv_staged, &mapdV, sQ) && store_acc(&sh.dk_staged, &mapdK, sK))
-                reduce_dq(n_it - 1);
+            while (tok) {
+                for (int it = 0; tok && it + 1 < s.x.n_it; ++it) tok = reduce_dq(it);  // the last tile's dQ follows dK and dV
+                if (!tok) break;
+                Items nx = s;
+                const bool more = next_item(nx, true);
+                tok = store_acc(!more, more) && store_acc(more, more) && reduce_dq(s.x.n_it - 1);
+                ++items;
+                if (!more) break;
+                s = nx;
+            }
             // the copies have read their shared-memory sources; they complete on their own
             bulk_wait_group_read_all();
         }
@@ -435,29 +532,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // scaled so that both enter the arithmetic as FMA addends, once the compute warps are through with the previous
         // tile's (they are when dS^T is stored).  A warp of its own: eight compute warps that did this beside their work,
         // and sixteen that waited for it, were ~400 cycles per tile longer at it.
-        if (n_it > 0) {
-            const float* lse_bh = a.LSE + (int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH;
-            const float* d_bh = a.D + (int64_t)b * a.d_sB + (int64_t)h * a.d_sH;
+        Items s{first, 0};
+        if (first.n_it > 0) {
             float l[TILE / 32], d[TILE / 32];
-            auto fetch = [&](int q0) {
+            auto fetch = [&](int it) {
+                const float* lse_bh = a.LSE + (int64_t)s.x.b * a.lse_sB + (int64_t)s.x.h * a.lse_sH;
+                const float* d_bh = a.D + (int64_t)s.x.b * a.d_sB + (int64_t)s.x.h * a.d_sH;
 #pragma unroll
                 for (int u = 0; u < TILE / 32; ++u) {
-                    const int q = q0 + 32 * u + lane;
+                    const int q = (s.x.it0 + it) * TILE + 32 * u + lane;
                     l[u] = q < a.Tq ? __ldg(lse_bh + q) : -INFINITY;
                     d[u] = q < a.Tq ? __ldg(d_bh + q) : 0.f;
                 }
             };
             pdl_wait();  // D
-            fetch(it0 * TILE);
-            for (int it = 0; it < n_it; ++it) {
-                if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(wc, &sh.p_ready, (it - 1) & 1, W_ROWSFREE, it))) break;
+            fetch(0);
+            int it = 0;
+            for (int g = 0;; ++g) {
+                if (g > 0 && !__all_sync(0xffffffffu, mbar_wait(wc, &sh.p_ready, (g - 1) & 1, W_ROWSFREE, g))) break;
 #pragma unroll
                 for (int u = 0; u < TILE / 32; ++u) {
                     sh.lse[32 * u + lane] = (l[u] == -INFINITY) ? -INFINITY : -l[u] * LOG2E;
                     sh.dsum[32 * u + lane] = -d[u] * a.scale;
                 }
                 mbar_arrive_warp(&sh.s_full, lane);
-                if (it + 1 < n_it) fetch((it0 + it + 1) * TILE);
+                if (++it == s.x.n_it) {
+                    if (!next_item(s, false)) break;
+                    it = 0;
+                }
+                fetch(it);
             }
         }
     } else {
@@ -466,12 +569,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const int part = warp >> 2;             // which 32 of the 128 query columns this thread owns
         const int row = quarter * 32 + lane;    // key row inside the tile = tensor-memory lane
         const int c0 = part * 32;
-        const int kvrow = kv0 + row;
-        const bool kv_ok = kvrow < a.Tk;
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
         bool ok = true;
         uint32_t rs[32], rp[32];
-        if (n_it == 0) pdl_wait();  // the rows written below; with query tiles the barriers order everything
 
         // dQ of query tile j out of tensor memory into the K-major dO tile (column groups 2 and 3 only: this thread's
         // query row `row`, 32 columns), in the layout of a 128-byte-swizzled TMA box: 16-byte chunk c of row r at
@@ -497,28 +597,36 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mbar_arrive_warp(&sh.dq_staged, lane);
         };
 
-        // V of this KV tile into tensor memory (A operand of dP^T = V dO^T): this thread's key row, 16 of the 64
-        // columns, read from the 128-byte-swizzled landing buffer (16-byte chunk c of row r at position c ^ (r & 7))
-        if (n_it > 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.v_full, 0, W_KVFULL, 3));
-            if (ok) {
-                uint32_t rv[16];
-                const uint8_t* vrow = sV + (part >> 1) * BOX_BYTES + row * 128;
+        // V of an item's KV tile into tensor memory (A operand of dP^T = V dO^T), by column groups 2 and 3, which are there
+        // first: this thread's key row, 32 of the 64 columns, read from the 128-byte-swizzled landing buffer (16-byte chunk
+        // c of row r at position c ^ (r & 7))
+        auto copy_v = [&](int item, uint32_t (&v)[32]) -> bool {
+            if (!__all_sync(0xffffffffu, mbar_wait(wc, &sh.v_full, item & 1, W_KVFULL, 3))) return false;
+            const uint8_t* vrow = sV + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(vrow + (((4 * (part & 1) + c) ^ (row & 7)) << 4));
-                    rv[4 * c] = x.x; rv[4 * c + 1] = x.y; rv[4 * c + 2] = x.z; rv[4 * c + 3] = x.w;
-                }
-                tmem_st16(trow + COL_V + 16 * part, rv);
-                tmem_wait_st();
-                tc_fence_before_sync();
-                mbar_arrive_warp(&sh.v_ready, lane);
+            for (int c = 0; c < 8; ++c) {
+                const uint4 x = *reinterpret_cast<const uint4*>(vrow + ((c ^ (row & 7)) << 4));
+                v[4 * c] = x.x; v[4 * c + 1] = x.y; v[4 * c + 2] = x.z; v[4 * c + 3] = x.w;
             }
-        }
+            tmem_st32(trow + COL_V + 32 * (part & 1), v);
+            tmem_wait_st();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&sh.v_ready, lane);
+            return true;
+        };
 
-        for (int it = 0; ok && it < n_it; ++it) {
+        int g = 0, item = 0;  // query tiles, items done with
+        Items s{first, 0};
+        for (;;) {
+        const int kv0 = s.x.kv0(), bh = s.x.bh, it0 = s.x.it0, n_it = s.x.n_it;
+        const int kvrow = kv0 + row;
+        const bool kv_ok = kvrow < a.Tk;
+        if (SPLIT && n_it == 0) pdl_wait();  // the rows written at the end; with query tiles the barriers order everything
+        for (int it = 0; it < n_it; ++it, ++g) {
             const int q0 = (it0 + it) * TILE;
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, it & 1, W_SFULL, it));
+            // V lands before the first S^T of the CTA is complete; that of later items while their first P^T is computed
+            if (g == 0 && part >= 2 && !(ok = copy_v(0, rp))) break;
+            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, g & 1, W_SFULL, g));
             if (!ok) break;
             tc_fence_after_sync();
 
@@ -616,11 +724,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tc_fence_before_sync();
                 mbar_arrive_warp(&sh.pt_ready, lane);
             }
-            if (it > 0 && part >= 2 && !(ok = read_dq(it - 1, rp))) break;  // rp is free until dP^T is loaded
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, it & 1, W_SFULL, 1000 + it));
+            if (g > 0 && part >= 2) {  // rp is free until dP^T is loaded
+                if (it == 0 && !(ok = copy_v(item, rp))) break;
+                if (!(ok = read_dq(g - 1, rp))) break;
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, g & 1, W_SFULL, 1000 + g));
             if (!ok) break;
             tc_fence_after_sync();
-            if (it > 0 && part >= 2) stage_dq(rp);
+            if (g > 0 && part >= 2) stage_dq(rp);
             tmem_ld32(trow + COL_DP + c0, rp);
             tmem_wait_ld();
 
@@ -661,10 +772,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // (before the first tile the buffer held V, which every thread has left once v_ready completes); boxes 2, 3 go over the MN-major dO tile as soon as dV of
             // this tile is done.
             if (part < 2) {
-                ok = __all_sync(0xffffffffu, it == 0 ? mbar_wait(wc, &sh.v_ready, 0, W_VREADY, 1)
-                                                      : mbar_wait(wc, &sh.dq_full, (it - 1) & 1, W_DQFULL, 1000 + it));
+                ok = __all_sync(0xffffffffu, it == 0 ? mbar_wait(wc, &sh.v_ready, item & 1, W_VREADY, 1)
+                                                      : mbar_wait(wc, &sh.dq_full, (g - 1) & 1, W_DQFULL, 1000 + g));
             } else {
-                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, it & 1, W_DVDONE, it));
+                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, g & 1, W_DVDONE, g));
             }
             if (!ok) break;
             {
@@ -685,17 +796,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mbar_arrive_warp(&sh.ds_ready, lane);
         }
 
-        // The accumulators: column groups 0, 1 put dV (times 1/(1-p) for inverted dropout), complete before the last dS
-        // was formed, into the K-major Q tile and groups 2, 3 put dK into the K-major K tile -- both dead after the last
-        // S^T -- as the boxes of a 128-byte-swizzled TMA tile: 16-byte chunk c of row r at position c ^ (r & 7).
-        if (ok && n_it > 0)
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, (part < 2) ? &sh.dv_done : &sh.dk_done, (n_it - 1) & 1, W_BDONE, n_it));
-        if (ok && n_it > 0) {
+        if (!ok) break;
+        Items nx = s;
+        const bool more = next_item(nx, false);
+        // The accumulators, as the boxes of a 128-byte-swizzled TMA tile (16-byte chunk c of row r at position c ^ (r & 7)):
+        // column groups 2, 3 put dK into the MN-major Q tile, dead with the last dK; groups 0, 1 put dV (times 1/(1-p) for
+        // inverted dropout) into the MN-major K tile, dead with the last dQ, or, if no item follows, at once into the
+        // K-major Q tile.  They are in registers when this warp hands over its next P^T, which the first dV of the next item
+        // waits for.
+        if (n_it > 0)
+            ok = __all_sync(0xffffffffu, mbar_wait(wc, (part >= 2) ? &sh.dk_done : more ? &sh.dq_full : &sh.dv_done, (g - 1) & 1, W_BDONE, g));
+        if (!ok) break;
+        if (n_it > 0) {
             tc_fence_after_sync();
             tmem_ld32(trow + ((part < 2) ? COL_DV + part * 32 : COL_DK + (part - 2) * 32), rs);
             tmem_wait_ld();
+            tc_fence_before_sync();
             const float f = (part < 2) ? a.dv_scale : 1.f;
-            uint8_t* srow = ((part < 2) ? sQ : sK) + (part & 1) * BOX_BYTES + row * 128;
+            uint8_t* srow = ((part >= 2) ? sQm : more ? sKm : sQ) + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c)
                 *reinterpret_cast<float4*>(srow + ((c ^ (row & 7)) << 4)) =
@@ -703,22 +821,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                                 __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
             fence_proxy_async_smem();
             mbar_arrive_warp((part < 2) ? &sh.dv_staged : &sh.dk_staged, lane);
-        } else if (n_it == 0 && !SPLIT && kv_ok && !a.accum_dkdv) {
-            // no query sees this KV tile: its dK and dV rows are zero
-            float* out_row = (part < 2)
-                                 ? a.dV + (int64_t)b * a.dv_sB + (int64_t)h * a.dv_sH + (int64_t)kvrow * a.dv_sM + part * 32
-                                 : a.dK + (int64_t)b * a.dk_sB + (int64_t)h * a.dk_sH + (int64_t)kvrow * a.dk_sM + (part - 2) * 32;
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(out_row + i) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+        if (!more) break;
+        s = nx;
+        ++item;
+        }  // items
 
         // dQ of the last query tile takes the same way out as the others: staged in the K-major dO tile (dead: its
         // last reader was dP^T of this tile) once the reduction of the previous tile has read that buffer, then
         // added to global memory by the store warp.  (From registers with red.global.add it took ~2 500 cycles per
         // CTA and held up the bulk stores of dV and dK behind it.)
-        if (ok && n_it > 0 && part >= 2) {
-            if (n_it > 1) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_out, (n_it - 2) & 1, W_DQOUT, n_it - 2));
-            if (ok) ok = read_dq(n_it - 1, rs);
+        if (ok && g > 0 && part >= 2) {
+            if (g > 1) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_out, (g - 2) & 1, W_DQOUT, g - 2));
+            if (ok) ok = read_dq(g - 1, rs);
             if (ok) stage_dq(rs);
         }
 
@@ -732,24 +847,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         cluster_wait();
         if (warp < W_LOAD) {
             // (rows of this thread) x (splits) = 8: all loads first, their latency is that of the other SM's memory
-            const int live = (n_all + run - 1) / max(run, 1);  // the splits that had query tiles
             const int ch = lane & 15;
             float4 v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int row = split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
-                const uint8_t* src = (lane < 16 ? sQ : sK) + (ch >> 3) * BOX_BYTES + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
-                v[u] = u % ns < live ? ld_cluster_f4(mapa(src, u % ns)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const uint8_t* src = (lane < 16 ? sQ : sQm) + (ch >> 3) * BOX_BYTES + row * 128 + (((ch & 7) ^ (row & 7)) << 4);
+                v[u] = u % ns < first.live ? ld_cluster_f4(mapa(src, u % ns)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
                 if ((u + 1) % ns != 0) continue;
-                const int64_t kvrow = kv0 + split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
+                const int64_t kvrow = first.kv0() + split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
                 if (kvrow < a.Tk) {
-                    float* dst = lane < 16 ? a.dV + (int64_t)b * a.dv_sB + (int64_t)h * a.dv_sH + kvrow * a.dv_sM
-                                           : a.dK + (int64_t)b * a.dk_sB + (int64_t)h * a.dk_sH + kvrow * a.dk_sM;
+                    float* dst = lane < 16 ? a.dV + (int64_t)first.b * a.dv_sB + (int64_t)first.h * a.dv_sH + kvrow * a.dv_sM
+                                           : a.dK + (int64_t)first.b * a.dk_sB + (int64_t)first.h * a.dk_sH + kvrow * a.dk_sM;
                     float4* out = reinterpret_cast<float4*>(dst) + ch;
                     if (a.accum_dkdv) {
                         const float4 old = *out;
@@ -768,10 +882,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     // ------------------------------ teardown ------------------------------
     tc_fence_before_sync();
     __syncthreads();
+    // A CTA that gave up does not leave while copies into its shared memory may be in flight (otherwise every copy was waited
+    // for by what it was for).
+    if (sh.abort.id)
+        for (const unsigned long long t0 = globaltimer_ns(); globaltimer_ns() - t0 < 100000ull;) {}
     if (warp == W_MMA) {
         __syncwarp();
         tc_fence_after_sync();
         tmem_dealloc(tmem, TMEM_COLS);
+        if (lane == 0) report_abort(sh.abort, a.status);
     }
 }
 
@@ -844,17 +963,34 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     BwdDevice* d = nullptr;
     const int device_rc = bwd_device(&d);
     if (device_rc != HK_OK) return device_rc;
-    const long long tiles = (long long)a.n_kvtiles * a.BH;
-    a.n_splits = plan_attn_bwd(tiles, a.Tq, a.Tk, d->slots);
-    const long long nblocks = tiles * a.n_splits;
-    if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
-    timing_mark(TIMED_BWD, true, stream);
-    LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn, m.dO_mn, m.dQ,
-                                              m.dK, m.dV, a);
-    timing_mark(TIMED_BWD, false, stream);
-    count_launch();
-    return rc == cudaSuccess ? HK_OK : check_launch();
+    // KV tiles that a query tile sees.  (The grid has no others: the store warp could not read past a run of items without
+    // query tiles, since it hands over the last dQ of an item beside the first tile of the next.)
+    int live = a.n_kvtiles;
+    if (a.causal) {
+        const long long last_q = (long long)(a.Tq + TILE - 1) / TILE * TILE - 1 + a.q_pos0 - a.k_pos0;  // in key positions
+        live = (int)std::max(0ll, std::min((long long)live, last_q < 0 ? 0 : last_q / TILE + 1));
+    }
+    a.n_splits = plan_attn_bwd((long long)a.n_kvtiles * a.BH, a.Tq, a.Tk, d->slots);
+    const long long nblocks = (long long)live * a.BH * a.n_splits;
+    if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
+    a.take_over = nblocks > d->slots[0];  // else every CTA starts at once
+    if (nblocks > 0) {
+        timing_mark(TIMED_BWD, true, stream);
+        LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
+        const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
+                                                  m.dO_mn, m.dQ, m.dK, m.dV, a);
+        timing_mark(TIMED_BWD, false, stream);
+        count_launch();
+        if (rc != cudaSuccess) return check_launch();
+    }
+    // the rows of the other KV tiles are zero
+    const int rows = a.Tk - live * TILE;
+    if (rows > 0 && !a.accum_dkdv) {
+        int rc = launch_zero_rows(a.dK + (int64_t)live * TILE * a.dk_sM, a.dk_sB, a.dk_sM, a.dk_sH, a.BH / a.H, a.H, rows, stream);
+        if (rc == HK_OK) rc = launch_zero_rows(a.dV + (int64_t)live * TILE * a.dv_sM, a.dv_sB, a.dv_sM, a.dv_sH, a.BH / a.H, a.H, rows, stream);
+        return rc;
+    }
+    return HK_OK;
 }
 
 }  // namespace hk

@@ -35,7 +35,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn get_encode_tiled();
 
 // Tensor map over a [B, H, T, inner] fp32 view (element strides sB, sM, sH; last
-// stride 1); box = 32 floats x `box_rows` rows, out-of-range rows read as zero.
+// stride 1; `inner` a multiple of 32).  A copy brings `box_rows` rows as boxes of 32 floats x box_rows, one behind the
+// other; out-of-range rows read as zero.
 // mn_major = false: 128-byte swizzle of 16-byte chunks (K-major MMA operand);
 // mn_major = true:  128-byte swizzle of 32-byte chunks (MN-major TF32 operand).
 // operand = true: the map of an MMA operand.  Its element type is TFLOAT32, with which a load rounds every fp32 value to

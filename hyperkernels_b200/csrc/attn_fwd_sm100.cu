@@ -63,7 +63,7 @@ struct __align__(16) Shared {
     float m[2][TILE], l[2][TILE];  // [stream]: row maxima and sums for the combination
     uint64_t q_full[2], kv_full[SLOTS], kv_empty[SLOTS], s_full[3], p_full[3], o_full[3];
     uint32_t tmem_base;
-    int abort_flag;
+    Abort abort;
 };
 
 constexpr int OFF_Q = 0;                          // two tiles
@@ -147,8 +147,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     auto row0_of = [&](int t) { return q0 + (keys ? 0 : t * TILE); };  // first row of stream t
     auto load_q = [&](int t) {
         mbar_arrive_expect_tx(&sh.q_full[t], TILE_BYTES);
-        tma_load_4d(sQ + t * TILE_BYTES, &mapQ, &sh.q_full[t], 0, row0_of(t), h, b);
-        tma_load_4d(sQ + t * TILE_BYTES + BOX_BYTES, &mapQ, &sh.q_full[t], HALF_D, row0_of(t), h, b);
+        tma_load_tile(sQ + t * TILE_BYTES, &mapQ, &sh.q_full[t], row0_of(t), h, b);
     };
     auto load_kv = [&](int i) {  // entry i of the ring sequence
         const bool v = i > 0 && (i & 1) == 0;
@@ -156,8 +155,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const CUtensorMap* map = v ? &mapV : &mapK;
         const int s = i % SLOTS;
         mbar_arrive_expect_tx(&sh.kv_full[s], TILE_BYTES);
-        tma_load_4d(sKV + s * TILE_BYTES, map, &sh.kv_full[s], 0, (jb + tile) * TILE, h, b);
-        tma_load_4d(sKV + s * TILE_BYTES + BOX_BYTES, map, &sh.kv_full[s], HALF_D, (jb + tile) * TILE, h, b);
+        tma_load_tile(sKV + s * TILE_BYTES, map, &sh.kv_full[s], (jb + tile) * TILE, h, b);
     };
     auto in_ring = [&](int i) { return i < 2 * nk - 1 || i == 2 * nk; };
 
@@ -189,7 +187,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mbar_init(&sh.p_full[bf], 4);  // one arrival per softmax warp of the stream
             mbar_init(&sh.o_full[bf], 1);
         }
-        sh.abort_flag = 0;
+        sh.abort.id = 0;
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -200,7 +198,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = uniform(sh.tmem_base);
-    WaitCtx wc{&sh.abort_flag, a.status};
+    WaitNote wc{&sh.abort};
     // all threads of the cluster (of the CTA, when it is alone)
     auto barrier_all = [&] {
         if (ns > 1) {
@@ -339,6 +337,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         if (warp == 1) {
             tc_fence_after_sync();
             tmem_dealloc(tmem, TMEM_COLS);
+            if (lane == 0) report_abort(sh.abort, a.status);
         }
     } else {
         // ------------------------------ softmax ------------------------------
@@ -572,8 +571,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // the end of the sequence are clipped by the copy
             asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
             if (row == 0 && row_ok && !keep_old) {
-                tma_store_4d(&mapO, sQ + t * TILE_BYTES, 0, qrow, h, b);
-                tma_store_4d(&mapO, sQ + t * TILE_BYTES + BOX_BYTES, HALF_D, qrow, h, b);
+                tma_store_tile(&mapO, sQ + t * TILE_BYTES, qrow, h, b);
                 bulk_commit_group();
                 bulk_wait_group_read_all();  // the copies have read their source; they complete on their own
             }

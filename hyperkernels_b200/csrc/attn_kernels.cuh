@@ -74,6 +74,7 @@ struct BwdArgs {
     int Tq, Tk;
     int n_kvtiles;
     int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; set by launch_attn_bwd
+    int take_over;     // 1: the grid is larger than the device; CTAs that are through take over others' work; set by launch_attn_bwd
     int q_pos0, k_pos0;
     float scale, scale_log2e;
     int causal;

@@ -108,11 +108,12 @@ int make_tile_map(CUtensorMap* map, const float* ptr, int inner, int B, int H, i
     // A size-1 dimension may carry any stride; give it a harmless valid one.
     if (H == 1) sH = sM * T;
     if (B == 1) sB = (sH * H > sM * T) ? sH * H : sM * T;
-    cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)sM * 4, (cuuint64_t)sH * 4, (cuuint64_t)sB * 4};
-    cuuint32_t box[4] = {(cuuint32_t)HALF_D, (cuuint32_t)box_rows, 1, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = enc(map, operand ? CU_TENSOR_MAP_DATA_TYPE_TFLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(ptr), dims, strides, box, estr,
+    const int boxes = inner / HALF_D;  // a row's 128-byte pieces are a dimension of their own: one copy takes them all
+    cuuint64_t dims[5] = {(cuuint64_t)HALF_D, (cuuint64_t)T, (cuuint64_t)boxes, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t strides[4] = {(cuuint64_t)sM * 4, (cuuint64_t)HALF_D * 4, (cuuint64_t)sH * 4, (cuuint64_t)sB * 4};
+    cuuint32_t box[5] = {(cuuint32_t)HALF_D, (cuuint32_t)box_rows, (cuuint32_t)boxes, 1, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r = enc(map, operand ? CU_TENSOR_MAP_DATA_TYPE_TFLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float*>(ptr), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE,
                      mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

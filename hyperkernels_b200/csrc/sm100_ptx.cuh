@@ -3,8 +3,8 @@
 // (TMEM) allocation / load / store, and tcgen05.mma with TF32 operands.
 //
 // Every wait is bounded: a spin that does not complete within HK_WAIT_LIMIT_NS
-// raises the CTA's abort flag and the global status word and returns false, so
-// no kernel built on these helpers can hang a device.
+// raises the CTA's abort record, sets the global status word (at once or as the
+// kernel ends) and returns false, so no kernel built on these helpers can hang a device.
 #pragma once
 
 #include <cuda.h>
@@ -18,12 +18,12 @@ namespace hk {
 // ---------------------------------------------------------------------------
 struct DeviceStatus {
     int code;        // 0 = ok, otherwise the id of the wait that timed out
-    int block;       // blockIdx.x + gridDim.x * blockIdx.y of the first reporter
+    int block;       // blockIdx.x of the first reporter
     int thread;      // threadIdx.x of the first reporter
     int aux;         // loop iteration the wait belonged to
 };
 
-constexpr unsigned long long HK_WAIT_LIMIT_NS = 2000000000ull;  // 2 s
+constexpr unsigned long long HK_WAIT_LIMIT_NS = 2000000000ull;  // 2 s; below 2^32, waits look at the clock's lower word
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -107,39 +107,66 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Per-CTA wait context: `abort` lives in shared memory and is raised by the
-// first wait that gives up; every later wait sees it and returns at once.
-struct WaitCtx {
+// Per-CTA wait contexts.  The record lives in shared memory and is raised by the first wait that gives up; every later wait
+// sees it and returns at once.
+struct WaitCtx {  // the wait that gives up tells the host
     volatile int* abort_flag;  // shared memory
     DeviceStatus* status;      // global memory
 };
+struct Abort {
+    volatile int id;  // of the wait, 0: none gave up
+    int thread, aux;
+};
+struct WaitNote {  // the kernel tells the host as it ends (report_abort): less code in each wait
+    Abort* abort;
+};
+__device__ __forceinline__ bool gave_up(const WaitCtx& ctx) { return *ctx.abort_flag != 0; }
+__device__ __forceinline__ bool gave_up(const WaitNote& ctx) { return ctx.abort->id != 0; }
+__device__ __forceinline__ void report_abort(const Abort& x, DeviceStatus* status) {
+    if (x.id != 0 && atomicCAS(&status->code, 0, x.id) == 0) {
+        status->block = blockIdx.x;
+        status->thread = x.thread;
+        status->aux = x.aux;
+    }
+}
+__device__ __forceinline__ void give_up(const WaitNote& ctx, int wait_id, int aux) {
+    ctx.abort->id = wait_id;
+    ctx.abort->thread = threadIdx.x;
+    ctx.abort->aux = aux;
+}
+__device__ __forceinline__ void give_up(const WaitCtx& ctx, int wait_id, int aux) {
+    *ctx.abort_flag = 1;
+    report_abort(Abort{wait_id, (int)threadIdx.x, aux}, ctx.status);
+}
 
-static __device__ __forceinline__ bool mbar_wait_slow(const WaitCtx& ctx, uint64_t* bar, uint32_t parity, int wait_id, int aux) {
-    const unsigned long long t0 = globaltimer_ns();
-    while (true) {
+__device__ __forceinline__ uint32_t globaltimer_lo() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(t));
+    return t;
+}
+
+template <class Ctx>
+__device__ __forceinline__ bool mbar_wait_slow(const Ctx& ctx, uint64_t* bar, uint32_t parity, int wait_id, int aux) {
+    const uint32_t t0 = globaltimer_lo();
 #pragma unroll 1
-        for (int i = 0; i < 64; ++i)
-            if (mbar_try_wait(bar, parity)) return true;
-        if (*ctx.abort_flag) return false;
-        if (globaltimer_ns() - t0 > HK_WAIT_LIMIT_NS) {
-            *ctx.abort_flag = 1;
-            if (atomicCAS(&ctx.status->code, 0, wait_id) == 0) {
-                ctx.status->block = blockIdx.x + gridDim.x * blockIdx.y;
-                ctx.status->thread = threadIdx.x;
-                ctx.status->aux = aux;
-            }
-            __threadfence();
+    while (!mbar_try_wait(bar, parity)) {
+        if (gave_up(ctx)) return false;
+        if (globaltimer_lo() - t0 > (uint32_t)HK_WAIT_LIMIT_NS) {
+            give_up(ctx, wait_id, aux);
             return false;
         }
     }
+    return true;
 }
 
 // Returns false if the wait was abandoned (the CTA must then wind down).
-// One try inline, the rest in a rolled loop.  Unrolled (32 + 64 tries at each of some thirty waits) the backward kernel
-// was 194 KiB of code, more than the instruction cache holds, and the first CTA on every SM spent ~11 000 cycles fetching
-// it: B8 H12 T1024 backward 115 -> 103 us, forward 51 -> 45.  Rolled without the inline try, with a suspend-time hint, or
+// One try inline, the rest in one short loop.  A wait stands in some thirty places of a kernel, and what the warps of an SM
+// run in turn has to stay in its instruction cache: with 32 + 64 tries unrolled the backward was 194 KiB of code and the first
+// CTA on every SM spent ~11 000 cycles fetching it (B8 H12 T1024 backward 115 -> 103 us, forward 51 -> 45); nested loops
+// round a 64-bit clock and the report in place were another 17 KiB.  Without the inline try, with a suspend-time hint, or
 // spinning on test_wait, the backward takes 4 - 15 % more cycles per query tile.
-__device__ __forceinline__ bool mbar_wait(const WaitCtx& ctx, uint64_t* bar, uint32_t parity, int wait_id, int aux = 0) {
+template <class Ctx>
+__device__ __forceinline__ bool mbar_wait(const Ctx& ctx, uint64_t* bar, uint32_t parity, int wait_id, int aux = 0) {
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(ctx, bar, parity, wait_id, aux);
 }
@@ -151,35 +178,32 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// 4-D tile load. Coordinates are element indices, innermost first; c0 must be
-// a multiple of 4 floats (16 bytes).
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
-                                            int c2, int c3) {
+// The tile of rows row .. of slice (b, h): every box of 32 floats x box_rows of a row's width, one after the other
+// (make_tile_map), in one copy.
+__device__ __forceinline__ void tma_load_tile(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int row, int h, int b) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2),
-        "r"(c3)
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %3, %5, %6}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(h), "r"(b)
         : "memory");
 }
 
-// 4-D tile reduction, shared -> global: global[tile] += shared tile (fp32 add performed by the
+// Tile reduction, shared -> global: global[tile] += shared tile (fp32 add performed by the
 // memory system).  Rows of the box that lie outside the tensor are skipped.  Completion is tracked
 // by the issuing thread's bulk async-group.  The shared-memory tile must have been written, and
 // fence_proxy_async_smem() executed by its writers, before the issuing thread learnt about it.
-__device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2,
-                                                  int c3) {
+__device__ __forceinline__ void tma_reduce_add_tile(const CUtensorMap* map, const void* smem_src, int row, int h, int b) {
     asm volatile(
-        "cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group"
-        " [%0, {%2, %3, %4, %5}], [%1];"
-        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        "cp.reduce.async.bulk.tensor.5d.global.shared::cta.add.tile.bulk_group"
+        " [%0, {%2, %3, %2, %4, %5}], [%1];"
+        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(0), "r"(row), "r"(h), "r"(b)
         : "memory");
 }
-// 4-D tile store, shared -> global; same rules as the reduction above.
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2, int c3) {
+// Tile store, shared -> global; same rules as the reduction above.
+__device__ __forceinline__ void tma_store_tile(const CUtensorMap* map, const void* smem_src, int row, int h, int b) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        "cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %2, %4, %5}], [%1];"
+        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(0), "r"(row), "r"(h), "r"(b)
         : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -436,6 +460,33 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 // kernel triggers only after its own pdl_wait, so that what precedes IT is complete too when its successor starts.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
+// cluster launch control (grids without clusters)
+// ---------------------------------------------------------------------------
+// Asks to take over the work of a CTA of this grid that has not started: the 16-byte answer arrives on `bar`.
+__device__ __forceinline__ void clc_try_cancel(uint4* answer, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+                 : "memory");
+}
+// blockIdx.x of the CTA taken over, or -1 if there was none left
+__device__ __forceinline__ int clc_read(const uint4* answer) {
+    int x;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b128 h;\n"
+        "ld.shared.b128 h, [%1];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n"
+        "mov.b32 %0, -1;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n"
+        "}\n"
+        : "=r"(x)
+        : "r"(smem_u32(answer))
+        : "memory");
+    return x;
+}
 
 // ---------------------------------------------------------------------------
 // thread-block clusters

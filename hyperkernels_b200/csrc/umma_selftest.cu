@@ -82,8 +82,8 @@ umma_selftest_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_cons
     if (threadIdx.x == 0) {
         const int a_boxes = (which == 0) ? 2 : (which == 2 ? 4 : 0);
         mbar_arrive_expect_tx(&sh.full, (a_boxes + 2) * BOX_BYTES);
-        for (int i = 0; i < a_boxes; ++i) tma_load_4d(sA + i * BOX_BYTES, &mapA, &sh.full, i * HALF_D, 0, 0, 0);
-        for (int i = 0; i < 2; ++i) tma_load_4d(sB + i * BOX_BYTES, &mapB, &sh.full, i * HALF_D, 0, 0, 0);
+        tma_load_tile(sA, &mapA, &sh.full, 0, 0, 0);
+        tma_load_tile(sB, &mapB, &sh.full, 0, 0, 0);
         if (mbar_wait(wc, &sh.full, 0, 901)) {
             tc_fence_after_sync();
             const uint32_t a_addr = smem_u32(sA), b_addr = smem_u32(sB);

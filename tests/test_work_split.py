@@ -157,6 +157,45 @@ def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
         assert float((s - (b + x)).abs().max()) <= 4 * 2.0 ** -23 * float(x.abs().max() + b.abs().max())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["none", "philox", "philox inverted"])
+@pytest.mark.parametrize("BH,Tq,Tk,causal", [(299, 128, 128, 0), (60, 640, 640, 1), (75, 100, 300, 0), (90, 257, 384, 1), (60, 130, 1000, 1), (5, 70, 200, 1)])
+def test_backward_ctas_take_over_key_tiles(BH, Tq, Tk, causal, kind):
+    """More KV tiles than CTAs start with, one to five query tiles each: the CTAs that are through take over the others.  First,
+    middle and last slice against the oracle, all of them against the same call on 20 slices at a time (every CTA starts with
+    its own tile: the same bits), and results added to what the buffers hold.  KV tiles that no query sees (Tk > Tq under the
+    mask; all of them where the keys lie behind the queries) leave zeros."""
+    from test_attention_gpu import gate, host, ok_status
+
+    q, g = _normal((1, BH, Tq, 64), 980), _normal((1, BH, Tq, 64), 981)
+    k, v = _normal((1, BH, Tk, 64), 982), _normal((1, BH, Tk, 64), 983)
+    kw, _ = _mask(kind, 1, 8, 8)
+    Q, K, V, G = map(_dev, (q, k, v, g))
+    for pos in (dict(), dict(k_pos0=1000)) if causal else (dict(),):
+        O, L = hk.attention_forward(Q, K, V, SCALE, bool(causal), **pos, **kw)
+        call = lambda s, **more: hk.attention_backward(Q[:, s], K[:, s], V[:, s], O[:, s], G[:, s], L[:, s], SCALE, bool(causal), **pos,  # noqa: E731
+                                                       **(dict(kw, bh_pos0=s.start) if kw else {}), **more)[:3]
+        whole = call(slice(0, BH), deterministic_dq=True)
+        ok_status()
+        for i in (0, BH // 2, BH - 1):
+            s = slice(i, i + 1)
+            mask = None if kind == "none" else ol.dropout_mask(BH, Tq, Tk, P, SEED, OFFSET, **pos)[s]
+            _, *refs = _oracle_backward(kind, mask, q[:, s], k[:, s], v[:, s], host(O[:, s]), g[:, s], host(L[:, s]), causal, **pos)
+            for name, got, ref in zip(("dQ", "dK", "dV"), whole, refs):
+                gate(name, host(got[:, s]), ref)
+        base = [_dev(_normal(tuple(x.shape), 984 + i)) for i, x in enumerate(whole)]
+        sums = [b.clone() for b in base]
+        call(slice(0, BH), deterministic_dq=True, accum_dq=True, accum_dkdv=True, dQ=sums[0], dK=sums[1], dV=sums[2])
+        for s0 in range(0, BH, 20):
+            s = slice(s0, min(BH, s0 + 20))
+            for got, ref in zip(call(s, deterministic_dq=True), whole):
+                assert torch.equal(got, ref[:, s])
+        ok_status()
+        for s, b, x in zip(sums, base, whole):
+            # fp32 sums of at most ceil(Tk / 128) + 1 terms in another order
+            assert float((s - (b + x)).abs().max()) <= 8 * 2.0 ** -23 * float(x.abs().max() + b.abs().max())
+
+
 # ---- what the cut may change ----------------------------------------------------------------------------------------
 @pytest.mark.gpu
 @pytest.mark.parametrize("Tq,Tk,causal,q_pos0", [(4096, 4096, 1, 0), (2048, 4095, 0, 0), (65, 129, 1, 64), (1023, 512, 0, 0), (1500, 1500, 1, 0)])
