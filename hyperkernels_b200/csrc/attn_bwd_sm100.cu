@@ -169,9 +169,12 @@ __device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split,
 }
 }  // namespace bwd
 
-// DROP: 0 none, 1 dense mask, 2 Philox.  SPLIT: a cluster shares the query tiles of a KV tile (an instantiation of its own:
-// the set-up and the registers it needs cost the plain kernel 1 - 3 %).
-template <int DROP, bool SPLIT>
+// DROP: 0 none, 1 dense mask, 2 Philox.  JOB: what a CTA does with its items.  SPLIT_ITEM: a cluster shares the query tiles of
+// a KV tile (the set-up and the registers it needs cost the plain kernel 1 - 3 %).  A kernel that contains cluster launch
+// control is not started under the tail of the one before it, programmatic dependent launch or not, so grids that fit the
+// device use one without.
+enum BwdJob { ONE_ITEM = 0, TAKE_OVER = 1, SPLIT_ITEM = 2 };
+template <int DROP, int JOB>
 __global__ void __launch_bounds__(bwd::NUM_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapdO,
@@ -180,6 +183,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const __grid_constant__ CUtensorMap mapdK, const __grid_constant__ CUtensorMap mapdV,
                 const __grid_constant__ BwdArgs a) {
     using namespace bwd;
+    constexpr bool SPLIT = JOB == SPLIT_ITEM, TAKES_OVER = JOB == TAKE_OVER;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {  // never expected; refuse to run on a misplaced buffer
         if (threadIdx.x == 0 && atomicCAS(&a.status->code, 0, 299) == 0) a.status->block = blockIdx.x;
@@ -286,7 +290,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     };
     // Goes on to the next item; false if there is none (or a wait gave up).  All lanes of a warp, or one thread alone (`solo`).
     auto next_item = [&](Items& s, bool solo) -> bool {
-        if (SPLIT) return false;
+        if (!TAKES_OVER) return false;
         const int buf = s.n % ITEMS;
         bool ok = mbar_wait(wc, &sh.item_full[buf], (s.n / ITEMS) & 1, W_ITEM, s.n);
         if (!solo) ok = __all_sync(0xffffffffu, ok);
@@ -303,17 +307,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             Item cur = first;
             int published = 0;
             int items = 0;  // whose accumulators have left
-            bool tok = true, more = !SPLIT;
-            // on to the next item: publishes what the request brought, if one was made
+            bool tok = true, more = TAKES_OVER;
+            // on to the next item: publishes what the request brought
             auto next = [&]() -> bool {
                 const int buf = published % ITEMS;
-                if (!more) return false;
-                int id = -1;
-                if (a.take_over) {
-                    if (!(tok = mbar_wait(wc, &sh.answered, published & 1, W_ITEM, published))) return false;
-                    id = clc_read(&sh.answer);
-                    fence_proxy_async_smem();  // the answer's buffer is next written by the async proxy
-                }
+                if (!more || !(tok = mbar_wait(wc, &sh.answered, published & 1, W_ITEM, published))) return false;
+                const int id = clc_read(&sh.answer);
+                fence_proxy_async_smem();  // the answer's buffer is next written by the async proxy
                 if (published >= ITEMS && !(tok = mbar_wait(wc, &sh.item_empty[buf], (published / ITEMS - 1) & 1, W_ITEM, 1000 + published)))
                     return false;
                 more = id >= 0;
@@ -342,7 +342,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 const bool have = t2.it < cur.n_it;
                 // Asked for a tile before it is needed: at the start of a long item it would be taken from a CTA that is
                 // through sooner (training step at B2 H16 T2000, reproducible: 190 instead of 183 us).
-                if (!SPLIT && a.take_over && t2.it + 1 == cur.n_it) {
+                if (TAKES_OVER && t2.it + 1 == cur.n_it) {
                     mbar_arrive_expect_tx(&sh.answered, sizeof(uint4));
                     clc_try_cancel(&sh.answer, &sh.answered);
                 }
@@ -903,8 +903,9 @@ struct BwdDevice {
 };
 typedef void (*BwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
                           CUtensorMap, CUtensorMap, BwdArgs);
-const BwdKernel bwd_kernels[6] = {attn_bwd_kernel<0, false>, attn_bwd_kernel<1, false>, attn_bwd_kernel<2, false>,
-                                  attn_bwd_kernel<0, true>,  attn_bwd_kernel<1, true>,  attn_bwd_kernel<2, true>};
+const BwdKernel bwd_kernels[9] = {attn_bwd_kernel<0, ONE_ITEM>,   attn_bwd_kernel<1, ONE_ITEM>,   attn_bwd_kernel<2, ONE_ITEM>,
+                                  attn_bwd_kernel<0, TAKE_OVER>,  attn_bwd_kernel<1, TAKE_OVER>,  attn_bwd_kernel<2, TAKE_OVER>,
+                                  attn_bwd_kernel<0, SPLIT_ITEM>, attn_bwd_kernel<1, SPLIT_ITEM>, attn_bwd_kernel<2, SPLIT_ITEM>};
 
 // of the current device; set up by the first call on it
 int bwd_device(BwdDevice** out) {
@@ -921,7 +922,7 @@ int bwd_device(BwdDevice** out) {
         for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
             LaunchConfig lc(8u << i, bwd::NUM_THREADS, bwd::SMEM_BYTES, nullptr, 1 << i, false);
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, bwd_kernels[3], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+            if (cudaOccupancyMaxActiveClusters(&n, bwd_kernels[6], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
         }
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
@@ -973,11 +974,11 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     a.n_splits = plan_attn_bwd((long long)a.n_kvtiles * a.BH, a.Tq, a.Tk, d->slots);
     const long long nblocks = (long long)live * a.BH * a.n_splits;
     if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
-    a.take_over = nblocks > d->slots[0];  // else every CTA starts at once
+    const int job = a.n_splits > 1 ? SPLIT_ITEM : nblocks > d->slots[0] ? TAKE_OVER : ONE_ITEM;
     if (nblocks > 0) {
         timing_mark(TIMED_BWD, true, stream);
         LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
-        const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + (a.n_splits > 1 ? 3 : 0)], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
+        const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + 3 * job], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
                                                   m.dO_mn, m.dQ, m.dK, m.dV, a);
         timing_mark(TIMED_BWD, false, stream);
         count_launch();

@@ -31,7 +31,7 @@
 //                 of a step.)  The running output is rescaled only when the running maximum grew by more than 2^8 (the
 //                 final O/l and LSE use the same maximum, so the result is the same function).
 // Tensor memory: three score buffers (128 columns each), O_0, O_1 (64 columns each): 512 of 512 columns.
-// Warps 0-3 give most of their registers to the softmax warps (setmaxnreg 56 / 224).
+// Warps 0-3 give most of their registers to the softmax warps (setmaxnreg 72 / 216).
 //
 // Key splits: a cluster of NS CTAs shares one block of query rows; split s takes a contiguous run of its key tiles, and at
 // the end every CTA combines a slice of the rows from the partial (O, m, l) the others left in their shared memory (keys
@@ -59,9 +59,24 @@ __device__ __forceinline__ uint32_t score_col(int b) { return b == 2 ? 384u : (u
 constexpr int SLOTS = 5;                    // K / V ring
 constexpr float RESCALE_THRESHOLD = 8.f;    // log2 units
 
+// What a CTA works on: one or two blocks of 128 query rows and the key tiles it takes them through.
+struct Item {
+    int b, h, bh, q0;  // q0: first query row
+    int n0, n1;        // steps of the streams; n0 < 0: there is no item
+    int nk, jb;        // key tiles loaded, the first of them (with splits: of this CTA's run)
+    int all0, all1;    // key tiles that the rows of the streams see, over all splits
+    __device__ __forceinline__ int steps(int t) const { return t == 0 ? n0 : n1; }
+};
+constexpr int ITEMS = 8;  // items that may be known beyond the one that the slowest warp is at
+
 struct __align__(16) Shared {
     float m[2][TILE], l[2][TILE];  // [stream]: row maxima and sums for the combination
-    uint64_t q_full[2], kv_full[SLOTS], kv_empty[SLOTS], s_full[3], p_full[3], o_full[3];
+    uint64_t q_full[2], q_empty[2], kv_full[SLOTS], kv_empty[SLOTS], s_full[3], p_full[3], o_full[3];
+    uint64_t o_staged[2];          // O of stream t is in its slot of the ring
+    uint64_t o_taken[2];           // the store warp knows: the stream may stage the next one
+    uint64_t item_full[ITEMS], item_empty[ITEMS], answered;
+    uint4 answer;                  // to a request for another item
+    Item item[ITEMS];              // the items taken over, decoded
     uint32_t tmem_base;
     Abort abort;
 };
@@ -72,18 +87,24 @@ constexpr int OFF_SH = OFF_KV + SLOTS * TILE_BYTES;
 constexpr int SMEM_BYTES = OFF_SH + sizeof(Shared);
 static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KiB a CTA may opt in to");
 
-enum WaitId { W_QFULL = 101, W_KFULL, W_KVEMPTY, W_VFULL, W_SFULL, W_PFULL, W_OFULL };
+enum WaitId { W_QFULL = 101, W_KFULL, W_KVEMPTY, W_VFULL, W_SFULL, W_PFULL, W_OFULL, W_QEMPTY, W_ITEM, W_OSLOT, W_OSTAGED };
 
-// 384 threads x 168 registers at launch = 128 x 56 + 256 x 224 after the hand-over (setmaxnreg.inc can only take what
+// 384 threads x 168 registers at launch = 128 x 72 + 256 x 216 after the hand-over (setmaxnreg.inc can only take what
 // the launch-time pool of the CTA holds)
-static_assert(128 * 56 + NUM_SOFTMAX * 224 <= NUM_THREADS * 168, "register hand-over exceeds the CTA's pool");
-__device__ __forceinline__ void reg_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n"); }
-__device__ __forceinline__ void reg_acquire() { asm volatile("setmaxnreg.inc.sync.aligned.u32 224;\n"); }
+static_assert(128 * 72 + NUM_SOFTMAX * 216 <= NUM_THREADS * 168, "register hand-over exceeds the CTA's pool");
+__device__ __forceinline__ void reg_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 72;\n"); }
+__device__ __forceinline__ void reg_acquire() { asm volatile("setmaxnreg.inc.sync.aligned.u32 216;\n"); }
 
-// Ring sequence: K0 K1 V0 K2 V1 K3 V2 ...: K(0) is entry 0, K(j) entry 2 j - 1, V(j) entry 2 j + 2 (so the entry before the
-// last V is skipped).
+// Ring sequence of an item of n key tiles: K0 K1 V0 K2 V1 .. K(n-1) V(n-2) - V(n-1): K(0) is entry 0, K(j) entry 2 j - 1, V(j)
+// entry 2 j + 2, so the entry before the last V is skipped.  Where other items follow (FOLLOWED) it is not, the last V is
+// entry 2 n - 1, and then comes one entry per stream that has rows: a slot through which its O leaves.
+template <bool FOLLOWED>
+__device__ __forceinline__ int ring_v(int j, int n) {
+    return FOLLOWED ? min(2 * j + 2, 2 * n - 1) : 2 * j + 2;
+}
 struct RingPos {
     uint32_t slot, phase;
+    __device__ __forceinline__ RingPos(uint32_t entry) : slot(entry % SLOTS), phase((entry / SLOTS) & 1u) {}
     __device__ __forceinline__ void advance(uint32_t by) {
         slot += by;
         if (slot >= SLOTS) {
@@ -105,13 +126,40 @@ __host__ __device__ inline int kv_tiles_for(int q0, int Tq, int Tk, int causal, 
     return (int)((kv_end + TILE - 1) / TILE);
 }
 
+__device__ __forceinline__ Item make_item(const FwdArgs& a, int work, int split, int ns) {
+    Item x;
+    // heavy (late) query blocks first: under the causal mask they have the most key tiles
+    x.bh = work % a.BH;
+    const int qb = a.n_qblocks - 1 - work / a.BH;
+    x.b = x.bh / a.H;
+    x.h = x.bh - x.b * a.H;
+    // rows mode: stream t = query rows q0 + 128 t ..; keys mode: both streams = rows q0 .., stream t = key tiles 2 j + t.
+    const bool keys = a.mode == FWD_KEYS;
+    x.q0 = qb * (a.mode == FWD_ROWS ? 2 * TILE : TILE);
+    x.all0 = kv_tiles_for(x.q0, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+    x.all1 = keys ? x.all0 : a.mode == FWD_ROW ? 0 : kv_tiles_for(x.q0 + TILE, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
+    const int all = max(x.all0, x.all1);
+    const int per = (all + ns - 1) / ns;  // split 0 is never empty while any key is seen
+    const int je = min(all, min(all, split * per) + per);
+    x.jb = min(all, split * per);
+    x.nk = je - x.jb;  // one per step (rows) or per product (keys)
+    x.n0 = keys ? (x.nk + 1) / 2 : max(0, min(je, x.all0) - x.jb);
+    x.n1 = keys ? x.nk / 2 : max(0, min(je, x.all1) - x.jb);
+    return x;
+}
+
 }  // namespace fwd
 
-template <int DROP>  // 0 none, 1 dense mask, 2 Philox
+// DROP: 0 none, 1 dense mask, 2 Philox.  JOB: what a CTA does with its items.  A kernel that contains cluster launch control is
+// not started under the tail of the one before it, programmatic dependent launch or not, so grids that fit the device use one
+// without (B1 H12 T512: 8.5 us, with it 9.5).
+enum FwdJob { ONE_ITEM = 0, TAKE_OVER = 1, COMBINE_ITEM = 2 };  // COMBINE_ITEM: keys mode or key splits, merged at the end
+template <int DROP, int JOB>
 __global__ void __launch_bounds__(fwd::NUM_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
-                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const FwdArgs a) {
+                const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdArgs a) {
     using namespace fwd;
+    constexpr bool COMBINE = JOB == COMBINE_ITEM, TAKES_OVER = JOB == TAKE_OVER;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sQ = smem + OFF_Q;
     uint8_t* sKV = smem + OFF_KV;
@@ -119,45 +167,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
     const int warp = (int)uniform(threadIdx.x >> 5);  // uniform for the compiler too: the issuing warp depends on it
     const int lane = threadIdx.x & 31;
-    const int ns = a.n_splits;  // cluster size
-    const int split = ns > 1 ? (int)cluster_ctarank() : 0;
-
-    // heavy (late) query blocks first: under the causal mask they have the most key tiles
-    const int work = blockIdx.x / ns;
-    const int bh = work % a.BH;
-    const int qb = a.n_qblocks - 1 - work / a.BH;
-    const int b = bh / a.H;
-    const int h = bh - b * a.H;
-    // rows mode: stream t = query rows q0 + 128 t ..; keys mode: both streams = rows q0 .., stream t = key tiles 2 j + t.
-    // q_end: end of the block's rows
-    // jb: this split's first key tile; n_t: steps of stream t; nk: key tiles this split loads, jb + 0 .. jb + nk - 1, one
-    // per step (rows) or per product (keys)
-    const bool keys = a.mode == FWD_KEYS;
+    const int ns = COMBINE ? a.n_splits : 1;  // cluster size
+    const int split = COMBINE && ns > 1 ? (int)cluster_ctarank() : 0;
+    const bool keys = COMBINE && a.mode == FWD_KEYS;
     const int block_rows = a.mode == FWD_ROWS ? 2 * TILE : TILE;
-    const int q0 = qb * block_rows, q_end = min(a.Tq, q0 + block_rows);
-    const int all0 = kv_tiles_for(q0, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
-    const int all1 = keys ? all0 : a.mode == FWD_ROW ? 0 : kv_tiles_for(q0 + TILE, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0);
-    const int all = max(all0, all1);
-    const int per = (all + ns - 1) / ns;  // split 0 is never empty while any key is seen
-    const int jb = min(all, split * per), je = min(all, jb + per);
-    const int nk = je - jb;
-    const int n0 = keys ? (nk + 1) / 2 : max(0, min(je, all0) - jb);
-    const int n1 = keys ? nk / 2 : max(0, min(je, all1) - jb);
+    const Item first = make_item(a, blockIdx.x / ns, split, ns);
 
-    auto row0_of = [&](int t) { return q0 + (keys ? 0 : t * TILE); };  // first row of stream t
-    auto load_q = [&](int t) {
+    auto end_of = [&](const Item& x) { return min(a.Tq, x.q0 + block_rows); };             // of the block's rows
+    auto row0_of = [&](const Item& x, int t) { return x.q0 + (keys ? 0 : t * TILE); };      // first row of stream t
+    // streams that have rows, whose O leaves through a slot of the ring
+    auto o_slots = [&](const Item& x) { return !TAKES_OVER ? 0 : row0_of(x, 1) < end_of(x) ? 2 : 1; };
+    auto load_q = [&](const Item& x, int t) {
         mbar_arrive_expect_tx(&sh.q_full[t], TILE_BYTES);
-        tma_load_tile(sQ + t * TILE_BYTES, &mapQ, &sh.q_full[t], row0_of(t), h, b);
+        tma_load_tile(sQ + t * TILE_BYTES, &mapQ, &sh.q_full[t], row0_of(x, t), x.h, x.b);
     };
-    auto load_kv = [&](int i) {  // entry i of the ring sequence
-        const bool v = i > 0 && (i & 1) == 0;
-        const int tile = v ? (i - 2) / 2 : (i + 1) / 2;
-        const CUtensorMap* map = v ? &mapV : &mapK;
-        const int s = i % SLOTS;
+    auto ring_end = [&](const Item& x) { return TAKES_OVER || x.nk == 0 ? 2 * x.nk : 2 * x.nk + 1; };
+    auto in_ring = [&](const Item& x, int i) { return TAKES_OVER || i != 2 * x.nk - 1; };
+    auto load_kv = [&](const Item& x, int i, uint32_t s) {  // entry i of the item's ring sequence, into slot s
+        const bool last = TAKES_OVER && i == 2 * x.nk - 1;
+        const bool v = i > 0 && ((i & 1) == 0 || last);
+        const int tile = x.jb + (last ? x.nk - 1 : v ? (i - 2) / 2 : (i + 1) / 2);
         mbar_arrive_expect_tx(&sh.kv_full[s], TILE_BYTES);
-        tma_load_tile(sKV + s * TILE_BYTES, map, &sh.kv_full[s], (jb + tile) * TILE, h, b);
+        tma_load_tile(sKV + s * TILE_BYTES, v ? &mapV : &mapK, &sh.kv_full[s], tile * TILE, x.h, x.b);
     };
-    auto in_ring = [&](int i) { return i < 2 * nk - 1 || i == 2 * nk; };
 
     // The producer initialises the barriers its copies complete on and issues the first loads at once (they wait for no
     // consumer): the rest of the set-up -- the other barriers, the tensor-memory allocation -- runs under their latency.
@@ -168,16 +200,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         fence_mbar_init();
         pdl_wait();  // whatever made Q, K, V
         pdl_trigger();
-        if (nk > 0) {
-            if (n0 > 0) load_q(0);
-            load_kv(0);
-            if (n1 > 0 && !keys) load_q(1);
+        if (first.nk > 0) {
+            if (first.n0 > 0) load_q(first, 0);
+            load_kv(first, 0, 0);
+            if (first.n1 > 0 && !keys) load_q(first, 1);
 #pragma unroll 1
-            for (int i = 1; i < SLOTS; ++i)
-                if (in_ring(i)) load_kv(i);
+            for (int i = 1; i < min(SLOTS, ring_end(first)); ++i)
+                if (in_ring(first, i)) load_kv(first, i, i);
         }
     }
-    if (threadIdx.x == 64) {  // an idle warp takes the rest of the barriers
+    if (threadIdx.x == 64) {  // another warp takes the rest of the barriers
         for (int s = 0; s < SLOTS; ++s) mbar_init(&sh.kv_empty[s], 1);
         // The score barriers belong to the score BUFFER, not to the stream: the warps of a stream may be a whole step
         // apart (the scores of the next step are there before the slowest warp has finished this one), and a
@@ -187,6 +219,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             mbar_init(&sh.p_full[bf], 4);  // one arrival per softmax warp of the stream
             mbar_init(&sh.o_full[bf], 1);
         }
+        for (int t = 0; t < 2; ++t) {
+            mbar_init(&sh.q_empty[t], 1);
+            mbar_init(&sh.o_staged[t], 4);
+            mbar_init(&sh.o_taken[t], 1);
+        }
+        for (int i = 0; i < ITEMS; ++i) {
+            mbar_init(&sh.item_full[i], 1);
+            mbar_init(&sh.item_empty[i], 10);  // the issuing, the storing and the softmax warps
+        }
+        mbar_init(&sh.answered, 1);
         sh.abort.id = 0;
         fence_mbar_init();
     }
@@ -197,11 +239,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     }
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem = uniform(sh.tmem_base);
+    // The CTA holds all 512 columns of tensor memory, so its allocation starts at address 0.
+    constexpr uint32_t tmem = 0;
+    if (sh.tmem_base != tmem) sh.abort.id = 198;  // never expected
     WaitNote wc{&sh.abort};
     // all threads of the cluster (of the CTA, when it is alone)
     auto barrier_all = [&] {
-        if (ns > 1) {
+        if (COMBINE && ns > 1) {
             __syncwarp();
             cluster_arrive();
             cluster_wait();
@@ -209,18 +253,72 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             __syncthreads();
         }
     };
-    const bool combine = ns > 1 || keys;  // the results of several streams or splits are merged at the end
+
+    // Work items.  A CTA that takes over starts with the item of its blockIdx and then, until none is left, takes over
+    // those of CTAs that have not started yet (cluster launch control): Q and the first keys of the next item are loaded, and
+    // its first scores computed, under the last steps of this one, and O leaves under the next one.  The producer asks, decodes
+    // the answer and puts the item into a ring that every warp reads in its own time: item r > 0 in entry r - 1.
+    auto read_item = [&](Item& x, int r, bool solo, bool release) -> bool {
+        if (!TAKES_OVER) return false;
+        const int buf = (r - 1) % ITEMS;
+        bool ok = mbar_wait(wc, &sh.item_full[buf], ((r - 1) / ITEMS) & 1, W_ITEM, r);
+        if (!solo) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
+        x = sh.item[buf];
+        if (!solo) __syncwarp();
+        if (release && (solo || lane == 0)) mbar_arrive(&sh.item_empty[buf]);
+        return x.n0 >= 0;
+    };
 
     if (warp < 4) {
         reg_release();
         if (warp == 0) {
             // ------------------------------ TMA producer ------------------------------
             if (lane == 0) {
+                Item x = first;
+                int q0_uses = first.n0 > 0 ? 1 : 0, q1_uses = first.n1 > 0 ? 1 : 0;  // loads of the streams' Q tiles
                 bool tok = true;
-                for (int i = SLOTS; tok && i <= 2 * nk; ++i) {
-                    if (!in_ring(i)) continue;
-                    if (!(tok = mbar_wait(wc, &sh.kv_empty[i % SLOTS], (i / SLOTS - 1) & 1, W_KVEMPTY, i))) break;
-                    load_kv(i);
+                // entry e of the ring: free when what it held SLOTS entries ago has been used up
+                auto free_slot = [&](int e) -> bool {
+                    return e < SLOTS || (tok = mbar_wait(wc, &sh.kv_empty[e % SLOTS], (e / SLOTS - 1) & 1, W_KVEMPTY, e));
+                };
+                for (int r = 0, base = 0;; ++r) {
+                    for (int i = r == 0 ? min(SLOTS, ring_end(x)) : 0; i < ring_end(x); ++i) {
+                        if (!in_ring(x, i)) continue;
+                        if (!free_slot(base + i)) break;
+                        load_kv(x, i, (base + i) % SLOTS);
+                        if (i == 0 && x.n1 > 0) {  // Q of the second stream behind the first keys
+                            if (q1_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[1], (q1_uses - 1) & 1, W_QEMPTY, r))) break;
+                            load_q(x, 1);
+                            ++q1_uses;
+                        }
+                    }
+                    if (!TAKES_OVER || !tok) break;
+                    base += 2 * x.nk;
+                    // asked for here, a step or two before this CTA is through
+                    mbar_arrive_expect_tx(&sh.answered, sizeof(uint4));
+                    clc_try_cancel(&sh.answer, &sh.answered);
+                    const int n_o = o_slots(x);
+                    for (int t = 0; tok && t < n_o; ++t, ++base)
+                        if (free_slot(base)) mbar_arrive(&sh.kv_full[base % SLOTS]);
+                    if (!tok || !(tok = mbar_wait(wc, &sh.answered, r & 1, W_ITEM, r))) break;
+                    const int id = clc_read(&sh.answer);
+                    fence_proxy_async_smem();  // the answer's buffer is next written by the async proxy
+                    const int buf = r % ITEMS;
+                    if (r >= ITEMS && !(tok = mbar_wait(wc, &sh.item_empty[buf], (r / ITEMS - 1) & 1, W_ITEM, 1000 + r))) break;
+                    if (id >= 0) {
+                        x = make_item(a, id, 0, 1);
+                        sh.item[buf] = x;
+                    } else {
+                        sh.item[buf].n0 = -1;
+                    }
+                    mbar_arrive(&sh.item_full[buf]);
+                    if (id < 0) break;
+                    if (x.n0 > 0) {
+                        if (q0_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[0], (q0_uses - 1) & 1, W_QEMPTY, r))) break;
+                        load_q(x, 0);
+                        ++q0_uses;
+                    }
                 }
                 // Every copy has landed once the softmax warps have seen the last product complete (they wait for it, and
                 // the barrier below waits for them).  Only a CTA that gave up may have some in flight still: give them
@@ -237,101 +335,166 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             // cycle this warp spends on something else than issuing leaves the pipe idle.  A wait costs some 150 cycles
             // even when the barrier completed long ago; each barrier is therefore looked at (test_wait) while the MMAs
             // before it are still being issued, and waited for only if that look came too early.
-            if (nk > 0) {
-                const uint32_t leader = elect_one_sync();
-                auto wait = [&](bool seen, uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
-                    if (__all_sync(0xffffffffu, seen)) return true;
-                    return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
-                };
-                constexpr uint32_t IDESC_S = make_idesc_tf32(TILE, TILE, false, false);
-                constexpr uint32_t IDESC_O = make_idesc_tf32(TILE, HEAD_DIM, false, true);
-                // products in issue order: step by step, stream 0 before stream 1 (a stream takes part while j < n_t)
-                struct Product {
-                    int j, t, buf;   // step, stream, score buffer
-                    uint32_t par;    // parity of the score buffer's barriers
-                    RingPos k, v;    // its key and value tile
-                    bool first;      // key tile 0
-                };
-                const int total = n0 + n1;
-                auto advance = [&](Product& p) {
-                    const bool next_step = p.t == 1 || p.j >= n1;
-                    if (next_step) ++p.j;
-                    p.t = (next_step && p.j < n0) ? 0 : 1;
-                    if (next_step || keys) {
-                        p.k.advance(p.first ? 1 : 2);
-                        p.v.advance(2);
-                        p.first = false;
+            const uint32_t leader = elect_one_sync();
+            auto wait = [&](bool seen, uint64_t* bar, uint32_t parity, int id, int aux) -> bool {
+                if (__all_sync(0xffffffffu, seen)) return true;
+                return __all_sync(0xffffffffu, mbar_wait(wc, bar, parity, id, aux));
+            };
+            constexpr uint32_t IDESC_S = make_idesc_tf32(TILE, TILE, false, false);
+            constexpr uint32_t IDESC_O = make_idesc_tf32(TILE, HEAD_DIM, false, true);
+            // products in issue order: step by step, stream 0 before stream 1 (a stream takes part while j < n_t), item by item
+            struct Product {
+                int n0, n1, nk, left;  // of the item: steps of the streams, key tiles, products from this one on
+                int j, t, idx;         // step, stream, number of its key tile
+                int buf;               // score buffer
+                uint32_t par;          // parity of the score buffer's barriers
+                int ke, ve;            // ring entries of its key and value tile
+                RingPos k, v;          // the same as slots
+                int base, r;           // ring entry behind the item, the item's number
+            };
+            auto start = [&](Product& p, const Item& x) {  // at the first product of an item
+                auto u = [](int v) { return TAKES_OVER ? (int)uniform(v) : v; };
+                p.n0 = u(x.n0), p.n1 = u(x.n1), p.nk = u(x.nk);
+                p.left = p.n0 + p.n1;
+                p.j = p.idx = 0;
+                p.t = p.n0 > 0 ? 0 : 1;
+                p.ke = p.base, p.ve = p.base + ring_v<TAKES_OVER>(0, p.nk);
+                p.k = RingPos(p.ke), p.v = RingPos(p.ve);
+                p.base += 2 * p.nk + u(o_slots(x));
+            };
+            auto step = [&](Product& p) {  // past a product, inside the item
+                if (++p.buf == 3) {
+                    p.buf = 0;
+                    p.par ^= 1u;
+                }
+                --p.left;
+                const bool next_step = p.t == 1 || p.j >= p.n1;
+                if (next_step) ++p.j;
+                p.t = (next_step && p.j < p.n0) ? 0 : 1;
+                if (next_step || keys) {
+                    ++p.idx;
+                    const int dk = p.idx == 1 ? 1 : 2, dv = TAKES_OVER && p.idx == p.nk - 1 ? 1 : 2;
+                    if (TAKES_OVER) p.ke += dk, p.ve += dv;
+                    p.k.advance(dk), p.v.advance(dv);
+                }
+            };
+            // first and last product that reads its K / V tile
+            auto new_kv = [&](const Product& p) { return keys || p.t == 0 || p.j >= p.n0; };
+            auto last_kv = [&](const Product& p) { return keys || p.t == 1 || p.j >= p.n1; };
+            const Desc q_desc = kmajor_desc(smem_u32(sQ), 0, BOX_BYTES), k_desc = kmajor_desc(smem_u32(sKV), 0, BOX_BYTES),
+                       v_desc = mnmajor_desc(smem_u32(sKV), 0, BOX_BYTES);
+            auto issue_qk = [&](const Product& p, int box) {  // 32 of the 64 d's
+                umma_ss4<KMAJOR_STEP, KMAJOR_STEP>(leader, tmem + score_col(p.buf),
+                                                   q_desc + ((keys ? 0 : p.t * TILE_BYTES) + box * BOX_BYTES),
+                                                   k_desc + (p.k.slot * TILE_BYTES + box * BOX_BYTES), IDESC_S, box);
+            };
+            const bool state_in = a.continue_state && split == 0;
+            Product pq{0, 0, 0, 0, 0, 0, 0, 0, 0u, 0, 0, RingPos(0u), RingPos(0u), 0, 0};  // the next S = Q K^T to issue
+            start(pq, first);
+            Product pv = pq;               // the next P V to issue
+            uint32_t q_par = 0u;           // bit t: parity of stream t's Q tile
+            int ahead = 0, released = 0;   // products between the two; items handed back
+            bool done = !TAKES_OVER, ok = true, seen_k = false, seen_v = false, seen_p = false;
+            auto release_to = [&](int r) {
+#pragma unroll 1
+                for (; released < r; ++released)
+                    if (lane == 0) mbar_arrive(&sh.item_empty[released % ITEMS]);
+            };
+            while (ok) {
+                // Scores are computed up to three products ahead, into the next item if that is known already.  Neither it nor a
+                // key tile is waited for while that may take a P V that is not issued yet: the ring entry five in front of
+                // the key tile's must have been used up by those that are.
+                if (TAKES_OVER && pq.left == 0 && !done && (ahead == 0 || __all_sync(0xffffffffu, mbar_test_wait(&sh.item_full[pq.r % ITEMS], (pq.r / ITEMS) & 1)))) {
+                    Item x;
+                    done = !__all_sync(0xffffffffu, read_item(x, ++pq.r, false, false));
+                    if (!done) start(pq, x);
+                    continue;
+                }
+                if (pq.left > 0 && ahead < 3 && (!TAKES_OVER || ahead == 0 || pq.ke < pv.ve + SLOTS)) {
+                    if (TAKES_OVER && ahead == 0) pv = pq;
+                    if (pq.j == 0) {
+                        if (!(ok = wait(false, &sh.q_full[keys ? 0 : pq.t], (q_par >> pq.t) & 1u, W_QFULL, pq.t))) break;
+                        if (!keys) q_par ^= 1u << pq.t;
                     }
-                    if (++p.buf == 3) {
-                        p.buf = 0;
-                        p.par ^= 1u;
-                    }
-                };
-                // first and last product that reads its K / V tile
-                auto new_kv = [&](const Product& p) { return keys || p.t == 0 || p.j >= n0; };
-                auto last_kv = [&](const Product& p) { return keys || p.t == 1 || p.j >= n1; };
-                const Desc q_desc = kmajor_desc(smem_u32(sQ), 0, BOX_BYTES), k_desc = kmajor_desc(smem_u32(sKV), 0, BOX_BYTES),
-                           v_desc = mnmajor_desc(smem_u32(sKV), 0, BOX_BYTES);
-                auto issue_qk = [&](const Product& p, int box) {  // 32 of the 64 d's
-                    umma_ss4<KMAJOR_STEP, KMAJOR_STEP>(leader, tmem + score_col(p.buf),
-                                                       q_desc + ((keys ? 0 : p.t * TILE_BYTES) + box * BOX_BYTES),
-                                                       k_desc + (p.k.slot * TILE_BYTES + box * BOX_BYTES), IDESC_S, box);
-                };
-                auto commit_qk = [&](const Product& p) {
-                    umma_commit_lead(leader, &sh.s_full[p.buf]);
-                    if (last_kv(p)) umma_commit_lead(leader, &sh.kv_empty[p.k.slot]);
-                };
-                auto issue_pv = [&](const Product& p, bool acc_first) {  // O_t += P V, P in the product's score buffer
-                    const uint32_t pc = tmem + score_col(p.buf), d = tmem + COL_O0 + p.t * HEAD_DIM;
-                    const Desc vd = v_desc + p.v.slot * TILE_BYTES;
-                    umma_ts4<MNMAJOR_STEP>(leader, d, pc, vd, IDESC_O, (p.j > 0 || (acc_first && !(keys && p.t == 1))) ? 1u : 0u);
-#pragma unroll
-                    for (int g = 1; g < 4; ++g) umma_ts4<MNMAJOR_STEP>(leader, d, pc + 32 * g, vd + 4096 * g, IDESC_O, 1u);
-                    umma_commit_lead(leader, &sh.o_full[p.buf]);
-                    if (last_kv(p)) umma_commit_lead(leader, &sh.kv_empty[p.v.slot]);
-                };
-                const bool state_in = a.continue_state && split == 0;
-                Product pq{0, (n0 > 0) ? 0 : 1, 0, 0u, {0u, 0u}, {2u, 0u}, true};  // the next S = Q K^T to issue
-                Product pv = pq;                                                   // the next P V to issue
-                int nq = 0;
-                bool ok = true;
-                for (; ok && nq < 3 && nq < total; ++nq) {
-                    if (pq.j == 0 && !(ok = wait(false, &sh.q_full[keys ? 0 : pq.t], 0, W_QFULL, pq.t))) break;
-                    if (new_kv(pq) && !(ok = wait(false, &sh.kv_full[pq.k.slot], pq.k.phase, W_KFULL, pq.j))) break;
+                    if (new_kv(pq) && !(ok = wait(seen_k, &sh.kv_full[pq.k.slot], pq.k.phase, W_KFULL, pq.j))) break;
                     tc_fence_after_sync();
                     issue_qk(pq, 0);
-                    issue_qk(pq, 1);
-                    commit_qk(pq);
-                    advance(pq);
-                }
-                bool seen_p = false, seen_v = false;
-                for (int q = 0; ok && q < total; ++q) {
-                    if (new_kv(pv) && !(ok = wait(seen_v, &sh.kv_full[pv.v.slot], pv.v.phase, W_VFULL, pv.j))) break;
-                    if (!(ok = wait(seen_p, &sh.p_full[pv.buf], pv.par, W_PFULL, pv.j))) break;
-                    tc_fence_after_sync();
-                    const bool more = nq < total;
-                    const bool seen_k = mbar_test_wait(&sh.kv_full[pq.k.slot], pq.k.phase);
-                    issue_pv(pv, state_in);
-                    advance(pv);
-                    if (more) {
-                        if (new_kv(pq) && !(ok = wait(seen_k, &sh.kv_full[pq.k.slot], pq.k.phase, W_KFULL, pq.j))) break;
-                        tc_fence_after_sync();
-                        issue_qk(pq, 0);
-                    }
                     seen_v = mbar_test_wait(&sh.kv_full[pv.v.slot], pv.v.phase);
                     seen_p = mbar_test_wait(&sh.p_full[pv.buf], pv.par);
-                    if (more) {
-                        issue_qk(pq, 1);
-                        commit_qk(pq);
-                        ++nq;
-                        advance(pq);
+                    // on to the next product between the MMAs, whose issue hides it (2 % at 512 queries against 8 192 keys); with
+                    // items to take over the copies cost more than that
+                    Product next = pq;
+                    if (!TAKES_OVER) step(next);
+                    issue_qk(pq, 1);
+                    umma_commit_lead(leader, &sh.s_full[pq.buf]);
+                    if (last_kv(pq)) umma_commit_lead(leader, &sh.kv_empty[pq.k.slot]);
+                    if (TAKES_OVER && pq.j + 1 == (pq.t == 0 ? pq.n0 : pq.n1)) umma_commit_lead(leader, &sh.q_empty[pq.t]);
+                    if (TAKES_OVER) step(next);
+                    pq = next;
+                    seen_k = false;
+                    if (++ahead < 3) continue;
+                }
+                if (ahead == 0) {
+                    if (!TAKES_OVER || done) break;
+                    continue;
+                }
+#pragma unroll 1
+                while (TAKES_OVER && pv.left == 0) {  // on to the item the scores went on to before
+                    Item x;
+                    if (!(ok = __all_sync(0xffffffffu, read_item(x, ++pv.r, false, false)))) break;
+                    start(pv, x);
+                    seen_v = false;  // that look was at another entry
+                }
+                if (!ok) break;
+                if (TAKES_OVER) release_to(pv.r);
+                if (new_kv(pv) && !(ok = wait(seen_v, &sh.kv_full[pv.v.slot], pv.v.phase, W_VFULL, pv.j))) break;
+                if (!(ok = wait(seen_p, &sh.p_full[pv.buf], pv.par, W_PFULL, pv.j))) break;
+                tc_fence_after_sync();
+                if (pq.left > 0) seen_k = mbar_test_wait(&sh.kv_full[pq.k.slot], pq.k.phase);
+                Product next = pv;
+                {  // O_t += P V, P in the product's score buffer
+                    const uint32_t pc = tmem + score_col(pv.buf), d = tmem + COL_O0 + pv.t * HEAD_DIM;
+                    const Desc vd = v_desc + pv.v.slot * TILE_BYTES;
+                    umma_ts4<MNMAJOR_STEP>(leader, d, pc, vd, IDESC_O, (pv.j > 0 || (state_in && !(keys && pv.t == 1))) ? 1u : 0u);
+                    umma_ts4<MNMAJOR_STEP>(leader, d, pc + 32, vd + 4096, IDESC_O, 1u);
+                    if (!TAKES_OVER) step(next);
+#pragma unroll
+                    for (int g = 2; g < 4; ++g) umma_ts4<MNMAJOR_STEP>(leader, d, pc + 32 * g, vd + 4096 * g, IDESC_O, 1u);
+                    umma_commit_lead(leader, &sh.o_full[pv.buf]);
+                    if (last_kv(pv)) umma_commit_lead(leader, &sh.kv_empty[pv.v.slot]);
+                }
+                if (TAKES_OVER) step(next);
+                pv = next;
+                --ahead;
+                seen_v = seen_p = false;
+            }
+        } else if (TAKES_OVER && warp == 2) {
+            // ------------------------------ store warp ------------------------------
+            if (lane == 0) {
+                pdl_wait();
+                Item x = first;
+                uint32_t par = 0u;  // bit t: parity of stream t's barrier
+                bool tok = true;
+                for (int r = 0, base = 0; tok; ) {
+                    base += 2 * x.nk;
+                    const int n_o = o_slots(x);
+                    for (int t = 0; t < n_o; ++t, ++base) {
+                        if (!(tok = mbar_wait(wc, &sh.o_staged[t], (par >> t) & 1u, W_OSTAGED, r))) break;
+                        par ^= 1u << t;
+                        mbar_arrive(&sh.o_taken[t]);
+                        // rows past the end of the sequence are clipped by the copy
+                        tma_store_tile(&mapO, sKV + base % SLOTS * TILE_BYTES, row0_of(x, t), x.h, x.b);
+                        bulk_commit_group();
+                        bulk_wait_group_read_all();  // the copy has read its source; it completes on its own
+                        mbar_arrive(&sh.kv_empty[base % SLOTS]);
                     }
+                    if (!tok || !read_item(x, ++r, true, true)) break;
                 }
             }
         }
         // teardown of the control warps (kept inside this branch: the two register regimes never
         // share code after the hand-over)
-        if (combine) barrier_all();  // partial results staged
+        if (COMBINE) barrier_all();  // partial results staged
         tc_fence_before_sync();
         barrier_all();
         if (warp == 1) {
@@ -346,25 +509,30 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         const int t = (warp - 4) >> 2;                   // stream
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;             // row inside the product = tensor-memory lane
-        const int qrow = row0_of(t) + row;               // row inside this (b,h)
-        const bool row_ok = qrow < q_end;
-        const bool warp_live = row0_of(t) + quarter * 32 < q_end;  // any row of this warp exists
-        const int nt = t == 0 ? n0 : n1;
         const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
         const uint32_t tO = trow + COL_O0 + t * HEAD_DIM;
+        const float cs = a.scale_log2e;
+        const float worst = (cs >= 0.f) ? -INFINITY : INFINITY;  // raw score that can never win the max
+        const bool scaled = a.drop_scaled != 0;
+        bool ok = true;
+        uint32_t r[128];
+
+        Item x = first;
+        int base = 0, q_base = 0, uses = 0;  // ring entries, products of the items before; items in which this stream had rows
+        for (int item = 0; ok;) {
+        const int n0 = x.n0, n1 = x.n1, b = x.b, h = x.h, bh = x.bh, q_end = end_of(x);
+        const int nt = x.steps(t);
+        const int qrow = row0_of(x, t) + row;               // row inside this (b,h)
+        const bool row_ok = qrow < q_end;
+        const bool warp_live = row0_of(x, t) + quarter * 32 < q_end;  // any row of this warp exists
         // last key index (local to this call's K) this row may see
         long long lim_ll = a.Tk - 1;
         if (a.causal) lim_ll = min(lim_ll, (long long)a.q_pos0 + qrow - a.k_pos0);
         const int kv_lim = row_ok ? (int)max(-1ll, lim_ll) : -1;
-        const float cs = a.scale_log2e;
-        const float worst = (cs >= 0.f) ? -INFINITY : INFINITY;  // raw score that can never win the max
-        const bool scaled = a.drop_scaled != 0;
         const bool state_in = a.continue_state && split == 0 && !(keys && t == 1);
 
         float m = -INFINITY;  // running max actually used as exponent reference, log2 units
         float l = 0.f;
-        bool ok = true;
-        uint32_t r[128];
         if (state_in && nt > 0) {
             // The result over the keys seen so far is the starting state: reference LSE, normaliser 1 and the running
             // output O itself (a row that has seen no key starts from nothing).  The output accumulator is written
@@ -387,7 +555,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         }
 
         // a product's number in the issue order picks its score buffer
-        auto product = [&](int j) { return min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0); };
+        auto product = [&](int j) { return q_base + min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0); };
         int q_prev = 0;  // number of this stream's previous product
         for (int j = 0; j < nt; ++j) {
             const int q = product(j);
@@ -402,7 +570,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tmem_ld32p(tS + 32, r + 32);
                 tmem_ld32p(tS + 64, r + 64);
                 tmem_ld32p(tS + 96, r + 96);
-                const int kv0 = (keys ? jb + 2 * j + t : jb + j) * TILE;
+                const int kv0 = (x.jb + (keys ? 2 * j + t : j)) * TILE;
                 const int lim_local = kv_lim - kv0;  // columns 0..lim_local are visible
                 tmem_wait_ld();
                 if (lim_local < TILE - 1) {
@@ -477,39 +645,44 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     }
                     s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
                 } else if constexpr (DROP == 2) {
-                    // One Philox call per eight keys of this row, four calls in flight; none for 32 keys that no row of
-                    // the warp sees (on the diagonal three in eight).  This integer arithmetic is what dropout costs:
-                    // H25 B32 T1024 takes 545 us with, 340 without it in one run (in another, where it took 477 - 495 with
-                    // it, all sixteen calls interleaved: 530; one at a time: 780; the calls in front of the wait for S:
-                    // 570 - 640; wide 32 x 32 multiplications: + 15 %).
+                    // One Philox call per eight keys of this row.  32 keys at a time, read from tensor memory once more, in a
+                    // rolled loop: the integer arithmetic is what dropout costs, and unrolled over the 128 registers
+                    // its code does not stay in the instruction cache.  None for 32 keys that no row of the warp
+                    // sees (on the diagonal three in eight).
                     const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
                     float2 sk = make_float2(0.f, 0.f), sa = make_float2(0.f, 0.f);  // kept terms, all terms
                     const int warp_lim = __reduce_max_sync(0xffffffffu, lim_local);
+#pragma unroll 1
+                    for (int c = 0; c < 128; c += 32) {
+                        if (c > warp_lim) {
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        if (q4 * 32 > warp_lim) {
-#pragma unroll
-                            for (int u = 0; u < 32; ++u) r[q4 * 32 + u] = 0u;
+                            for (int u = 0; u < 32; ++u) r[u] = 0u;
                         } else {
+                            tmem_ld32p(tS + c, r);
+                            hk_philox4_t w[4];
 #pragma unroll
-                            for (int g = 4 * q4; g < 4 * q4 + 4; ++g) {
-                                const uint32_t kpos = (uint32_t)(a.k_pos0 + kv0 + g * 8);
-                                const hk_philox4_t w = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
-                                                                      (uint32_t)(a.q_pos0 + qrow), kpos >> 3);
+                            for (int g = 0; g < 4; ++g)
+                                w[g] = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh, (uint32_t)(a.q_pos0 + qrow),
+                                                           (uint32_t)(a.k_pos0 + kv0 + c + 8 * g) >> 3);
+                            tmem_wait_ld();
+                            if (lim_local < c + 31) {
 #pragma unroll
-                                for (int u = 0; u < 8; u += 2) {
-                                    const int i = g * 8 + u;
-                                    const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
-                                    float2 p = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
-                                    if (scaled) sa = __fadd2_rn(sa, p);  // the normaliser ignores the mask
-                                    if (!hk_philox_keep1(w, u, a.drop_thr)) p.x = 0.f;
-                                    if (!hk_philox_keep1(w, u + 1, a.drop_thr)) p.y = 0.f;
-                                    sk = __fadd2_rn(sk, p);
-                                    r[i] = tf32_round_bits_mma(__float_as_uint(p.x));
-                                    r[i + 1] = tf32_round_bits_mma(__float_as_uint(p.y));
-                                }
+                                for (int i = 0; i < 32; ++i)
+                                    if (c + i > lim_local) r[i] = __float_as_uint(worst);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 32; i += 2) {
+                                const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
+                                float2 p = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
+                                if (scaled) sa = __fadd2_rn(sa, p);  // the normaliser ignores the mask
+                                if (!hk_philox_keep1(w[i >> 3], i & 7, a.drop_thr)) p.x = 0.f;
+                                if (!hk_philox_keep1(w[i >> 3], (i & 7) + 1, a.drop_thr)) p.y = 0.f;
+                                sk = __fadd2_rn(sk, p);
+                                r[i] = tf32_round_bits_mma(__float_as_uint(p.x));
+                                r[i + 1] = tf32_round_bits_mma(__float_as_uint(p.y));
                             }
                         }
+                        tmem_st32p(tS + c, r);
                     }
                     s0 = sk.x; s1 = sk.y; s2 = sa.x; s3 = sa.y;
                 } else {
@@ -523,10 +696,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                         r[i] = tf32_round_bits_mma(__float_as_uint(p));
                     }
                 }
-                tmem_st32p(tS, r);
-                tmem_st32p(tS + 32, r + 32);
-                tmem_st32p(tS + 64, r + 64);
-                tmem_st32p(tS + 96, r + 96);
+                if constexpr (DROP != 2) {
+                    tmem_st32p(tS, r);
+                    tmem_st32p(tS + 32, r + 32);
+                    tmem_st32p(tS + 64, r + 64);
+                    tmem_st32p(tS + 96, r + 96);
+                }
                 // inverted dropout: s2, s3 hold the sums over all visible keys, s0, s1 the kept ones
                 l = l * alpha + ((scaled && DROP != 0) ? (s2 + s3) : ((s0 + s1) + (s2 + s3)));
                 m = m_new;
@@ -540,42 +715,64 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // epilogue: O / l and LSE
         if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, nt));
         tc_fence_after_sync();
-        const float inv_l = combine ? 1.f : (l > 0.f) ? a.keep_scale / l : 0.f;
+        const float inv_l = COMBINE ? 1.f : (l > 0.f) ? a.keep_scale / l : 0.f;
         if (ok && nt > 0) {
             tmem_ld32p(tO, r);
             tmem_ld32p(tO + 32, r + 32);
             tmem_wait_ld();
+            tc_fence_before_sync();  // the next item's first P V overwrites it
         } else {
 #pragma unroll
             for (int i = 0; i < 64; ++i) r[i] = 0u;
         }
-        // O leaves through shared memory (a thread-per-row store would touch 32 lines per instruction).  The stream's own Q
-        // buffer is dead -- o_full covered its last S = Q K^T, and in keys mode, where the streams share Q, every S: the
-        // last one is issued before the last two P V -- and takes the two 32-column boxes of a 128-byte-swizzled TMA tile:
-        // 16-byte chunk i of row r at position i ^ (r & 7).
-        {
-            uint8_t* srow = sQ + t * TILE_BYTES + row * 128;
+        // O leaves through shared memory (a thread-per-row store would touch 32 lines per instruction): a slot of the ring or, with
+        // one item, the stream's own Q buffer, which is dead -- o_full covered its last S = Q K^T, and in keys mode,
+        // where the streams share Q, every S: the last one is issued before the last two P V.  Either way as the two
+        // 32-column boxes of a 128-byte-swizzled TMA tile: 16-byte chunk i of row r at position i ^ (r & 7).
+        auto stage = [&](uint8_t* dst) {
+            uint8_t* srow = dst + row * 128;
 #pragma unroll
             for (int ch = 0; ch < 16; ++ch)
                 *reinterpret_cast<float4*>(srow + (ch >> 3) * BOX_BYTES + (((ch & 7) ^ (row & 7)) << 4)) =
                     make_float4(__uint_as_float(r[4 * ch]) * inv_l, __uint_as_float(r[4 * ch + 1]) * inv_l,
                                 __uint_as_float(r[4 * ch + 2]) * inv_l, __uint_as_float(r[4 * ch + 3]) * inv_l);
-        }
-        // a block none of whose rows sees a key of this call leaves a continued result untouched
-        const bool keep_old = a.continue_state && (t == 0 ? all0 : all1) == 0;
-        if (!combine) {
+        };
+        if constexpr (TAKES_OVER) {
+            const int n_o = o_slots(x);
+            if (ok && t < n_o) {
+                const int e = base + 2 * x.nk + t;
+                ok = (uses == 0 || mbar_wait(wc, &sh.o_taken[t], (uses - 1) & 1, W_OSLOT, 1000 + item)) &&
+                     mbar_wait(wc, &sh.kv_full[e % SLOTS], (e / SLOTS) & 1, W_OSLOT, item);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                ++uses;
+                stage(sKV + e % SLOTS * TILE_BYTES);
+                fence_proxy_async_smem();
+                mbar_arrive_warp(&sh.o_staged[t], lane);
+                if (row_ok)
+                    a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
+            }
+            base += 2 * x.nk + n_o;
+            q_base += n0 + n1;
+            if (!ok || !read_item(x, ++item, false, true)) break;
+        } else if constexpr (!COMBINE) {
+            stage(sQ + t * TILE_BYTES);
             fence_proxy_async_smem();
+            // a block none of whose rows sees a key of this call leaves a continued result untouched
+            const bool keep_old = a.continue_state && nt == 0;
             if (row_ok && !keep_old)
                 a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
-            // the 128 threads of this stream (every one gets here, whatever `ok` is), then one of them stores; rows past
-            // the end of the sequence are clipped by the copy
+            // the 128 threads of this stream (every one gets here, whatever `ok` is), then one of them stores
             asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
             if (row == 0 && row_ok && !keep_old) {
                 tma_store_tile(&mapO, sQ + t * TILE_BYTES, qrow, h, b);
                 bulk_commit_group();
-                bulk_wait_group_read_all();  // the copies have read their source; they complete on their own
+                bulk_wait_group_read_all();  // the copy has read its source; it completes on its own
             }
+            break;
         } else {
+            const int all0 = x.all0, all1 = x.all1;
+            stage(sQ + t * TILE_BYTES);
             // Combine: O = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M) over the splits and, in keys mode, the two
             // streams.  Each CTA takes an equal slice of the rows it shares with its counterparts, 16 threads per row.
             sh.m[t][row] = m;
@@ -586,7 +783,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             for (int i = threadIdx.x - 128; i < rows * 16; i += NUM_SOFTMAX) {
                 const int rr = split * rows + (i >> 4), ch = i & 15;
                 const int tt = rr / TILE, r1 = rr % TILE;
-                const int qr = row0_of(tt) + r1;
+                const int qr = row0_of(x, tt) + r1;
                 if (qr >= q_end || (a.continue_state && (tt == 0 ? all0 : all1) == 0)) continue;
                 const uint8_t* src = sQ + tt * TILE_BYTES + (ch >> 3) * BOX_BYTES + r1 * 128 + (((ch & 7) ^ (r1 & 7)) << 4);
                 float M = -INFINITY, L = 0.f;
@@ -623,7 +820,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 if (ch == 0)
                     a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qr] = (L > 0.f) ? (M + log2f(L)) * LN2 : -INFINITY;
             }
+            break;
         }
+        }  // items
         tc_fence_before_sync();
         barrier_all();  // pairs with the control warps' barrier before tensor memory is freed
     }
@@ -637,7 +836,9 @@ struct FwdDevice {
     int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
 typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
-const FwdKernel fwd_kernels[3] = {attn_fwd_kernel<0>, attn_fwd_kernel<1>, attn_fwd_kernel<2>};
+const FwdKernel fwd_kernels[9] = {attn_fwd_kernel<0, ONE_ITEM>,     attn_fwd_kernel<1, ONE_ITEM>,     attn_fwd_kernel<2, ONE_ITEM>,
+                                  attn_fwd_kernel<0, TAKE_OVER>,    attn_fwd_kernel<1, TAKE_OVER>,    attn_fwd_kernel<2, TAKE_OVER>,
+                                  attn_fwd_kernel<0, COMBINE_ITEM>, attn_fwd_kernel<1, COMBINE_ITEM>, attn_fwd_kernel<2, COMBINE_ITEM>};
 
 // of the current device; set up by the first call on it
 int fwd_device(FwdDevice** out) {
@@ -654,7 +855,7 @@ int fwd_device(FwdDevice** out) {
         for (int i = 1; i < 4 && d.rc == cudaSuccess; ++i) {
             LaunchConfig lc(8u << i, fwd::NUM_THREADS, fwd::SMEM_BYTES, nullptr, 1 << i, false);
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, fwd_kernels[0], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
+            if (cudaOccupancyMaxActiveClusters(&n, fwd_kernels[6], &lc.cfg) == cudaSuccess && n > 0) d.slots[i] = n;
         }
     });
     if (d.rc != cudaSuccess) return HK_ERR_CUDA;
@@ -704,7 +905,7 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
             const double cost = std::max(one, mean + 0.5 * one);
             if ((mode == FWD_ROWS && i == 0) || cost < 0.95 * best_cost) {
                 best_cost = cost;
-                plan = {mode, 1 << i, nb};
+                plan = {mode, 1 << i, nb, sum / nb};
             }
         }
     }
@@ -722,9 +923,19 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.n_qblocks = plan.n_qblocks;
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
+    // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
+    // then more than the bookkeeping costs per step (about 2 %).  Steps per item on average, one item per CTA -> taken over:
+    // 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same without a mask)
+    // 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
+    // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
+    // storing warp counts on a product in every item.
+    const bool sees_keys = !a.causal || a.q_pos0 >= a.k_pos0;
+    const int job = plan.mode == FWD_KEYS || plan.n_splits > 1                        ? COMBINE_ITEM
+                    : nblocks > d->slots[0] && plan.mean_steps <= 12.0 && sees_keys ? TAKE_OVER
+                                                                                     : ONE_ITEM;
     timing_mark(TIMED_FWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode], mq, mk, mv, mo, a);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * job], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();

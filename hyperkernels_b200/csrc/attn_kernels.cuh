@@ -33,6 +33,7 @@ struct FwdArgs {
 // How a forward's work is cut, from sizes and the resident clusters of 1, 2, 4, 8 CTAs (slots) alone.
 struct FwdPlan {
     int mode, n_splits, n_qblocks;
+    double mean_steps;  // of a block of query rows, before splits
 };
 FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]);
 int attn_fwd_slots(const int** slots);  // of the current device; status
@@ -74,7 +75,6 @@ struct BwdArgs {
     int Tq, Tk;
     int n_kvtiles;
     int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; set by launch_attn_bwd
-    int take_over;     // 1: the grid is larger than the device; CTAs that are through take over others' work; set by launch_attn_bwd
     int q_pos0, k_pos0;
     float scale, scale_log2e;
     int causal;

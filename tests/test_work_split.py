@@ -158,6 +158,52 @@ def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["none", "philox", "dense inverted"])
+@pytest.mark.parametrize("BH,Tq,Tk,causal,pos", [
+    (299, 128, 128, 0, {}), (160, 200, 200, 1, {}), (75, 600, 640, 1, {}), (40, 1000, 1100, 0, {}), (200, 100, 150, 0, {}), (40, 1300, 1800, 0, {}),
+    (60, 1100, 1100, 1, dict(k_pos0=512)), (200, 70, 100, 1, dict(k_pos0=128))])
+def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
+    """More blocks of query rows than CTAs start with, of one to nine steps in one or two streams: first, middle and last slice
+    against the oracle, every one against the same call on few enough slices that no CTA takes anything over (the same bits),
+    and as a continued state.  Beside them the calls that take none over for another reason: long items, and blocks that see
+    no key (k_pos0 behind their rows; all of them in the last case)."""
+    from test_attention_gpu import gate, host, lse_check, ok_status
+
+    q, k, v = _normal((1, BH, Tq, 64), 990), _normal((1, BH, Tk, 64), 991), _normal((1, BH, Tk, 64), 992)
+    Q, K, V = map(_dev, (q, k, v))
+    mode, splits = forward_plan(BH, Tq, Tk, causal, 0, pos.get("k_pos0", 0))
+    assert splits == 1 and BH * -(-Tq // (256 if mode == ROWS else 128)) > 148
+    mask = None if kind == "none" else ol.dropout_mask(BH, Tq, Tk, P, SEED, OFFSET, **pos)
+    kw = {} if kind == "none" else dict(_mask(kind, 1, 8, 8)[0])
+    if "dropout_mask" in kw:
+        kw["dropout_mask"] = _dev(mask)
+    O, L = hk.attention_forward(Q, K, V, SCALE, bool(causal), **pos, **kw)
+    ok_status()
+    for i in (0, BH // 2, BH - 1):
+        s = slice(i, i + 1)
+        O_ref, L_ref = _oracle_forward(kind, None if mask is None else mask[s], q[:, s], k[:, s], v[:, s], causal, **pos)
+        gate("O", host(O[:, s]), O_ref)
+        lse_check(host(L[:, s]), L_ref)
+    if kind == "philox":
+        n = 128 // -(-Tq // 128)  # slices whose blocks all start at once
+        for s0 in range(0, BH, n):
+            s = slice(s0, min(BH, s0 + n))
+            one = hk.attention_forward(Q[:, s], K[:, s], V[:, s], SCALE, bool(causal), **pos, **dict(kw, bh_pos0=s0))
+            assert torch.equal(one[0], O[:, s]) and torch.equal(one[1], L[:, s])
+    if kind == "none":
+        # a block that sees no key of the second call keeps what the first one left
+        O2, L2 = hk.attention_forward(Q, K, V, SCALE, False, q_pos0=0)
+        keep = O2.clone(), L2.clone()
+        hk.attention_forward(Q, K, V, SCALE, bool(causal), **pos, continue_state=True, out=O2, lse=L2)
+        ok_status()
+        blind = min(Tq, pos.get("k_pos0", 0)) if causal else 0
+        assert torch.equal(O2[:, :, :blind], keep[0][:, :, :blind]) and torch.equal(L2[:, :, :blind], keep[1][:, :, :blind])
+        # twice the same keys: the same O, a normaliser twice as large, where every row sees them all
+        if not causal:
+            assert float((O2 - keep[0]).norm() / keep[0].norm()) < 1e-3 and float((L2 - keep[1] - np.log(2.0)).abs().max()) < 2e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["none", "philox", "philox inverted"])
 @pytest.mark.parametrize("BH,Tq,Tk,causal", [(299, 128, 128, 0), (60, 640, 640, 1), (75, 100, 300, 0), (90, 257, 384, 1), (60, 130, 1000, 1), (5, 70, 200, 1)])
 def test_backward_ctas_take_over_key_tiles(BH, Tq, Tk, causal, kind):
