@@ -254,8 +254,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         mbar_init(&sh.dk_done, 1);
         mbar_init(&sh.ds_ready, NUM_COMPUTE / 32);
         mbar_init(&sh.dq_full, 1);
-        mbar_init(&sh.dq_empty, 8);   // column groups 2, 3 drain dQ
-        mbar_init(&sh.dq_staged, 8);
+        mbar_init(&sh.dq_empty, NUM_COMPUTE / 32);
+        mbar_init(&sh.dq_staged, NUM_COMPUTE / 32);
         mbar_init(&sh.dq_out, 1);
         mbar_init(&sh.dv_staged, 8);  // column groups 0, 1
         mbar_init(&sh.dk_staged, 8);  // column groups 2, 3
@@ -573,25 +573,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         bool ok = true;
         uint32_t rs[32], rp[32];
 
-        // dQ of query tile j out of tensor memory into the K-major dO tile (column groups 2 and 3 only: this thread's
-        // query row `row`, 32 columns), in the layout of a 128-byte-swizzled TMA box: 16-byte chunk c of row r at
+        // dQ of query tile j out of tensor memory into the K-major dO tile (this thread's query row `row`, 16 of the 64
+        // columns), in the layout of a 128-byte-swizzled TMA box: 16-byte chunk c of row r at
         // position c ^ (r & 7).  Done in the middle of the NEXT tile, in two parts: read while dP^T of that tile is still
         // being computed, stored when it is done: its operand, the K-major dO tile, is then dead until the tile after it
         // is prefetched, long enough for the bulk reduction, which keeps its source for ~1 600 cycles.
-        auto read_dq = [&](int j, uint32_t (&v)[32]) -> bool {
+        auto read_dq = [&](int j, uint32_t* v) -> bool {
             if (!__all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_full, j & 1, W_DQFULL, j))) return false;
             tc_fence_after_sync();
-            tmem_ld32(trow + COL_DQ + 32 * (part & 1), v);
+            tmem_ld16(trow + COL_DQ + 16 * part, v);
             tmem_wait_ld();
             tc_fence_before_sync();
             mbar_arrive_warp(&sh.dq_empty, lane);  // dQ is in registers: the next dQ = dS K may overwrite tensor memory
             return true;
         };
-        auto stage_dq = [&](const uint32_t (&v)[32]) {
-            uint8_t* srow = sdO + (part & 1) * BOX_BYTES + row * 128;
+        auto stage_dq = [&](const uint32_t* v) {
+            uint8_t* srow = sdO + (part >> 1) * BOX_BYTES + row * 128;
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<uint4*>(srow + ((c ^ (row & 7)) << 4)) =
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4*>(srow + (((4 * (part & 1) + c) ^ (row & 7)) << 4)) =
                     make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
             fence_proxy_async_smem();
             mbar_arrive_warp(&sh.dq_staged, lane);
@@ -724,14 +724,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 tc_fence_before_sync();
                 mbar_arrive_warp(&sh.pt_ready, lane);
             }
-            if (g > 0 && part >= 2) {  // rp is free until dP^T is loaded
-                if (it == 0 && !(ok = copy_v(item, rp))) break;
+            if (g > 0) {  // rp is free until dP^T is loaded
+                if (it == 0 && part >= 2 && !(ok = copy_v(item, rp))) break;
                 if (!(ok = read_dq(g - 1, rp))) break;
             }
             ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, g & 1, W_SFULL, 1000 + g));
             if (!ok) break;
             tc_fence_after_sync();
-            if (g > 0 && part >= 2) stage_dq(rp);
+            if (g > 0) stage_dq(rp);
             tmem_ld32(trow + COL_DP + c0, rp);
             tmem_wait_ld();
 
@@ -768,16 +768,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
             // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns
             // 32*part..32*part+31, one 128-byte row per key row, 32-byte chunks XOR-swizzled with (row & 3).  Boxes 0, 1
-            // -- the groups that get here first -- have a buffer of their own, free once dQ of the previous tile is done
-            // (before the first tile the buffer held V, which every thread has left once v_ready completes); boxes 2, 3 go over the MN-major dO tile as soon as dV of
-            // this tile is done.
-            if (part < 2) {
-                ok = __all_sync(0xffffffffu, it == 0 ? mbar_wait(wc, &sh.v_ready, item & 1, W_VREADY, 1)
-                                                      : mbar_wait(wc, &sh.dq_full, (g - 1) & 1, W_DQFULL, 1000 + g));
-            } else {
+            // have a buffer of their own, free once dQ of the previous tile is done -- and, at the first tile of an item, V
+            // has left it --: dP^T of this tile, complete here, was issued behind either.  Boxes 2, 3 go over the MN-major dO
+            // tile as soon as dV of this tile is done.
+            if (part >= 2) {
                 ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, g & 1, W_DVDONE, g));
+                if (!ok) break;
             }
-            if (!ok) break;
             {
                 // Rows r and r + 4 share a 32-byte chunk position; they store its two halves in opposite order so
                 // that the eight lanes of a quarter-warp hit eight different 16-byte bank groups.
@@ -831,7 +828,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // last reader was dP^T of this tile) once the reduction of the previous tile has read that buffer, then
         // added to global memory by the store warp.  (From registers with red.global.add it took ~2 500 cycles per
         // CTA and held up the bulk stores of dV and dK behind it.)
-        if (ok && g > 0 && part >= 2) {
+        if (ok && g > 0) {
             if (g > 1) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dq_out, (g - 2) & 1, W_DQOUT, g - 2));
             if (ok) ok = read_dq(g - 1, rs);
             if (ok) stage_dq(rs);
