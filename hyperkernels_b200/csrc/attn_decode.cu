@@ -9,9 +9,7 @@
 // loads of 2 * UNROLL rows before it uses the first.  Scores are reduced over the 16 lanes with shuffles; the running
 // maximum is raised once per batch of rows.  The partial (m, l, O) of the warps are merged in shared memory, those of the
 // CTAs of a slice (a cluster) through distributed shared memory.
-//   B16 H12, one query, 2 047 keys (201 MB, 31 us at the copy bandwidth): 37 us, 55 with the tensor-core kernel.
-#include <algorithm>
-
+//   B16 H12, one query, 2 047 keys (201 MB, 31 us at the copy bandwidth): 33 us, 55 with the tensor-core kernel.
 #include "attn_kernels.cuh"
 
 namespace hk {
@@ -168,20 +166,32 @@ __global__ void __launch_bounds__(WARPS * 32, (NQ == 1 ? 24 : 16) / WARPS) attn_
     }
 }
 
-// CTAs per slice: up to eight (the portable cluster size), each warp with at least one batch of rows.  Warps per CTA:
-// four, more where the slices are so few that eight CTAs each do not put ~16 warps on every SM.
-DecodePlan plan_attn_decode(int BH, int Tk, int sms) {
-    DecodePlan p{4, 8};
-    for (int w = 0; w < 2 && (long long)BH * 8 * p.warps < sms * 16; ++w) p.warps *= 2;
-    while (p.n_splits > 1 && (long long)p.n_splits * p.warps * 2 * dec::UNROLL > Tk) p.n_splits /= 2;
-    return p;
+// Warps of a CTA and CTAs of a slice (a cluster of up to eight, the portable size): as many warps per slice as can all be
+// resident at once, each with at least one batch of rows.  A second wave finds a chip that the first is leaving a CTA at a
+// time.  B4 H8, 8 191 keys: 25.0 us with 14 warps per SM, 37.7 with 28 wanted and 24 that fit; B16 H12, 2 047 keys: 33.0 with 21, 37.1
+// with 42, 36.6 with 10; B64 H16, 511 keys: 45.3 one CTA per slice, 48 - 63 with more.  Of equal numbers eight warps come
+// first, then larger CTAs in smaller clusters.  Slices that do not fit at all take one CTA each.
+DecodePlan plan_attn_decode(int BH, int Tq, int Tk, int sms) {
+    static const DecodePlan order[] = {{8, 4}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}};
+    DecodePlan best{Tq == 1 ? 8 : 4, 1};
+    int most = 0;
+    for (const DecodePlan& p : order) {
+        const double filled = p.n_splits == 8 ? 0.85 : p.n_splits == 4 ? 0.92 : 1.0;  // clusters do not pack every SM
+        const double ctas = sms * filled * ((Tq == 1 ? 24 : 16) / p.warps);           // resident, by the kernels' launch bounds
+        const int n = p.warps * p.n_splits;
+        if ((double)BH * p.n_splits <= ctas && (long long)n * 2 * dec::UNROLL <= Tk && n > most) {
+            most = n;
+            best = p;
+        }
+    }
+    return best;
 }
 
 int launch_attn_decode(DecodeArgs a, cudaStream_t stream) {
     typedef void (*Kernel)(DecodeArgs);
     static const Kernel kernels[2][3] = {{attn_decode_kernel<1, 4>, attn_decode_kernel<1, 8>, attn_decode_kernel<1, 16>},
                                          {attn_decode_kernel<2, 4>, attn_decode_kernel<2, 8>, attn_decode_kernel<2, 16>}};
-    const DecodePlan plan = plan_attn_decode(a.BH, a.Tk, sm_count());
+    const DecodePlan plan = plan_attn_decode(a.BH, a.Tq, a.Tk, sm_count());
     const int warps = plan.warps;
     const Kernel k = kernels[a.Tq - 1][warps == 4 ? 0 : warps == 8 ? 1 : 2];
     a.n_splits = plan.n_splits;

@@ -59,7 +59,7 @@ struct DecodeArgs {
 struct DecodePlan {
     int warps, n_splits;
 };
-DecodePlan plan_attn_decode(int BH, int Tk, int sms);
+DecodePlan plan_attn_decode(int BH, int Tq, int Tk, int sms);
 int launch_attn_decode(DecodeArgs a, cudaStream_t stream);
 
 struct BwdArgs {

@@ -494,7 +494,7 @@ int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* pla
     int mode = 0, rc = validate_dropout(p->dropout_p, p->dropout_mask, p->flags, p->k_pos0, &mode);
     if (rc != HK_OK) return rc;
     if (decodes(p->T, Tk, mode, p->flags)) {
-        const DecodePlan d = plan_attn_decode(p->B * p->nh, (int)Tk, slots ? slots[0] : sm_count());
+        const DecodePlan d = plan_attn_decode(p->B * p->nh, (int)p->T, (int)Tk, slots ? slots[0] : sm_count());
         plan[0] = -1; plan[1] = d.n_splits; plan[2] = d.warps;
         return HK_OK;
     }

@@ -101,6 +101,47 @@ def _oracle_backward(kind, mask, q, k, v, O, g, L, causal, **pos):
     return ol.attn_backward_mt(q, k, v, O, g, L, SCALE, causal, mask, **pos)
 
 
+def decode_plan(BH, Tq, Tk, slots=B200):
+    """(warps of a CTA, CTAs of a slice)"""
+    p = hk.MemEfficientFwdParams()
+    p.B, p.nh, p.T, p.kv_len = 1, BH, Tq, Tk
+    out = (C.c_int * 3)()
+    assert hk.lib().hk_attn_forward_plan(C.byref(p), slots, out) == 0 and out[0] == DECODE
+    return out[2], out[1]
+
+
+def test_decode_puts_one_wave_of_warps_on_the_chip():
+    """As many warps as are resident together, unless one CTA per slice is more already; each with a batch of rows."""
+    rnd = random.Random(2)
+    for _ in range(3000):
+        BH, Tq, Tk = int(2 ** rnd.uniform(0, 12)), rnd.choice([1, 2]), int(2 ** rnd.uniform(7, 15))
+        warps, splits = decode_plan(BH, Tq, Tk)
+        assert warps in (4, 8, 16) and splits in (1, 2, 4, 8) and warps * splits * 8 <= Tk
+        per_sm = 24 if Tq == 1 else 16
+        assert BH * splits <= 148 * (per_sm // warps) or splits == 1
+        # twice the splits would not fit any more, or leave warps without rows
+        if splits < 8 and BH * splits * 2 <= 0.85 * 148 * (per_sm // warps):
+            assert warps * splits * 2 * 8 > Tk
+    assert decode_plan(192, 1, 2047) == (8, 2) and decode_plan(1024, 1, 511) == (8, 1) and decode_plan(12, 1, 2047) == (16, 8)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("BH,Tq,Tk,causal,warps,splits", [
+    (4, 1, 129, 1, 8, 2), (4, 2, 257, 0, 8, 4), (2, 1, 2049, 1, 16, 8), (30, 1, 515, 1, 16, 4), (60, 2, 131, 1, 8, 2), (40, 1, 1025, 0, 8, 8),
+    (160, 1, 140, 1, 8, 2), (300, 1, 200, 0, 8, 1), (500, 1, 130, 1, 4, 1), (1000, 1, 130, 1, 8, 1), (700, 2, 129, 0, 4, 1), (90, 2, 300, 1, 8, 2)])
+def test_every_decode_cut(BH, Tq, Tk, causal, warps, splits):
+    from test_attention_gpu import gate, host, lse_check, ok_status
+
+    q, k, v = _normal((1, BH, Tq, 64), 950), _normal((1, BH, Tk, 64), 951), _normal((1, BH, Tk, 64), 952)
+    pos = Tk - Tq if causal else 0
+    assert decode_plan(BH, Tq, Tk) == (warps, splits)
+    O_ref, L_ref = ol.attn_forward_mt(q, k, v, SCALE, causal, q_pos0=pos)
+    O, LSE = hk.attention_forward(_dev(q), _dev(k), _dev(v), SCALE, bool(causal), q_pos0=pos)
+    ok_status()
+    gate("O", host(O), O_ref)
+    lse_check(host(LSE), L_ref)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", MASKS)
 @pytest.mark.parametrize("mode,splits,BH,Tq,Tk,causal", [
