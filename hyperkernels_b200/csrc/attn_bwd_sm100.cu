@@ -470,6 +470,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // ------------------------------ store warp ------------------------------
         // Everything that leaves the CTA: the staged dQ tiles (bulk reductions) and, at the end of an item, dK and dV (bulk
         // stores).  A thread of its own, so that a reduction is issued the moment its tile is staged.
+        if constexpr (SPLIT) cluster_arrive();
         if (lane == 0) {
             pdl_wait();
             tma_prefetch_desc(&mapdK);
@@ -824,6 +825,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         ++item;
         }  // items
 
+        if constexpr (SPLIT) {
+            __syncwarp();
+            cluster_arrive();
+        }
+
         // dQ of the last query tile takes the same way out as the others: staged in the K-major dO tile (dead: its
         // last reader was dP^T of this tile) once the reduction of the previous tile has read that buffer, then
         // added to global memory by the store warp.  (From registers with red.global.add it took ~2 500 cycles per
@@ -838,9 +844,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
     if constexpr (SPLIT) {
         // dV and dK of the KV tile: the sum over the splits, always in the same order, from what each left in its shared
-        // memory; each CTA adds up an equal slice of the rows, 32 threads per row (16 for dV, 16 for dK).
+        // memory; each CTA adds up an equal slice of the rows, 32 threads per row (16 for dV, 16 for dK).  The compute warps
+        // have arrived once their dV and dK were staged, the store warp at its start: no CTA waits for another's last dQ, and
+        // the sums are stored while the others leave (24.7 -> 22.7 us for B=4 H=6, 777 queries, 333 keys).
         __syncwarp();
-        cluster_arrive();
+        if (warp >= W_LOAD && warp != W_STORE) cluster_arrive();
         cluster_wait();
         if (warp < W_LOAD) {
             // (rows of this thread) x (splits) = 8: all loads first, their latency is that of the other SM's memory
@@ -856,6 +864,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
+                if (u == 7) {  // every v is in: the others may leave
+                    __syncwarp();
+                    cluster_arrive();
+                }
                 if ((u + 1) % ns != 0) continue;
                 const int64_t kvrow = first.kv0() + split * (TILE / ns) + warp + NUM_COMPUTE / 32 * (u / ns);
                 if (kvrow < a.Tk) {
@@ -872,8 +884,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
             }
         }
         __syncwarp();
-        cluster_arrive();  // the others have read this CTA's shared memory
-        cluster_wait();
+        if (warp >= W_LOAD) cluster_arrive();
+        cluster_wait();  // the others have read this CTA's shared memory
     }
 
     // ------------------------------ teardown ------------------------------
