@@ -25,6 +25,7 @@
 //                 P V(1) S(4) | ...: the scores of a stream's NEXT step are computed while its softmax works on the
 //                 current one (the tensor pipe executes in issue order, so S(q+3) cannot overtake the P V(q) that
 //                 reads the same buffer).
+//   warp 2        where further blocks of rows follow: O of a finished one to global memory, by TMA
 //   warps 4-7     softmax of stream 0, warps 8-11 softmax of stream 1: thread r owns query row r (tensor-memory lane
 //                 r), holds the 128 scores of a step in registers (one tensor-memory read per score) and writes P back
 //                 over S.  (Two threads per row, sixteen warps: the exchange of the row maximum alone takes 300 cycles
@@ -32,6 +33,10 @@
 //                 final O/l and LSE use the same maximum, so the result is the same function).
 // Tensor memory: three score buffers (128 columns each), O_0, O_1 (64 columns each): 512 of 512 columns.
 // Warps 0-3 give most of their registers to the softmax warps (setmaxnreg 72 / 216).
+//
+// Where there are more blocks of rows than SMs and they are short, a CTA that is through with one takes over another of a CTA
+// not started yet (cluster launch control, FwdJob::TAKE_OVER): its loads, scores and first softmax run under the last products
+// of the block before it.
 //
 // Key splits: a cluster of NS CTAs shares one block of query rows; split s takes a contiguous run of its key tiles, and at
 // the end every CTA combines a slice of the rows from the partial (O, m, l) the others left in their shared memory (keys
@@ -872,44 +877,87 @@ int attn_fwd_slots(const int** slots) {
     return rc;
 }
 
-FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]) {
-    // Mode and splits by an estimate of the makespan: the mean load of a slot plus half of the longest cluster, but at
-    // least that cluster.  A CTA costs ~3.5 us and ~2.1 us per step of two products (1.5 with one stream, 2.3 in keys
-    // mode), ~2 us more when it merges streams and ~3 us more when it combines splits.  Rows mode loads a key tile once
-    // for two products and is the fastest where it fills the chip; row mode where it does not; keys mode and splits
-    // when even those leave most SMs idle (512 queries of 32 heads against 8 192 keys: 64 CTAs of 64 steps on 148 SMs).
-    // Those two sum in another order, and the choice depends on batch x heads: they are left out for sequences of
-    // training length, so that a batch cut into calls gives the bits of the single call.
+FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, bool drop, const int slots[4]) {
+    // Mode and splits by estimates of the makespan.  Rows mode loads a key tile once for two products and is the fastest
+    // where it fills the chip; row mode where it does not; keys mode and splits when even those leave most SMs idle (512
+    // queries of 32 heads against 8 192 keys: 64 CTAs of 64 steps on 148 SMs).  Those two sum in another order, and the choice
+    // depends on batch x heads: they are left out for sequences of training length, so that a batch cut into calls gives the
+    // bits of the single call.
+    //
+    // Two estimates.  The coarse one takes the mean load of a slot plus half of the longest cluster, but at least that
+    // cluster, whether or not one wave holds all of them; a CTA costs ~3.5 us and ~2.1 us per step of two products (1.5 with
+    // one stream, 2.3 in keys mode), ~2 us more when it merges streams and ~3 us more when it combines splits.  The fine one
+    // tells one wave from several and is fitted to kernel times of every cut of 330 shapes, with dropout and without (1 - 400
+    // slices, 16 - 12 000 queries, 64 - 18 000 keys).  It is off by 9 % on average, so it replaces the coarse one's cut only
+    // where it expects a gain of 15 % (13 % between rows and row mode): a quarter of those shapes, chosen close to the lines
+    // between the cuts.  Of 1 000 further ones 103 are cut differently, 1.23 times as fast on average; three of them are 3 - 4 %
+    // slower and one 10 %.  (By itself the fine estimate slows 7 % of the fitted shapes, by up to 25 %.)  H16, 512 queries, 4 096
+    // keys 27.7 -> 21.4 us; H32, 128 queries, 2 048 keys 16.0 -> 12.2; H24 T525 without a mask, with dropout 19.3 -> 16.2.
     const bool may_split = Tk > 4096 || Tk >= 2 * (long long)Tq;
-    FwdPlan plan{};
-    double best_cost = 0;
+    // Of the cuts of splits of eight key tiles or fewer 2 us are at stake; there the coarse estimate stays alone, and with it
+    // the small shapes that reach each mode.
+    const bool refine = !may_split || Tk > 8 * TILE;
+    const int n_kvtiles = (Tk + TILE - 1) / TILE;
+    FwdPlan plan{}, fine_plan{};
+    double coarse_cost = 0, cost_of_plan = 0, fine_cost = 0;  // cost_of_plan: of the coarse one's cut, by the fine one
     for (int mode = FWD_ROWS; mode <= (may_split ? FWD_KEYS : FWD_ROW); ++mode) {
         const int rows = mode == FWD_ROWS ? 2 * TILE : TILE;
         const int nb = (Tq + rows - 1) / rows;
-        double sum = 0, longest = 0;  // steps of one (batch, head) slice, of its longest block
+        // steps of one (batch, head) slice, of its longest block, of its last, of the shortest of the others
+        double sum = 0, longest = 0, last_block = 0, shortest = 1e30;
         const int sampled = std::min(nb, 64);  // the work per block is linear in its position: long sequences are sampled
         for (int i = 0; i < sampled; ++i) {
             const long long blk = sampled == nb ? i : (long long)i * (nb - 1) / (sampled - 1);
             const int last = (int)(std::min<long long>(Tq, (blk + 1) * rows) - 1);  // its tile sees the most keys of the block
             const int tiles = fwd::kv_tiles_for(last / TILE * TILE, Tq, Tk, causal, q_pos0, k_pos0);
-            const double st = mode == FWD_KEYS ? 0.5 * tiles : tiles;
-            sum += st;
-            longest = std::max(longest, st);
+            if (i > 0) shortest = std::min(shortest, last_block);
+            last_block = mode == FWD_KEYS ? 0.5 * tiles : tiles;
+            sum += last_block;
+            longest = std::max(longest, last_block);
         }
         sum *= (double)nb / sampled;
+        // in rows mode the last block may be of a single row tile: its steps are those of row mode
+        const bool single = mode == FWD_ROWS && (Tq + TILE - 1) / TILE % 2 == 1;
         for (int i = 0; i < (may_split ? 4 : 1); ++i) {
+            const int ns = 1 << i;
+            const FwdPlan cut = {mode, ns, nb, sum / nb};
+            double fine = 1e30;
+            if (refine && (mode != FWD_KEYS || n_kvtiles >= 2 * ns)) {
+                // A CTA, adding up a cluster, a step (with dropout), how much longer a step is on a full device; a key tile's
+                // share of the L2's bandwidth (keys mode loads two per step) and, once per slice, of the memory's.  All in us.
+                static const double CTA[3] = {3.7, 3.4, 3.9}, CLUSTER[3] = {5.3, 2.4, 2.3}, BUSY[3] = {0.07, 0.04, 0.16};
+                static const double STEP[2][3] = {{1.5, 1.3, 1.7}, {3.0, 2.5, 2.9}};
+                const double L2_TILE = 0.007, HBM_TILE = 0.0024, TAKING_OVER = 0.6;
+                const double n = (double)BH * nb, busy = std::min(1.0, n / slots[i]), waves = std::ceil(n / slots[i]);
+                const double fixed = CTA[mode] + (i ? CLUSTER[mode] : 0.0);
+                const double step = STEP[drop][mode] * (1.0 + BUSY[mode] * busy);
+                const double last_step = single ? STEP[drop][FWD_ROW] * (1.0 + BUSY[FWD_ROW] * busy) : step;
+                const double loads = BH * (L2_TILE * sum * (mode == FWD_KEYS ? 2 : 1) + HBM_TILE * n_kvtiles);
+                fine = fixed + std::max(loads, (nb == 1 ? last_step : step) * std::ceil(longest / ns));
+                if (waves > 1) {  // longest first: about a third of the shortest CTA is left over
+                    const double least = fixed + std::min(nb == 1 ? 1e30 : step * std::ceil(shortest / ns), last_step * std::ceil(last_block / ns));
+                    const double mean = (n * fixed + BH * (step * (sum - last_block) + last_step * last_block) / ns) / slots[i];
+                    fine = std::max(fine, std::max(mean + 0.3 * least, waves * least));
+                    if (mode != FWD_KEYS && i == 0) fine += TAKING_OVER;
+                }
+                if (fine_plan.n_splits == 0 || fine < fine_cost) {
+                    fine_cost = fine;
+                    fine_plan = cut;
+                }
+            }
             const double fixed = 3.5 + (mode == FWD_KEYS ? 2.0 : 0.0) + (i ? 3.0 : 0.0);
             const double step = mode == FWD_ROWS ? 2.1 : mode == FWD_ROW ? 1.5 : 2.3;
-            const double one = fixed + step * std::ceil(longest / (1 << i));
-            const double mean = BH * (nb * fixed + step * sum / (1 << i)) / slots[i];
+            const double one = fixed + step * std::ceil(longest / ns);
+            const double mean = BH * (nb * fixed + step * sum / ns) / slots[i];
             const double cost = std::max(one, mean + 0.5 * one);
-            if ((mode == FWD_ROWS && i == 0) || cost < 0.95 * best_cost) {
-                best_cost = cost;
-                plan = {mode, 1 << i, nb, sum / nb};
+            if ((mode == FWD_ROWS && i == 0) || cost < 0.95 * coarse_cost) {
+                coarse_cost = cost;
+                cost_of_plan = fine;
+                plan = cut;
             }
         }
     }
-    return plan;
+    return refine && fine_cost < (may_split ? 0.85 : 0.87) * cost_of_plan ? fine_plan : plan;
 }
 
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
@@ -917,7 +965,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     FwdDevice* d = nullptr;
     const int device_rc = fwd_device(&d);
     if (device_rc != HK_OK) return device_rc;
-    const FwdPlan plan = plan_attn_fwd(a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, d->slots);
+    const FwdPlan plan = plan_attn_fwd(a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, a.dropout_mode != 0, d->slots);
     a.mode = plan.mode;
     a.n_splits = plan.n_splits;
     a.n_qblocks = plan.n_qblocks;

@@ -35,7 +35,7 @@ struct FwdPlan {
     int mode, n_splits, n_qblocks;
     double mean_steps;  // of a block of query rows, before splits
 };
-FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]);
+FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, bool drop, const int slots[4]);
 int attn_fwd_slots(const int** slots);  // of the current device; status
 
 // mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.

@@ -499,7 +499,7 @@ int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* pla
         return HK_OK;
     }
     if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
-    const FwdPlan f = plan_attn_fwd(p->B * p->nh, (int)p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, slots);
+    const FwdPlan f = plan_attn_fwd(p->B * p->nh, (int)p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode != 0, slots);
     plan[0] = f.mode; plan[1] = f.n_splits; plan[2] = 12;
     return HK_OK;
 }

@@ -162,6 +162,34 @@ def test_every_forward_cut_with_every_mask(mode, splits, BH, Tq, Tk, causal, kin
     lse_check(host(LSE), L_ref)
 
 
+# where the fine estimate of the forward's plan decides: (BH, Tq, Tk, causal, dropout) -> its cut, the coarse one's cut
+FINER = [(24, 525, 525, 0, 1, (ROW, 1), (ROWS, 1)), (64, 282, 2017, 1, 0, (ROWS, 1), (KEYS, 1)), (4, 804, 1906, 1, 0, (KEYS, 4), (ROWS, 4)),
+         (16, 22, 8399, 1, 0, (KEYS, 4), (ROW, 8)), (8, 390, 8868, 1, 1, (KEYS, 4), (ROWS, 8))]
+
+
+@pytest.mark.parametrize("BH,Tq,Tk,causal,drop,fine,coarse", FINER)
+def test_the_finer_estimate_decides_by_sizes_alone(BH, Tq, Tk, causal, drop, fine, coarse):
+    kw = dict(flags=hk.FLAG_PHILOX_DROPOUT, dropout_p=0.1) if drop else {}
+    assert forward_plan(BH, Tq, Tk, causal, Tk - Tq if causal else 0, slots=B200, **kw) == fine != coarse
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("BH,Tq,Tk,causal,drop,fine,coarse", FINER)
+def test_forward_cut_by_the_finer_estimate(BH, Tq, Tk, causal, drop, fine, coarse):
+    from test_attention_gpu import gate, host, lse_check, ok_status
+
+    q, k, v = _normal((1, BH, Tq, 64), 970), _normal((1, BH, Tk, 64), 971), _normal((1, BH, Tk, 64), 972)
+    kind, pos = "philox" if drop else "none", Tk - Tq if causal else 0
+    kw, mask = _mask(kind, 1, Tq, Tk, q_pos0=pos)  # the first slice's
+    assert forward_plan(BH, Tq, Tk, causal, pos, **(dict(flags=hk.FLAG_PHILOX_DROPOUT, dropout_p=0.1) if drop else {})) == fine
+    O, LSE = hk.attention_forward(_dev(q), _dev(k), _dev(v), SCALE, bool(causal), q_pos0=pos, **kw)
+    ok_status()
+    s = slice(0, 1)
+    O_ref, L_ref = _oracle_forward(kind, mask, q[:, s], k[:, s], v[:, s], causal, q_pos0=pos)
+    gate("O", host(O)[:, s], O_ref)
+    lse_check(host(LSE)[:, s], L_ref)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", MASKS)
 @pytest.mark.parametrize("splits,BH,Tq,Tk,causal", [
