@@ -2,7 +2,7 @@
 //
 // Computes what mem_efficient_bwd_unified_kernel_exp12<64,Causal> computes
 // (kernels/attention/mem_efficient_bwd_unified_kernel_exp12.cu:54-329 of the
-// reference), one KV tile per CTA, looping over the query tiles that can see it:
+// reference), a KV tile at a time, looping over the query tiles that can see it:
 //   S = Q K^T, dP = dO V^T                    (:186-212)
 //   p = exp2(log2e * (S*scale - LSE)), 0 outside bounds / above the diagonal   (:224-227)
 //   dS = p * (dP - D) * scale                 (:228)
@@ -11,13 +11,13 @@
 // plus the dropout keep-mask (p is multiplied by it), which the reference
 // backward lacks but its forward implies.
 //
-// Blackwell structure (one CTA = one 128-row KV tile, 128-row query tiles):
+// Blackwell structure (a CTA works on one 128-row KV tile at a time, 128-row query tiles):
 // the transposed products S^T = K Q^T and dP^T = V dO^T put key rows on the 128
 // tensor-memory lanes, so P^T and dS^T -- written back over S^T and dP^T by the
 // compute warps -- are directly the tensor-memory A operands of dV += P^T dO and
 // dK += dS^T Q.  dS is also staged once through shared memory (MN-major) as the
 // A operand of dQ = dS K.  dV, dK (64 columns each) stay in tensor memory for
-// the whole CTA; dQ (64 columns) is drained per query tile; V (64 columns) is
+// the whole KV tile; dQ (64 columns) is drained per query tile; V (64 columns) is
 // copied into tensor memory once and is the A operand of dP^T, which frees its
 // 32 KiB of shared memory for dS.  Everything the kernel writes leaves through
 // shared memory and the TMA unit: dQ tiles are added to global memory with bulk
@@ -49,15 +49,21 @@
 // Splits: where few KV tiles have many query tiles (cross-attention of a long sequence to a short one), a cluster of 2, 4
 // or 8 CTAs shares the query tiles of a KV tile; at the end each adds up a slice of the rows of dV and dK from the partial
 // sums the others left in their shared memory (plan_attn_bwd picks the number).  B1 H4, 5 000 queries,
-// 200 keys: 107 -> 25 us; B1 H1, 16 384 and 4 096: 330 -> 100; B4 H6, 777 and 333: 26.5 -> 24.6.
+// 200 keys: 107 -> 25 us; B1 H1, 16 384 and 4 096: 330 -> 100.
+//
+// Where there are more KV tiles than SMs, a CTA that is through with one takes over another of a CTA not started yet (cluster
+// launch control, BwdJob::TAKE_OVER): loads and S^T of the next KV tile run under the last products of this one.  B8 H12 T1024
+// 108 -> 94 us.  All roles run different code at the same time, so it is kept short: at 194 KiB of text (waits unrolled) the
+// first tile of a CTA took 11 000 cycles more than the others, at 108 KiB the loop over the items was 13 - 30 % slower per
+// tile than one item per CTA, at 60 KiB no slower.
 //
 //   warps 0-15  compute: four threads per key row (tensor-memory lane), each
 //               owning 32 of the 128 query columns, all held in registers so
 //               that S^T and dP^T are read from tensor memory exactly once
-//   warp 16     TMA loads (K, V once; Q and dO per query tile, each in two layouts)
+//   warp 16     TMA loads (K, V per KV tile; Q and dO per query tile, each in two layouts)
 //   warp 17     MMA issuer (the whole warp runs the issuing code, one elected lane
 //               issues)
-//   warp 18     TMA reductions of dQ (per query tile) and stores of dK, dV (at the end)
+//   warp 18     TMA reductions of dQ (per query tile) and stores of dK, dV (per KV tile)
 //   warp 19     LSE and D of the query rows into shared memory
 #include <algorithm>
 #include <cmath>

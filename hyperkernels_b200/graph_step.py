@@ -1,10 +1,10 @@
 """Forward + backward captured once in a CUDA graph and replayed.
 
 A training step of the attention path is four launches (dQ zeroing, forward, D
-pre-pass, backward).  A replay takes the host 3.3 us instead of 18 for the two
+pre-pass, backward).  A replay takes the host 3.4 us instead of 17.5 for the two
 calls, which it has for other work; the device is no faster for it where the
-host keeps ahead (B=8, H=12, T=1024: 172 us replayed, 169 by calls; B=2, H=4,
-T=256: 25.0 and 22.3), since the launches of a call are dependent launches
+host keeps ahead (B=8, H=12, T=1024: 142-149 us replayed, 142-146 by calls; B=2,
+H=4, T=256: 22.0 and 17.8), since the launches of a call are dependent launches
 already and the zeroing is one of its own here.  Zeroing dQ depends on nothing, so it is a
 branch beside the forward: its stores (25 MB at B=8, H=12, T=1024) leave the
 D pre-pass and fill SMs the forward's last wave leaves idle.  Capture goes through
