@@ -162,6 +162,13 @@ def test_every_forward_cut_with_every_mask(mode, splits, BH, Tq, Tk, causal, kin
     lse_check(host(LSE), L_ref)
 
 
+@pytest.mark.parametrize("tiles,n_q,splits", [
+    (148, 20, 1), (149, 20, 2), (74, 4, 2), (75, 4, 1), (80, 58, 4), (33, 40, 4), (34, 40, 2), (15, 80, 8), (16, 80, 4), (150, 1, 1), (1, 2, 1), (1, 4, 4)])
+def test_query_splits_by_whole_waves(tiles, n_q, splits):
+    """One CTA more than a wave holds is another wave: either side of each line, for 148, 74, 33 and 15 clusters at once."""
+    assert backward_splits(tiles, 128 * n_q, 64, slots=B200) == splits
+
+
 # where the fine estimate of the forward's plan decides: (BH, Tq, Tk, causal, dropout) -> its cut, the coarse one's cut
 FINER = [(24, 525, 525, 0, 1, (ROW, 1), (ROWS, 1)), (64, 282, 2017, 1, 0, (ROWS, 1), (KEYS, 1)), (4, 804, 1906, 1, 0, (KEYS, 4), (ROWS, 4)),
          (16, 22, 8399, 1, 0, (KEYS, 4), (ROW, 8)), (8, 390, 8868, 1, 1, (KEYS, 4), (ROWS, 8))]
