@@ -957,11 +957,11 @@ int attn_bwd_slots(const int** slots) {
 int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]) {
     // Splits by an estimate of the makespan: whole waves of CTAs that cost ~7 us and ~2.5 us per query tile, ~2.5 - 3 us more
     // where they add dV and dK up over a cluster.  They pay where few KV tiles have many query tiles (cross-attention of a
-    // long sequence to a short one).  Of 110 such shapes the number is the best one or within 2 % of it in all but a few (0.2 %
-    // on average; with half a wave for what the last one leaves over 1.3 %: B2 H2, 9 851 queries, 2 554 keys took two CTAs
-    // per tile, 80 clusters in 74 slots, 208 us; four take 173; of 500 further shapes 36 are cut
-    // differently, 1.10 times as fast on average, one of them 2 % slower).  The sum is taken in another order and the choice depends on
-    // batch x heads, so sequences of training length do without: a batch cut into calls gives the bits of the single call.
+    // long sequence to a short one).  Over 110 such shapes the number is 0.2 % from the best one on average; with half a wave
+    // for what the last one leaves over it was 1.3 % (B2 H2, 9 851 queries, 2 554 keys took two CTAs per tile, 80 clusters in
+    // 74 slots, 208 us; four take 173).  Of 500 further shapes 36 are cut differently, 1.10 times as fast on average, one of
+    // them 2 % slower.  The sum is taken in another order and the choice depends on batch x heads, so sequences of training
+    // length do without: a batch cut into calls gives the bits of the single call.
     int n_splits = 1;
     if (Tq >= 2 * (long long)Tk) {
         const double n_q = (Tq + TILE - 1) / TILE;

@@ -10,6 +10,8 @@
 // maximum is raised once per batch of rows.  The partial (m, l, O) of the warps are merged in shared memory, those of the
 // CTAs of a slice (a cluster) through distributed shared memory.
 //   B16 H12, one query, 2 047 keys (201 MB, 31 us at the copy bandwidth): 33 us, 55 with the tensor-core kernel.
+#include <algorithm>
+
 #include "attn_kernels.cuh"
 
 namespace hk {
@@ -169,17 +171,24 @@ __global__ void __launch_bounds__(WARPS * 32, (NQ == 1 ? 24 : 16) / WARPS) attn_
 // Warps of a CTA and CTAs of a slice (a cluster of up to eight, the portable size): as many warps per slice as can all be
 // resident at once, each with at least one batch of rows.  A second wave finds a chip that the first is leaving a CTA at a
 // time.  B4 H8, 8 191 keys: 25.0 us with 14 warps per SM, 37.7 with 28 wanted and 24 that fit; B16 H12, 2 047 keys: 33.0 with 21, 37.1
-// with 42, 36.6 with 10; B64 H16, 511 keys: 45.3 one CTA per slice, 48 - 63 with more.  Of equal numbers eight warps come
-// first, then larger CTAs in smaller clusters.  Slices that do not fit at all take one CTA each.
-DecodePlan plan_attn_decode(int BH, int Tq, int Tk, int sms) {
-    static const DecodePlan order[] = {{8, 4}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}};
+// with 42, 36.6 with 10; B64 H16, 511 keys: 45.3 one CTA per slice, 48 - 63 with more.  Slices that do not fit at all take
+// one CTA each.
+// Of equal numbers the order decides.  One CTA of sixteen warps is faster than two of eight (120 slices of 2 056 keys 22.1 and
+// 24.8 us); two of sixteen than four of eight only where these no longer get an SM each (68 slices 15.5 and 16.2; 4 slices of
+// 359 keys 4.9 and 4.3; two query rows: 64 slices 15.9 and 15.6).
+// What fits is known from the clusters of one CTA per SM that the device holds.  Clusters of eight pack better two and three
+// to an SM: 48 slices run at once (12.7 us), 52 do not (19.0), with 15 clusters of one CTA per SM.
+DecodePlan plan_attn_decode(int BH, int Tq, int Tk, const int slots[4]) {
+    static const DecodePlan order[2][9] = {{{8, 4}, {16, 1}, {16, 2}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}},
+                                           {{16, 2}, {16, 1}, {8, 4}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}}};
     DecodePlan best{Tq == 1 ? 8 : 4, 1};
     int most = 0;
-    for (const DecodePlan& p : order) {
-        const double filled = p.n_splits == 8 ? 0.85 : p.n_splits == 4 ? 0.92 : 1.0;  // clusters do not pack every SM
-        const double ctas = sms * filled * ((Tq == 1 ? 24 : 16) / p.warps);           // resident, by the kernels' launch bounds
+    for (const DecodePlan& p : order[Tq == 1 && 2 * BH > 3 * slots[2]]) {
+        const int per_sm = (Tq == 1 ? 24 : 16) / p.warps;  // by the kernels' launch bounds
+        int fit = per_sm * slots[p.n_splits == 8 ? 3 : p.n_splits == 4 ? 2 : p.n_splits == 2 ? 1 : 0];
+        if (p.n_splits == 8 && per_sm > 1) fit = std::max(fit, (int)(0.87 * slots[0] * per_sm / 8));
         const int n = p.warps * p.n_splits;
-        if ((double)BH * p.n_splits <= ctas && (long long)n * 2 * dec::UNROLL <= Tk && n > most) {
+        if (BH <= fit && (long long)n * 2 * dec::UNROLL <= Tk && n > most) {
             most = n;
             best = p;
         }
@@ -191,7 +200,10 @@ int launch_attn_decode(DecodeArgs a, cudaStream_t stream) {
     typedef void (*Kernel)(DecodeArgs);
     static const Kernel kernels[2][3] = {{attn_decode_kernel<1, 4>, attn_decode_kernel<1, 8>, attn_decode_kernel<1, 16>},
                                          {attn_decode_kernel<2, 4>, attn_decode_kernel<2, 8>, attn_decode_kernel<2, 16>}};
-    const DecodePlan plan = plan_attn_decode(a.BH, a.Tq, a.Tk, sm_count());
+    const int* slots = nullptr;
+    const int slots_rc = attn_fwd_slots(&slots);
+    if (slots_rc != HK_OK) return slots_rc;
+    const DecodePlan plan = plan_attn_decode(a.BH, a.Tq, a.Tk, slots);
     const int warps = plan.warps;
     const Kernel k = kernels[a.Tq - 1][warps == 4 ? 0 : warps == 8 ? 1 : 2];
     a.n_splits = plan.n_splits;

@@ -59,7 +59,7 @@ struct DecodeArgs {
 struct DecodePlan {
     int warps, n_splits;
 };
-DecodePlan plan_attn_decode(int BH, int Tq, int Tk, int sms);
+DecodePlan plan_attn_decode(int BH, int Tq, int Tk, const int slots[4]);  // slots: as attn_fwd_slots gives them
 int launch_attn_decode(DecodeArgs a, cudaStream_t stream);
 
 struct BwdArgs {

@@ -493,12 +493,12 @@ int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* pla
     const int64_t Tk = p->kv_len > 0 ? p->kv_len : p->T;
     int mode = 0, rc = validate_dropout(p->dropout_p, p->dropout_mask, p->flags, p->k_pos0, &mode);
     if (rc != HK_OK) return rc;
+    if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
     if (decodes(p->T, Tk, mode, p->flags)) {
-        const DecodePlan d = plan_attn_decode(p->B * p->nh, (int)p->T, (int)Tk, slots ? slots[0] : sm_count());
+        const DecodePlan d = plan_attn_decode(p->B * p->nh, (int)p->T, (int)Tk, slots);
         plan[0] = -1; plan[1] = d.n_splits; plan[2] = d.warps;
         return HK_OK;
     }
-    if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
     const FwdPlan f = plan_attn_fwd(p->B * p->nh, (int)p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode != 0, slots);
     plan[0] = f.mode; plan[1] = f.n_splits; plan[2] = 12;
     return HK_OK;
