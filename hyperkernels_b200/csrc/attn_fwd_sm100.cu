@@ -219,6 +219,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         // The score barriers belong to the score BUFFER, not to the stream: the warps of a stream may be a whole step
         // apart (the scores of the next step are there before the slowest warp has finished this one), and a
         // buffer is only refilled after every warp has handed over the P it held.
+        // A wait by parity needs to know that the phase before it is complete: whoever waits for s_full of product q, that
+        // S(q - 3) is.  A stream with a product among the last three has seen it.  One that sat out the item before (the last
+        // block of a slice may be of one row tile, without stream 1) has not: with two key tiles its next product is number
+        // three, and on the fresh barrier of buffer 0 the wait would pass before S(0).  An item is therefore made known
+        // only when every score of such a one before it is complete (q_empty[0], in the producer).
         for (int bf = 0; bf < 3; ++bf) {
             mbar_init(&sh.s_full[bf], 1);
             mbar_init(&sh.p_full[bf], 4);  // one arrival per softmax warp of the stream
@@ -312,6 +317,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     const int buf = r % ITEMS;
                     if (r >= ITEMS && !(tok = mbar_wait(wc, &sh.item_empty[buf], (r / ITEMS - 1) & 1, W_ITEM, 1000 + r))) break;
                     if (id >= 0) {
+                        // The next item is made known behind the last score of stream 0 in this one: see s_full.  Q and K of the
+                        // next item wait for it anyway.
+                        if (q0_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[0], (q0_uses - 1) & 1, W_QEMPTY, r))) break;
                         x = make_item(a, id, 0, 1);
                         sh.item[buf] = x;
                     } else {
@@ -320,7 +328,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     mbar_arrive(&sh.item_full[buf]);
                     if (id < 0) break;
                     if (x.n0 > 0) {
-                        if (q0_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[0], (q0_uses - 1) & 1, W_QEMPTY, r))) break;
                         load_q(x, 0);
                         ++q0_uses;
                     }

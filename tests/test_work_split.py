@@ -241,7 +241,9 @@ def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
 @pytest.mark.parametrize("kind", ["none", "philox", "dense inverted"])
 @pytest.mark.parametrize("BH,Tq,Tk,causal,pos", [
     (299, 128, 128, 0, {}), (160, 200, 200, 1, {}), (75, 600, 640, 1, {}), (40, 1000, 1100, 0, {}), (200, 100, 150, 0, {}), (40, 1300, 1800, 0, {}),
-    (60, 1100, 1100, 1, dict(k_pos0=512)), (200, 70, 100, 1, dict(k_pos0=128))])
+    (60, 1100, 1100, 1, dict(k_pos0=512)), (200, 70, 100, 1, dict(k_pos0=128)),
+    # two key tiles, an odd number of row tiles: blocks of one stream before blocks of two
+    (96, 379, 200, 0, {}), (96, 640, 256, 1, {}), (48, 1152, 256, 0, {}), (200, 379, 200, 0, {})])
 def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
     """More blocks of query rows than CTAs start with, of one to nine steps in one or two streams: first, middle and last slice
     against the oracle, every one against the same call on few enough slices that no CTA takes anything over (the same bits),
@@ -264,12 +266,12 @@ def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
         O_ref, L_ref = _oracle_forward(kind, None if mask is None else mask[s], q[:, s], k[:, s], v[:, s], causal, **pos)
         gate("O", host(O[:, s]), O_ref)
         lse_check(host(L[:, s]), L_ref)
-    if kind == "philox":
-        n = 128 // -(-Tq // 128)  # slices whose blocks all start at once
-        for s0 in range(0, BH, n):
-            s = slice(s0, min(BH, s0 + n))
-            one = hk.attention_forward(Q[:, s], K[:, s], V[:, s], SCALE, bool(causal), **pos, **dict(kw, bh_pos0=s0))
-            assert torch.equal(one[0], O[:, s]) and torch.equal(one[1], L[:, s])
+    n = 128 // -(-Tq // 128)  # slices whose blocks all start at once
+    for s0 in range(0, BH, n):
+        s = slice(s0, min(BH, s0 + n))
+        part = dict(kw, dropout_mask=kw["dropout_mask"][s]) if "dropout_mask" in kw else dict(kw, bh_pos0=s0) if kw else {}
+        one = hk.attention_forward(Q[:, s], K[:, s], V[:, s], SCALE, bool(causal), **pos, **part)
+        assert torch.equal(one[0], O[:, s]) and torch.equal(one[1], L[:, s])
     if kind == "none":
         # a block that sees no key of the second call keeps what the first one left
         O2, L2 = hk.attention_forward(Q, K, V, SCALE, False, q_pos0=0)
