@@ -954,7 +954,15 @@ int attn_bwd_slots(const int** slots) {
     return rc;
 }
 
-int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]) {
+BwdPlan plan_attn_bwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]) {
+    // KV tiles that a query tile sees.  (The grid has no others: the store warp could not read past a run of items without
+    // query tiles, since it hands over the last dQ of an item beside the first tile of the next.)
+    const int n_kvtiles = (Tk + TILE - 1) / TILE;
+    BwdPlan plan{1, n_kvtiles, ONE_ITEM};
+    if (causal) {
+        const long long last_q = (long long)(Tq + TILE - 1) / TILE * TILE - 1 + q_pos0 - k_pos0;  // in key positions
+        plan.live = (int)std::max(0ll, std::min((long long)n_kvtiles, last_q < 0 ? 0 : last_q / TILE + 1));
+    }
     // Splits by an estimate of the makespan: whole waves of CTAs that cost ~7 us and ~2.5 us per query tile, ~2.5 - 3 us more
     // where they add dV and dK up over a cluster.  They pay where few KV tiles have many query tiles (cross-attention of a
     // long sequence to a short one).  Over 110 such shapes the number is 0.2 % from the best one on average; with half a wave
@@ -962,41 +970,35 @@ int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]) {
     // 74 slots, 208 us; four take 173).  Of 500 further shapes 36 are cut differently, 1.10 times as fast on average, one of
     // them 2 % slower.  The sum is taken in another order and the choice depends on batch x heads, so sequences of training
     // length do without: a batch cut into calls gives the bits of the single call.
-    int n_splits = 1;
     if (Tq >= 2 * (long long)Tk) {
         const double n_q = (Tq + TILE - 1) / TILE;
         double best_cost = 0;
         for (int i = 0; i < 4; ++i) {
             const double one = 7.0 + (i ? 2.2 + 0.3 * i : 0.0) + 2.5 * std::ceil(n_q / (1 << i));
-            const double cost = one * std::ceil(tiles / (double)slots[i]);
+            const double cost = one * std::ceil((double)n_kvtiles * BH / slots[i]);
             if (i == 0 || cost < 0.95 * best_cost) {
                 best_cost = cost;
-                n_splits = 1 << i;
+                plan.n_splits = 1 << i;
             }
         }
     }
-    return n_splits;
+    plan.job = plan.n_splits > 1 ? SPLIT_ITEM : (long long)plan.live * BH > slots[0] ? TAKE_OVER : ONE_ITEM;
+    return plan;
 }
 
 int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream) {
     BwdDevice* d = nullptr;
     const int device_rc = bwd_device(&d);
     if (device_rc != HK_OK) return device_rc;
-    // KV tiles that a query tile sees.  (The grid has no others: the store warp could not read past a run of items without
-    // query tiles, since it hands over the last dQ of an item beside the first tile of the next.)
-    int live = a.n_kvtiles;
-    if (a.causal) {
-        const long long last_q = (long long)(a.Tq + TILE - 1) / TILE * TILE - 1 + a.q_pos0 - a.k_pos0;  // in key positions
-        live = (int)std::max(0ll, std::min((long long)live, last_q < 0 ? 0 : last_q / TILE + 1));
-    }
-    a.n_splits = plan_attn_bwd((long long)a.n_kvtiles * a.BH, a.Tq, a.Tk, d->slots);
+    const BwdPlan plan = plan_attn_bwd(a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, d->slots);
+    const int live = plan.live;
+    a.n_splits = plan.n_splits;
     const long long nblocks = (long long)live * a.BH * a.n_splits;
     if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
-    const int job = a.n_splits > 1 ? SPLIT_ITEM : nblocks > d->slots[0] ? TAKE_OVER : ONE_ITEM;
     if (nblocks > 0) {
         timing_mark(TIMED_BWD, true, stream);
         LaunchConfig lc((unsigned)nblocks, bwd::NUM_THREADS, bwd::SMEM_BYTES, stream, a.n_splits, after_prepass);
-        const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + 3 * job], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
+        const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, bwd_kernels[a.dropout_mode + 3 * plan.job], m.q, m.k, m.v, m.dO, m.q_mn, m.k_mn,
                                                   m.dO_mn, m.dQ, m.dK, m.dV, a);
         timing_mark(TIMED_BWD, false, stream);
         count_launch();

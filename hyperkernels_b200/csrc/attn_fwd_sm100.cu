@@ -905,6 +905,14 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     // the small shapes that reach each mode.
     const bool refine = !may_split || Tk > 8 * TILE;
     const int n_kvtiles = (Tk + TILE - 1) / TILE;
+    // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
+    // then more than the bookkeeping costs per step (about 2 %).  Steps per item on average, one item per CTA -> taken over:
+    // 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same without a mask)
+    // 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
+    // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
+    // storing warp counts on a product in every item.
+    const bool sees_keys = !causal || q_pos0 >= k_pos0;
+    auto taken_over = [&](int nb, double mean_steps) { return (long long)nb * BH > slots[0] && mean_steps <= 12.0 && sees_keys; };
     FwdPlan plan{}, fine_plan{};
     double coarse_cost = 0, cost_of_plan = 0, fine_cost = 0;  // cost_of_plan: of the coarse one's cut, by the fine one
     for (int mode = FWD_ROWS; mode <= (may_split ? FWD_KEYS : FWD_ROW); ++mode) {
@@ -927,7 +935,7 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
         const bool single = mode == FWD_ROWS && (Tq + TILE - 1) / TILE % 2 == 1;
         for (int i = 0; i < (may_split ? 4 : 1); ++i) {
             const int ns = 1 << i;
-            const FwdPlan cut = {mode, ns, nb, sum / nb};
+            const FwdPlan cut = {mode, ns, nb, mode == FWD_KEYS || ns > 1 ? COMBINE_ITEM : taken_over(nb, sum / nb) ? TAKE_OVER : ONE_ITEM};
             double fine = 1e30;
             if (refine && (mode != FWD_KEYS || n_kvtiles >= 2 * ns)) {
                 // A CTA, adding up a cluster, a step (with dropout), how much longer a step is on a full device; a key tile's
@@ -978,19 +986,9 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.n_qblocks = plan.n_qblocks;
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
-    // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
-    // then more than the bookkeeping costs per step (about 2 %).  Steps per item on average, one item per CTA -> taken over:
-    // 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same without a mask)
-    // 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
-    // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
-    // storing warp counts on a product in every item.
-    const bool sees_keys = !a.causal || a.q_pos0 >= a.k_pos0;
-    const int job = plan.mode == FWD_KEYS || plan.n_splits > 1                        ? COMBINE_ITEM
-                    : nblocks > d->slots[0] && plan.mean_steps <= 12.0 && sees_keys ? TAKE_OVER
-                                                                                     : ONE_ITEM;
     timing_mark(TIMED_FWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * job], mq, mk, mv, mo, a);
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * plan.job], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();

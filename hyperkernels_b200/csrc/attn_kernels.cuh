@@ -33,7 +33,7 @@ struct FwdArgs {
 // How a forward's work is cut, from sizes and the resident clusters of 1, 2, 4, 8 CTAs (slots) alone.
 struct FwdPlan {
     int mode, n_splits, n_qblocks;
-    double mean_steps;  // of a block of query rows, before splits
+    int job;  // FwdJob (attn_fwd_sm100.cu): the kernel that runs it
 };
 FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, bool drop, const int slots[4]);
 int attn_fwd_slots(const int** slots);  // of the current device; status
@@ -73,7 +73,6 @@ struct BwdArgs {
     int64_t dq_sB, dq_sM, dq_sH, dk_sB, dk_sM, dk_sH, dv_sB, dv_sM, dv_sH;
     int H, BH;
     int Tq, Tk;
-    int n_kvtiles;
     int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; set by launch_attn_bwd
     int q_pos0, k_pos0;
     float scale, scale_log2e;
@@ -100,8 +99,13 @@ struct BwdMaps {
     CUtensorMap q, k, v, dO, q_mn, k_mn, dO_mn, dQ, dK, dV;
 };
 
-// CTAs that share the query tiles of each of `tiles` KV tiles
-int plan_attn_bwd(long long tiles, int Tq, int Tk, const int slots[4]);
+// How a backward's work is cut, from the same.
+struct BwdPlan {
+    int n_splits;  // CTAs that share the query tiles of a KV tile
+    int live;      // KV tiles that a query tile sees: the others are not in the grid
+    int job;       // BwdJob (attn_bwd_sm100.cu): the kernel that runs it
+};
+BwdPlan plan_attn_bwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]);
 int attn_bwd_slots(const int** slots);
 
 // after_prepass: the launch before it in the stream is this call's D pre-pass, the only kernel whose results it waits for
@@ -117,7 +121,8 @@ extern "C" int hk_attn_forward_noscratch(const hk_attn_fwd_params* p, void* stre
 extern "C" int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* stream);
 // How the call of this block would be cut, for tests: nothing is launched and no pointer is read.  slots: resident clusters
 // of 1, 2, 4, 8 CTAs, or null for those of the current device.  Forward: plan = {FwdMode, or -1 for the decode kernel; CTAs
-// that share a block of rows (decode: a slice); warps of a CTA}.  Backward: plan = {CTAs that share a KV tile}.
+// that share a block of rows (decode: a slice); FwdJob (decode: warps of a CTA)}.  Backward: plan = {CTAs that share a KV tile;
+// BwdJob}.
 extern "C" int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* plan);
 extern "C" int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slots, int* plan);
 // zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ

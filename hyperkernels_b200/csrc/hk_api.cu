@@ -339,7 +339,6 @@ int attn_backward(const hk_attn_bwd_params& pr, cudaStream_t stream, bool check_
     a.dk_sB = p->dk_strideB; a.dk_sM = p->dk_strideM; a.dk_sH = p->dk_strideH;
     a.dv_sB = p->dv_strideB; a.dv_sM = p->dv_strideM; a.dv_sH = p->dv_strideH;
     a.H = H; a.BH = BH; a.Tq = (int)Tq; a.Tk = (int)Tk;
-    a.n_kvtiles = n_kvtiles;
     a.det_dq = det_dq ? 1 : 0;
     a.B = B;
     a.q_pos0 = (int)p->q_pos0; a.k_pos0 = (int)p->k_pos0;
@@ -500,7 +499,7 @@ int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* pla
         return HK_OK;
     }
     const FwdPlan f = plan_attn_fwd(p->B * p->nh, (int)p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode != 0, slots);
-    plan[0] = f.mode; plan[1] = f.n_splits; plan[2] = 12;
+    plan[0] = f.mode; plan[1] = f.n_splits; plan[2] = f.job;
     return HK_OK;
 }
 
@@ -508,7 +507,8 @@ int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slots, int* pl
     const int64_t Tk = p->kv_len > 0 ? p->kv_len : p->T;
     int rc = HK_OK;
     if (!slots && (rc = attn_bwd_slots(&slots))) return rc;
-    plan[0] = plan_attn_bwd((Tk + TILE - 1) / TILE * p->B * p->nh, p->T, (int)Tk, slots);
+    const BwdPlan b = plan_attn_bwd(p->B * p->nh, p->T, (int)Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, slots);
+    plan[0] = b.n_splits; plan[1] = b.job;
     return HK_OK;
 }
 

@@ -12,25 +12,39 @@ import oracle_lib as ol
 
 SCALE = 0.125
 ROWS, ROW, KEYS, DECODE = 0, 1, 2, -1
+ONE_ITEM, TAKE_OVER, TOGETHER = 0, 1, 2  # a CTA's items: one, then others that have not started, one that a cluster or two streams share
 B200 = (C.c_int * 4)(148, 74, 33, 15)  # resident clusters of 1, 2, 4, 8 CTAs, one CTA per SM
 
 
 def forward_plan(BH, Tq, Tk, causal=False, q_pos0=0, k_pos0=0, flags=0, dropout_p=0.0, slots=None):
     """(mode, CTAs per block of rows or decoded slice); slots=None: those of the current device"""
+    return _forward_plan(BH, Tq, Tk, causal, q_pos0, k_pos0, flags, dropout_p, slots)[:2]
+
+
+def forward_job(BH, Tq, Tk, causal=False, q_pos0=0, k_pos0=0, slots=None):
+    return _forward_plan(BH, Tq, Tk, causal, q_pos0, k_pos0, 0, 0.0, slots)[2]
+
+
+def _forward_plan(BH, Tq, Tk, causal, q_pos0, k_pos0, flags, dropout_p, slots):
     p = hk.MemEfficientFwdParams()
     p.B, p.nh, p.T, p.kv_len, p.is_causal = 1, BH, Tq, Tk, bool(causal)
     p.q_pos0, p.k_pos0, p.flags, p.dropout_p = q_pos0, k_pos0, flags, dropout_p
     out = (C.c_int * 3)()
     assert hk.lib().hk_attn_forward_plan(C.byref(p), slots, out) == 0
-    return out[0], out[1]
+    return tuple(out)
+
+
+def backward_plan(BH, Tq, Tk, causal=False, q_pos0=0, k_pos0=0, slots=None):
+    """(CTAs per KV tile, job)"""
+    p = hk.MemEfficientBwdParams()
+    p.B, p.nh, p.T, p.kv_len, p.is_causal, p.q_pos0, p.k_pos0 = 1, BH, Tq, Tk, bool(causal), q_pos0, k_pos0
+    out = (C.c_int * 2)()
+    assert hk.lib().hk_attn_backward_plan(C.byref(p), slots, out) == 0
+    return tuple(out)
 
 
 def backward_splits(BH, Tq, Tk, slots=None):
-    p = hk.MemEfficientBwdParams()
-    p.B, p.nh, p.T, p.kv_len = 1, BH, Tq, Tk
-    out = (C.c_int * 1)()
-    assert hk.lib().hk_attn_backward_plan(C.byref(p), slots, out) == 0
-    return out[0]
+    return backward_plan(BH, Tq, Tk, slots=slots)[0]
 
 
 # ---- the choice -----------------------------------------------------------------------------------------------------
@@ -65,6 +79,25 @@ def test_decode_kernel_for_one_or_two_rows():
     assert plan(1, 128) == plan(2, 128) == plan(1, 5000, causal=True) == DECODE
     assert DECODE not in (plan(3, 128), plan(1, 127), plan(1, 500, flags=hk.FLAG_CONTINUE_SOFTMAX_STATE),
                           plan(1, 500, flags=hk.FLAG_PHILOX_DROPOUT, dropout_p=0.1))
+
+
+@pytest.mark.parametrize("job,BH,Tq,Tk,causal,pos", [
+    (ONE_ITEM, 148, 128, 128, 0, {}), (TAKE_OVER, 149, 128, 128, 0, {}),  # one CTA more than the device holds
+    (TAKE_OVER, 96, 1024, 1536, 0, {}), (ONE_ITEM, 96, 1024, 1537, 0, {}),  # twelve and thirteen steps
+    (TAKE_OVER, 96, 2816, 2816, 1, {}), (ONE_ITEM, 96, 2817, 2817, 1, {}),  # 12 and 12.9 on average under the mask
+    (TAKE_OVER, 60, 1100, 1100, 1, dict(q_pos0=512, k_pos0=512)), (ONE_ITEM, 60, 1100, 1100, 1, dict(q_pos0=511, k_pos0=512)),
+    (TAKE_OVER, 60, 1100, 1100, 0, dict(k_pos0=512)), (TOGETHER, 16, 257, 1000, 0, {}), (TOGETHER, 24, 257, 1000, 1, dict(q_pos0=743))])
+def test_row_blocks_that_are_taken_over(job, BH, Tq, Tk, causal, pos):
+    """Short ones of a grid larger than the device, each with a key: either side of each line."""
+    assert forward_job(BH, Tq, Tk, causal, slots=B200, **pos) == job
+
+
+@pytest.mark.parametrize("plan,BH,Tq,Tk,causal,pos", [
+    ((1, ONE_ITEM), 148, 128, 128, 0, {}), ((1, TAKE_OVER), 149, 128, 128, 0, {}), ((2, TOGETHER), 24, 777, 333, 0, {}),
+    ((1, ONE_ITEM), 74, 256, 1000, 1, {}), ((1, TAKE_OVER), 75, 256, 1000, 1, {}), ((1, ONE_ITEM), 75, 256, 1000, 1, dict(k_pos0=128))])
+def test_key_tiles_that_are_taken_over(plan, BH, Tq, Tk, causal, pos):
+    """A grid larger than the device; KV tiles that no query sees are not in it."""
+    assert backward_plan(BH, Tq, Tk, causal, slots=B200, **pos) == plan
 
 
 # ---- every cut, with every mask -------------------------------------------------------------------------------------
@@ -240,21 +273,22 @@ def test_every_backward_cut_with_every_mask(splits, BH, Tq, Tk, causal, kind):
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["none", "philox", "dense inverted"])
 @pytest.mark.parametrize("BH,Tq,Tk,causal,pos", [
-    (299, 128, 128, 0, {}), (160, 200, 200, 1, {}), (75, 600, 640, 1, {}), (40, 1000, 1100, 0, {}), (200, 100, 150, 0, {}), (40, 1300, 1800, 0, {}),
-    (60, 1100, 1100, 1, dict(k_pos0=512)), (200, 70, 100, 1, dict(k_pos0=128)),
+    (299, 128, 128, 0, {}), (160, 200, 200, 1, {}), (75, 600, 640, 1, {}), (40, 1000, 1100, 0, {}), (200, 100, 150, 0, {}), (40, 1300, 1500, 0, {}),
+    (40, 1300, 1800, 0, {}), (60, 1100, 1100, 1, dict(k_pos0=512)), (200, 70, 100, 1, dict(k_pos0=128)),
     # two key tiles, an odd number of row tiles: blocks of one stream before blocks of two
     (96, 379, 200, 0, {}), (96, 640, 256, 1, {}), (48, 1152, 256, 0, {}), (200, 379, 200, 0, {})])
 def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
-    """More blocks of query rows than CTAs start with, of one to nine steps in one or two streams: first, middle and last slice
+    """More blocks of query rows than CTAs start with, of one to twelve steps in one or two streams: first, middle and last slice
     against the oracle, every one against the same call on few enough slices that no CTA takes anything over (the same bits),
-    and as a continued state.  Beside them the calls that take none over for another reason: long items, and blocks that see
-    no key (k_pos0 behind their rows; all of them in the last case)."""
+    and as a continued state.  Beside them the calls that take none over for another reason: long items (1 800 keys), and blocks
+    that see no key (k_pos0 behind their rows; all of them at 70 queries)."""
     from test_attention_gpu import gate, host, lse_check, ok_status
 
     q, k, v = _normal((1, BH, Tq, 64), 990), _normal((1, BH, Tk, 64), 991), _normal((1, BH, Tk, 64), 992)
     Q, K, V = map(_dev, (q, k, v))
     mode, splits = forward_plan(BH, Tq, Tk, causal, 0, pos.get("k_pos0", 0))
     assert splits == 1 and BH * -(-Tq // (256 if mode == ROWS else 128)) > 148
+    assert forward_job(BH, Tq, Tk, causal, **pos) == (ONE_ITEM if Tk == 1800 or pos else TAKE_OVER)
     mask = None if kind == "none" else ol.dropout_mask(BH, Tq, Tk, P, SEED, OFFSET, **pos)
     kw = {} if kind == "none" else dict(_mask(kind, 1, 8, 8)[0])
     if "dropout_mask" in kw:
@@ -267,6 +301,7 @@ def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
         gate("O", host(O[:, s]), O_ref)
         lse_check(host(L[:, s]), L_ref)
     n = 128 // -(-Tq // 128)  # slices whose blocks all start at once
+    assert forward_job(n, Tq, Tk, causal, **pos) == ONE_ITEM
     for s0 in range(0, BH, n):
         s = slice(s0, min(BH, s0 + n))
         part = dict(kw, dropout_mask=kw["dropout_mask"][s]) if "dropout_mask" in kw else dict(kw, bh_pos0=s0) if kw else {}
@@ -289,7 +324,8 @@ def test_forward_ctas_take_over_row_blocks(BH, Tq, Tk, causal, pos, kind):
 @pytest.mark.parametrize("kind", ["none", "philox", "philox inverted"])
 @pytest.mark.parametrize("BH,Tq,Tk,causal", [(299, 128, 128, 0), (60, 640, 640, 1), (75, 100, 300, 0), (90, 257, 384, 1), (60, 130, 1000, 1), (5, 70, 200, 1)])
 def test_backward_ctas_take_over_key_tiles(BH, Tq, Tk, causal, kind):
-    """More KV tiles than CTAs start with, one to five query tiles each: the CTAs that are through take over the others.  First,
+    """More KV tiles than CTAs start with, one to five query tiles each: the CTAs that are through take over the others (not
+    where the keys that a query sees make 120 tiles, or none).  First,
     middle and last slice against the oracle, all of them against the same call on 20 slices at a time (every CTA starts with
     its own tile: the same bits), and results added to what the buffers hold.  KV tiles that no query sees (Tk > Tq under the
     mask; all of them where the keys lie behind the queries) leave zeros."""
@@ -300,6 +336,8 @@ def test_backward_ctas_take_over_key_tiles(BH, Tq, Tk, causal, kind):
     kw, _ = _mask(kind, 1, 8, 8)
     Q, K, V, G = map(_dev, (q, k, v, g))
     for pos in (dict(), dict(k_pos0=1000)) if causal else (dict(),):
+        assert backward_plan(BH, Tq, Tk, causal, **pos)[1] == (ONE_ITEM if pos or Tk in (200, 1000) else TAKE_OVER)
+        assert backward_plan(20, Tq, Tk, causal, **pos)[1] == ONE_ITEM
         O, L = hk.attention_forward(Q, K, V, SCALE, bool(causal), **pos, **kw)
         call = lambda s, **more: hk.attention_backward(Q[:, s], K[:, s], V[:, s], O[:, s], G[:, s], L[:, s], SCALE, bool(causal), **pos,  # noqa: E731
                                                        **(dict(kw, bh_pos0=s.start) if kw else {}), **more)[:3]
