@@ -42,9 +42,10 @@
 // four 32-column boxes of dS(i) go over the MN-major dO tile as soon as dV(i) has
 // consumed it, so that tile can be loaded for i+1 only when dQ(i) is done, and
 // dV(i+1) waits for it: with dQ(i) in front of dP^T(i+1) half of that load is
-// hidden (B4 H16 T2048 433 -> 388 us, H32 T8192 1 670 -> 1 500, against dQ last).  Measured tensor-pipe time of the 72 instructions of a tile:
-// about 3 050 cycles (M128 N128 K8: 74 cycles, M128 N64 K8: 36 from tensor
-// memory, 52 from shared memory).
+// hidden (B4 H16 T2048 433 -> 388 us, H32 T8192 1 670 -> 1 500, against dQ last).
+// Measured tensor-pipe time of the 72 instructions of a tile: about 3 050 cycles
+// (M128 N128 K8: 74 cycles, M128 N64 K8: 36 from tensor memory, 52 from shared
+// memory).
 //
 // Splits: where few KV tiles have many query tiles (cross-attention of a long sequence to a short one), a cluster of 2, 4
 // or 8 CTAs shares the query tiles of a KV tile; at the end each adds up a slice of the rows of dV and dK from the partial
@@ -625,210 +626,210 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         int g = 0, item = 0;  // query tiles, items done with
         Items s{first, 0};
         for (;;) {
-        const int kv0 = s.x.kv0(), bh = s.x.bh, it0 = s.x.it0, n_it = s.x.n_it;
-        const int kvrow = kv0 + row;
-        const bool kv_ok = kvrow < a.Tk;
-        if (SPLIT && n_it == 0) pdl_wait();  // the rows written at the end; with query tiles the barriers order everything
-        for (int it = 0; it < n_it; ++it, ++g) {
-            const int q0 = (it0 + it) * TILE;
-            // V lands before the first S^T of the CTA is complete; that of later items while their first P^T is computed
-            if (g == 0 && part >= 2 && !(ok = copy_v(0, rp))) break;
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, g & 1, W_SFULL, g));
-            if (!ok) break;
-            tc_fence_after_sync();
+            const int kv0 = s.x.kv0(), bh = s.x.bh, it0 = s.x.it0, n_it = s.x.n_it;
+            const int kvrow = kv0 + row;
+            const bool kv_ok = kvrow < a.Tk;
+            if (SPLIT && n_it == 0) pdl_wait();  // the rows written at the end; with query tiles the barriers order everything
+            for (int it = 0; it < n_it; ++it, ++g) {
+                const int q0 = (it0 + it) * TILE;
+                // V lands before the first S^T of the CTA is complete; that of later items while their first P^T is computed
+                if (g == 0 && part >= 2 && !(ok = copy_v(0, rp))) break;
+                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full, g & 1, W_SFULL, g));
+                if (!ok) break;
+                tc_fence_after_sync();
 
-            tmem_ld32(trow + COL_S + c0, rs);
+                tmem_ld32(trow + COL_S + c0, rs);
 
-            // first query column (local to the tile) this key row is visible to
-            int cmin = 0;
-            if (a.causal) {
-                const long long c = (long long)a.k_pos0 + kvrow - a.q_pos0 - q0;
-                cmin = (int)max(0ll, min((long long)TILE, c));
-            }
-            if (!kv_ok) cmin = TILE;
-
-            // dropout keep bits of this thread's 32 (query, key) pairs
-            uint32_t keep = 0xffffffffu;
-            if constexpr (DROP == 2) {
-                // One Philox call covers the eight keys kpos & ~7 .. of one query row, i.e. the key rows of eight
-                // adjacent lanes (k_pos0 and kv0 are multiples of 8, so row & 7 == lane & 7).  Lane j of such a
-                // group evaluates the query columns 8m + j (m = 0..3) and keeps 8 bits per call; the group then
-                // swaps them with shuffles, so every lane does 4 calls for its 32 columns instead of 32.
-                const int j8 = lane & 7;
-                const uint32_t kgrp = (uint32_t)(a.k_pos0 + kvrow) >> 3;
-                uint32_t mine = 0u;  // bit 8m + u: query column c0 + 8m + j8, key row (row & ~7) + u
-#pragma unroll
-                for (int mI = 0; mI < 4; ++mI) {
-                    const hk_philox4_t w = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
-                                                          (uint32_t)(a.q_pos0 + q0 + c0 + 8 * mI + j8), kgrp);
-                    mine |= hk_philox_keep8(w, a.drop_thr) << (8 * mI);
+                // first query column (local to the tile) this key row is visible to
+                int cmin = 0;
+                if (a.causal) {
+                    const long long c = (long long)a.k_pos0 + kvrow - a.q_pos0 - q0;
+                    cmin = (int)max(0ll, min((long long)TILE, c));
                 }
-                keep = 0u;
+                if (!kv_ok) cmin = TILE;
+
+                // dropout keep bits of this thread's 32 (query, key) pairs
+                uint32_t keep = 0xffffffffu;
+                if constexpr (DROP == 2) {
+                    // One Philox call covers the eight keys kpos & ~7 .. of one query row, i.e. the key rows of eight
+                    // adjacent lanes (k_pos0 and kv0 are multiples of 8, so row & 7 == lane & 7).  Lane j of such a
+                    // group evaluates the query columns 8m + j (m = 0..3) and keeps 8 bits per call; the group then
+                    // swaps them with shuffles, so every lane does 4 calls for its 32 columns instead of 32.
+                    const int j8 = lane & 7;
+                    const uint32_t kgrp = (uint32_t)(a.k_pos0 + kvrow) >> 3;
+                    uint32_t mine = 0u;  // bit 8m + u: query column c0 + 8m + j8, key row (row & ~7) + u
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t other = __shfl_sync(0xffffffffu, mine, (lane & ~7) | j);  // lane j's columns 8m + j
-                    keep |= ((other >> j8) & 0x01010101u) << j;                              // its bit for MY key row
-                }
-            } else if constexpr (DROP == 1) {
-                keep = 0u;
-                if (kv_ok) {
+                    for (int mI = 0; mI < 4; ++mI) {
+                        const hk_philox4_t w = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
+                                                              (uint32_t)(a.q_pos0 + q0 + c0 + 8 * mI + j8), kgrp);
+                        mine |= hk_philox_keep8(w, a.drop_thr) << (8 * mI);
+                    }
+                    keep = 0u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t other = __shfl_sync(0xffffffffu, mine, (lane & ~7) | j);  // lane j's columns 8m + j
+                        keep |= ((other >> j8) & 0x01010101u) << j;                              // its bit for MY key row
+                    }
+                } else if constexpr (DROP == 1) {
+                    keep = 0u;
+                    if (kv_ok) {
 #pragma unroll 4
-                    for (int i = 0; i < 32; ++i) {
-                        const int q = q0 + c0 + i;
-                        if (q < a.Tq && __ldg(a.mask + ((size_t)bh * a.Tq + q) * (size_t)a.Tk + kvrow) != 0.f)
-                            keep |= 1u << i;
+                        for (int i = 0; i < 32; ++i) {
+                            const int q = q0 + c0 + i;
+                            if (q < a.Tq && __ldg(a.mask + ((size_t)bh * a.Tq + q) * (size_t)a.Tk + kvrow) != 0.f)
+                                keep |= 1u << i;
+                        }
                     }
                 }
-            }
-            // fold the causal / tail mask into the keep bits: column cc is visible iff cc >= cmin
-            uint32_t vis = 0xffffffffu;
-            {
-                const int lo = cmin - c0;  // first visible local index, may be <= 0 or >= 32
-                if (lo > 0) vis = (lo >= 32) ? 0u : (0xffffffffu << lo);
-                keep &= vis;
-            }
-            // pairs whose p is zero: hidden ones, and dropped ones unless the dropout is the inverted kind
-            const uint32_t live = DROP != 0 && a.drop_scaled ? vis : keep;
-            tmem_wait_ld();
+                // fold the causal / tail mask into the keep bits: column cc is visible iff cc >= cmin
+                uint32_t vis = 0xffffffffu;
+                {
+                    const int lo = cmin - c0;  // first visible local index, may be <= 0 or >= 32
+                    if (lo > 0) vis = (lo >= 32) ? 0u : (0xffffffffu << lo);
+                    keep &= vis;
+                }
+                // pairs whose p is zero: hidden ones, and dropped ones unless the dropout is the inverted kind
+                const uint32_t live = DROP != 0 && a.drop_scaled ? vis : keep;
+                tmem_wait_ld();
 
-            // p = exp2(s*scale*log2e - LSE*log2e) needs S^T only: dP^T is still being computed.  Two scores per
-            // packed FMA (fma.rn.f32x2 gives the same bits as two scalar FMAs).
-            {
-                const float4* lse4 = reinterpret_cast<const float4*>(sh.lse + c0);
-                const float2 c2 = make_float2(a.scale_log2e, a.scale_log2e);
+                // p = exp2(s*scale*log2e - LSE*log2e) needs S^T only: dP^T is still being computed.  Two scores per
+                // packed FMA (fma.rn.f32x2 gives the same bits as two scalar FMAs).
+                {
+                    const float4* lse4 = reinterpret_cast<const float4*>(sh.lse + c0);
+                    const float2 c2 = make_float2(a.scale_log2e, a.scale_log2e);
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const float4 L = lse4[g];
-                    const float2 x01 = __ffma2_rn(make_float2(__uint_as_float(rs[4 * g]), __uint_as_float(rs[4 * g + 1])), c2,
-                                                  make_float2(L.x, L.y));
-                    const float2 x23 = __ffma2_rn(make_float2(__uint_as_float(rs[4 * g + 2]), __uint_as_float(rs[4 * g + 3])), c2,
-                                                  make_float2(L.z, L.w));
-                    rs[4 * g] = __float_as_uint(ex2_approx(x01.x));
-                    rs[4 * g + 1] = __float_as_uint(ex2_approx(x01.y));
-                    rs[4 * g + 2] = __float_as_uint(ex2_approx(x23.x));
-                    rs[4 * g + 3] = __float_as_uint(ex2_approx(x23.y));
+                    for (int f = 0; f < 8; ++f) {
+                        const float4 L = lse4[f];
+                        const float2 x01 = __ffma2_rn(make_float2(__uint_as_float(rs[4 * f]), __uint_as_float(rs[4 * f + 1])), c2,
+                                                      make_float2(L.x, L.y));
+                        const float2 x23 = __ffma2_rn(make_float2(__uint_as_float(rs[4 * f + 2]), __uint_as_float(rs[4 * f + 3])), c2,
+                                                      make_float2(L.z, L.w));
+                        rs[4 * f] = __float_as_uint(ex2_approx(x01.x));
+                        rs[4 * f + 1] = __float_as_uint(ex2_approx(x01.y));
+                        rs[4 * f + 2] = __float_as_uint(ex2_approx(x23.x));
+                        rs[4 * f + 3] = __float_as_uint(ex2_approx(x23.y));
+                    }
+                    if (live != 0xffffffffu) {  // tiles on the diagonal, the ragged end, dropout
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (!((live >> i) & 1u)) rs[i] = 0u;
+                    }
                 }
-                if (live != 0xffffffffu) {  // tiles on the diagonal, the ragged end, dropout
+                // P^T goes to tensor memory at once (rounded; a pair dropped by inverted dropout counts as zero in dV but
+                // keeps its p for dS below): dV += P^T dO and, behind it, the next tile's S^T run while dS is computed,
+                // and the store has drained by the time its first reader starts.  rp is free until dP^T is loaded.
+                {
+                    const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (!((live >> i) & 1u)) rs[i] = 0u;
+                    for (int i = 0; i < 32; ++i) rp[i] = tf32_round_bits_mma(rs[i]);
+                    if (dropped_some) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (!((keep >> i) & 1u)) rp[i] = 0u;
+                    }
+                    tmem_st32(trow + COL_S + c0, rp);
+                    tmem_wait_st();
+                    tc_fence_before_sync();
+                    mbar_arrive_warp(&sh.pt_ready, lane);
                 }
-            }
-            // P^T goes to tensor memory at once (rounded; a pair dropped by inverted dropout counts as zero in dV but
-            // keeps its p for dS below): dV += P^T dO and, behind it, the next tile's S^T run while dS is computed,
-            // and the store has drained by the time its first reader starts.  rp is free until dP^T is loaded.
-            {
-                const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) rp[i] = tf32_round_bits_mma(rs[i]);
-                if (dropped_some) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (!((keep >> i) & 1u)) rp[i] = 0u;
+                if (g > 0) {  // rp is free until dP^T is loaded
+                    if (it == 0 && part >= 2 && !(ok = copy_v(item, rp))) break;
+                    if (!(ok = read_dq(g - 1, rp))) break;
                 }
-                tmem_st32(trow + COL_S + c0, rp);
+                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, g & 1, W_SFULL, 1000 + g));
+                if (!ok) break;
+                tc_fence_after_sync();
+                if (g > 0) stage_dq(rp);
+                tmem_ld32(trow + COL_DP + c0, rp);
+                tmem_wait_ld();
+
+                // dS = p * (dP*scale - D*scale), two elements per packed instruction
+                {
+                    const float4* ds4 = reinterpret_cast<const float4*>(sh.dsum + c0);
+                    const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
+                    if (dropped_some) {
+                        // inverted dropout: a dropped pair keeps the -D term of dS but contributes neither dP (zeroed
+                        // here) nor to dV (its P^T entry was stored as zero above)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (!((keep >> i) & 1u)) rp[i] = 0u;
+                    }
+                    const float2 dps2 = make_float2(a.dp_scale, a.dp_scale);
+#pragma unroll
+                    for (int f = 0; f < 8; ++f) {
+                        const float4 Dv = ds4[f];  // -D * scale
+#pragma unroll
+                        for (int h2 = 0; h2 < 2; ++h2) {
+                            const int i = 4 * f + 2 * h2;
+                            const float2 nd = h2 ? make_float2(Dv.z, Dv.w) : make_float2(Dv.x, Dv.y);
+                            const float2 t = __ffma2_rn(make_float2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), dps2, nd);
+                            const float2 ds = __fmul2_rn(make_float2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), t);
+                            rp[i] = tf32_round_bits_mma(__float_as_uint(ds.x));
+                            rp[i + 1] = tf32_round_bits_mma(__float_as_uint(ds.y));
+                        }
+                    }
+                }
+                tmem_st32(trow + COL_DP + c0, rp);
                 tmem_wait_st();
                 tc_fence_before_sync();
-                mbar_arrive_warp(&sh.pt_ready, lane);
-            }
-            if (g > 0) {  // rp is free until dP^T is loaded
-                if (it == 0 && part >= 2 && !(ok = copy_v(item, rp))) break;
-                if (!(ok = read_dq(g - 1, rp))) break;
-            }
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dp_full, g & 1, W_SFULL, 1000 + g));
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (g > 0) stage_dq(rp);
-            tmem_ld32(trow + COL_DP + c0, rp);
-            tmem_wait_ld();
+                mbar_arrive_warp(&sh.p_ready, lane);
 
-            // dS = p * (dP*scale - D*scale), two elements per packed instruction
-            {
-                const float4* ds4 = reinterpret_cast<const float4*>(sh.dsum + c0);
-                const bool dropped_some = DROP != 0 && a.drop_scaled && keep != 0xffffffffu;
-                if (dropped_some) {
-                    // inverted dropout: a dropped pair keeps the -D term of dS but contributes neither dP (zeroed
-                    // here) nor to dV (its P^T entry was stored as zero above)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (!((keep >> i) & 1u)) rp[i] = 0u;
+                // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns
+                // 32*part..32*part+31, one 128-byte row per key row, 32-byte chunks XOR-swizzled with (row & 3).  Boxes 0, 1
+                // have a buffer of their own, free once dQ of the previous tile is done -- and, at the first tile of an item, V
+                // has left it --: dP^T of this tile, complete here, was issued behind either.  Boxes 2, 3 go over the MN-major dO
+                // tile as soon as dV of this tile is done.
+                if (part >= 2) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, g & 1, W_DVDONE, g));
+                    if (!ok) break;
                 }
-                const float2 dps2 = make_float2(a.dp_scale, a.dp_scale);
+                {
+                    // Rows r and r + 4 share a 32-byte chunk position; they store its two halves in opposite order so
+                    // that the eight lanes of a quarter-warp hit eight different 16-byte bank groups.
+                    uint8_t* drow = sdS + part * BOX_BYTES + row * 128;
+                    const bool swap = (row >> 2) & 1;
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const float4 Dv = ds4[g];  // -D * scale
-#pragma unroll
-                    for (int h2 = 0; h2 < 2; ++h2) {
-                        const int i = 4 * g + 2 * h2;
-                        const float2 nd = h2 ? make_float2(Dv.z, Dv.w) : make_float2(Dv.x, Dv.y);
-                        const float2 t = __ffma2_rn(make_float2(__uint_as_float(rp[i]), __uint_as_float(rp[i + 1])), dps2, nd);
-                        const float2 ds = __fmul2_rn(make_float2(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), t);
-                        rp[i] = tf32_round_bits_mma(__float_as_uint(ds.x));
-                        rp[i + 1] = tf32_round_bits_mma(__float_as_uint(ds.y));
+                    for (int u = 0; u < 4; ++u) {
+                        const uint4 lo = make_uint4(rp[8 * u], rp[8 * u + 1], rp[8 * u + 2], rp[8 * u + 3]);
+                        const uint4 hi = make_uint4(rp[8 * u + 4], rp[8 * u + 5], rp[8 * u + 6], rp[8 * u + 7]);
+                        uint8_t* chunk = drow + ((u ^ (row & 3)) << 5);
+                        *reinterpret_cast<uint4*>(chunk + (swap ? 16 : 0)) = swap ? hi : lo;
+                        *reinterpret_cast<uint4*>(chunk + (swap ? 0 : 16)) = swap ? lo : hi;
                     }
                 }
+                fence_proxy_async_smem();
+                mbar_arrive_warp(&sh.ds_ready, lane);
             }
-            tmem_st32(trow + COL_DP + c0, rp);
-            tmem_wait_st();
-            tc_fence_before_sync();
-            mbar_arrive_warp(&sh.p_ready, lane);
 
-            // dS into shared memory, the MN-major A operand of dQ = dS K: box `part` holds query columns
-            // 32*part..32*part+31, one 128-byte row per key row, 32-byte chunks XOR-swizzled with (row & 3).  Boxes 0, 1
-            // have a buffer of their own, free once dQ of the previous tile is done -- and, at the first tile of an item, V
-            // has left it --: dP^T of this tile, complete here, was issued behind either.  Boxes 2, 3 go over the MN-major dO
-            // tile as soon as dV of this tile is done.
-            if (part >= 2) {
-                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.dv_done, g & 1, W_DVDONE, g));
-                if (!ok) break;
-            }
-            {
-                // Rows r and r + 4 share a 32-byte chunk position; they store its two halves in opposite order so
-                // that the eight lanes of a quarter-warp hit eight different 16-byte bank groups.
-                uint8_t* drow = sdS + part * BOX_BYTES + row * 128;
-                const bool swap = (row >> 2) & 1;
+            if (!ok) break;
+            Items nx = s;
+            const bool more = next_item(nx, false);
+            // The accumulators, as the boxes of a 128-byte-swizzled TMA tile (16-byte chunk c of row r at position c ^ (r & 7)):
+            // column groups 2, 3 put dK into the MN-major Q tile, dead with the last dK; groups 0, 1 put dV (times 1/(1-p) for
+            // inverted dropout) into the MN-major K tile, dead with the last dQ, or, if no item follows, at once into the
+            // K-major Q tile.  They are in registers when this warp hands over its next P^T, which the first dV of the next item
+            // waits for.
+            if (n_it > 0)
+                ok = __all_sync(0xffffffffu, mbar_wait(wc, (part >= 2) ? &sh.dk_done : more ? &sh.dq_full : &sh.dv_done, (g - 1) & 1, W_BDONE, g));
+            if (!ok) break;
+            if (n_it > 0) {
+                tc_fence_after_sync();
+                tmem_ld32(trow + ((part < 2) ? COL_DV + part * 32 : COL_DK + (part - 2) * 32), rs);
+                tmem_wait_ld();
+                tc_fence_before_sync();
+                const float f = (part < 2) ? a.dv_scale : 1.f;
+                uint8_t* srow = ((part >= 2) ? sQm : more ? sKm : sQ) + (part & 1) * BOX_BYTES + row * 128;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint4 lo = make_uint4(rp[8 * u], rp[8 * u + 1], rp[8 * u + 2], rp[8 * u + 3]);
-                    const uint4 hi = make_uint4(rp[8 * u + 4], rp[8 * u + 5], rp[8 * u + 6], rp[8 * u + 7]);
-                    uint8_t* chunk = drow + ((u ^ (row & 3)) << 5);
-                    *reinterpret_cast<uint4*>(chunk + (swap ? 16 : 0)) = swap ? hi : lo;
-                    *reinterpret_cast<uint4*>(chunk + (swap ? 0 : 16)) = swap ? lo : hi;
-                }
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<float4*>(srow + ((c ^ (row & 7)) << 4)) =
+                        make_float4(__uint_as_float(rs[4 * c]) * f, __uint_as_float(rs[4 * c + 1]) * f,
+                                    __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
+                fence_proxy_async_smem();
+                mbar_arrive_warp((part < 2) ? &sh.dv_staged : &sh.dk_staged, lane);
             }
-            fence_proxy_async_smem();
-            mbar_arrive_warp(&sh.ds_ready, lane);
-        }
-
-        if (!ok) break;
-        Items nx = s;
-        const bool more = next_item(nx, false);
-        // The accumulators, as the boxes of a 128-byte-swizzled TMA tile (16-byte chunk c of row r at position c ^ (r & 7)):
-        // column groups 2, 3 put dK into the MN-major Q tile, dead with the last dK; groups 0, 1 put dV (times 1/(1-p) for
-        // inverted dropout) into the MN-major K tile, dead with the last dQ, or, if no item follows, at once into the
-        // K-major Q tile.  They are in registers when this warp hands over its next P^T, which the first dV of the next item
-        // waits for.
-        if (n_it > 0)
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, (part >= 2) ? &sh.dk_done : more ? &sh.dq_full : &sh.dv_done, (g - 1) & 1, W_BDONE, g));
-        if (!ok) break;
-        if (n_it > 0) {
-            tc_fence_after_sync();
-            tmem_ld32(trow + ((part < 2) ? COL_DV + part * 32 : COL_DK + (part - 2) * 32), rs);
-            tmem_wait_ld();
-            tc_fence_before_sync();
-            const float f = (part < 2) ? a.dv_scale : 1.f;
-            uint8_t* srow = ((part >= 2) ? sQm : more ? sKm : sQ) + (part & 1) * BOX_BYTES + row * 128;
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<float4*>(srow + ((c ^ (row & 7)) << 4)) =
-                    make_float4(__uint_as_float(rs[4 * c]) * f, __uint_as_float(rs[4 * c + 1]) * f,
-                                __uint_as_float(rs[4 * c + 2]) * f, __uint_as_float(rs[4 * c + 3]) * f);
-            fence_proxy_async_smem();
-            mbar_arrive_warp((part < 2) ? &sh.dv_staged : &sh.dk_staged, lane);
-        }
-        if (!more) break;
-        s = nx;
-        ++item;
+            if (!more) break;
+            s = nx;
+            ++item;
         }  // items
 
         if constexpr (SPLIT) {

@@ -532,308 +532,308 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
         Item x = first;
         int base = 0, q_base = 0, uses = 0;  // ring entries, products of the items before; items in which this stream had rows
         for (int item = 0; ok;) {
-        const int n0 = x.n0, n1 = x.n1, b = x.b, h = x.h, bh = x.bh, q_end = end_of(x);
-        const int nt = x.steps(t);
-        const int qrow = row0_of(x, t) + row;               // row inside this (b,h)
-        const bool row_ok = qrow < q_end;
-        const bool warp_live = row0_of(x, t) + quarter * 32 < q_end;  // any row of this warp exists
-        // last key index (local to this call's K) this row may see
-        long long lim_ll = a.Tk - 1;
-        if (a.causal) lim_ll = min(lim_ll, (long long)a.q_pos0 + qrow - a.k_pos0);
-        const int kv_lim = row_ok ? (int)max(-1ll, lim_ll) : -1;
-        const bool state_in = a.continue_state && split == 0 && !(keys && t == 1);
+            const int n0 = x.n0, n1 = x.n1, b = x.b, h = x.h, bh = x.bh, q_end = end_of(x);
+            const int nt = x.steps(t);
+            const int qrow = row0_of(x, t) + row;               // row inside this (b,h)
+            const bool row_ok = qrow < q_end;
+            const bool warp_live = row0_of(x, t) + quarter * 32 < q_end;  // any row of this warp exists
+            // last key index (local to this call's K) this row may see
+            long long lim_ll = a.Tk - 1;
+            if (a.causal) lim_ll = min(lim_ll, (long long)a.q_pos0 + qrow - a.k_pos0);
+            const int kv_lim = row_ok ? (int)max(-1ll, lim_ll) : -1;
+            const bool state_in = a.continue_state && split == 0 && !(keys && t == 1);
 
-        float m = -INFINITY;  // running max actually used as exponent reference, log2 units
-        float l = 0.f;
-        if (state_in && nt > 0) {
-            // The result over the keys seen so far is the starting state: reference LSE, normaliser 1 and the running
-            // output O itself (a row that has seen no key starts from nothing).  The output accumulator is written
-            // before this warp's first arrival on p_full, which the first P V of the stream waits for.
-            const float lse0 = row_ok ? a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] : -INFINITY;
-            const bool have = lse0 > -INFINITY;
-            m = have ? lse0 * LOG2E : -INFINITY;
-            l = have ? 1.f : 0.f;
-            const float4* orow = reinterpret_cast<const float4*>(a.O + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH +
-                                                                 (int64_t)(row_ok ? qrow : 0) * a.o_sM);
+            float m = -INFINITY;  // running max actually used as exponent reference, log2 units
+            float l = 0.f;
+            if (state_in && nt > 0) {
+                // The result over the keys seen so far is the starting state: reference LSE, normaliser 1 and the running
+                // output O itself (a row that has seen no key starts from nothing).  The output accumulator is written
+                // before this warp's first arrival on p_full, which the first P V of the stream waits for.
+                const float lse0 = row_ok ? a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] : -INFINITY;
+                const bool have = lse0 > -INFINITY;
+                m = have ? lse0 * LOG2E : -INFINITY;
+                l = have ? 1.f : 0.f;
+                const float4* orow = reinterpret_cast<const float4*>(a.O + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH +
+                                                                     (int64_t)(row_ok ? qrow : 0) * a.o_sM);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float4 v = have ? orow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                r[4 * i] = __float_as_uint(v.x); r[4 * i + 1] = __float_as_uint(v.y);
-                r[4 * i + 2] = __float_as_uint(v.z); r[4 * i + 3] = __float_as_uint(v.w);
-            }
-            tmem_st32p(tO, r);
-            tmem_st32p(tO + 32, r + 32);
-            tmem_wait_st();
-        }
-
-        // a product's number in the issue order picks its score buffer
-        auto product = [&](int j) { return q_base + min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0); };
-        int q_prev = 0;  // number of this stream's previous product
-        for (int j = 0; j < nt; ++j) {
-            const int q = product(j);
-            const int buf = q % 3;
-            const uint32_t tS = trow + score_col(buf);
-            // the vote keeps the warp converged for the .sync.aligned tensor-memory accesses below
-            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full[buf], (q / 3) & 1, W_SFULL, j));
-            if (!ok) break;
-            if (warp_live) {
-                tc_fence_after_sync();
-                tmem_ld32p(tS, r);
-                tmem_ld32p(tS + 32, r + 32);
-                tmem_ld32p(tS + 64, r + 64);
-                tmem_ld32p(tS + 96, r + 96);
-                const int kv0 = (x.jb + (keys ? 2 * j + t : j)) * TILE;
-                const int lim_local = kv_lim - kv0;  // columns 0..lim_local are visible
-                tmem_wait_ld();
-                if (lim_local < TILE - 1) {
-#pragma unroll
-                    for (int i = 0; i < 128; ++i)
-                        if (i > lim_local) r[i] = __float_as_uint(worst);
+                for (int i = 0; i < 16; ++i) {
+                    const float4 v = have ? orow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    r[4 * i] = __float_as_uint(v.x); r[4 * i + 1] = __float_as_uint(v.y);
+                    r[4 * i + 2] = __float_as_uint(v.z); r[4 * i + 3] = __float_as_uint(v.w);
                 }
-                // row max of the raw scores (min if the scale is negative), four chains
-                float mx0 = __uint_as_float(r[0]), mx1 = __uint_as_float(r[1]), mx2 = __uint_as_float(r[2]),
-                      mx3 = __uint_as_float(r[3]);
-                if (cs >= 0.f) {
-#pragma unroll
-                    for (int i = 4; i < 124; i += 8) {
-                        mx0 = fmax3(mx0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                        mx1 = fmax3(mx1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
-                        mx2 = fmax3(mx2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
-                        mx3 = fmax3(mx3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
-                    }
-                    mx0 = fmax3(mx0, __uint_as_float(r[124]), __uint_as_float(r[125]));
-                    mx1 = fmax3(mx1, __uint_as_float(r[126]), __uint_as_float(r[127]));
-                    mx0 = fmax3(fmaxf(mx0, mx1), mx2, mx3);
-                } else {
-#pragma unroll
-                    for (int i = 4; i < 128; i += 4) {
-                        mx0 = fminf(mx0, __uint_as_float(r[i]));
-                        mx1 = fminf(mx1, __uint_as_float(r[i + 1]));
-                        mx2 = fminf(mx2, __uint_as_float(r[i + 2]));
-                        mx3 = fminf(mx3, __uint_as_float(r[i + 3]));
-                    }
-                    mx0 = fminf(fminf(mx0, mx1), fminf(mx2, mx3));
-                }
-                const float m_cand = mx0 * cs;  // -inf when nothing is visible
-                // raise the reference only when it pays: a stale m makes p at most 2^8 larger, which fp32 absorbs
-                const bool raise = (m == -INFINITY) ? (m_cand > -INFINITY) : (m_cand > m + RESCALE_THRESHOLD);
-                const float m_new = raise ? m_cand : m;
-                const float alpha = raise ? ((m == -INFINITY) ? 0.f : ex2_approx(m - m_cand)) : 1.f;
-                if ((j > 0 || state_in) && __any_sync(0xffffffffu, raise)) {
-                    // rescale the running output, once the P V of the previous step has completed
-                    if (j > 0) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, j));
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                    }
-#pragma unroll 1
-                    for (int cc = 0; cc < 2; ++cc) {
-                        uint32_t o[32];
-                        tmem_ld32(tO + cc * 32, o);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st32(tO + cc * 32, o);
-                    }
-                }
-                const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
-                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-                if constexpr (DROP == 0) {
-                    // two scores per FMA and per add (fma.rn.f32x2 / add.rn.f32x2: the same roundings as the scalar forms)
-                    const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
-                    float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int i = 0; i < 128; i += 4) {
-                        const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
-                        const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), c2, nm2);
-                        const float2 p01 = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
-                        const float2 p23 = make_float2(ex2_approx(t23.x), ex2_approx(t23.y));
-                        s01 = __fadd2_rn(s01, p01);
-                        s23 = __fadd2_rn(s23, p23);
-                        r[i] = tf32_round_bits_mma(__float_as_uint(p01.x));
-                        r[i + 1] = tf32_round_bits_mma(__float_as_uint(p01.y));
-                        r[i + 2] = tf32_round_bits_mma(__float_as_uint(p23.x));
-                        r[i + 3] = tf32_round_bits_mma(__float_as_uint(p23.y));
-                    }
-                    s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
-                } else if constexpr (DROP == 2) {
-                    // One Philox call per eight keys of this row.  32 keys at a time, read from tensor memory once more, in a
-                    // rolled loop: the integer arithmetic is what dropout costs, and unrolled over the 128 registers
-                    // its code does not stay in the instruction cache.  None for 32 keys that no row of the warp
-                    // sees (on the diagonal three in eight).
-                    const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
-                    float2 sk = make_float2(0.f, 0.f), sa = make_float2(0.f, 0.f);  // kept terms, all terms
-                    const int warp_lim = __reduce_max_sync(0xffffffffu, lim_local);
-#pragma unroll 1
-                    for (int c = 0; c < 128; c += 32) {
-                        if (c > warp_lim) {
-#pragma unroll
-                            for (int u = 0; u < 32; ++u) r[u] = 0u;
-                        } else {
-                            tmem_ld32p(tS + c, r);
-                            hk_philox4_t w[4];
-#pragma unroll
-                            for (int g = 0; g < 4; ++g)
-                                w[g] = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh, (uint32_t)(a.q_pos0 + qrow),
-                                                           (uint32_t)(a.k_pos0 + kv0 + c + 8 * g) >> 3);
-                            tmem_wait_ld();
-                            if (lim_local < c + 31) {
-#pragma unroll
-                                for (int i = 0; i < 32; ++i)
-                                    if (c + i > lim_local) r[i] = __float_as_uint(worst);
-                            }
-#pragma unroll
-                            for (int i = 0; i < 32; i += 2) {
-                                const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
-                                float2 p = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
-                                if (scaled) sa = __fadd2_rn(sa, p);  // the normaliser ignores the mask
-                                if (!hk_philox_keep1(w[i >> 3], i & 7, a.drop_thr)) p.x = 0.f;
-                                if (!hk_philox_keep1(w[i >> 3], (i & 7) + 1, a.drop_thr)) p.y = 0.f;
-                                sk = __fadd2_rn(sk, p);
-                                r[i] = tf32_round_bits_mma(__float_as_uint(p.x));
-                                r[i + 1] = tf32_round_bits_mma(__float_as_uint(p.y));
-                            }
-                        }
-                        tmem_st32p(tS + c, r);
-                    }
-                    s0 = sk.x; s1 = sk.y; s2 = sa.x; s3 = sa.y;
-                } else {
-                    const float* mrow = a.mask + ((size_t)bh * a.Tq + (row_ok ? qrow : 0)) * (size_t)a.Tk + kv0;
-#pragma unroll
-                    for (int i = 0; i < 128; ++i) {
-                        float p = ex2_approx(fmaf(__uint_as_float(r[i]), cs, neg_m));
-                        if (scaled) s2 += (i <= lim_local) ? p : 0.f;
-                        p = (i <= lim_local) ? p * __ldg(mrow + i) : 0.f;
-                        s0 += p;
-                        r[i] = tf32_round_bits_mma(__float_as_uint(p));
-                    }
-                }
-                if constexpr (DROP != 2) {
-                    tmem_st32p(tS, r);
-                    tmem_st32p(tS + 32, r + 32);
-                    tmem_st32p(tS + 64, r + 64);
-                    tmem_st32p(tS + 96, r + 96);
-                }
-                // inverted dropout: s2, s3 hold the sums over all visible keys, s0, s1 the kept ones
-                l = l * alpha + ((scaled && DROP != 0) ? (s2 + s3) : ((s0 + s1) + (s2 + s3)));
-                m = m_new;
+                tmem_st32p(tO, r);
+                tmem_st32p(tO + 32, r + 32);
                 tmem_wait_st();
-                tc_fence_before_sync();
             }
-            mbar_arrive_warp(&sh.p_full[buf], lane);
-            q_prev = q;
-        }
 
-        // epilogue: O / l and LSE
-        if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, nt));
-        tc_fence_after_sync();
-        const float inv_l = COMBINE ? 1.f : (l > 0.f) ? a.keep_scale / l : 0.f;
-        if (ok && nt > 0) {
-            tmem_ld32p(tO, r);
-            tmem_ld32p(tO + 32, r + 32);
-            tmem_wait_ld();
-            tc_fence_before_sync();  // the next item's first P V overwrites it
-        } else {
-#pragma unroll
-            for (int i = 0; i < 64; ++i) r[i] = 0u;
-        }
-        // O leaves through shared memory (a thread-per-row store would touch 32 lines per instruction): a slot of the ring or, with
-        // one item, the stream's own Q buffer, which is dead -- o_full covered its last S = Q K^T, and in keys mode,
-        // where the streams share Q, every S: the last one is issued before the last two P V.  Either way as the two
-        // 32-column boxes of a 128-byte-swizzled TMA tile: 16-byte chunk i of row r at position i ^ (r & 7).
-        auto stage = [&](uint8_t* dst) {
-            uint8_t* srow = dst + row * 128;
-#pragma unroll
-            for (int ch = 0; ch < 16; ++ch)
-                *reinterpret_cast<float4*>(srow + (ch >> 3) * BOX_BYTES + (((ch & 7) ^ (row & 7)) << 4)) =
-                    make_float4(__uint_as_float(r[4 * ch]) * inv_l, __uint_as_float(r[4 * ch + 1]) * inv_l,
-                                __uint_as_float(r[4 * ch + 2]) * inv_l, __uint_as_float(r[4 * ch + 3]) * inv_l);
-        };
-        if constexpr (TAKES_OVER) {
-            const int n_o = o_slots(x);
-            if (ok && t < n_o) {
-                const int e = base + 2 * x.nk + t;
-                ok = (uses == 0 || mbar_wait(wc, &sh.o_taken[t], (uses - 1) & 1, W_OSLOT, 1000 + item)) &&
-                     mbar_wait(wc, &sh.kv_full[e % SLOTS], (e / SLOTS) & 1, W_OSLOT, item);
-                ok = __all_sync(0xffffffffu, ok);
+            // a product's number in the issue order picks its score buffer
+            auto product = [&](int j) { return q_base + min(j, n0) + min(j, n1) + ((t == 1 && j < n0) ? 1 : 0); };
+            int q_prev = 0;  // number of this stream's previous product
+            for (int j = 0; j < nt; ++j) {
+                const int q = product(j);
+                const int buf = q % 3;
+                const uint32_t tS = trow + score_col(buf);
+                // the vote keeps the warp converged for the .sync.aligned tensor-memory accesses below
+                ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.s_full[buf], (q / 3) & 1, W_SFULL, j));
                 if (!ok) break;
-                ++uses;
-                stage(sKV + e % SLOTS * TILE_BYTES);
-                fence_proxy_async_smem();
-                mbar_arrive_warp(&sh.o_staged[t], lane);
-                if (row_ok)
-                    a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
-            }
-            base += 2 * x.nk + n_o;
-            q_base += n0 + n1;
-            if (!ok || !read_item(x, ++item, false, true)) break;
-        } else if constexpr (!COMBINE) {
-            stage(sQ + t * TILE_BYTES);
-            fence_proxy_async_smem();
-            // a block none of whose rows sees a key of this call leaves a continued result untouched
-            const bool keep_old = a.continue_state && nt == 0;
-            if (row_ok && !keep_old)
-                a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
-            // the 128 threads of this stream (every one gets here, whatever `ok` is), then one of them stores
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
-            if (row == 0 && row_ok && !keep_old) {
-                tma_store_tile(&mapO, sQ + t * TILE_BYTES, qrow, h, b);
-                bulk_commit_group();
-                bulk_wait_group_read_all();  // the copy has read its source; it completes on its own
-            }
-            break;
-        } else {
-            const int all0 = x.all0, all1 = x.all1;
-            stage(sQ + t * TILE_BYTES);
-            // Combine: O = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M) over the splits and, in keys mode, the two
-            // streams.  Each CTA takes an equal slice of the rows it shares with its counterparts, 16 threads per row.
-            sh.m[t][row] = m;
-            sh.l[t][row] = l;
-            barrier_all();
-            const int rows = block_rows / ns, streams = keys ? 2 : 1;
-#pragma unroll 1
-            for (int i = threadIdx.x - 128; i < rows * 16; i += NUM_SOFTMAX) {
-                const int rr = split * rows + (i >> 4), ch = i & 15;
-                const int tt = rr / TILE, r1 = rr % TILE;
-                const int qr = row0_of(x, tt) + r1;
-                if (qr >= q_end || (a.continue_state && (tt == 0 ? all0 : all1) == 0)) continue;
-                const uint8_t* src = sQ + tt * TILE_BYTES + (ch >> 3) * BOX_BYTES + r1 * 128 + (((ch & 7) ^ (r1 & 7)) << 4);
-                float M = -INFINITY, L = 0.f;
-                float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                auto fold = [&](float ms, float ls, const float4& v) {
-                    const float Mn = fmaxf(M, ms);
-                    const float wa = M == -INFINITY ? 0.f : ex2_approx(M - Mn), w = ms == -INFINITY ? 0.f : ex2_approx(ms - Mn);
-                    L = L * wa + w * ls;
-                    acc.x = acc.x * wa + w * v.x; acc.y = acc.y * wa + w * v.y;
-                    acc.z = acc.z * wa + w * v.z; acc.w = acc.w * wa + w * v.w;
-                    M = Mn;
-                };
-                for (int u = 0; u < streams; ++u) {
-                    if (ns == 1) {
-                        fold(sh.m[tt + u][r1], sh.l[tt + u][r1], *reinterpret_cast<const float4*>(src + u * TILE_BYTES));
-                    } else {
-                        for (int s0 = 0; s0 < ns; s0 += 2) {
-                            float ms[2], ls[2];
-                            float4 v[2];
+                if (warp_live) {
+                    tc_fence_after_sync();
+                    tmem_ld32p(tS, r);
+                    tmem_ld32p(tS + 32, r + 32);
+                    tmem_ld32p(tS + 64, r + 64);
+                    tmem_ld32p(tS + 96, r + 96);
+                    const int kv0 = (x.jb + (keys ? 2 * j + t : j)) * TILE;
+                    const int lim_local = kv_lim - kv0;  // columns 0..lim_local are visible
+                    tmem_wait_ld();
+                    if (lim_local < TILE - 1) {
 #pragma unroll
-                            for (int s = 0; s < 2; ++s) {
-                                ms[s] = ld_cluster_f(mapa(&sh.m[tt + u][r1], s0 + s));
-                                ls[s] = ld_cluster_f(mapa(&sh.l[tt + u][r1], s0 + s));
-                                v[s] = ld_cluster_f4(mapa(src + u * TILE_BYTES, s0 + s));
-                            }
-                            fold(ms[0], ls[0], v[0]);
-                            fold(ms[1], ls[1], v[1]);
+                        for (int i = 0; i < 128; ++i)
+                            if (i > lim_local) r[i] = __float_as_uint(worst);
+                    }
+                    // row max of the raw scores (min if the scale is negative), four chains
+                    float mx0 = __uint_as_float(r[0]), mx1 = __uint_as_float(r[1]), mx2 = __uint_as_float(r[2]),
+                          mx3 = __uint_as_float(r[3]);
+                    if (cs >= 0.f) {
+#pragma unroll
+                        for (int i = 4; i < 124; i += 8) {
+                            mx0 = fmax3(mx0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                            mx1 = fmax3(mx1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                            mx2 = fmax3(mx2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
+                            mx3 = fmax3(mx3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
+                        }
+                        mx0 = fmax3(mx0, __uint_as_float(r[124]), __uint_as_float(r[125]));
+                        mx1 = fmax3(mx1, __uint_as_float(r[126]), __uint_as_float(r[127]));
+                        mx0 = fmax3(fmaxf(mx0, mx1), mx2, mx3);
+                    } else {
+#pragma unroll
+                        for (int i = 4; i < 128; i += 4) {
+                            mx0 = fminf(mx0, __uint_as_float(r[i]));
+                            mx1 = fminf(mx1, __uint_as_float(r[i + 1]));
+                            mx2 = fminf(mx2, __uint_as_float(r[i + 2]));
+                            mx3 = fminf(mx3, __uint_as_float(r[i + 3]));
+                        }
+                        mx0 = fminf(fminf(mx0, mx1), fminf(mx2, mx3));
+                    }
+                    const float m_cand = mx0 * cs;  // -inf when nothing is visible
+                    // raise the reference only when it pays: a stale m makes p at most 2^8 larger, which fp32 absorbs
+                    const bool raise = (m == -INFINITY) ? (m_cand > -INFINITY) : (m_cand > m + RESCALE_THRESHOLD);
+                    const float m_new = raise ? m_cand : m;
+                    const float alpha = raise ? ((m == -INFINITY) ? 0.f : ex2_approx(m - m_cand)) : 1.f;
+                    if ((j > 0 || state_in) && __any_sync(0xffffffffu, raise)) {
+                        // rescale the running output, once the P V of the previous step has completed
+                        if (j > 0) {
+                            ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, j));
+                            if (!ok) break;
+                            tc_fence_after_sync();
+                        }
+#pragma unroll 1
+                        for (int cc = 0; cc < 2; ++cc) {
+                            uint32_t o[32];
+                            tmem_ld32(tO + cc * 32, o);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                            tmem_st32(tO + cc * 32, o);
                         }
                     }
+                    const float neg_m = (m_new == -INFINITY) ? 0.f : -m_new;
+                    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+                    if constexpr (DROP == 0) {
+                        // two scores per FMA and per add (fma.rn.f32x2 / add.rn.f32x2: the same roundings as the scalar forms)
+                        const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
+                        float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int i = 0; i < 128; i += 4) {
+                            const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
+                            const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), c2, nm2);
+                            const float2 p01 = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
+                            const float2 p23 = make_float2(ex2_approx(t23.x), ex2_approx(t23.y));
+                            s01 = __fadd2_rn(s01, p01);
+                            s23 = __fadd2_rn(s23, p23);
+                            r[i] = tf32_round_bits_mma(__float_as_uint(p01.x));
+                            r[i + 1] = tf32_round_bits_mma(__float_as_uint(p01.y));
+                            r[i + 2] = tf32_round_bits_mma(__float_as_uint(p23.x));
+                            r[i + 3] = tf32_round_bits_mma(__float_as_uint(p23.y));
+                        }
+                        s0 = s01.x; s1 = s01.y; s2 = s23.x; s3 = s23.y;
+                    } else if constexpr (DROP == 2) {
+                        // One Philox call per eight keys of this row.  32 keys at a time, read from tensor memory once more, in a
+                        // rolled loop: the integer arithmetic is what dropout costs, and unrolled over the 128 registers
+                        // its code does not stay in the instruction cache.  None for 32 keys that no row of the warp
+                        // sees (on the diagonal three in eight).
+                        const float2 c2 = make_float2(cs, cs), nm2 = make_float2(neg_m, neg_m);
+                        float2 sk = make_float2(0.f, 0.f), sa = make_float2(0.f, 0.f);  // kept terms, all terms
+                        const int warp_lim = __reduce_max_sync(0xffffffffu, lim_local);
+#pragma unroll 1
+                        for (int c = 0; c < 128; c += 32) {
+                            if (c > warp_lim) {
+#pragma unroll
+                                for (int u = 0; u < 32; ++u) r[u] = 0u;
+                            } else {
+                                tmem_ld32p(tS + c, r);
+                                hk_philox4_t w[4];
+#pragma unroll
+                                for (int g = 0; g < 4; ++g)
+                                    w[g] = hk_philox_row8_keys(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh, (uint32_t)(a.q_pos0 + qrow),
+                                                               (uint32_t)(a.k_pos0 + kv0 + c + 8 * g) >> 3);
+                                tmem_wait_ld();
+                                if (lim_local < c + 31) {
+#pragma unroll
+                                    for (int i = 0; i < 32; ++i)
+                                        if (c + i > lim_local) r[i] = __float_as_uint(worst);
+                                }
+#pragma unroll
+                                for (int i = 0; i < 32; i += 2) {
+                                    const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, nm2);
+                                    float2 p = make_float2(ex2_approx(t01.x), ex2_approx(t01.y));
+                                    if (scaled) sa = __fadd2_rn(sa, p);  // the normaliser ignores the mask
+                                    if (!hk_philox_keep1(w[i >> 3], i & 7, a.drop_thr)) p.x = 0.f;
+                                    if (!hk_philox_keep1(w[i >> 3], (i & 7) + 1, a.drop_thr)) p.y = 0.f;
+                                    sk = __fadd2_rn(sk, p);
+                                    r[i] = tf32_round_bits_mma(__float_as_uint(p.x));
+                                    r[i + 1] = tf32_round_bits_mma(__float_as_uint(p.y));
+                                }
+                            }
+                            tmem_st32p(tS + c, r);
+                        }
+                        s0 = sk.x; s1 = sk.y; s2 = sa.x; s3 = sa.y;
+                    } else {
+                        const float* mrow = a.mask + ((size_t)bh * a.Tq + (row_ok ? qrow : 0)) * (size_t)a.Tk + kv0;
+#pragma unroll
+                        for (int i = 0; i < 128; ++i) {
+                            float p = ex2_approx(fmaf(__uint_as_float(r[i]), cs, neg_m));
+                            if (scaled) s2 += (i <= lim_local) ? p : 0.f;
+                            p = (i <= lim_local) ? p * __ldg(mrow + i) : 0.f;
+                            s0 += p;
+                            r[i] = tf32_round_bits_mma(__float_as_uint(p));
+                        }
+                    }
+                    if constexpr (DROP != 2) {
+                        tmem_st32p(tS, r);
+                        tmem_st32p(tS + 32, r + 32);
+                        tmem_st32p(tS + 64, r + 64);
+                        tmem_st32p(tS + 96, r + 96);
+                    }
+                    // inverted dropout: s2, s3 hold the sums over all visible keys, s0, s1 the kept ones
+                    l = l * alpha + ((scaled && DROP != 0) ? (s2 + s3) : ((s0 + s1) + (s2 + s3)));
+                    m = m_new;
+                    tmem_wait_st();
+                    tc_fence_before_sync();
                 }
-                const float f = (L > 0.f) ? a.keep_scale / L : 0.f;
-                reinterpret_cast<float4*>(a.O + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH + (int64_t)qr * a.o_sM)[ch] =
-                    make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
-                if (ch == 0)
-                    a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qr] = (L > 0.f) ? (M + log2f(L)) * LN2 : -INFINITY;
+                mbar_arrive_warp(&sh.p_full[buf], lane);
+                q_prev = q;
             }
-            break;
-        }
+
+            // epilogue: O / l and LSE
+            if (ok && nt > 0) ok = __all_sync(0xffffffffu, mbar_wait(wc, &sh.o_full[q_prev % 3], (q_prev / 3) & 1, W_OFULL, nt));
+            tc_fence_after_sync();
+            const float inv_l = COMBINE ? 1.f : (l > 0.f) ? a.keep_scale / l : 0.f;
+            if (ok && nt > 0) {
+                tmem_ld32p(tO, r);
+                tmem_ld32p(tO + 32, r + 32);
+                tmem_wait_ld();
+                tc_fence_before_sync();  // the next item's first P V overwrites it
+            } else {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) r[i] = 0u;
+            }
+            // O leaves through shared memory (a thread-per-row store would touch 32 lines per instruction): a slot of the ring or, with
+            // one item, the stream's own Q buffer, which is dead -- o_full covered its last S = Q K^T, and in keys mode,
+            // where the streams share Q, every S: the last one is issued before the last two P V.  Either way as the two
+            // 32-column boxes of a 128-byte-swizzled TMA tile: 16-byte chunk i of row r at position i ^ (r & 7).
+            auto stage = [&](uint8_t* dst) {
+                uint8_t* srow = dst + row * 128;
+#pragma unroll
+                for (int ch = 0; ch < 16; ++ch)
+                    *reinterpret_cast<float4*>(srow + (ch >> 3) * BOX_BYTES + (((ch & 7) ^ (row & 7)) << 4)) =
+                        make_float4(__uint_as_float(r[4 * ch]) * inv_l, __uint_as_float(r[4 * ch + 1]) * inv_l,
+                                    __uint_as_float(r[4 * ch + 2]) * inv_l, __uint_as_float(r[4 * ch + 3]) * inv_l);
+            };
+            if constexpr (TAKES_OVER) {
+                const int n_o = o_slots(x);
+                if (ok && t < n_o) {
+                    const int e = base + 2 * x.nk + t;
+                    ok = (uses == 0 || mbar_wait(wc, &sh.o_taken[t], (uses - 1) & 1, W_OSLOT, 1000 + item)) &&
+                         mbar_wait(wc, &sh.kv_full[e % SLOTS], (e / SLOTS) & 1, W_OSLOT, item);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    ++uses;
+                    stage(sKV + e % SLOTS * TILE_BYTES);
+                    fence_proxy_async_smem();
+                    mbar_arrive_warp(&sh.o_staged[t], lane);
+                    if (row_ok)
+                        a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
+                }
+                base += 2 * x.nk + n_o;
+                q_base += n0 + n1;
+                if (!ok || !read_item(x, ++item, false, true)) break;
+            } else if constexpr (!COMBINE) {
+                stage(sQ + t * TILE_BYTES);
+                fence_proxy_async_smem();
+                // a block none of whose rows sees a key of this call leaves a continued result untouched
+                const bool keep_old = a.continue_state && nt == 0;
+                if (row_ok && !keep_old)
+                    a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qrow] = (l > 0.f) ? (m + log2f(l)) * LN2 : -INFINITY;
+                // the 128 threads of this stream (every one gets here, whatever `ok` is), then one of them stores
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + t) : "memory");
+                if (row == 0 && row_ok && !keep_old) {
+                    tma_store_tile(&mapO, sQ + t * TILE_BYTES, qrow, h, b);
+                    bulk_commit_group();
+                    bulk_wait_group_read_all();  // the copy has read its source; it completes on its own
+                }
+                break;
+            } else {
+                const int all0 = x.all0, all1 = x.all1;
+                stage(sQ + t * TILE_BYTES);
+                // Combine: O = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M) over the splits and, in keys mode, the two
+                // streams.  Each CTA takes an equal slice of the rows it shares with its counterparts, 16 threads per row.
+                sh.m[t][row] = m;
+                sh.l[t][row] = l;
+                barrier_all();
+                const int rows = block_rows / ns, streams = keys ? 2 : 1;
+#pragma unroll 1
+                for (int i = threadIdx.x - 128; i < rows * 16; i += NUM_SOFTMAX) {
+                    const int rr = split * rows + (i >> 4), ch = i & 15;
+                    const int tt = rr / TILE, r1 = rr % TILE;
+                    const int qr = row0_of(x, tt) + r1;
+                    if (qr >= q_end || (a.continue_state && (tt == 0 ? all0 : all1) == 0)) continue;
+                    const uint8_t* src = sQ + tt * TILE_BYTES + (ch >> 3) * BOX_BYTES + r1 * 128 + (((ch & 7) ^ (r1 & 7)) << 4);
+                    float M = -INFINITY, L = 0.f;
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    auto fold = [&](float ms, float ls, const float4& v) {
+                        const float Mn = fmaxf(M, ms);
+                        const float wa = M == -INFINITY ? 0.f : ex2_approx(M - Mn), w = ms == -INFINITY ? 0.f : ex2_approx(ms - Mn);
+                        L = L * wa + w * ls;
+                        acc.x = acc.x * wa + w * v.x; acc.y = acc.y * wa + w * v.y;
+                        acc.z = acc.z * wa + w * v.z; acc.w = acc.w * wa + w * v.w;
+                        M = Mn;
+                    };
+                    for (int u = 0; u < streams; ++u) {
+                        if (ns == 1) {
+                            fold(sh.m[tt + u][r1], sh.l[tt + u][r1], *reinterpret_cast<const float4*>(src + u * TILE_BYTES));
+                        } else {
+                            for (int s0 = 0; s0 < ns; s0 += 2) {
+                                float ms[2], ls[2];
+                                float4 v[2];
+#pragma unroll
+                                for (int s = 0; s < 2; ++s) {
+                                    ms[s] = ld_cluster_f(mapa(&sh.m[tt + u][r1], s0 + s));
+                                    ls[s] = ld_cluster_f(mapa(&sh.l[tt + u][r1], s0 + s));
+                                    v[s] = ld_cluster_f4(mapa(src + u * TILE_BYTES, s0 + s));
+                                }
+                                fold(ms[0], ls[0], v[0]);
+                                fold(ms[1], ls[1], v[1]);
+                            }
+                        }
+                    }
+                    const float f = (L > 0.f) ? a.keep_scale / L : 0.f;
+                    reinterpret_cast<float4*>(a.O + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH + (int64_t)qr * a.o_sM)[ch] =
+                        make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f);
+                    if (ch == 0)
+                        a.LSE[(int64_t)b * a.lse_sB + (int64_t)h * a.lse_sH + qr] = (L > 0.f) ? (M + log2f(L)) * LN2 : -INFINITY;
+                }
+                break;
+            }
         }  // items
         tc_fence_before_sync();
         barrier_all();  // pairs with the control warps' barrier before tensor memory is freed
