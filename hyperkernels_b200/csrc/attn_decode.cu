@@ -168,16 +168,19 @@ __global__ void __launch_bounds__(WARPS * 32, (NQ == 1 ? 24 : 16) / WARPS) attn_
     }
 }
 
-// Warps of a CTA and CTAs of a slice (a cluster of up to eight, the portable size): as many warps per slice as can all be
-// resident at once, each with at least one batch of rows.  A second wave finds a chip that the first is leaving a CTA at a
+// Warps of a CTA and CTAs of a slice (a cluster of up to eight, the portable size): as many warps per slice as should all be
+// resident at once by the estimate below, each with at least one batch of rows.  A second wave finds a chip that the first is leaving a CTA at a
 // time.  B4 H8, 8 191 keys: 25.0 us with 14 warps per SM, 37.7 with 28 wanted and 24 that fit; B16 H12, 2 047 keys: 33.0 with 21, 37.1
 // with 42, 36.6 with 10; B64 H16, 511 keys: 45.3 one CTA per slice, 48 - 63 with more.  Slices that do not fit at all take
 // one CTA each.
 // Of equal numbers the order decides.  One CTA of sixteen warps is faster than two of eight (120 slices of 2 056 keys 22.1 and
 // 24.8 us); two of sixteen than four of eight only where these no longer get an SM each (68 slices 15.5 and 16.2; 4 slices of
 // 359 keys 4.9 and 4.3; two query rows: 64 slices 15.9 and 15.6).
-// What fits is known from the clusters of one CTA per SM that the device holds.  Clusters of eight pack better two and three
-// to an SM: 48 slices run at once (12.7 us), 52 do not (19.0), with 15 clusters of one CTA per SM.
+// What fits is an estimate.  The device is asked how many clusters of the forward kernel, one CTA per SM, it holds
+// (attn_fwd_slots); here an SM holds two to six CTAs by the kernels' launch bounds, and the number of clusters is taken to grow
+// with that.  Clusters of eight pack better than this two and three to an SM: with 15 of them at one CTA per SM, 48 slices
+// still run at once at three (12.7 us), 52 do not (19.0), hence 0.87 of the places.  That share is measured on a chip of 148
+// SMs; elsewhere, and where the estimate is off, a call takes a wave more or leaves places empty, nothing else.
 DecodePlan plan_attn_decode(int BH, int Tq, int Tk, const int slots[4]) {
     static const DecodePlan order[2][9] = {{{8, 4}, {16, 1}, {16, 2}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}},
                                            {{16, 2}, {16, 1}, {8, 4}, {8, 2}, {8, 1}, {16, 8}, {16, 4}, {8, 8}, {4, 1}}};

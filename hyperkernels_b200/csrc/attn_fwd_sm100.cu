@@ -901,14 +901,15 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     // slower and one 10 %.  (By itself the fine estimate slows 7 % of the fitted shapes, by up to 25 %.)  H16, 512 queries, 4 096
     // keys 27.7 -> 21.4 us; H32, 128 queries, 2 048 keys 16.0 -> 12.2; H24 T525 without a mask, with dropout 19.3 -> 16.2.
     const bool may_split = Tk > 4096 || Tk >= 2 * (long long)Tq;
-    // Of the cuts of splits of eight key tiles or fewer 2 us are at stake; there the coarse estimate stays alone, and with it
-    // the small shapes that reach each mode.
+    // Where eight key tiles or fewer may be split, 2 us are at stake between the cuts, and the coarse estimate stays alone.  (The
+    // tests of every cut use such shapes: they hold on to the cuts that it gives.)
     const bool refine = !may_split || Tk > 8 * TILE;
     const int n_kvtiles = (Tk + TILE - 1) / TILE;
     // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
-    // then more than the bookkeeping costs per step (about 2 %).  Steps per item on average, one item per CTA -> taken over:
-    // 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same without a mask)
-    // 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
+    // then more than the bookkeeping costs per step (about 2 %, of which some may be registers: the kernels that take over spill
+    // 76 to 152 bytes per thread, those for one item none, or 88 with a dense mask).  Steps per item on average, one item per
+    // CTA -> taken over: 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same
+    // without a mask) 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
     // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
     // storing warp counts on a product in every item.
     const bool sees_keys = !causal || q_pos0 >= k_pos0;

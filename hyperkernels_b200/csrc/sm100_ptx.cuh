@@ -109,7 +109,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 
 // Per-CTA wait contexts.  The record lives in shared memory and is raised by the first wait that gives up; every later wait
 // sees it and returns at once.
-struct WaitCtx {  // the wait that gives up tells the host
+struct WaitCtx {  // the wait that gives up tells the host: for short kernels (self-test, rate probe)
     volatile int* abort_flag;  // shared memory
     DeviceStatus* status;      // global memory
 };
@@ -117,7 +117,7 @@ struct Abort {
     volatile int id;  // of the wait, 0: none gave up
     int thread, aux;
 };
-struct WaitNote {  // the kernel tells the host as it ends (report_abort): less code in each wait
+struct WaitNote {  // the kernel tells the host as it ends (report_abort): less code in each wait, for the attention kernels
     Abort* abort;
 };
 __device__ __forceinline__ bool gave_up(const WaitCtx& ctx) { return *ctx.abort_flag != 0; }

@@ -144,7 +144,8 @@ def decode_plan(BH, Tq, Tk, slots=B200):
 
 
 def test_decode_puts_one_wave_of_warps_on_the_chip():
-    """As many warps as are resident together, unless one CTA per slice is more already; each with a batch of rows."""
+    """As many warps as the plan's own estimate of what is resident together (clusters of one CTA per SM, times the CTAs of an
+    SM; 0.87 of the places for eight of them), unless one CTA per slice is more already; each with a batch of rows."""
     rnd = random.Random(2)
     for _ in range(3000):
         BH, Tq, Tk = int(2 ** rnd.uniform(0, 12)), rnd.choice([1, 2]), int(2 ** rnd.uniform(7, 15))
@@ -152,7 +153,7 @@ def test_decode_puts_one_wave_of_warps_on_the_chip():
         assert warps in (4, 8, 16) and splits in (1, 2, 4, 8) and warps * splits * 8 <= Tk
         per_sm = 24 if Tq == 1 else 16
         k = per_sm // warps
-        fit = dict(zip((1, 2, 4, 8), (k * s for s in B200)))  # clusters that the device holds
+        fit = dict(zip((1, 2, 4, 8), (k * s for s in B200)))  # clusters that the device is taken to hold
         if k > 1:
             fit[8] = max(fit[8], int(0.87 * 148 * k / 8))
         assert BH <= fit[splits] or splits == 1
