@@ -153,8 +153,7 @@ namespace bwd {
 __device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split, int ns) {
     Item x;
     // early KV tiles first: under the causal mask they see the most query tiles
-    x.bh = item % a.BH;
-    x.kt = item / a.BH;
+    take_in_groups(item, a.BH, a.live, a.group, x.bh, x.kt);
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
     const int n_qtiles = (a.Tq + TILE - 1) / TILE;
@@ -994,6 +993,8 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     const BwdPlan plan = plan_attn_bwd(a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, d->slots);
     const int live = plan.live;
     a.n_splits = plan.n_splits;
+    a.live = live;
+    a.group = slices_in_l2(a.BH, 256.0 * (3.0 * a.Tq + 4.0 * a.Tk));  // Q, dO, dQ; K, V, dK, dV
     const long long nblocks = (long long)live * a.BH * a.n_splits;
     if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     if (nblocks > 0) {

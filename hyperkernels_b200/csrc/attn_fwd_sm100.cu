@@ -134,8 +134,9 @@ __host__ __device__ inline int kv_tiles_for(int q0, int Tq, int Tk, int causal, 
 __device__ __forceinline__ Item make_item(const FwdArgs& a, int work, int split, int ns) {
     Item x;
     // heavy (late) query blocks first: under the causal mask they have the most key tiles
-    x.bh = work % a.BH;
-    const int qb = a.n_qblocks - 1 - work / a.BH;
+    int qb;
+    take_in_groups(work, a.BH, a.n_qblocks, a.group, x.bh, qb);
+    qb = a.n_qblocks - 1 - qb;
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
     // rows mode: stream t = query rows q0 + 128 t ..; keys mode: both streams = rows q0 .., stream t = key tiles 2 j + t.
@@ -985,6 +986,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.mode = plan.mode;
     a.n_splits = plan.n_splits;
     a.n_qblocks = plan.n_qblocks;
+    a.group = slices_in_l2(a.BH, 256.0 * (2.0 * a.Tq + 2.0 * a.Tk));  // Q, O; K, V
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);

@@ -1,9 +1,33 @@
 // attn_kernels.cuh -- argument blocks and launchers of the two tensor-core kernels.
 #pragma once
+#include <algorithm>
+
 #include "attn_common.cuh"
 #include "philox.h"
 
 namespace hk {
+
+// Order of work items: slice `bh` (batch x head) and part `part` of it (a KV tile or a block of rows, 0 the longest) of item
+// `item`, where the `n` parts of each of `all` slices are handed out part by part inside runs of `group` slices.  With all slices
+// in one run a slice's second part came up when its tensors had long left the L2 again, and every part fetched them (the
+// backward's dQ both ways) from memory.  Runs whose tensors take half of the L2 (slices_in_l2), one order -> the other:
+// backward B32 H25 T1024 815 -> 701 us, B16 H16 T2048 without a mask 1 741 -> 1 395, H32 T32768 23 820 -> 21 126, forward of the
+// first two 288 -> 279 and 514 -> 484.  A run also has to be long enough for the CTAs to finish together (longest parts first, and
+// the last run takes what is left over): with 8 MB per run B2 H16 T2000 took 115 us, with 64 MB or more 93.  24 to 96 MB
+// are within 4 % of each other for most shapes.
+__device__ __forceinline__ void take_in_groups(int item, int all, int n, int group, int& bh, int& part) {
+    int first = 0, size = all;
+    if (group < all) {  // (two divisions before the first load: 1 % of the smallest calls)
+        first = min(item / (n * group), all / group - 1) * group;
+        if (all - first >= 2 * group) size = group;
+        item -= first * n;
+    }
+    part = item / size;
+    bh = first + (item - part * size);
+}
+
+// Slices in a run: as many as 64 MB hold (about half of the 126 MB of L2, the rest for what the next run loads), at least one.
+inline int slices_in_l2(int all, double slice_bytes) { return std::max(1, (int)std::min((double)all, 67108864.0 / slice_bytes + 0.5)); }
 
 // what the two streams of a forward CTA are (attn_fwd_sm100.cu)
 enum FwdMode { FWD_ROWS = 0, FWD_ROW = 1, FWD_KEYS = 2 };
@@ -15,7 +39,8 @@ struct FwdArgs {
     int64_t o_sB, o_sM, o_sH, lse_sB, lse_sH;
     int H, BH;
     int Tq, Tk;
-    int n_qblocks, n_splits, mode;  // how the work is cut: set by launch_attn_fwd
+    int n_qblocks, n_splits, mode;  // how the work is cut: set by launch_attn_fwd, as is
+    int group;                      // slices whose blocks of rows come before those of others (take_in_groups)
     int q_pos0, k_pos0;
     float scale_log2e;
     int causal;
@@ -73,7 +98,9 @@ struct BwdArgs {
     int64_t dq_sB, dq_sM, dq_sH, dk_sB, dk_sM, dk_sH, dv_sB, dv_sM, dv_sH;
     int H, BH;
     int Tq, Tk;
-    int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; set by launch_attn_bwd
+    int n_splits;      // CTAs (a cluster) that share the query tiles of a KV tile; this and the next two set by launch_attn_bwd
+    int live;          // KV tiles of a slice in the grid
+    int group;         // slices whose KV tiles come before those of others (take_in_groups)
     int q_pos0, k_pos0;
     float scale, scale_log2e;
     int causal;

@@ -389,6 +389,31 @@ def test_a_slice_keeps_its_bits_in_any_batch_at_training_lengths(Tq, Tk, causal,
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("BH,Tq,Tk,causal", [(530, 300, 300, True), (530, 300, 400, False), (171, 1000, 700, False), (2100, 64, 100, True)])
+def test_slices_handed_out_in_runs_keep_their_bits(BH, Tq, Tk, causal):
+    """More slices than one run of the grid holds (64 MB), the last run longer than the others: every slice equals the same
+    slice in calls of one run."""
+    def run(seq):  # slices of a run
+        return max(1, int(min(BH, 2 ** 26 / (256 * seq) + 0.5)))
+    fwd, bwd = run(2 * Tq + 2 * Tk), run(3 * Tq + 4 * Tk)
+    part = min(fwd, bwd)
+    assert BH >= 2 * bwd and BH % bwd  # several, with a remainder
+    gen = torch.Generator(device="cuda").manual_seed(79)
+    Q, dO = (torch.randn((1, BH, Tq, 64), generator=gen, device="cuda") for _ in range(2))
+    K, V = (torch.randn((1, BH, Tk, 64), generator=gen, device="cuda") for _ in range(2))
+    O, LSE = hk.attention_forward(Q, K, V, SCALE, causal)
+    got = (O, LSE) + hk.attention_backward(Q, K, V, O, dO, LSE, SCALE, causal, deterministic_dq=True)[:3]
+    for i in range(0, BH, part):
+        s = slice(i, min(BH, i + part))
+        o, l = hk.attention_forward(Q[:, s], K[:, s], V[:, s], SCALE, causal)
+        want = (o, l) + hk.attention_backward(Q[:, s], K[:, s], V[:, s], o, dO[:, s], l, SCALE, causal, deterministic_dq=True)[:3]
+        for g, w in zip(got, want):
+            assert torch.equal(g[:, s], w)
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+
+
+@pytest.mark.gpu
 def test_a_chunked_host_step_beyond_them_agrees_within_rounding():
     """One long sequence, its heads one by one or in one call: the forward is cut differently, so a probability is rounded
     to TF32 (2^-11 of itself) relative to another maximum on either side."""
