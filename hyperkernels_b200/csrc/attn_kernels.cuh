@@ -15,11 +15,12 @@ namespace hk {
 // first two 288 -> 279 and 514 -> 484.  A run also has to be long enough for the CTAs to finish together (longest parts first, and
 // the last run takes what is left over): with 8 MB per run B2 H16 T2000 took 115 us, with 64 MB or more 93.  24 to 96 MB
 // are within 4 % of each other for most shapes.
-__device__ __forceinline__ void take_in_groups(int item, int all, int n, int group, int& bh, int& part) {
+__host__ __device__ __forceinline__ void take_in_groups(int item, int all, int n, int group, int& bh, int& part) {
     int first = 0, size = all;
     if (group < all) {  // (two divisions before the first load: 1 % of the smallest calls)
-        first = min(item / (n * group), all / group - 1) * group;
-        if (all - first >= 2 * group) size = group;
+        const int run = item / (n * group), last = all / group - 1;
+        first = (run < last ? run : last) * group;
+        size = run < last ? group : all - first;
         item -= first * n;
     }
     part = item / size;
@@ -152,6 +153,9 @@ extern "C" int hk_attn_backward_noscratch(const hk_attn_bwd_params* p, void* str
 // BwdJob}.
 extern "C" int hk_attn_forward_plan(const hk_attn_fwd_params* p, const int* slots, int* plan);
 extern "C" int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slots, int* plan);
+// The order of the work items (take_in_groups) of `all` slices of `slice_bytes` and `n` parts each, for tests: all * n pairs
+// {slice, part}.
+extern "C" void hk_attn_item_order(int all, int n, double slice_bytes, int* pairs);
 // zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ
 extern "C" int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream);
 

@@ -388,6 +388,21 @@ def test_a_slice_keeps_its_bits_in_any_batch_at_training_lengths(Tq, Tk, causal,
     assert hk.last_device_status() == 0
 
 
+@pytest.mark.parametrize("all_", [1, 2, 7, 96, 126, 127, 128, 333, 800])
+@pytest.mark.parametrize("n", [1, 2, 9, 64])
+def test_every_item_is_handed_out_once(all_, n):
+    """Runs of 1, 2, 5, 64 and of more slices than there are: every part of every slice once, a run's slices before those of
+    the next, longest parts first inside a run, and only the last run longer (up to, not including, two)."""
+    for group in (1, 2, 5, 64, 1000):
+        pairs = np.zeros((all_ * n, 2), np.int32)
+        hk.lib().hk_attn_item_order(all_, n, C.c_double(2 ** 26 / group), pairs.ctypes.data_as(C.c_void_p))
+        assert len({tuple(p) for p in pairs.tolist()}) == all_ * n
+        assert pairs.min() == 0 and pairs[:, 0].max() == all_ - 1 and pairs[:, 1].max() == n - 1
+        run = np.minimum(pairs[:, 0] // group, max(all_ // group, 1) - 1)
+        key = run * n + pairs[:, 1]
+        assert (np.diff(key) >= 0).all()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("BH,Tq,Tk,causal", [(530, 300, 300, True), (530, 300, 400, False), (171, 1000, 700, False), (2100, 64, 100, True)])
 def test_slices_handed_out_in_runs_keep_their_bits(BH, Tq, Tk, causal):
