@@ -783,18 +783,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     if (!ok) break;
                 }
                 {
-                    // Rows r and r + 4 share a 32-byte chunk position; they store its two halves in opposite order so
-                    // that the eight lanes of a quarter-warp hit eight different 16-byte bank groups.
+                    // Rows r and r + 4 share a 32-byte chunk position, so two of the eight lanes of a quarter-warp meet in a
+                    // 16-byte bank group.  Storing the two halves in opposite order avoids that, but the 32 selects that it
+                    // takes cost what it gains (B8 H12 T1024 84.4 us either way), and more where the warps have keep bits to
+                    // draw too (with dropout 97.0 -> 94.6 without them).
                     uint8_t* drow = sdS + part * BOX_BYTES + row * 128;
-                    const bool swap = (row >> 2) & 1;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint4 lo = make_uint4(rp[8 * u], rp[8 * u + 1], rp[8 * u + 2], rp[8 * u + 3]);
-                        const uint4 hi = make_uint4(rp[8 * u + 4], rp[8 * u + 5], rp[8 * u + 6], rp[8 * u + 7]);
-                        uint8_t* chunk = drow + ((u ^ (row & 3)) << 5);
-                        *reinterpret_cast<uint4*>(chunk + (swap ? 16 : 0)) = swap ? hi : lo;
-                        *reinterpret_cast<uint4*>(chunk + (swap ? 0 : 16)) = swap ? lo : hi;
-                    }
+                    for (int u = 0; u < 8; ++u)
+                        *reinterpret_cast<uint4*>(drow + (((u >> 1) ^ (row & 3)) << 5) + ((u & 1) << 4)) =
+                            make_uint4(rp[4 * u], rp[4 * u + 1], rp[4 * u + 2], rp[4 * u + 3]);
                 }
                 fence_proxy_async_smem();
                 mbar_arrive_warp(&sh.ds_ready, lane);
