@@ -90,6 +90,44 @@ __device__ __forceinline__ hk_philox4_t hk_philox_row8_keys(const hk_philox_keys
     out.v[0] = c0; out.v[1] = c1; out.v[2] = c2; out.v[3] = c3;
     return out;
 }
+
+/* Both halves of a product by one instruction.  With the calls in parts (below) this is faster than the two of hk_mulhilo32,
+ * with whole calls it is not. */
+__device__ __forceinline__ void hk_mulwide32(uint32_t a, uint32_t b, uint32_t* hi, uint32_t* lo) {
+    unsigned long long p;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(p) : "r"(a), "r"(b));
+    *lo = (uint32_t)p;
+    *hi = (uint32_t)(p >> 32);
+}
+/* The same call in parts.  Of the first two and a half rounds every product has a factor that depends on the query row alone
+ * or on the keys alone (the other words enter by exclusive or): 5 of the 20 wide products of a call. */
+__device__ __forceinline__ uint4 hk_philox_key_part(const hk_philox_keys_t& k, uint32_t offset, uint32_t bh, uint32_t kj8) {
+    uint32_t hi, lo0, lo1, hi2, lo2;
+    hk_mulwide32(HK_PHILOX_M0, kj8, &hi, &lo0);
+    hk_mulwide32(HK_PHILOX_M1, hi ^ offset ^ k.k1[0], &hi, &lo1);
+    hk_mulwide32(HK_PHILOX_M0, hi ^ (HK_PHILOX_M1 * bh) ^ k.k0[1], &hi2, &lo2);
+    return make_uint4(lo0 ^ k.k1[1], lo1 ^ k.k0[2], hi2 ^ k.k1[2], lo2);
+}
+__device__ __forceinline__ uint2 hk_philox_row_part(const hk_philox_keys_t& k, uint32_t bh, uint32_t qi) {
+    uint32_t hi, lo;
+    hk_mulwide32(HK_PHILOX_M0, __umulhi(HK_PHILOX_M1, bh) ^ qi ^ k.k0[0], &hi, &lo);
+    return make_uint2(hi, lo);
+}
+__device__ __forceinline__ hk_philox4_t hk_philox_join(const hk_philox_keys_t& k, const uint4& key, const uint2& row) {
+    uint32_t hi0, lo0, hi1, lo1;
+    hk_mulwide32(HK_PHILOX_M1, row.x ^ key.x, &hi1, &lo1);
+    uint32_t c0 = hi1 ^ key.y, c1 = lo1, c2 = key.z ^ row.y, c3 = key.w;
+#pragma unroll
+    for (int r = 3; r < 10; ++r) {
+        hk_mulwide32(HK_PHILOX_M0, c0, &hi0, &lo0);
+        hk_mulwide32(HK_PHILOX_M1, c2, &hi1, &lo1);
+        const uint32_t n0 = hi1 ^ c1 ^ k.k0[r], n2 = hi0 ^ c3 ^ k.k1[r];
+        c0 = n0; c1 = lo1; c2 = n2; c3 = lo0;
+    }
+    hk_philox4_t out;
+    out.v[0] = c0; out.v[1] = c1; out.v[2] = c2; out.v[3] = c3;
+    return out;
+}
 #endif
 
 /* floor(p * 2^16), in [0, 65535]; p in [0,1). */
