@@ -150,10 +150,12 @@ enum WaitId {
 }  // namespace bwd
 
 namespace bwd {
+// GROUPS: the items come in runs of slices (take_in_groups)
+template <bool GROUPS>
 __device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split, int ns) {
     Item x;
     // early KV tiles first: under the causal mask they see the most query tiles
-    take_in_groups(item, a.BH, a.live, a.group, x.bh, x.kt);
+    take_in_groups(item, a.BH, a.live, GROUPS ? a.group : a.BH, x.bh, x.kt);
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
     const int n_qtiles = (a.Tq + TILE - 1) / TILE;
@@ -210,7 +212,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
 
     const int ns = SPLIT ? a.n_splits : 1;  // cluster size
     const int split = SPLIT ? (int)cluster_ctarank() : 0;
-    const Item first = make_item(a, (int)blockIdx.x / ns, split, ns);
+    const Item first = make_item<TAKES_OVER>(a, (int)blockIdx.x / ns, split, ns);
 
     auto load_tile = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row, const Item& x) {
         mbar_arrive_expect_tx(bar, TILE_BYTES);
@@ -324,7 +326,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                     return false;
                 more = id >= 0;
                 if (more) {
-                    cur = make_item(a, id, 0, 1);
+                    cur = make_item<true>(a, id, 0, 1);
                     sh.item[buf] = cur;
                 } else {
                     sh.item[buf].n_it = -1;

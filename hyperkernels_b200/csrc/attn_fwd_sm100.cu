@@ -131,11 +131,13 @@ __host__ __device__ inline int kv_tiles_for(int q0, int Tq, int Tk, int causal, 
     return (int)((kv_end + TILE - 1) / TILE);
 }
 
+// GROUPS: the items come in runs of slices (take_in_groups)
+template <bool GROUPS>
 __device__ __forceinline__ Item make_item(const FwdArgs& a, int work, int split, int ns) {
     Item x;
     // heavy (late) query blocks first: under the causal mask they have the most key tiles
     int qb;
-    take_in_groups(work, a.BH, a.n_qblocks, a.group, x.bh, qb);
+    take_in_groups(work, a.BH, a.n_qblocks, GROUPS ? a.group : a.BH, x.bh, qb);
     qb = a.n_qblocks - 1 - qb;
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
@@ -177,7 +179,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int split = COMBINE && ns > 1 ? (int)cluster_ctarank() : 0;
     const bool keys = COMBINE && a.mode == FWD_KEYS;
     const int block_rows = a.mode == FWD_ROWS ? 2 * TILE : TILE;
-    const Item first = make_item(a, blockIdx.x / ns, split, ns);
+    const Item first = make_item<!COMBINE>(a, blockIdx.x / ns, split, ns);
 
     auto end_of = [&](const Item& x) { return min(a.Tq, x.q0 + block_rows); };             // of the block's rows
     auto row0_of = [&](const Item& x, int t) { return x.q0 + (keys ? 0 : t * TILE); };      // first row of stream t
@@ -321,7 +323,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                         // The next item is made known behind the last score of stream 0 in this one: see s_full.  Q and K of the
                         // next item wait for it anyway.
                         if (q0_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[0], (q0_uses - 1) & 1, W_QEMPTY, r))) break;
-                        x = make_item(a, id, 0, 1);
+                        x = make_item<true>(a, id, 0, 1);
                         sh.item[buf] = x;
                     } else {
                         sh.item[buf].n0 = -1;

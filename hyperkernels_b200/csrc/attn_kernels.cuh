@@ -17,7 +17,7 @@ namespace hk {
 // are within 4 % of each other for most shapes.
 __host__ __device__ __forceinline__ void take_in_groups(int item, int all, int n, int group, int& bh, int& part) {
     int first = 0, size = all;
-    if (group < all) {  // (two divisions before the first load: 1 % of the smallest calls)
+    if (group < all) {  // with one run the divisions before the first load would cost the smallest calls 1 %
         const int run = item / (n * group), last = all / group - 1;
         first = (run < last ? run : last) * group;
         size = run < last ? group : all - first;
@@ -27,8 +27,12 @@ __host__ __device__ __forceinline__ void take_in_groups(int item, int all, int n
     bh = first + (item - part * size);
 }
 
-// Slices in a run: as many as 64 MB hold (about half of the 126 MB of L2, the rest for what the next run loads), at least one.
-inline int slices_in_l2(int all, double slice_bytes) { return std::max(1, (int)std::min((double)all, 67108864.0 / slice_bytes + 0.5)); }
+// Slices in a run: as many as 64 MB hold (about half of the 126 MB of L2, the rest for what the next run loads), at least one;
+// all, if that leaves one run.
+inline int slices_in_l2(int all, double slice_bytes) {
+    const int group = std::max(1, (int)std::min((double)all, 67108864.0 / slice_bytes + 0.5));
+    return all < 2 * group ? all : group;
+}
 
 // what the two streams of a forward CTA are (attn_fwd_sm100.cu)
 enum FwdMode { FWD_ROWS = 0, FWD_ROW = 1, FWD_KEYS = 2 };
