@@ -150,12 +150,12 @@ enum WaitId {
 }  // namespace bwd
 
 namespace bwd {
-// GROUPS: the items come in runs of slices (take_in_groups)
-template <bool GROUPS>
+// RUNS: the items come in runs of slices (take_in_groups)
+template <bool RUNS>
 __device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split, int ns) {
     Item x;
     // early KV tiles first: under the causal mask they see the most query tiles
-    take_in_groups(item, a.BH, a.live, GROUPS ? a.group : a.BH, x.bh, x.kt);
+    take_in_groups(item, a.BH, a.live, RUNS ? a.group : a.BH, x.bh, x.kt);
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
     const int n_qtiles = (a.Tq + TILE - 1) / TILE;
