@@ -131,13 +131,13 @@ __host__ __device__ inline int kv_tiles_for(int q0, int Tq, int Tk, int causal, 
     return (int)((kv_end + TILE - 1) / TILE);
 }
 
-// GROUPS: the items come in runs of slices (take_in_groups)
-template <bool GROUPS>
+// RUNS: the items come in runs of slices (take_in_groups)
+template <bool RUNS>
 __device__ __forceinline__ Item make_item(const FwdArgs& a, int work, int split, int ns) {
     Item x;
     // heavy (late) query blocks first: under the causal mask they have the most key tiles
     int qb;
-    take_in_groups(work, a.BH, a.n_qblocks, GROUPS ? a.group : a.BH, x.bh, qb);
+    take_in_groups(work, a.BH, a.n_qblocks, RUNS ? a.group : a.BH, x.bh, qb);
     qb = a.n_qblocks - 1 - qb;
     x.b = x.bh / a.H;
     x.h = x.bh - x.b * a.H;
@@ -162,7 +162,9 @@ __device__ __forceinline__ Item make_item(const FwdArgs& a, int work, int split,
 // not started under the tail of the one before it, programmatic dependent launch or not, so grids that fit the device use one
 // without (B1 H12 T512: 8.5 us, with it 9.5).
 enum FwdJob { ONE_ITEM = 0, TAKE_OVER = 1, COMBINE_ITEM = 2 };  // COMBINE_ITEM: keys mode or key splits, merged at the end
-template <int DROP, int JOB>
+// RUNS: the blocks come in runs of slices (take_in_groups).  A kernel without them is 1 % faster where there is one run (B8 H12
+// T1024 39.3 -> 38.9 us), so there are both.
+template <int DROP, int JOB, bool RUNS>
 __global__ void __launch_bounds__(fwd::NUM_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                 const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO, const __grid_constant__ FwdArgs a) {
@@ -179,7 +181,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
     const int split = COMBINE && ns > 1 ? (int)cluster_ctarank() : 0;
     const bool keys = COMBINE && a.mode == FWD_KEYS;
     const int block_rows = a.mode == FWD_ROWS ? 2 * TILE : TILE;
-    const Item first = make_item<!COMBINE>(a, blockIdx.x / ns, split, ns);
+    const Item first = make_item<RUNS>(a, blockIdx.x / ns, split, ns);
 
     auto end_of = [&](const Item& x) { return min(a.Tq, x.q0 + block_rows); };             // of the block's rows
     auto row0_of = [&](const Item& x, int t) { return x.q0 + (keys ? 0 : t * TILE); };      // first row of stream t
@@ -323,7 +325,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                         // The next item is made known behind the last score of stream 0 in this one: see s_full.  Q and K of the
                         // next item wait for it anyway.
                         if (q0_uses > 0 && !(tok = mbar_wait(wc, &sh.q_empty[0], (q0_uses - 1) & 1, W_QEMPTY, r))) break;
-                        x = make_item<true>(a, id, 0, 1);
+                        x = make_item<RUNS>(a, id, 0, 1);
                         sh.item[buf] = x;
                     } else {
                         sh.item[buf].n0 = -1;
@@ -861,9 +863,12 @@ struct FwdDevice {
     int slots[4] = {148, 74, 33, 15};  // resident clusters of 1, 2, 4, 8 CTAs; the device is asked
 };
 typedef void (*FwdKernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, FwdArgs);
-const FwdKernel fwd_kernels[9] = {attn_fwd_kernel<0, ONE_ITEM>,     attn_fwd_kernel<1, ONE_ITEM>,     attn_fwd_kernel<2, ONE_ITEM>,
-                                  attn_fwd_kernel<0, TAKE_OVER>,    attn_fwd_kernel<1, TAKE_OVER>,    attn_fwd_kernel<2, TAKE_OVER>,
-                                  attn_fwd_kernel<0, COMBINE_ITEM>, attn_fwd_kernel<1, COMBINE_ITEM>, attn_fwd_kernel<2, COMBINE_ITEM>};
+const FwdKernel fwd_kernels[15] = {
+    attn_fwd_kernel<0, ONE_ITEM, false>,     attn_fwd_kernel<1, ONE_ITEM, false>,     attn_fwd_kernel<2, ONE_ITEM, false>,
+    attn_fwd_kernel<0, TAKE_OVER, false>,    attn_fwd_kernel<1, TAKE_OVER, false>,    attn_fwd_kernel<2, TAKE_OVER, false>,
+    attn_fwd_kernel<0, COMBINE_ITEM, false>, attn_fwd_kernel<1, COMBINE_ITEM, false>, attn_fwd_kernel<2, COMBINE_ITEM, false>,
+    attn_fwd_kernel<0, ONE_ITEM, true>,      attn_fwd_kernel<1, ONE_ITEM, true>,      attn_fwd_kernel<2, ONE_ITEM, true>,
+    attn_fwd_kernel<0, TAKE_OVER, true>,     attn_fwd_kernel<1, TAKE_OVER, true>,     attn_fwd_kernel<2, TAKE_OVER, true>};
 
 // of the current device; set up by the first call on it
 int fwd_device(FwdDevice** out) {
@@ -920,7 +925,7 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     const int n_kvtiles = (Tk + TILE - 1) / TILE;
     // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
     // then more than the bookkeeping costs per step (about 2 %, of which some may be registers: the kernels that take over spill
-    // 76 to 152 bytes per thread, those for one item none, or 88 with a dense mask).  Steps per item on average, one item per
+    // 76 to 160 bytes per thread, those for one item none, or 172 with a dense mask).  Steps per item on average, one item per
     // CTA -> taken over: 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same
     // without a mask) 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
     // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
@@ -1003,7 +1008,8 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
-    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * plan.job], mq, mk, mv, mo, a);
+    const bool runs = a.group < a.BH && plan.job != COMBINE_ITEM;
+    const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * plan.job + (runs ? 9 : 0)], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();
     return rc == cudaSuccess ? HK_OK : check_launch();
