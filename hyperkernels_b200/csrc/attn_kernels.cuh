@@ -58,7 +58,13 @@ struct FwdArgs {
     hk_philox_keys_t philox_keys;
     uint32_t philox_offset;
     DeviceStatus* status;
+    uint64_t unused[6];  // up to a size that launches fast: FWD_PARAM_BYTES
 };
+// The smallest forwards are bound by how fast the host launches them, and that depends on the bytes of parameters, four maps and this
+// block: 24 or 32 beyond a multiple of 64 take 2.1 us per launch of an empty kernel, any other number 2.4 to 2.5 (640 to 808 and
+// 1 536 to 1 656 bytes in steps of 8).  B2 H25 T68 with 736 or 792 bytes 5.95 us per call, with 744 6.3.
+constexpr size_t FWD_PARAM_BYTES = 4 * sizeof(CUtensorMap) + sizeof(FwdArgs);
+static_assert(FWD_PARAM_BYTES % 64 == 24 || FWD_PARAM_BYTES % 64 == 32, "a forward's launch would take 0.3 us longer");
 
 // How a forward's work is cut, from sizes and the resident clusters of 1, 2, 4, 8 CTAs (slots) alone.
 struct FwdPlan {
