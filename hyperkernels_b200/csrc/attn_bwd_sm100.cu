@@ -993,7 +993,7 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     const int live = plan.live;
     a.n_splits = plan.n_splits;
     a.live = live;
-    a.group = slices_in_l2(a.BH, 256.0 * (3.0 * a.Tq + 4.0 * a.Tk));  // Q, dO, dQ; K, V, dK, dV
+    a.group = bwd_run(a.BH, a.Tq, a.Tk);
     const long long nblocks = (long long)live * a.BH * a.n_splits;
     if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     if (nblocks > 0) {

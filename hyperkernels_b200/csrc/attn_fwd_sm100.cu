@@ -1003,7 +1003,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.mode = plan.mode;
     a.n_splits = plan.n_splits;
     a.n_qblocks = plan.n_qblocks;
-    a.group = slices_in_l2(a.BH, 256.0 * (2.0 * a.Tq + 2.0 * a.Tk));  // Q, O; K, V
+    a.group = fwd_run(a.BH, a.Tq, a.Tk);
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);

@@ -33,6 +33,9 @@ inline int slices_in_l2(int all, double slice_bytes) {
     const int group = std::max(1, (int)std::min((double)all, 67108864.0 / slice_bytes + 0.5));
     return all < 2 * group ? all : group;
 }
+// of a forward (Q, O; K, V) and of a backward (Q, dO, dQ; K, V, dK, dV)
+inline int fwd_run(int BH, int Tq, int Tk) { return slices_in_l2(BH, 256.0 * (2.0 * Tq + 2.0 * Tk)); }
+inline int bwd_run(int BH, int Tq, int Tk) { return slices_in_l2(BH, 256.0 * (3.0 * Tq + 4.0 * Tk)); }
 
 // what the two streams of a forward CTA are (attn_fwd_sm100.cu)
 enum FwdMode { FWD_ROWS = 0, FWD_ROW = 1, FWD_KEYS = 2 };
@@ -166,6 +169,8 @@ extern "C" int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slo
 // The order of the work items (take_in_groups) of `all` slices of `slice_bytes` and `n` parts each, for tests: all * n pairs
 // {slice, part}.
 extern "C" void hk_attn_item_order(int all, int n, double slice_bytes, int* pairs);
+// Slices in a run of such a call, `all` where it has one run; for tests.
+extern "C" int hk_attn_slices_per_run(int backward, int all, int Tq, int Tk);
 // zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ
 extern "C" int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream);
 

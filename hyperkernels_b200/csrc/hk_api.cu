@@ -516,6 +516,8 @@ void hk_attn_item_order(int all, int n, double slice_bytes, int* pairs) {
     for (int i = 0; i < all * n; ++i) take_in_groups(i, all, n, slices_in_l2(all, slice_bytes), pairs[2 * i], pairs[2 * i + 1]);
 }
 
+int hk_attn_slices_per_run(int backward, int all, int Tq, int Tk) { return backward ? bwd_run(all, Tq, Tk) : fwd_run(all, Tq, Tk); }
+
 int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream) {
     if (!p || !p->dQ) return HK_ERR_NULL_POINTER;
     if (p->B <= 0 || p->nh <= 0 || p->T <= 0) return HK_ERR_BAD_SHAPE;

@@ -1,0 +1,94 @@
+"""Calls of more slices than a run of work items holds (csrc/attn_kernels.cuh, take_in_groups), in every kind of call: each slice
+equals the same slice in calls of one run, which other tests compare with the oracle.  Run sizes are asked for, not restated."""
+import pytest
+import torch
+
+import hyperkernels_b200 as hk
+from test_work_split import B200, ONE_ITEM, TAKE_OVER, backward_plan, forward_job
+
+SCALE, P, SEED = 0.125, 0.25, 99
+
+# (BH, Tq, Tk, causal, the forward's job): KV tiles that no query sees, so that the backward's grid has 3 of 4; blocks of more than
+# twelve steps; blocks and KV tiles of one tile
+SHAPES = [(400, 300, 500, True, TAKE_OVER), (111, 1000, 1600, False, ONE_ITEM), (2100, 64, 100, True, TAKE_OVER)]
+
+
+def run_of(backward, BH, Tq, Tk):
+    return hk.lib().hk_attn_slices_per_run(backward, BH, Tq, Tk)
+
+
+@pytest.mark.parametrize("BH,Tq,Tk,causal,job", SHAPES)
+def test_shapes_take_several_runs(BH, Tq, Tk, causal, job):
+    """Two runs or more in both directions, the last one longer, on the route that the shape stands for."""
+    for backward in (0, 1):
+        n = run_of(backward, BH, Tq, Tk)
+        assert 2 * n <= BH and BH % n
+        assert run_of(backward, 2 * n - 1, Tq, Tk) == 2 * n - 1 and run_of(backward, 2 * n, Tq, Tk) == n
+    assert forward_job(BH, Tq, Tk, causal, slots=B200) == job
+    assert backward_plan(BH, Tq, Tk, causal, slots=B200) == (1, TAKE_OVER)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["none", "philox", "philox inverted", "dense", "dense inverted"])
+@pytest.mark.parametrize("BH,Tq,Tk,causal,job", SHAPES)
+def test_every_kind_of_call_in_runs_keeps_its_bits(BH, Tq, Tk, causal, job, kind):
+    """O, LSE, dK, dV and the reproducible dQ, stored [B, T, H, 64], and a forward that goes on from a state; gradients added to
+    what the buffers hold."""
+    part = min(run_of(0, BH, Tq, Tk), run_of(1, BH, Tq, Tk))
+    gen = torch.Generator(device="cuda").manual_seed(83)
+    normal = lambda T: torch.randn((1, T, BH, 64), generator=gen, device="cuda").transpose(1, 2)  # noqa: E731
+    Q, dO, K, V = normal(Tq), normal(Tq), normal(Tk), normal(Tk)
+    mask = (torch.rand((BH, Tq, Tk), generator=gen, device="cuda") >= P).float() if kind.startswith("dense") else None
+
+    def calls(s):
+        """every output of the slices `s`"""
+        kw = {} if kind == "none" else dict(dropout_p=P, dropout_scaled=kind.endswith("inverted"))
+        if kind.startswith("philox"):
+            kw.update(philox_seed=SEED, bh_pos0=s.start)
+        second, half = dict(kw), Tk // 16 * 8  # keys in two calls
+        if mask is not None:
+            kw["dropout_mask"] = mask[s]
+        q, k, v, g = Q[:, s], K[:, s], V[:, s], dO[:, s]
+        O, L = hk.attention_forward(q, k, v, SCALE, causal, **kw)
+        back = lambda **more: hk.attention_backward(q, k, v, O, g, L, SCALE, causal, deterministic_dq=True, **kw, **more)[:3]  # noqa: E731
+        grads = back()
+        sums = [torch.full_like(x, 0.5) for x in grads]
+        back(accum_dq=True, accum_dkdv=True, dQ=sums[0], dK=sums[1], dV=sums[2])
+        out = [O, L, *grads, *sums]
+        if not kind.endswith("inverted"):
+            first = dict(second, dropout_mask=mask[s][:, :, :half].contiguous()) if mask is not None else second
+            O2, L2 = hk.attention_forward(q, k[:, :, :half], v[:, :, :half], SCALE, causal, **first)
+            if mask is not None:
+                second["dropout_mask"] = mask[s][:, :, half:].contiguous()
+            hk.attention_forward(q, k[:, :, half:], v[:, :, half:], SCALE, causal, k_pos0=half, continue_state=True, out=O2, lse=L2, **second)
+            out += [O2, L2]
+        torch.cuda.synchronize()
+        assert hk.last_device_status() == 0
+        return out
+
+    whole = calls(slice(0, BH))
+    for i in range(0, BH, part):
+        s = slice(i, min(BH, i + part))
+        for got, want in zip(whole, calls(s)):
+            assert torch.equal(got[:, s], want)
+
+
+@pytest.mark.gpu
+def test_default_dq_in_runs_differs_by_the_order_of_its_sum():
+    """The default dQ adds one term per KV tile in the order of arrival: n terms in two orders, (n - 1) roundings of at most 2^-24 of
+    the sum of the magnitudes each."""
+    BH, Tq, Tk, causal, _ = SHAPES[0]
+    gen = torch.Generator(device="cuda").manual_seed(89)
+    normal = lambda T: torch.randn((1, BH, T, 64), generator=gen, device="cuda")  # noqa: E731
+    Q, dO, K, V = normal(Tq), normal(Tq), normal(Tk), normal(Tk)
+    O, L = hk.attention_forward(Q, K, V, SCALE, causal)
+    want, _, _, D = hk.attention_backward(Q, K, V, O, dO, L, SCALE, causal, deterministic_dq=True)
+    got = hk.attention_backward(Q, K, V, O, dO, L, SCALE, causal)[0]
+    size, tiles = torch.zeros_like(want), -(-Tk // 128)
+    for i in range(tiles):  # a KV tile alone
+        k, v = (x[:, :, 128 * i:128 * (i + 1)].contiguous() for x in (K, V))
+        size += hk.attention_backward(Q, k, v, O, dO, L, SCALE, causal, k_pos0=128 * i, D=D, d_precomputed=True)[0].abs()
+    torch.cuda.synchronize()
+    assert hk.last_device_status() == 0
+    # the sum of magnitudes is itself rounded (n - 1) times, and the zero that dQ starts with is a term without a rounding
+    assert bool(((got - want).abs() <= 2 * (tiles - 1) * 2.0 ** -24 * (1 + tiles * 2.0 ** -23) * size).all())
