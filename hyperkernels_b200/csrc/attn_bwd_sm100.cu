@@ -985,6 +985,18 @@ BwdPlan plan_attn_bwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     return plan;
 }
 
+// As in the forward, several runs cost balance at the end of the grid, the more the more KV tiles a slice has.  us, one run ->
+// several, at 2.2 times the slices of a run: T512 55.8 -> 54.9, T768 69.0 -> 66.7, T1024 78.2 -> 78.0, without a causal mask 129.3 ->
+// 130.4, with Philox 89.1 -> 90.2; T2048 123.6 -> 124.7, T3000 170.8 -> 173.9, T4096 213.6 -> 216.5; at 2.7 times T1024 94.6 -> 92.9,
+// T2048 146.7 -> 143.9, T4096 255.3 -> 254.8.  With a dense mask T1024 377 -> 386 and 469 -> 463; T2048 at 2.6, 3.3 and 4.1 times
+// 808 -> 819, 1 010 -> 1 012, 1 261 -> 1 239; T4096 at 2.6, 3.5 and 5 times 1 547 -> 1 562, 2 043 -> 2 061, 2 924 -> 2 895.
+int bwd_run(const BwdPlan& plan, int BH, int Tq, int Tk, int dropout_mode) {
+    const int group = slices_in_l2(BH, 256.0 * (3.0 * Tq + 4.0 * Tk));  // Q, dO, dQ; K, V, dK, dV
+    if (plan.job != TAKE_OVER || plan.live == 1) return BH;
+    const double least = plan.live < 8 ? 2.0 : dropout_mode == 1 && plan.live >= 16 ? 4.0 : 2.5;
+    return BH < least * group ? BH : group;
+}
+
 int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_t stream) {
     BwdDevice* d = nullptr;
     const int device_rc = bwd_device(&d);
@@ -993,7 +1005,7 @@ int launch_attn_bwd(const BwdMaps& m, BwdArgs a, bool after_prepass, cudaStream_
     const int live = plan.live;
     a.n_splits = plan.n_splits;
     a.live = live;
-    a.group = bwd_run(a.BH, a.Tq, a.Tk);
+    a.group = bwd_run(plan, a.BH, a.Tq, a.Tk, a.dropout_mode);
     const long long nblocks = (long long)live * a.BH * a.n_splits;
     if (nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     if (nblocks > 0) {

@@ -994,6 +994,22 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     return refine && fine_cost < (may_split ? 0.85 : 0.87) * cost_of_plan ? fine_plan : plan;
 }
 
+// Runs save loads from memory, and what they cost is the balance at the end of the grid: under the causal mask blocks are of
+// different lengths, and the short ones of the last run alone even it out less than those of all slices.  us, one run -> several,
+// at 2, 3 and 4 to 5 times the slices of a run: T512 37.7 -> 39.1, 55.4 -> 55.9, 70.4 -> 71.0; T1024 48.4 -> 51.4, 71.2 -> 72.7,
+// 95.1 -> 93.0; T2048 74.0 -> 75.7, 109.0 -> 109.7, 148.9 -> 143.3; T4096 127.8 -> 128.9, 189 -> 188, 258 -> 248.  Without a causal
+// mask T512 47.4 -> 46.4, 67.7 -> 65.7, 86.3 -> 84.0; T1024 73.2 -> 73.1, 109.7 -> 106.4, 145.9 -> 137.3; T2048 129.0 -> 130.0,
+// 195.5 -> 190.0, 268.9 -> 249.5.  Blocks that are alone in their slice come in one order either way, and the kernels without runs
+// take less to decode them: T256 45.7 -> 47.2.
+// A dense mask goes through the L2 as well, and its kernels for runs are the faster ones whatever the order: T512 301 -> 287,
+// T1024 514 -> 455, T2048 984 -> 869 at twice the slices, blocks alone in their slice (T256) 260 -> 247.
+int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int dropout_mode) {
+    const int group = slices_in_l2(BH, 256.0 * (2.0 * Tq + 2.0 * Tk));  // Q, O; K, V
+    if (plan.job == COMBINE_ITEM) return BH;
+    if (dropout_mode != 1 && (plan.n_qblocks == 1 || (causal && BH < 4 * (long long)group))) return BH;
+    return group;
+}
+
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                     FwdArgs a, cudaStream_t stream) {
     FwdDevice* d = nullptr;
@@ -1003,12 +1019,12 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.mode = plan.mode;
     a.n_splits = plan.n_splits;
     a.n_qblocks = plan.n_qblocks;
-    a.group = fwd_run(a.BH, a.Tq, a.Tk);
+    a.group = fwd_run(plan, a.BH, a.Tq, a.Tk, a.causal, a.dropout_mode);
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);
     LaunchConfig lc((unsigned)nblocks, fwd::NUM_THREADS, fwd::SMEM_BYTES, stream, a.n_splits, true);
-    const bool runs = a.group < a.BH && plan.job != COMBINE_ITEM;
+    const bool runs = a.group < a.BH;
     const cudaError_t rc = cudaLaunchKernelEx(&lc.cfg, fwd_kernels[a.dropout_mode + 3 * plan.job + (runs ? 9 : 0)], mq, mk, mv, mo, a);
     timing_mark(TIMED_FWD, false, stream);
     count_launch();

@@ -10,11 +10,12 @@ namespace hk {
 // Order of work items: slice `bh` (batch x head) and part `part` of it (a KV tile or a block of rows, 0 the longest) of item
 // `item`, where the `n` parts of each of `all` slices are handed out part by part inside runs of `group` slices.  With all slices
 // in one run a slice's second part came up when its tensors had long left the L2 again, and every part fetched them (the
-// backward's dQ both ways) from memory.  Runs whose tensors take half of the L2 (slices_in_l2), one order -> the other:
-// backward B32 H25 T1024 815 -> 701 us, B16 H16 T2048 without a mask 1 741 -> 1 395, H32 T32768 23 820 -> 21 126, forward of the
-// first two 288 -> 279 and 514 -> 484.  A run also has to be long enough for the CTAs to finish together (longest parts first, and
-// the last run takes what is left over): with 8 MB per run B2 H16 T2000 took 115 us, with 64 MB or more 93.  24 to 96 MB
-// are within 4 % of each other for most shapes.
+// backward's dQ both ways) from memory.  One run -> runs whose tensors take half of the L2 (slices_in_l2), kernels alone, ten launches
+// after a pause of 50 ms, 1 965 MHz: backward B32 H25 T1024 780 -> 634 us, B16 H16 T2048 without a mask 1 637 -> 1 258, H32 T32768
+// 20 565 -> 18 551; forward 266 -> 254, 495 -> 441, 6 526 -> 5 945.  From memory at B16 H20 T1024: the backward 1 736 -> 631 MB, the
+// forward 553 -> 314.  A run also has to be long enough for the CTAs to finish together (longest parts first, and the last run takes
+// what is left over): with 8 MB per run the backward of B2 H16 T2000 took 1.24 times as long as with 64 MB or more.  24 to 96 MB are
+// within 4 % of each other for most shapes.  How many runs there have to be: fwd_run, bwd_run.
 __host__ __device__ __forceinline__ void take_in_groups(int item, int all, int n, int group, int& bh, int& part) {
     int first = 0, size = all;
     if (group < all) {  // with one run the divisions before the first load would cost the smallest calls 1 %
@@ -27,15 +28,14 @@ __host__ __device__ __forceinline__ void take_in_groups(int item, int all, int n
     bh = first + (item - part * size);
 }
 
-// Slices in a run: as many as 64 MB hold (about half of the 126 MB of L2, the rest for what the next run loads), at least one;
-// all, if that leaves one run.
+// Slices in a run: the number whose tensors come closest to 64 MB, about half of the 126 MB of L2 of the one chip this is built for,
+// and at least one; all, if that leaves one run.  So a run of two slices may be of 85 MB, and one slice of any size; the last run
+// holds up to twice the number, which its balance needs more than its loads need the L2.  The slabs of a reproducible dQ and a dense
+// mask, which go through once, are not counted, nor is it that a causal mask leaves half of the loads.
 inline int slices_in_l2(int all, double slice_bytes) {
     const int group = std::max(1, (int)std::min((double)all, 67108864.0 / slice_bytes + 0.5));
     return all < 2 * group ? all : group;
 }
-// of a forward (Q, O; K, V) and of a backward (Q, dO, dQ; K, V, dK, dV)
-inline int fwd_run(int BH, int Tq, int Tk) { return slices_in_l2(BH, 256.0 * (2.0 * Tq + 2.0 * Tk)); }
-inline int bwd_run(int BH, int Tq, int Tk) { return slices_in_l2(BH, 256.0 * (3.0 * Tq + 4.0 * Tk)); }
 
 // what the two streams of a forward CTA are (attn_fwd_sm100.cu)
 enum FwdMode { FWD_ROWS = 0, FWD_ROW = 1, FWD_KEYS = 2 };
@@ -76,6 +76,8 @@ struct FwdPlan {
 };
 FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, bool drop, const int slots[4]);
 int attn_fwd_slots(const int** slots);  // of the current device; status
+// slices in a run of its work items, BH where they come in one
+int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int dropout_mode);
 
 // mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
@@ -148,6 +150,7 @@ struct BwdPlan {
 };
 BwdPlan plan_attn_bwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, const int slots[4]);
 int attn_bwd_slots(const int** slots);
+int bwd_run(const BwdPlan& plan, int BH, int Tq, int Tk, int dropout_mode);
 
 // after_prepass: the launch before it in the stream is this call's D pre-pass, the only kernel whose results it waits for
 // itself (Q, K, V and dO are complete when the pre-pass lets it start)
@@ -169,8 +172,9 @@ extern "C" int hk_attn_backward_plan(const hk_attn_bwd_params* p, const int* slo
 // The order of the work items (take_in_groups) of `all` slices of `slice_bytes` and `n` parts each, for tests: all * n pairs
 // {slice, part}.
 extern "C" void hk_attn_item_order(int all, int n, double slice_bytes, int* pairs);
-// Slices in a run of such a call, `all` where it has one run; for tests.
-extern "C" int hk_attn_slices_per_run(int backward, int all, int Tq, int Tk);
+// Slices in a run of the call of this block, all of them where it has one run; for tests, as the plans above.
+extern "C" int hk_attn_forward_run(const hk_attn_fwd_params* p, const int* slots, int* slices);
+extern "C" int hk_attn_backward_run(const hk_attn_bwd_params* p, const int* slots, int* slices);
 // zeroes dQ (fields dQ, dq_stride*, B, nh, T), for a caller that runs the backward with HK_FLAG_ACCUM_DQ
 extern "C" int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream);
 

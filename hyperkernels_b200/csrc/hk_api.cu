@@ -516,7 +516,25 @@ void hk_attn_item_order(int all, int n, double slice_bytes, int* pairs) {
     for (int i = 0; i < all * n; ++i) take_in_groups(i, all, n, slices_in_l2(all, slice_bytes), pairs[2 * i], pairs[2 * i + 1]);
 }
 
-int hk_attn_slices_per_run(int backward, int all, int Tq, int Tk) { return backward ? bwd_run(all, Tq, Tk) : fwd_run(all, Tq, Tk); }
+int hk_attn_forward_run(const hk_attn_fwd_params* p, const int* slots, int* slices) {
+    const int BH = p->B * p->nh, Tq = (int)p->T, Tk = (int)(p->kv_len > 0 ? p->kv_len : p->T);
+    int mode = 0, rc = validate_dropout(p->dropout_p, p->dropout_mask, p->flags, p->k_pos0, &mode);
+    if (rc != HK_OK) return rc;
+    if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
+    const FwdPlan f = plan_attn_fwd(BH, Tq, Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode != 0, slots);
+    *slices = fwd_run(f, BH, Tq, Tk, p->is_causal, mode);
+    return HK_OK;
+}
+
+int hk_attn_backward_run(const hk_attn_bwd_params* p, const int* slots, int* slices) {
+    const int BH = p->B * p->nh, Tk = (int)(p->kv_len > 0 ? p->kv_len : p->T);
+    int mode = 0, rc = validate_dropout(p->dropout_p, p->dropout_mask, p->flags, p->k_pos0, &mode);
+    if (rc != HK_OK) return rc;
+    if (!slots && (rc = attn_bwd_slots(&slots))) return rc;
+    const BwdPlan b = plan_attn_bwd(BH, p->T, Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, slots);
+    *slices = bwd_run(b, BH, p->T, Tk, mode);
+    return HK_OK;
+}
 
 int hk_attn_zero_dq(const hk_attn_bwd_params* p, void* stream) {
     if (!p || !p->dQ) return HK_ERR_NULL_POINTER;

@@ -1,29 +1,64 @@
-"""Calls of more slices than a run of work items holds (csrc/attn_kernels.cuh, take_in_groups), in every kind of call: each slice
-equals the same slice in calls of one run, which other tests compare with the oracle.  Run sizes are asked for, not restated."""
+"""Calls whose work items come in several runs of slices (csrc/attn_kernels.cuh, take_in_groups): which calls do, and that each
+slice equals the same slice in calls of one run, which other tests compare with the oracle.  Run sizes are asked for, not restated."""
+import ctypes as C
+
 import pytest
 import torch
 
 import hyperkernels_b200 as hk
-from test_work_split import B200, ONE_ITEM, TAKE_OVER, backward_plan, forward_job
+from test_work_split import B200, ONE_ITEM, TAKE_OVER, TOGETHER, backward_plan, forward_job
 
 SCALE, P, SEED = 0.125, 0.25, 99
 
 # (BH, Tq, Tk, causal, the forward's job): KV tiles that no query sees, so that the backward's grid has 3 of 4; blocks of more than
-# twelve steps; blocks and KV tiles of one tile
-SHAPES = [(400, 300, 500, True, TAKE_OVER), (111, 1000, 1600, False, ONE_ITEM), (2100, 64, 100, True, TAKE_OVER)]
+# twelve steps; two KV tiles and a second block of few rows
+SHAPES = [(700, 300, 500, True, TAKE_OVER), (111, 1000, 1600, False, ONE_ITEM), (1000, 280, 256, True, TAKE_OVER)]
 
 
-def run_of(backward, BH, Tq, Tk):
-    return hk.lib().hk_attn_slices_per_run(backward, BH, Tq, Tk)
+def run_of(backward, BH, Tq, Tk, causal, kind="none"):
+    """slices in a run, BH where there is one"""
+    p = hk.MemEfficientBwdParams() if backward else hk.MemEfficientFwdParams()
+    p.B, p.nh, p.T, p.kv_len, p.is_causal = 1, BH, Tq, Tk, causal
+    if kind != "none":
+        p.dropout_p = P
+    if kind.startswith("philox"):
+        p.flags = hk.FLAG_PHILOX_DROPOUT
+    elif kind.startswith("dense"):
+        p.dropout_mask = 16  # not read
+    n = C.c_int()
+    assert (hk.lib().hk_attn_backward_run if backward else hk.lib().hk_attn_forward_run)(C.byref(p), B200, C.byref(n)) == 0
+    return n.value
 
 
+@pytest.mark.parametrize("backward,Tq,Tk,causal,kind,least,run", [
+    # least: the fewest slices that come in several runs; blocks of different lengths cost more than they save below four runs
+    (0, 1024, 1024, True, "none", 256, 64), (0, 1024, 1024, True, "philox", 256, 64), (0, 1024, 1024, True, "dense", 128, 64),
+    (0, 1024, 1024, False, "none", 128, 64), (0, 257, 257, False, "philox", 510, 255),
+    # KV tiles: fewer than eight, eight, sixteen
+    (1, 512, 512, True, "none", 146, 73), (1, 897, 896, True, "philox", 84, 42), (1, 1024, 1024, True, "none", 93, 37),
+    (1, 1024, 1024, False, "dense", 93, 37), (1, 2048, 2048, True, "philox", 45, 18), (1, 2048, 2048, True, "dense", 72, 18),
+    (1, 2048, 1920, False, "dense", 48, 19)])
+def test_calls_of_several_runs(backward, Tq, Tk, causal, kind, least, run):
+    assert run_of(backward, least - 1, Tq, Tk, causal, kind) == least - 1
+    assert run_of(backward, least, Tq, Tk, causal, kind) == run
+
+
+@pytest.mark.parametrize("backward,BH,Tq,Tk,causal", [
+    (0, 3000, 256, 256, True), (0, 3000, 100, 128, False), (1, 3000, 128, 128, True), (1, 3000, 100, 300, True),  # alone in their slice
+    (0, 8, 512, 65536, False), (1, 4, 60000, 300, False)])  # shared by a cluster
+def test_calls_of_one_run(backward, BH, Tq, Tk, causal):
+    assert run_of(backward, BH, Tq, Tk, causal) == BH
+    if BH < 10:
+        assert (backward_plan(BH, Tq, Tk, causal, slots=B200)[1] if backward else forward_job(BH, Tq, Tk, causal, slots=B200)) == TOGETHER
+
+
+@pytest.mark.parametrize("kind", ["none", "philox", "dense"])
 @pytest.mark.parametrize("BH,Tq,Tk,causal,job", SHAPES)
-def test_shapes_take_several_runs(BH, Tq, Tk, causal, job):
+def test_shapes_take_several_runs(BH, Tq, Tk, causal, job, kind):
     """Two runs or more in both directions, the last one longer, on the route that the shape stands for."""
     for backward in (0, 1):
-        n = run_of(backward, BH, Tq, Tk)
+        n = run_of(backward, BH, Tq, Tk, causal, kind)
         assert 2 * n <= BH and BH % n
-        assert run_of(backward, 2 * n - 1, Tq, Tk) == 2 * n - 1 and run_of(backward, 2 * n, Tq, Tk) == n
     assert forward_job(BH, Tq, Tk, causal, slots=B200) == job
     assert backward_plan(BH, Tq, Tk, causal, slots=B200) == (1, TAKE_OVER)
 
@@ -34,7 +69,8 @@ def test_shapes_take_several_runs(BH, Tq, Tk, causal, job):
 def test_every_kind_of_call_in_runs_keeps_its_bits(BH, Tq, Tk, causal, job, kind):
     """O, LSE, dK, dV and the reproducible dQ, stored [B, T, H, 64], and a forward that goes on from a state; gradients added to
     what the buffers hold."""
-    part = min(run_of(0, BH, Tq, Tk), run_of(1, BH, Tq, Tk))
+    part = min(run_of(backward, BH, Tq, Tk, causal, kind) for backward in (0, 1))
+    assert all(run_of(backward, part, Tq, Tk, causal, kind) == part for backward in (0, 1))
     gen = torch.Generator(device="cuda").manual_seed(83)
     normal = lambda T: torch.randn((1, T, BH, 64), generator=gen, device="cuda").transpose(1, 2)  # noqa: E731
     Q, dO, K, V = normal(Tq), normal(Tq), normal(Tk), normal(Tk)
