@@ -150,7 +150,8 @@ enum WaitId {
 }  // namespace bwd
 
 namespace bwd {
-// RUNS: the items come in runs of slices (take_in_groups)
+// RUNS: the items may come in runs of slices (take_in_groups), which the kernels that take over decide as they run: kernels of their
+// own for one run, as the forward has them, gain nothing here (B16 H12 T256 22.54 us either way).
 template <bool RUNS>
 __device__ __forceinline__ Item make_item(const BwdArgs& a, int item, int split, int ns) {
     Item x;
@@ -787,8 +788,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                 {
                     // Rows r and r + 4 share a 32-byte chunk position, so two of the eight lanes of a quarter-warp meet in a
                     // 16-byte bank group.  Storing the two halves in opposite order avoids that, but the 32 selects that it
-                    // takes cost what it gains (B8 H12 T1024 84.4 us either way), and more where the warps have keep bits to
-                    // draw too (with dropout 97.0 -> 94.6 without them).
+                    // takes cost what it gains (B8 H12 T1024 87.6 us with them, 88.0 without; ten launches after a pause, 1 965
+                    // MHz), and more where the warps have keep bits to draw too (with dropout 101.5 -> 99.9, B32 H25 T1024 736 -> 723).
                     uint8_t* drow = sdS + part * BOX_BYTES + row * 128;
 #pragma unroll
                     for (int u = 0; u < 8; ++u)

@@ -673,7 +673,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant_
                         // The part of the 16 calls that depends on the keys alone is the same for all rows: a lane works out one,
                         // and the others read it from where the warp's m and l go at the end.  The integer products are what
                         // dropout costs: 15 instead of 20 per call, each by one wide multiplication, took B16 H16 T2048 without
-                        // a mask from 902 to 867 us, B8 H12 T1024 from 62.0 to 60.7.
+                        // a mask from 846 to 809 us, B8 H12 T1024 from 58.7 to 56.8 (ten launches after a pause, 1 965 MHz).
                         uint4 *keys0 = reinterpret_cast<uint4*>(&sh.m[t][quarter * 32]), *keys8 = reinterpret_cast<uint4*>(&sh.l[t][quarter * 32]);
                         if (lane < 16)
                             (lane < 8 ? keys0 : keys8)[lane & 7] = hk_philox_key_part(a.philox_keys, a.philox_offset, a.bh_pos0 + (uint32_t)bh,
@@ -925,8 +925,9 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     const int n_kvtiles = (Tk + TILE - 1) / TILE;
     // CTAs take over further items where the grid is larger than the device and items are short: what overlaps at their ends is
     // then more than the bookkeeping costs per step (about 2 %, of which some may be registers: the kernels that take over spill
-    // 76 to 160 bytes per thread, those for one item none, or 172 with a dense mask).  Steps per item on average, one item per
-    // CTA -> taken over: 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same
+    // 76 to 160 bytes per thread, those for one item none).  (With a dense mask the latter spill 172 bytes and are the faster for it:
+    // in another schedule of the same code with 88, H36 T512 took 87.1 instead of 62.5 us, H8 T4096 815 instead of 548.)
+    // Steps per item on average, one item per CTA -> taken over: 1.5 (H384 T256) 26.9 -> 23.9 us, 5 (H96 T1024) 41.3 -> 39.8, 9 (H96 T2048) 128 -> 124.5, 16 (the same
     // without a mask) 224 -> 225, 17 (H48 T4096) 206 -> 208, 33 (H32 T8192) 494 -> 505.
     // Every block sees a key then (q_pos0 >= k_pos0 under the mask): the hand-over between the streams, the issuing and the
     // storing warp counts on a product in every item.
