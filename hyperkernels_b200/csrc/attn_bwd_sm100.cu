@@ -990,11 +990,15 @@ BwdPlan plan_attn_bwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
 // several, at 2.2 times the slices of a run: T512 55.8 -> 54.9, T768 69.0 -> 66.7, T1024 78.2 -> 78.0, without a causal mask 129.3 ->
 // 130.4, with Philox 89.1 -> 90.2; T2048 123.6 -> 124.7, T3000 170.8 -> 173.9, T4096 213.6 -> 216.5; at 2.7 times T1024 94.6 -> 92.9,
 // T2048 146.7 -> 143.9, T4096 255.3 -> 254.8.  With a dense mask T1024 377 -> 386 and 469 -> 463; T2048 at 2.6, 3.3 and 4.1 times
-// 808 -> 819, 1 010 -> 1 012, 1 261 -> 1 239; T4096 at 2.6, 3.5 and 5 times 1 547 -> 1 562, 2 043 -> 2 061, 2 924 -> 2 895.
+// 808 -> 819, 1 010 -> 1 012, 1 261 -> 1 239; T4096 at 2.6, 3.5 and 5 times 1 547 -> 1 562, 2 043 -> 2 061, 2 924 -> 2 895.  With
+// Philox T4096 at 3.5 times 404.9 -> 401.6, T5067 at 3.2 and 5.4 times 463 -> 474, 762 -> 751, T8192 at 3.5 and 5.2 times 754 -> 768,
+// 1 118 -> 1 105.  Without dropout T8192 at 3.5 times 631 -> 630, but T16384 at 2.6, 3.5 and 7 times 912 -> 921, 1 209 -> 1 212,
+// 2 467 -> 2 382 and T24000 at 3.2 and 5.1 times 1 596 -> 1 619, 2 574 -> 2 544: runs of one or two slices.
 int bwd_run(const BwdPlan& plan, int BH, int Tq, int Tk, int dropout_mode) {
     const int group = slices_in_l2(BH, 256.0 * (3.0 * Tq + 4.0 * Tk));  // Q, dO, dQ; K, V, dK, dV
     if (plan.job != TAKE_OVER || plan.live == 1) return BH;
-    const double least = plan.live < 8 ? 2.0 : dropout_mode == 1 && plan.live >= 16 ? 4.0 : 2.5;
+    const bool many = dropout_mode == 1 ? plan.live >= 16 : dropout_mode == 2 ? plan.live > 32 : group <= 2;
+    const double least = plan.live < 8 ? 2.0 : many ? 4.0 : 2.5;  // in runs
     return BH < least * group ? BH : group;
 }
 

@@ -34,10 +34,11 @@ def run_of(backward, BH, Tq, Tk, causal, kind="none"):
     # least: the fewest slices that come in several runs; blocks of different lengths cost more than they save below four runs
     (0, 1024, 1024, True, "none", 256, 64), (0, 1024, 1024, True, "philox", 256, 64), (0, 1024, 1024, True, "dense", 128, 64),
     (0, 1024, 1024, False, "none", 128, 64), (0, 257, 257, False, "philox", 510, 255),
-    # KV tiles: fewer than eight, eight, sixteen
+    # KV tiles: fewer than eight, eight, sixteen, more than 32; runs of two slices
     (1, 512, 512, True, "none", 146, 73), (1, 897, 896, True, "philox", 84, 42), (1, 1024, 1024, True, "none", 93, 37),
     (1, 1024, 1024, False, "dense", 93, 37), (1, 2048, 2048, True, "philox", 45, 18), (1, 2048, 2048, True, "dense", 72, 18),
-    (1, 2048, 1920, False, "dense", 48, 19)])
+    (1, 2048, 1920, False, "dense", 48, 19), (1, 4096, 4096, True, "philox", 23, 9), (1, 5067, 5067, True, "philox", 28, 7),
+    (1, 5067, 5067, True, "none", 18, 7), (1, 16384, 16384, False, "none", 8, 2)])
 def test_calls_of_several_runs(backward, Tq, Tk, causal, kind, least, run):
     assert run_of(backward, least - 1, Tq, Tk, causal, kind) == least - 1
     assert run_of(backward, least, Tq, Tk, causal, kind) == run
