@@ -995,19 +995,24 @@ FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0
     return refine && fine_cost < (may_split ? 0.85 : 0.87) * cost_of_plan ? fine_plan : plan;
 }
 
-// Runs save loads from memory, and what they cost is the balance at the end of the grid: under the causal mask blocks are of
-// different lengths, and the short ones of the last run alone even it out less than those of all slices.  us, one run -> several,
-// at 2, 3 and 4 to 5 times the slices of a run: T512 37.7 -> 39.1, 55.4 -> 55.9, 70.4 -> 71.0; T1024 48.4 -> 51.4, 71.2 -> 72.7,
-// 95.1 -> 93.0; T2048 74.0 -> 75.7, 109.0 -> 109.7, 148.9 -> 143.3; T4096 127.8 -> 128.9, 189 -> 188, 258 -> 248.  Without a causal
-// mask T512 47.4 -> 46.4, 67.7 -> 65.7, 86.3 -> 84.0; T1024 73.2 -> 73.1, 109.7 -> 106.4, 145.9 -> 137.3; T2048 129.0 -> 130.0,
-// 195.5 -> 190.0, 268.9 -> 249.5.  Blocks that are alone in their slice come in one order either way, and the kernels without runs
-// take less to decode them: T256 45.7 -> 47.2.
+// Runs save loads from memory, and what they cost is the balance at the end of the grid: where a causal mask makes blocks of very
+// different lengths, the short ones of the last run alone even it out less than those of all slices.  us, one run -> several, at
+// 2, 3.2 and 4.3 times the slices of a run: T512 37.7 -> 39.1, 55.4 -> 55.9, 70.4 -> 71.0; T768 3.2 times 63.3 -> 64.5, 4.3 times 82.6 ->
+// 82.0; T1024 48.4 -> 51.4, 71.2 -> 72.7, 95.1 -> 93.0.  Of more than four blocks they pay earlier, at 2.6, 2.9, 3.5 and 3.8 times: T1100
+// 73.7 -> 72.1, 80.4 -> 79.4, 95.6 -> 93.6, 101.8 -> 100.4; T1536 75.0 -> 77.7, 83.5 -> 84.5, 100.1 -> 98.9, 107.9 -> 106.2; T2048 90.7 ->
+// 93.0, 100.6 -> 100.8, 121.5 -> 119.4, 132.5 -> 128.1.  Without a causal mask, at 2, 3.2 and 4.3 times, T512 47.4 -> 46.4, 67.7 -> 65.7,
+// 86.3 -> 84.0; T1024 73.2 -> 73.1, 109.7 -> 106.4, 145.9 -> 137.3; T2048 129.0 -> 130.0, 195.5 -> 190.0, 268.9 -> 249.5; with one,
+// but keys in front of the queries, 512 of 2 048 at 2.5 times 62.8 -> 60.9, 1 024 of 1 400 at 2.3 and 3.1 times 69.4 -> 65.8, 90.0 ->
+// 87.7.  Blocks that are alone in their slice come in one order either way, and the kernels without runs take less to decode
+// them: T256 45.7 -> 47.2.
 // A dense mask goes through the L2 as well, and its kernels for runs are the faster ones whatever the order: T512 301 -> 287,
 // T1024 514 -> 455, T2048 984 -> 869 at twice the slices, blocks alone in their slice (T256) 260 -> 247.
-int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int dropout_mode) {
+int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, int dropout_mode) {
     const int group = slices_in_l2(BH, 256.0 * (2.0 * Tq + 2.0 * Tk));  // Q, O; K, V
     if (plan.job == COMBINE_ITEM) return BH;
-    if (dropout_mode != 1 && (plan.n_qblocks == 1 || (causal && BH < 4 * (long long)group))) return BH;
+    const bool uneven = causal && q_pos0 <= k_pos0;
+    const int least = !uneven ? 2 : plan.n_qblocks <= 4 ? 4 : 3;  // in runs
+    if (dropout_mode != 1 && (plan.n_qblocks == 1 || BH < least * (long long)group)) return BH;
     return group;
 }
 
@@ -1020,7 +1025,7 @@ int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensor
     a.mode = plan.mode;
     a.n_splits = plan.n_splits;
     a.n_qblocks = plan.n_qblocks;
-    a.group = fwd_run(plan, a.BH, a.Tq, a.Tk, a.causal, a.dropout_mode);
+    a.group = fwd_run(plan, a.BH, a.Tq, a.Tk, a.causal, a.q_pos0, a.k_pos0, a.dropout_mode);
     const long long nblocks = (long long)a.n_qblocks * a.BH * a.n_splits;
     if (nblocks <= 0 || nblocks > 0x7fffffffLL) return HK_ERR_BAD_SHAPE;
     timing_mark(TIMED_FWD, true, stream);

@@ -77,7 +77,7 @@ struct FwdPlan {
 FwdPlan plan_attn_fwd(int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, bool drop, const int slots[4]);
 int attn_fwd_slots(const int** slots);  // of the current device; status
 // slices in a run of its work items, BH where they come in one
-int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int dropout_mode);
+int fwd_run(const FwdPlan& plan, int BH, int Tq, int Tk, int causal, int q_pos0, int k_pos0, int dropout_mode);
 
 // mq, mk, mv: TMA maps of the operands (rounded to TF32 by the copy); mo: map of O, the destination of the kernel's bulk stores.
 int launch_attn_fwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,

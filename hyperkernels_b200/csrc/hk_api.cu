@@ -522,7 +522,7 @@ int hk_attn_forward_run(const hk_attn_fwd_params* p, const int* slots, int* slic
     if (rc != HK_OK) return rc;
     if (!slots && (rc = attn_fwd_slots(&slots))) return rc;
     const FwdPlan f = plan_attn_fwd(BH, Tq, Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode != 0, slots);
-    *slices = fwd_run(f, BH, Tq, Tk, p->is_causal, mode);
+    *slices = fwd_run(f, BH, Tq, Tk, p->is_causal, (int)p->q_pos0, (int)p->k_pos0, mode);
     return HK_OK;
 }
 

@@ -15,10 +15,10 @@ SCALE, P, SEED = 0.125, 0.25, 99
 SHAPES = [(700, 300, 500, True, TAKE_OVER), (111, 1000, 1600, False, ONE_ITEM), (1000, 280, 256, True, TAKE_OVER)]
 
 
-def run_of(backward, BH, Tq, Tk, causal, kind="none"):
+def run_of(backward, BH, Tq, Tk, causal, kind="none", q_pos0=0):
     """slices in a run, BH where there is one"""
     p = hk.MemEfficientBwdParams() if backward else hk.MemEfficientFwdParams()
-    p.B, p.nh, p.T, p.kv_len, p.is_causal = 1, BH, Tq, Tk, causal
+    p.B, p.nh, p.T, p.kv_len, p.is_causal, p.q_pos0 = 1, BH, Tq, Tk, causal, q_pos0
     if kind != "none":
         p.dropout_p = P
     if kind.startswith("philox"):
@@ -31,9 +31,9 @@ def run_of(backward, BH, Tq, Tk, causal, kind="none"):
 
 
 @pytest.mark.parametrize("backward,Tq,Tk,causal,kind,least,run", [
-    # least: the fewest slices that come in several runs; blocks of different lengths cost more than they save below four runs
+    # least: the fewest slices that come in several runs; up to four blocks of different lengths, and more
     (0, 1024, 1024, True, "none", 256, 64), (0, 1024, 1024, True, "philox", 256, 64), (0, 1024, 1024, True, "dense", 128, 64),
-    (0, 1024, 1024, False, "none", 128, 64), (0, 257, 257, False, "philox", 510, 255),
+    (0, 1025, 1025, True, "none", 192, 64), (0, 1024, 1024, False, "none", 128, 64), (0, 257, 257, False, "philox", 510, 255),
     # KV tiles: fewer than eight, eight, sixteen, more than 32; runs of two slices
     (1, 512, 512, True, "none", 146, 73), (1, 897, 896, True, "philox", 84, 42), (1, 1024, 1024, True, "none", 93, 37),
     (1, 1024, 1024, False, "dense", 93, 37), (1, 2048, 2048, True, "philox", 45, 18), (1, 2048, 2048, True, "dense", 72, 18),
@@ -42,6 +42,13 @@ def run_of(backward, BH, Tq, Tk, causal, kind="none"):
 def test_calls_of_several_runs(backward, Tq, Tk, causal, kind, least, run):
     assert run_of(backward, least - 1, Tq, Tk, causal, kind) == least - 1
     assert run_of(backward, least, Tq, Tk, causal, kind) == run
+
+
+@pytest.mark.parametrize("q_pos0,least", [(0, 408), (1, 204), (256, 204)])
+def test_runs_of_chunks_behind_keys(q_pos0, least):
+    """Keys in front of the queries even out the blocks: two runs of 102 slices, four where there are none."""
+    assert run_of(0, least - 1, 512, 768, True, q_pos0=q_pos0) == least - 1
+    assert run_of(0, least, 512, 768, True, q_pos0=q_pos0) == 102
 
 
 @pytest.mark.parametrize("backward,BH,Tq,Tk,causal", [
